@@ -339,6 +339,90 @@ def work(case):
                 flops=6 * tokens * per_token + pairs * 2 * (4 * head + 3 * value) + polar)
 
 
+# ---- the same in 64 bits -------------------------------------------------------------------------------------------------
+def _visible(rows, cols, start, window):
+    """rows x cols truth values: query i sits at position start + i and looks `window` positions back (None: all the way)."""
+    q = torch.arange(start, start + rows, device="cuda")[:, None]
+    k = torch.arange(cols, device="cuda")[None, :]
+    keep = k <= q
+    return keep if window is None else keep & (q - k <= window)
+
+
+def _exact_attention(case, seed):
+    state = _prepare_attention(case, seed)
+    q, k, v, d_out = (state[n].detach().double() for n in ("q", "k", "v", "d_out"))
+    b, t, h, d = q.shape
+    group, window, cap = h // k.shape[2], state["window"], state["softcap"]
+    out, dq, dk, dv = torch.empty_like(d_out), torch.empty_like(q), torch.zeros_like(k), torch.zeros_like(v)
+    step = max(1, min(t, (1 << 27) // t))                # rows at a time: a gigabyte of scores
+    for i in range(b):
+        for j in range(h):
+            kj, vj = k[i, :, j // group], v[i, :, j // group]
+            for r in range(0, t, step):
+                rows = slice(r, min(r + step, t))
+                s = q[i, rows, j] @ kj.t() * d ** -0.5
+                slope = None
+                if cap:
+                    th = torch.tanh(s / cap)
+                    s, slope = cap * th, 1 - th * th
+                p = torch.softmax(s.masked_fill(~_visible(s.shape[0], t, r, window), -math.inf), dim=-1)
+                o, g = p @ vj, d_out[i, rows, j]
+                out[i, rows, j] = o
+                dv[i, :, j // group] += p.t() @ g
+                ds = p * (g @ vj.t() - (g * o).sum(-1, keepdim=True)) * d ** -0.5
+                if slope is not None:
+                    ds = ds * slope
+                dq[i, rows, j] = ds @ kj
+                dk[i, :, j // group] += ds.t() @ q[i, rows, j]
+    return out, dq, dk, dv
+
+
+def _exact_mla(case, seed):
+    state = _prepare_mla(case, seed)
+    gc, _ = get_preset("mla")
+    attn, cache, x, start = state["attn"], state["cache"], state["x"].double(), state["start"]
+    par = {name: p.detach().double() for name, p in attn.named_parameters()}
+    b, t, _ = x.shape
+    h, r, dr, c, dv = gc.n_heads, gc.mla_kv_rank, gc.mla_qk_rope_dim, gc.mla_qk_content_dim, gc.mla_value_dim
+
+    def rotate(y):                                       # [b, t, heads, dr], pairs of neighbours
+        freq = gc.rope_base_theta ** (-torch.arange(0, dr, 2, device="cuda", dtype=torch.float64) / dr)
+        angle = torch.arange(start, start + t, device="cuda", dtype=torch.float64)[:, None] * freq
+        cos, sin = angle.cos()[None, :, None], angle.sin()[None, :, None]
+        a, o = y[..., 0::2], y[..., 1::2]
+        return torch.stack((a * cos - o * sin, a * sin + o * cos), dim=-1).flatten(-2)
+
+    def gain(y, scale):
+        return torch.rsqrt(y.pow(2).mean(-1, keepdim=True) + gc.qk_eps) * scale.clamp(gc.qk_scale_min, gc.qk_scale_max).view(1, 1, -1, 1)
+
+    q = (x @ par["q_proj.weight"].t()).view(b, t, h, c + dr)
+    q = torch.cat((q[..., :c], rotate(q[..., c:])), dim=-1)
+    low = x @ par["kv_down_proj.weight"].t()
+    lat = low[..., :r]
+    lat = lat * torch.rsqrt(lat.pow(2).mean(-1, keepdim=True) + gc.mla_norm_eps) * par["kv_norm.weight"]
+    rope = rotate(low[..., None, r:])
+    w = par["kv_up_proj.weight"].view(h, c + dv, r)
+    key = torch.cat((torch.einsum("btr,hdr->bthd", lat, w[:, :c]), rope.expand(-1, -1, h, -1)), dim=-1)
+    new_gain = gain(key, par["k_scale"])[..., 0]
+    q = q * gain(q, par["q_scale"])
+    q_lat = torch.einsum("bthd,hdr->bthr", q[..., :c], w[:, :c])
+    context = torch.empty(b, t, h, r, device="cuda", dtype=torch.float64)
+    for i in range(b):
+        ci, ri, gi = (torch.cat((old[i, :start].double(), new[i]), dim=0) for old, new in ((cache.latent, lat), (cache.rope, rope[:, :, 0]), (cache.key_gain, new_gain)))
+        keep = _visible(t, start + t, start, state["window"])
+        for j in range(h):
+            s = (q_lat[i, :, j] @ ci.t() + q[i, :, j, c:] @ ri.t()) * gi[:, j] * (c + dr) ** -0.5
+            context[i, :, j] = torch.softmax(s.masked_fill(~keep, -math.inf), dim=-1) @ ci
+    out = torch.einsum("bthr,hdr->bthd", context, w[:, c:]).flatten(-2) @ par["out_proj.weight"].t()
+    return out, lat, rope[:, :, 0], new_gain
+
+
+def exact(case, seed):
+    """The single layers in 64 bits; a whole model has no such answer that its roundings would not hide."""
+    with torch.no_grad():
+        return _exact_attention(case, seed) if case["kind"] == "attention" else _exact_mla(case, seed) if case["kind"] == "mla" else None
+
+
 def tolerance(case):
     """About four times what was measured between correct ways of computing the same: attention by another kernel with another
     order of its sums, or in fp32 on whole score matrices.  Training compares the fourth step of a run, gradients included."""
