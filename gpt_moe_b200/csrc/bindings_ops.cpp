@@ -201,7 +201,7 @@ Tensor mla_decode(const Tensor& q_latent, const Tensor& q_rope, const Tensor& la
                  c->stride(1) == c->size(2), "mla_decode: bf16 cache tensors [B, S, width] with packed rows");
     GM_CHECK(latent.size(2) == r && rope.size(2) == dr && mla_decode_supported(H, Hkv, r, dr),
              "mla_decode: latent rank 256/512/768/1024, 8/16/32 heads (rank/32 * heads/8 <= 64), rope width even and <= 64");
-    const int splits = mla_decode_splits(B, T, S);
+    const int splits = mla_decode_splits(B, T, H, r, S);
     Tensor part_ctx = gm::out_empty({B, T, H, splits, r}, q_latent.options());
     Tensor part_ml = gm::out_empty({B, T, H, splits, 2}, q_latent.options());
     Tensor context = gm::out_empty({B, T, H, r}, q_latent.options());
@@ -210,6 +210,85 @@ Tensor mla_decode(const Tensor& q_latent, const Tensor& q_rope, const Tensor& la
                                context.data_ptr<float>(), B, T, H, Hkv, r, dr, S, splits, start, window, static_cast<float>(scale),
                                static_cast<float>(softcap), stream()), "mla_decode: unsupported shape");
     return context;
+}
+
+// y = x w^T for at most 32 rows (see rows_linear_kernel): x [rows, K] bf16 with packed columns, w [N, K] bf16 contiguous.
+Tensor rows_linear(const Tensor& x, const Tensor& w) {
+    c10::cuda::CUDAGuard guard(x.device());
+    check_bf16(w, "w");
+    GM_CHECK(x.is_cuda() && x.scalar_type() == torch::kBFloat16 && x.dim() == 2 && w.dim() == 2 && x.size(1) == w.size(1) && x.stride(1) == 1 &&
+             x.stride(0) % 8 == 0, "rows_linear: x [rows, K] bf16 with rows of whole 16-byte pieces, w [N, K]");
+    GM_CHECK(reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 && reinterpret_cast<uintptr_t>(w.data_ptr()) % 16 == 0, "rows_linear: 16-byte aligned operands");
+    Tensor y = gm::out_empty({x.size(0), w.size(0)}, x.options());
+    GM_CHECK(launch_rows_linear(x.data_ptr(), w.data_ptr(), y.data_ptr(), x.size(0), w.size(0), w.size(1), x.stride(0), w.size(0), stream()),
+             "rows_linear: at most 32 rows, K a multiple of 32");
+    return y;
+}
+
+// Latent-cache attention of T new tokens per sequence from their projections (attention/mla_decode.cu): appends them to the cache and
+// returns bf16 [B * T, H * value].  query [B*T, H * (content + dr)] and low [B*T, r + dr] bf16 (any row pitch), w_up fp32
+// [Hkv * (content + value), r], cos / sin fp32 tables [>= start + T, dr / 2], caches bf16 [B, capacity, width] with packed rows.
+Tensor mla_cached(const Tensor& query, const Tensor& low, const Tensor& w_up, const OptTensor& norm_w, double norm_eps, const Tensor& cos,
+                  const Tensor& sin, const OptTensor& q_scale, const OptTensor& k_scale, double qk_eps, bool rms, double smin, double smax,
+                  Tensor& latent, Tensor& rope, Tensor& key_gain, int64_t start, int64_t heads, int64_t content, int64_t value, double scale,
+                  double softcap, int64_t window) {
+    c10::cuda::CUDAGuard guard(query.device());
+    MlaCachedArgs a;
+    a.B = latent.size(0); a.H = heads; a.Hkv = key_gain.size(2); a.r = latent.size(2); a.dr = rope.size(2);
+    a.content = content; a.value = value; a.start = start; a.window = static_cast<int>(std::max<int64_t>(-1, window));
+    GM_CHECK(query.is_cuda() && query.scalar_type() == torch::kBFloat16 && query.dim() == 2 && query.stride(1) == 1 && a.B > 0 && query.size(0) % a.B == 0 &&
+             query.size(1) == heads * (content + a.dr), "mla_cached: query [B * T, H * (content + rope)] bf16");
+    GM_CHECK(low.is_cuda() && low.scalar_type() == torch::kBFloat16 && low.dim() == 2 && low.stride(1) == 1 && low.size(0) == query.size(0) &&
+             low.size(1) == a.r + a.dr, "mla_cached: low [B * T, rank + rope] bf16");
+    a.T = query.size(0) / a.B;
+    const int64_t capacity = latent.size(1);
+    GM_CHECK(start >= 0 && a.T >= 1 && start + a.T <= capacity, "mla_cached: cache capacity");
+    for (const Tensor* c : {&latent, &rope, &key_gain})
+        GM_CHECK(c->is_cuda() && c->scalar_type() == torch::kBFloat16 && c->dim() == 3 && c->size(0) == a.B && c->size(1) == capacity && c->stride(2) == 1 &&
+                 c->stride(1) == c->size(2), "mla_cached: bf16 cache tensors [B, capacity, width] with packed rows");
+    GM_CHECK(mla_decode_supported(a.H, a.Hkv, a.r, a.dr), "mla_cached: unsupported shape");
+    GM_CHECK(w_up.is_cuda() && w_up.scalar_type() == torch::kFloat32 && w_up.is_contiguous() && w_up.numel() == static_cast<int64_t>(a.Hkv) * (content + value) * a.r &&
+             reinterpret_cast<uintptr_t>(w_up.data_ptr()) % 16 == 0, "mla_cached: w_up fp32 [Hkv * (content + value), rank], 16-byte aligned");
+    for (const Tensor* c : {&cos, &sin})
+        GM_CHECK(c->is_cuda() && c->scalar_type() == torch::kFloat32 && c->is_contiguous() && c->dim() == 2 && c->size(1) == a.dr / 2 && c->size(0) >= start + a.T,
+                 "mla_cached: rotary tables");
+    auto vec = [&](const OptTensor& t, int64_t n) {
+        GM_CHECK(!t.has_value() || (t->is_cuda() && t->scalar_type() == torch::kFloat32 && t->is_contiguous() && t->numel() == n), "mla_cached: fp32 vectors");
+        return fptr(t);
+    };
+    a.norm_w = vec(norm_w, a.r); a.q_scale = vec(q_scale, heads); a.k_scale = vec(k_scale, a.Hkv);
+    GM_CHECK((a.q_scale == nullptr) == (a.k_scale == nullptr), "mla_cached: both QK scales or none");
+    a.cos = cos.data_ptr<float>() + start * (a.dr / 2); a.sin = sin.data_ptr<float>() + start * (a.dr / 2);
+    a.query = query.data_ptr(); a.low = low.data_ptr(); a.q_pitch = query.stride(0); a.low_pitch = low.stride(0);
+    a.w_up = w_up.data_ptr<float>();
+    a.latent = latent.data_ptr(); a.rope = rope.data_ptr(); a.key_gain = key_gain.data_ptr();
+    a.latent_bs = latent.stride(0); a.rope_bs = rope.stride(0); a.gain_bs = key_gain.stride(0);
+    a.norm_eps = norm_eps; a.qk_eps = qk_eps; a.smin = smin; a.smax = smax; a.scale = scale; a.softcap = softcap; a.rms = rms;
+    a.splits = mla_decode_splits(a.B, a.T, a.H, a.r, start + a.T);
+    const int64_t rows = static_cast<int64_t>(a.B) * a.T * a.H;
+    // one fp32 workspace: queries in latent space, rotary queries, partial contexts, partial maxima and sums
+    Tensor ws = gm::out_empty({rows * (a.r + 64) + rows * a.splits * (a.r + 2)}, query.options().dtype(torch::kFloat32));
+    a.q_latent = ws.data_ptr<float>();
+    a.part_ctx = a.q_latent + rows * a.r;
+    a.q_rope = a.part_ctx + rows * a.splits * a.r;
+    a.part_ml = a.q_rope + rows * 64;
+    Tensor out = gm::out_empty({query.size(0), heads * value}, query.options());
+    a.out = out.data_ptr();
+    GM_CHECK(launch_mla_cached(a, stream()), "mla_cached: unsupported shape");
+    return out;
+}
+
+// The whole cached step of at most 32 rows: [query | latent, rotary key] projection, attention over the cache, output projection.
+Tensor mla_step(const Tensor& x, const Tensor& w_in, const Tensor& w_out, const Tensor& w_up, const OptTensor& norm_w, double norm_eps, const Tensor& cos,
+                const Tensor& sin, const OptTensor& q_scale, const OptTensor& k_scale, double qk_eps, bool rms, double smin, double smax, Tensor& latent,
+                Tensor& rope, Tensor& key_gain, int64_t start, int64_t heads, int64_t content, int64_t value, double scale, double softcap,
+                int64_t window) {
+    Tensor both = rows_linear(x, w_in);
+    const int64_t nq = heads * (content + rope.size(2));
+    GM_CHECK(both.size(1) == nq + latent.size(2) + rope.size(2), "mla_step: w_in holds the query rows, then the latent and rotary rows");
+    Tensor out = mla_cached(both.narrow(1, 0, nq), both.narrow(1, nq, both.size(1) - nq), w_up, norm_w, norm_eps, cos, sin, q_scale, k_scale, qk_eps, rms, smin,
+                            smax, latent, rope, key_gain, start, heads, content, value, scale, softcap, window);
+    return rows_linear(out, w_out);
 }
 
 // (issue clocks, completion clocks) of `count` chained tcgen05.mma instructions of shape code `shape` (csrc/bench/mma_issue.cu)
@@ -584,6 +663,9 @@ void register_kernels(pybind11::module_& m) {
           py::arg("smin"), py::arg("smax"), py::arg("dq32") = py::none(), py::arg("quantize") = false);
     m.def("mla_decode", &mla_decode);
     m.def("mla_decode_ok", &mla_decode_ok);
+    m.def("rows_linear", &rows_linear);
+    m.def("mla_cached", &mla_cached);
+    m.def("mla_step", &mla_step);
     m.def("mma_issue_bench", &mma_issue_bench, py::arg("shape"), py::arg("count") = 64);
     m.def("router_fwd", &router_fwd);
     m.def("router_bwd", &router_bwd);

@@ -42,11 +42,27 @@ void launch_activation_bwd(const void* dact, const void* pre, void* dpre, const 
                            cudaStream_t s);
 
 // attention/mla_decode.cu
-int mla_decode_splits(int B, int T, int S);
+int mla_decode_splits(int B, int T, int H, int r, int S);
 bool mla_decode_supported(int H, int Hkv, int r, int dr);
 bool launch_mla_decode(const float* q_latent, const float* q_rope, const void* latent, const void* rope, const void* key_gain,
                        long long latent_bs, long long rope_bs, long long gain_bs, float* part_ctx, float* part_ml, float* context, int B, int T,
                        int H, int Hkv, int r, int dr, int S, int splits, int start, int window, float scale, float softcap, cudaStream_t s);
+// New tokens of a latent cache from their projections to the attention output (pointers as in the kernels of the file; `latent`,
+// `rope` and `key_gain` are whole caches whose rows start .. start + T - 1 are written).
+struct MlaCachedArgs {
+    const void *query, *low;
+    long long q_pitch, low_pitch;
+    const float *norm_w, *cos, *sin, *w_up, *q_scale, *k_scale;
+    void *latent, *rope, *key_gain;
+    long long latent_bs, rope_bs, gain_bs;
+    float *q_latent, *q_rope, *part_ctx, *part_ml;
+    void* out;                       // bf16 [B, T, H, value]
+    int B, T, H, Hkv, r, dr, content, value, start, splits, window, rms;
+    float norm_eps, qk_eps, smin, smax, scale, softcap;
+};
+bool launch_mla_cached(const MlaCachedArgs& a, cudaStream_t s);
+bool rows_linear_supported(int rows, int N, int K);
+bool launch_rows_linear(const void* x, const void* w, void* y, int rows, int N, int K, long long x_pitch, long long y_pitch, cudaStream_t s);
 
 // fused/router.cu
 int router_blocks(int tokens);

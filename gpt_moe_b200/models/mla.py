@@ -184,6 +184,10 @@ class MLAttention(nn.Module):
         start, end = cache.length, cache.length + t
         if end > cache.latent.size(1) or b != cache.latent.size(0):
             raise ValueError("MLA cache capacity or batch size mismatch")
+        fused = self._cached_on_gpu(x, cache, start, window)
+        if fused is not None:
+            cache.length = end
+            return fused
         query, latent, rope = self._project(x, start)
         cache.latent[:, start:end] = latent
         cache.rope[:, start:end] = rope[:, :, 0]
@@ -207,6 +211,44 @@ class MLAttention(nn.Module):
         context = context.view(b, t, self.n_kv_heads, self.group, self.kv_rank)
         out = torch.einsum("bthgr,hdr->bthgd", context, w_v).reshape(b, t, self.attn_dim)
         return self.out_proj(out.to(x.dtype))
+
+
+    def _cached_on_gpu(self, x: Tensor, cache: MLACache, start: int, window: Optional[int]) -> Optional[Tensor]:
+        """The cached step as five launches (`csrc/attention/mla_decode.cu`): projections; norm, rotation, QK gains, absorbed
+        queries and the cache entries; attention over the cache in splits; merge and W_v; output projection.  The general path
+        of `forward_cached` issues some sixty.  None when a shape, type or option needs that path."""
+        b, t, hidden = x.shape
+        caches = (cache.latent, cache.rope, cache.key_gain)
+        w_up = self.kv_up_proj.weight
+        if not (x.is_cuda and self.rotary is not None and t > 0 and all(c.dtype == torch.bfloat16 and c.is_cuda and c.stride(2) == 1
+                and c.stride(1) == c.size(2) for c in caches) and all(m.bias is None for m in (self.q_proj, self.kv_down_proj, self.kv_up_proj))
+                and w_up.dtype == torch.float32 and w_up.is_contiguous() and w_up.data_ptr() % 16 == 0 and self.content_dim <= 256
+                and (self.softcap <= 0.0 or self.tanh_backend == "exact") and start + t <= self.rotary.cos_cached.shape[0]
+                and cache.rope.size(1) == cache.latent.size(1) == cache.key_gain.size(1) and self.rotary.cos_cached.dtype == torch.float32):
+            return None
+        from ..ops import cuda_ops
+        c = cuda_ops.ext()
+        if not c.mla_decode_ok(self.n_heads, self.n_kv_heads, self.kv_rank, self.rope_dim):
+            return None
+        cuda_ops.count_path("mla_decode:kernel")
+        qs = ks = None
+        if self.use_qk_norm:
+            qs, ks = self.q_scale.detach().float().reshape(-1), self.k_scale.detach().float().reshape(-1)
+        norm_w = None if self.kv_norm.weight is None else self.kv_norm.weight.detach().float()
+        rest = (w_up.detach(), norm_w, self.kv_norm.eps, self.rotary.cos_cached, self.rotary.sin_cached, qs, ks, self.qk_eps, self.qk_norm_type == "rms",
+                max(self.qk_scale_min, -3.0e38), min(self.qk_scale_max, 3.0e38), *caches, start, self.n_heads, self.content_dim, self.value_dim,
+                self.softmax_scale, max(self.softcap, 0.0), -1 if (self.is_full_attention or window is None) else int(window))
+        plain = (self.q_proj, self.kv_down_proj, self.out_proj)
+        if (b * t <= 32 and not self.q_rank and hidden % 32 == 0 and self.attn_dim % 32 == 0 and self.out_proj.bias is None
+                and all(type(m) is Linear and m.precision == "default" and not m._forward_hooks and not m._forward_pre_hooks for m in plain)):
+            return c.mla_step(cuda_ops._as_bf16_2d(x), cuda_ops.bf16_weight((self.q_proj.weight, self.kv_down_proj.weight)),
+                              cuda_ops.bf16_weight((self.out_proj.weight,)), *rest).view(b, t, -1)
+        query = x
+        if self.q_rank:
+            query = api.rms_norm(self.q_down_proj(query), self.q_norm.weight, self.q_norm.eps)
+        query = self.q_proj(query).reshape(b * t, -1)
+        out = c.mla_cached(query, self.kv_down_proj(x).reshape(b * t, -1), *rest)
+        return self.out_proj(out.view(b, t, self.attn_dim))
 
 
 def api_mla_decode(q_latent: Tensor, q_rope: Tensor, latent: Tensor, rope: Tensor, key_gain: Tensor,

@@ -1,0 +1,78 @@
+"""The cached step of multi-head latent attention (`MLAttention.forward_cached`) on the GPU against the plain fp32 path on the CPU."""
+import copy
+
+import pytest
+import torch
+
+from gpt_moe_b200.config import get_preset
+from gpt_moe_b200.models.mla import MLAttention
+
+pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    a, b = a.detach().double().cpu(), b.detach().double().cpu()
+    return ((a - b).norm() / b.norm().clamp_min(1e-30)).item()
+
+
+# batch, new tokens, heads, kv heads, latent rank, rope width, content width, tokens already there, window, QK-norm, query rank
+CASES = [
+    (3, 1, 16, 16, 512, 64, 64, 333, None, True, 0),         # one token, cache no multiple of the tile
+    (1, 1, 16, 16, 512, 64, 64, 0, None, True, 0),           # first token of an empty cache
+    (33, 1, 16, 4, 512, 64, 64, 65, 40, True, 0),            # more rows than the skinny projection takes; groups of heads; window
+    (2, 16, 16, 16, 512, 64, 64, 31, None, True, 0),         # 32 rows: largest skinny projection, tokens straddle tiles
+    (1, 37, 8, 8, 256, 16, 48, 100, 20, True, 0),            # two tokens to a 16-row tile, odd count, narrow rotary part
+    (2, 3, 32, 8, 256, 10, 54, 62, None, False, 0),          # 32 heads, rotary width no multiple of 8, no QK-norm
+    (1, 70, 16, 16, 768, 32, 32, 5, None, True, 64),         # wide latent, low-rank queries, many tokens per weight pass
+    (2, 1, 8, 2, 1024, 64, 64, 200, 64, True, 0),            # widest latent
+]
+
+
+@pytest.mark.parametrize("b,t,h,hkv,r,dr,c,start,window,norm,q_rank", CASES)
+def test_cached_step_matches_the_plain_path(b, t, h, hkv, r, dr, c, start, window, norm, q_rank):
+    torch.manual_seed(11)
+    gc, tc = get_preset("mla")
+    gc.hidden_size, gc.n_heads, gc.n_kv_heads, gc.use_qk_norm = 256, h, hkv, norm
+    gc.mla_kv_rank, gc.mla_qk_rope_dim, gc.mla_qk_content_dim, gc.mla_value_dim, gc.mla_q_rank = r, dr, c, 32, q_rank
+    tc.resolve(1)
+    cpu = MLAttention(gc, tc).eval()
+    for p in cpu.parameters():
+        if p.dim() == 2:
+            torch.nn.init.normal_(p, std=0.05)
+            p.data = p.data.bfloat16().float()                # both sides then project with the same weights
+    gpu = copy.deepcopy(cpu).cuda()
+    x = torch.randn(b, t, 256).bfloat16()
+    cache = gpu.allocate_cache(b, start + t + 3, device="cuda", dtype=torch.bfloat16)
+    cache.latent.normal_(), cache.rope.normal_(), cache.key_gain.uniform_(0.5, 2.0)
+    poison = start + t
+    for part in (cache.latent, cache.rope, cache.key_gain):
+        part[:, poison:] = float("nan")                       # rows past the new tokens are not read
+    cache.length = start
+    plain = cpu.allocate_cache(b, start + t + 3, device="cpu", dtype=torch.float32)
+    for mine, theirs in ((plain.latent, cache.latent), (plain.rope, cache.rope), (plain.key_gain, cache.key_gain)):
+        mine.copy_(theirs.float().cpu())
+        mine[:, poison:] = 0.0
+    plain.length = start
+    from gpt_moe_b200.ops import cuda_ops
+    before = cuda_ops.path_counts().get("mla_decode:kernel", 0)
+    got = gpu.forward_cached(x.cuda(), cache, window)
+    assert cuda_ops.path_counts().get("mla_decode:kernel", 0) == before + 1
+    want = cpu.forward_cached(x.float(), plain, window)
+    assert got.dtype == torch.bfloat16 and cache.length == plain.length == start + t
+    new = slice(start, start + t)
+    # one rounding to bf16 is 2^-9 / sqrt(3) = 1.1e-3 on average.  Cache entries: the projection's, the norm's and the stored one.
+    # Output: those of query, latent and attention output (several thousand roundings average out in the sums) and its own; the
+    # scores are the exponents of the probabilities, which doubles the share of query and key
+    for name in ("latent", "rope", "key_gain"):
+        assert rel(getattr(cache, name)[:, new], getattr(plain, name)[:, new]) < 5e-3, name
+    assert rel(got, want) < 1.2e-2, rel(got, want)
+    cuda_ops.check_status()
+
+
+@pytest.mark.parametrize("rows,n,k", [(1, 16, 32), (8, 576, 1024), (9, 8, 96), (17, 2624, 1024), (32, 24, 64)])
+def test_rows_linear_matches_matmul(rows, n, k):
+    from gpt_moe_b200.ops import cuda_ops
+    torch.manual_seed(3)
+    x, w = torch.randn(rows, k, device="cuda").bfloat16(), torch.randn(n, k, device="cuda").bfloat16()
+    want = x.double() @ w.double().t()
+    assert rel(cuda_ops.ext().rows_linear(x, w), want) < 3e-3         # fp32 sums, one rounding of the result
