@@ -140,7 +140,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     const int kv_tile = blockIdx.x, kv_head = blockIdx.y, batch = blockIdx.z;
     const int kv0 = kv_tile * TILE;
     const int window = p.window_ptr ? min(max(*p.window_ptr, 0), p.seq_len) : p.window;
-    const int q_tiles_total = p.seq_len / TILE;
+    const int q_tiles_total = (p.seq_len + TILE - 1) / TILE;
     int last_q_tile = (kv0 + TILE - 1 + window) / TILE;
     if (last_q_tile > q_tiles_total - 1) last_q_tile = q_tiles_total - 1;
     const int n_q = last_q_tile - kv_tile + 1;        // query tiles per head that see this key tile
@@ -174,13 +174,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
                 mbar_expect_tx(&bar_qdo[st], QK_BYTES + T_BYTES);
 #pragma unroll
                 for (int sl = 0; sl < QK_SLABS; ++sl)
-                    tma_load_3d(sq + st * QK_BYTES + sl * T_BYTES, &tmap_q, &bar_qdo[st], head * DQK + 64 * sl, row0 + q0, 0);
-                tma_load_3d(sdo + st * T_BYTES, &tmap_do, &bar_qdo[st], head * HD, row0 + q0, 0);
+                    tma_load_3d(sq + st * QK_BYTES + sl * T_BYTES, &tmap_q, &bar_qdo[st], head * DQK + 64 * sl, q0, batch);
+                tma_load_3d(sdo + st * T_BYTES, &tmap_do, &bar_qdo[st], head * HD, q0, batch);
             };
             mbar_expect_tx(bar_kv, QK_BYTES + T_BYTES);
 #pragma unroll
-            for (int sl = 0; sl < QK_SLABS; ++sl) tma_load_3d(sk + sl * T_BYTES, &tmap_k, bar_kv, kv_head * DQK + 64 * sl, row0 + kv0, 0);
-            tma_load_3d(sv, &tmap_v, bar_kv, kv_head * HD, row0 + kv0, 0);
+            for (int sl = 0; sl < QK_SLABS; ++sl) tma_load_3d(sk + sl * T_BYTES, &tmap_k, bar_kv, kv_head * DQK + 64 * sl, kv0, batch);
+            tma_load_3d(sv, &tmap_v, bar_kv, kv_head * HD, kv0, batch);
             for (int it = 0; it < QDO_STAGES && it < n_iter; ++it) load_qdo(it);
             if (!mbar_wait(bar_kv, 0)) { atomicExch(p.status, 301); ok = false; }
             auto issue_sdp = [&](int it) -> bool {               // S = Q K^T ; dP = dO V^T for iteration `it`
@@ -254,12 +254,15 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
             const int q0 = (kv_tile + it % n_q) * TILE;
             const int qpos = q0 + r;
             const long long stat = (static_cast<long long>(batch) * p.heads + head) * p.seq_len + qpos;
-            const float lse2 = p.lse[stat] * 1.4426950408889634f;
-            const float delta = p.delta[stat];
+            // rows past the sequence end are zeros; an infinite log-sum-exp makes their probabilities 0
+            const bool live = qpos < p.seq_len;
+            const float lse2 = live ? p.lse[stat] * 1.4426950408889634f : INFINITY;
+            const float delta = live ? p.delta[stat] : 0.f;
             int w_row = window, w_last = window;                        // document masking: see the forward kernel
             if (p.doc_start) {
-                w_row = min(window, qpos - p.doc_start[row0 + qpos]);
-                w_last = min(window, q0 + TILE - 1 - p.doc_start[row0 + q0 + TILE - 1]);
+                const int last = min(q0 + TILE, p.seq_len) - 1;
+                if (live) w_row = min(window, qpos - p.doc_start[row0 + qpos]);
+                w_last = min(window, last - p.doc_start[row0 + last]);
             }
             const bool need_mask = (q0 == kv0) || (q0 + TILE - 1 - kv0 > w_last);
             if (!mbar_wait(bar_sdp, ph)) { atomicExch(p.status, 305); ok = false; break; }
@@ -309,13 +312,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 #pragma unroll
                 for (int sl = 0; sl < DQK / 32; ++sl) {
                     asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.bulk_group [%0, {%2, %3, %4}], [%1];"
-                                 ::"l"(&tmap_dq), "r"(smem_u32(stg + sl * (TILE * 128))), "r"(head * DQK + sl * 32), "r"(row0 + q0), "r"(0) : "memory");
+                                 ::"l"(&tmap_dq), "r"(smem_u32(stg + sl * (TILE * 128))), "r"(head * DQK + sl * 32), "r"(q0), "r"(batch) : "memory");
                 }
                 asm volatile("cp.async.bulk.commit_group;" ::: "memory");
             }
         }
         if (ok && n_iter > 0) {
             // dK, dV: TMEM lanes are the 128 keys of this CTA; each thread writes half of the columns of its key row
+            const bool live = kv0 + r < p.seq_len;
             const long long token = static_cast<long long>(row0) + kv0 + r;
             __nv_bfloat16* dk = reinterpret_cast<__nv_bfloat16*>(p.dk) + token * p.dkv_stride + kv_head * DQK + half * (DQK / 2);
             __nv_bfloat16* dv = reinterpret_cast<__nv_bfloat16*>(p.dv) + token * p.dv_stride + kv_head * HD + half * 32;
@@ -329,7 +333,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
                 wv.y = pack_bf16x2(__uint_as_float(vreg[8 * q + 2]), __uint_as_float(vreg[8 * q + 3]));
                 wv.z = pack_bf16x2(__uint_as_float(vreg[8 * q + 4]), __uint_as_float(vreg[8 * q + 5]));
                 wv.w = pack_bf16x2(__uint_as_float(vreg[8 * q + 6]), __uint_as_float(vreg[8 * q + 7]));
-                *reinterpret_cast<uint4*>(dv + 8 * q) = wv;
+                if (live) *reinterpret_cast<uint4*>(dv + 8 * q) = wv;
             }
 #pragma unroll
             for (int j = 0; j < DQK / 64; ++j) {
@@ -343,7 +347,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
                     wk.y = pack_bf16x2(__uint_as_float(kreg[8 * q + 2]) * p.scale, __uint_as_float(kreg[8 * q + 3]) * p.scale);
                     wk.z = pack_bf16x2(__uint_as_float(kreg[8 * q + 4]) * p.scale, __uint_as_float(kreg[8 * q + 5]) * p.scale);
                     wk.w = pack_bf16x2(__uint_as_float(kreg[8 * q + 6]) * p.scale, __uint_as_float(kreg[8 * q + 7]) * p.scale);
-                    *reinterpret_cast<uint4*>(dk + j * 32 + 8 * q) = wk;
+                    if (live) *reinterpret_cast<uint4*>(dk + j * 32 + 8 * q) = wk;
                 }
             }
         }
@@ -374,7 +378,7 @@ static cudaError_t launch_bwd_variant(const CUtensorMap& tq, const CUtensorMap& 
         if (e != cudaSuccess) return e;
         configured = true;
     }
-    dim3 grid(p.seq_len / TILE, p.heads / p.group, p.batch);
+    dim3 grid((p.seq_len + TILE - 1) / TILE, p.heads / p.group, p.batch);
     kernel<<<grid, BW_THREADS, smem, stream>>>(tq, tk, tv, tdo, tdq, p);
     return cudaGetLastError();
 }

@@ -1,7 +1,7 @@
 // Causal sliding-window attention backward for sm_100a, 64-wide heads, with the score products of the next query tile issued
 // ahead of the gradient products of the current one.
 //
-// Same tiling and products as attn_bwd.cu (one CTA owns 128 keys of one (batch, kv head) and walks the query tiles that see
+// Same tiling and products as attn_bwd.cu (sequences of any length: the tensor maps end at the sequence's last row; one CTA owns 128 keys of one (batch, kv head) and walks the query tiles that see
 // them; S = Q K^T and dP = dO V^T into TMEM, P and dS to shared memory, dV += P^T dO, dK += dS^T Q, dQ = dS K reduced into a
 // fp32 buffer by TMA).  What differs is the order.  In attn_bwd.cu one iteration is a chain: S/dP -> softmax warps -> three
 // gradient products -> dQ read-out, and the S/dP of the next iteration queue behind the gradient products, so the tensor
@@ -108,7 +108,7 @@ attn_bwd_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     const int kv_tile = blockIdx.x, kv_head = blockIdx.y, batch = blockIdx.z;
     const int kv0 = kv_tile * BP_TILE;
     const int window = p.window_ptr ? min(max(*p.window_ptr, 0), p.seq_len) : p.window;
-    const int q_tiles_total = p.seq_len / BP_TILE;
+    const int q_tiles_total = (p.seq_len + BP_TILE - 1) / BP_TILE;
     int last_q_tile = (kv0 + BP_TILE - 1 + window) / BP_TILE;
     if (last_q_tile > q_tiles_total - 1) last_q_tile = q_tiles_total - 1;
     const int n_q = last_q_tile - kv_tile + 1;        // query tiles per head that see this key tile
@@ -134,12 +134,12 @@ attn_bwd_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
                 const int head = kv_head * p.group + it / n_q;
                 const int q0 = (kv_tile + it % n_q) * BP_TILE;
                 mbar_expect_tx(&bar_qdo[st], 2 * BP_T_BYTES);
-                tma_load_3d(sq + st * BP_T_BYTES, &tmap_q, &bar_qdo[st], head * BP_HD, row0 + q0, 0);
-                tma_load_3d(sdo + st * BP_T_BYTES, &tmap_do, &bar_qdo[st], head * BP_HD, row0 + q0, 0);
+                tma_load_3d(sq + st * BP_T_BYTES, &tmap_q, &bar_qdo[st], head * BP_HD, q0, batch);
+                tma_load_3d(sdo + st * BP_T_BYTES, &tmap_do, &bar_qdo[st], head * BP_HD, q0, batch);
             };
             mbar_expect_tx(bar_kv, 2 * BP_T_BYTES);
-            tma_load_3d(sk, &tmap_k, bar_kv, kv_head * BP_HD, row0 + kv0, 0);
-            tma_load_3d(sv, &tmap_v, bar_kv, kv_head * BP_HD, row0 + kv0, 0);
+            tma_load_3d(sk, &tmap_k, bar_kv, kv_head * BP_HD, kv0, batch);
+            tma_load_3d(sv, &tmap_v, bar_kv, kv_head * BP_HD, kv0, batch);
             for (int it = 0; it < BP_STAGES && it < n_iter; ++it) load_qdo(it);
             for (int it = BP_STAGES; it < n_iter; ++it) {
                 // the stage was read by S/dP and by the gradient products of iteration it - BP_STAGES
@@ -238,24 +238,24 @@ attn_bwd_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
 #pragma unroll
                 for (int sl = 0; sl < 2; ++sl) {
                     asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.bulk_group [%0, {%2, %3, %4}], [%1];"
-                                 ::"l"(&tmap_dq), "r"(smem_u32(stg + sl * (BP_TILE * 128))), "r"(head * BP_HD + sl * 32), "r"(row0 + q0), "r"(0) : "memory");
+                                 ::"l"(&tmap_dq), "r"(smem_u32(stg + sl * (BP_TILE * 128))), "r"(head * BP_HD + sl * 32), "r"(q0), "r"(batch) : "memory");
                 }
                 asm volatile("cp.async.bulk.commit_group;" ::: "memory");
             }
             return true;
         };
-        // index of this thread's query row of iteration `jt` in the [batch, head, seq] statistics
-        auto row_stat_index = [&](int jt) -> long long {
+        // statistics of this thread's query row of iteration `jt`, [batch, head, seq].  Rows past the sequence end are zeros; an
+        // infinite log-sum-exp makes their probabilities 0
+        float lse_next = INFINITY, delta_next = 0.f;
+        auto fetch_stats = [&](int jt) {
             const int head_j = kv_head * p.group + jt / n_q;
             const int qpos_j = (kv_tile + jt % n_q) * BP_TILE + r;
-            return (static_cast<long long>(batch) * p.heads + head_j) * p.seq_len + qpos_j;
+            const bool live = qpos_j < p.seq_len;
+            const long long stat = (static_cast<long long>(batch) * p.heads + head_j) * p.seq_len + qpos_j;
+            lse_next = live ? p.lse[stat] : INFINITY;
+            delta_next = live ? p.delta[stat] : 0.f;
         };
-        float lse_next = 0.f, delta_next = 0.f;
-        if (n_iter > 0) {
-            const long long stat0 = row_stat_index(0);
-            lse_next = p.lse[stat0];
-            delta_next = p.delta[stat0];
-        }
+        if (n_iter > 0) fetch_stats(0);
         for (int it = 0; it < n_iter && ok; ++it) {
             const uint32_t ph = it & 1;
             const int head = kv_head * p.group + it / n_q;
@@ -265,15 +265,12 @@ attn_bwd_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
             // latency runs under this iteration's arithmetic instead of in front of it
             const float lse2 = lse_next * 1.4426950408889634f;
             const float delta = delta_next;
-            if (it + 1 < n_iter) {
-                const long long stat_next = row_stat_index(it + 1);
-                lse_next = p.lse[stat_next];
-                delta_next = p.delta[stat_next];
-            }
+            if (it + 1 < n_iter) fetch_stats(it + 1);
             int w_row = window, w_last = window;                        // document masking: see the forward kernel
             if (p.doc_start) {
-                w_row = min(window, qpos - p.doc_start[row0 + qpos]);
-                w_last = min(window, q0 + BP_TILE - 1 - p.doc_start[row0 + q0 + BP_TILE - 1]);
+                const int last = min(q0 + BP_TILE, p.seq_len) - 1;
+                if (qpos < p.seq_len) w_row = min(window, qpos - p.doc_start[row0 + qpos]);
+                w_last = min(window, last - p.doc_start[row0 + last]);
             }
             const bool need_mask = (q0 == kv0) || (q0 + BP_TILE - 1 - kv0 > w_last);
             if (!mbar_wait(bar_sdp, ph)) { atomicExch(p.status, 305); ok = false; break; }
@@ -297,6 +294,7 @@ attn_bwd_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         if (ok && n_iter > 0 && !drain_dq(n_iter - 1)) { atomicExch(p.status, 306); ok = false; }
         if (ok && n_iter > 0) {
             // dK, dV: TMEM lanes are the 128 keys of this CTA; each thread writes half of the columns of its key row
+            const bool live = kv0 + r < p.seq_len;
             const long long token = static_cast<long long>(row0) + kv0 + r;
             __nv_bfloat16* dk = reinterpret_cast<__nv_bfloat16*>(p.dk) + token * p.dkv_stride + kv_head * BP_HD + half * 32;
             __nv_bfloat16* dv = reinterpret_cast<__nv_bfloat16*>(p.dv) + token * p.dv_stride + kv_head * BP_HD + half * 32;
@@ -311,12 +309,12 @@ attn_bwd_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
                 wv.y = pack_bf16x2(__uint_as_float(vreg[8 * q + 2]), __uint_as_float(vreg[8 * q + 3]));
                 wv.z = pack_bf16x2(__uint_as_float(vreg[8 * q + 4]), __uint_as_float(vreg[8 * q + 5]));
                 wv.w = pack_bf16x2(__uint_as_float(vreg[8 * q + 6]), __uint_as_float(vreg[8 * q + 7]));
-                *reinterpret_cast<uint4*>(dv + 8 * q) = wv;
+                if (live) *reinterpret_cast<uint4*>(dv + 8 * q) = wv;
                 wk.x = pack_bf16x2(__uint_as_float(kreg[8 * q]) * p.scale, __uint_as_float(kreg[8 * q + 1]) * p.scale);
                 wk.y = pack_bf16x2(__uint_as_float(kreg[8 * q + 2]) * p.scale, __uint_as_float(kreg[8 * q + 3]) * p.scale);
                 wk.z = pack_bf16x2(__uint_as_float(kreg[8 * q + 4]) * p.scale, __uint_as_float(kreg[8 * q + 5]) * p.scale);
                 wk.w = pack_bf16x2(__uint_as_float(kreg[8 * q + 6]) * p.scale, __uint_as_float(kreg[8 * q + 7]) * p.scale);
-                *reinterpret_cast<uint4*>(dk + 8 * q) = wk;
+                if (live) *reinterpret_cast<uint4*>(dk + 8 * q) = wk;
             }
         }
         if (leader) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
@@ -346,7 +344,7 @@ static cudaError_t launch_pipe_variant(const CUtensorMap& tq, const CUtensorMap&
         if (e != cudaSuccess) return e;
         configured = true;
     }
-    dim3 grid(p.seq_len / BP_TILE, p.heads / p.group, p.batch);
+    dim3 grid((p.seq_len + BP_TILE - 1) / BP_TILE, p.heads / p.group, p.batch);
     kernel<<<grid, BP_THREADS, smem, stream>>>(tq, tk, tv, tdo, tdq, p);
     return cudaGetLastError();
 }

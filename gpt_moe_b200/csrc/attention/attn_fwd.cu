@@ -15,8 +15,10 @@
 // halves of a row exchange only their running maximum, through shared memory, once per key tile.  K and V each use a
 // two-deep ring of shared-memory tiles refilled as soon as the MMA reading a tile has committed; two CTAs fit per SM
 // (80 KB shared memory, 256 TMEM columns each), so one CTA's softmax overlaps the other's MMAs.
-// Calls with 64-wide heads, no document mask and a sequence length that is a multiple of 256 go to attn_fwd_dual.cu instead
-// (two query tiles per CTA); this kernel serves the rest and is the one that kernel is tested against.
+// The tensor maps are [column, position, sequence]: a tile that reaches past the end of its sequence is filled with zeros instead of
+// the next sequence's rows, its query rows are not stored and its keys lie past every query (the causal mask), so any length runs.
+// Most calls with 64-wide heads and no document mask go to attn_fwd_dual.cu instead (two query tiles per CTA, see
+// attn_fwd_dual_supported); this kernel serves the rest and is the one that kernel is tested against.
 // Reference counterpart: FlexAttention with the causal + sliding-window BlockMask (model/gpt.py:311-687,
 // model/attention/self_attention.py:250-255); here the window test is exact per token in every tile.
 #include "../common/ptx.cuh"
@@ -32,10 +34,6 @@ constexpr int SLAB_BYTES = AT_BM * 64 * 2;          // 128 rows x 64 bf16 column
 constexpr int V_BYTES = AT_BN * AT_D * 2;
 constexpr uint32_t AT_TMEM_COLS = 256;
 constexpr int KV_STAGES = 2;      // key/value tiles in flight: the global->shared latency of a strided tile spans more than one tile of work
-
-__device__ __forceinline__ void tma_load_2d_as3d(void* dst, const void* tmap, uint64_t* bar, int col, int row) {
-    tma_load_3d(dst, tmap, bar, col, row, 0);
-}
 
 // Softmax of one thread's 64 scores of the current key tile (two 32-column TMEM reads per pass).
 // Pass 1 finds the row maximum (combined with the other half of the row through shared memory); pass 2 forms the
@@ -131,7 +129,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     int w_first = window, w_last = window;
     if (p.doc_start) {
         w_first = min(window, q0 - p.doc_start[row0 + q0]);
-        w_last = min(window, q0 + AT_BM - 1 - p.doc_start[row0 + q0 + AT_BM - 1]);
+        const int last = min(q0 + AT_BM, p.seq_len) - 1;
+        w_last = min(window, last - p.doc_start[row0 + last]);
     }
     int kv_lo = q0 - w_first;
     if (kv_lo < 0) kv_lo = 0;
@@ -172,16 +171,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
                 mbar_expect_tx(&bar_k[st], K_BYTES);
 #pragma unroll
                 for (int sl = 0; sl < QK_SLABS; ++sl)
-                    tma_load_2d_as3d(sk + st * K_BYTES + sl * SLAB_BYTES, &tmap_k, &bar_k[st], k_col + 64 * sl, row0 + kv_lo + tile * AT_BN);
+                    tma_load_3d(sk + st * K_BYTES + sl * SLAB_BYTES, &tmap_k, &bar_k[st], k_col + 64 * sl, kv_lo + tile * AT_BN, batch);
             };
             auto load_v = [&](int tile) {
                 const int st = tile % KV_STAGES;
                 mbar_expect_tx(&bar_v[st], V_BYTES);
-                tma_load_2d_as3d(sv + st * V_BYTES, &tmap_v, &bar_v[st], v_col, row0 + kv_lo + tile * AT_BN);
+                tma_load_3d(sv + st * V_BYTES, &tmap_v, &bar_v[st], v_col, kv_lo + tile * AT_BN, batch);
             };
             mbar_expect_tx(bar_q, Q_BYTES);
 #pragma unroll
-            for (int sl = 0; sl < QK_SLABS; ++sl) tma_load_2d_as3d(sq + sl * SLAB_BYTES, &tmap_q, bar_q, q_col + 64 * sl, row0 + q0);
+            for (int sl = 0; sl < QK_SLABS; ++sl) tma_load_3d(sq + sl * SLAB_BYTES, &tmap_q, bar_q, q_col + 64 * sl, q0, batch);
             for (int t = 0; t < KV_STAGES && t < n_tiles; ++t) { load_k(t); load_v(t); }
             if (!mbar_wait(bar_q, 0) || !mbar_wait(&bar_k[0], 0)) { atomicExch(p.status, 201); ok = false; }
             if (ok) { tc_fence_after(); issue_s(0); }
@@ -214,7 +213,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         const int quad = warp & 3, half = warp >> 2;         // TMEM lanes 32*quad..+31; key / output columns of this half
         const int r = quad * 32 + lane;
         const int qpos = q0 + r;
-        const int w_row = p.doc_start ? min(window, qpos - p.doc_start[row0 + qpos]) : window;     // this row's look-back
+        const bool live = qpos < p.seq_len;                     // rows past the sequence end are computed on zeros and not stored
+        const int w_row = p.doc_start && live ? min(window, qpos - p.doc_start[row0 + qpos]) : window;     // this row's look-back
         const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
         const float c = p.scale_log2e;
         constexpr bool capped = CAPPED;
@@ -263,6 +263,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
             row_stat[half * AT_BM + r] = l;
             asm volatile("bar.sync %0, 64;" ::"r"(bar_id) : "memory");
             l += row_stat[(half ^ 1) * AT_BM + r];
+        }
+        if (ok && live) {
             const float inv = 1.f / l;
             const long long token = static_cast<long long>(row0) + qpos;
             __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.out) + token * p.out_stride + head * AT_D + half * 32;
@@ -325,7 +327,7 @@ static cudaError_t launch_fwd_variant(const CUtensorMap& tq, const CUtensorMap& 
         if (e != cudaSuccess) return e;
         configured = true;
     }
-    dim3 grid(p.seq_len / AT_BM, p.heads, p.batch);
+    dim3 grid((p.seq_len + AT_BM - 1) / AT_BM, p.heads, p.batch);
     kernel<<<grid, AT_THREADS, smem, stream>>>(tq, tk, tv, p);
     return cudaGetLastError();
 }

@@ -115,7 +115,7 @@ class SelfAttention(nn.Module):
         optional logit soft-capping and document masking, no padding mask).  Returns None when the shapes or options call for the general path."""
         b, t, _ = x.shape
         d, hq, hk = self.head_size, self.n_heads, self.n_kv_heads
-        if not (x.is_cuda and self.q_proj.bias is None and d == 64 and hq + hk <= 64 and hq % hk == 0 and t % 128 == 0
+        if not (x.is_cuda and self.q_proj.bias is None and d == 64 and hq + hk <= 64 and hq % hk == 0 and (t % 128 == 0 or self.softcap == 0.0)
                 and self.is_causal and ctx.attn_mask is None):
             return None
         from ..ops import cuda_ops

@@ -131,7 +131,7 @@ class MLAttention(nn.Module):
         b, t, _ = x.shape
         h, hk, d = self.n_heads, self.n_kv_heads, self.head_size
         if not (x.is_cuda and d == 128 and self.value_dim == 64 and self.rope_dim > 0 and self.rotary is not None and h + hk <= 64
-                and t % 128 == 0 and self.is_causal and self.softcap == 0.0 and ctx.attn_mask is None and ctx.document_ids is None
+                and self.is_causal and self.softcap == 0.0 and ctx.attn_mask is None and ctx.document_ids is None
                 and self.q_proj.bias is None):
             return None
         from ..ops import cuda_ops

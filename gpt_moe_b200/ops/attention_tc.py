@@ -9,10 +9,13 @@ from torch import Tensor
 
 
 def supported(q: Tensor, k: Tensor, v: Tensor, softcap_value: float) -> bool:
+    """Any sequence length; with soft-capping multiples of 128 only (the kernels cap with the hardware's approximate tanh, other
+    lengths keep the backend that the caller names)."""
     b, t, h, d = q.shape
-    return (q.dtype == torch.bfloat16 and k.dtype == torch.bfloat16 and v.dtype == torch.bfloat16 and d in (64, 128) and k.shape[-1] == d
-            and v.shape[-1] == 64 and t % 128 == 0 and softcap_value >= 0.0 and h % k.shape[2] == 0
-            and all(x.stride(3) == 1 and x.stride(2) == x.shape[3] and x.stride(0) == t * x.stride(1) and x.stride(1) % 8 == 0 for x in (q, k, v)))
+    return (b > 0 and q.dtype == torch.bfloat16 and k.dtype == torch.bfloat16 and v.dtype == torch.bfloat16 and d in (64, 128) and k.shape[-1] == d
+            and v.shape[-1] == 64 and t > 0 and (softcap_value == 0.0 or (softcap_value > 0.0 and t % 128 == 0)) and h % k.shape[2] == 0
+            and all(x.stride(3) == 1 and x.stride(2) == x.shape[3] and x.stride(0) == t * x.stride(1) and x.stride(1) % 8 == 0 and x.data_ptr() % 16 == 0
+                    for x in (q, k, v)))
 
 
 def document_starts(document_ids: Tensor) -> Tensor:
@@ -43,7 +46,8 @@ class _AttentionFn(torch.autograd.Function):
         window, scale, softcap = ctx.cfg
         b, t, h, d = q.shape
         hk = k.shape[2]
-        d_out = d_out if (d_out.stride(3) == 1 and d_out.stride(2) == 64 and d_out.stride(0) == t * d_out.stride(1)) else d_out.contiguous()
+        d_out = d_out if (t > 1 and d_out.stride(3) == 1 and d_out.stride(2) == 64 and d_out.stride(0) == t * d_out.stride(1)
+                          and d_out.stride(1) % 8 == 0 and d_out.data_ptr() % 16 == 0) else d_out.contiguous()
         if d != 64:                   # wide query / key heads: separate gradient tensors
             dk = torch.empty((b, t, hk, d), dtype=q.dtype, device=q.device)
             dv = torch.empty((b, t, hk, 64), dtype=q.dtype, device=q.device)

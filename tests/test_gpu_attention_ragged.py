@@ -1,0 +1,59 @@
+"""The attention kernels at sequence lengths that are no multiple of a tile, against the fp32 definition."""
+import pytest
+import torch
+
+from gpt_moe_b200.ops import attention_cuda, cuda_ops
+from gpt_moe_b200.ops import reference as ref
+
+pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    a, b = a.detach().double(), b.detach().double()
+    return ((a - b).norm() / b.norm().clamp_min(1e-30)).item()
+
+
+# one row, inside a tile, edges of one and two tiles, an odd number of tiles on both sides of the two-tile kernel's rule
+@pytest.mark.parametrize("t,window,hq,hk,d", [(1, None, 2, 2, 64), (45, None, 4, 4, 64), (127, 20, 2, 1, 64), (129, None, 4, 2, 64),
+                                               (184, 64, 2, 2, 64), (300, None, 2, 2, 64), (1000, 256, 3, 3, 64), (1100, None, 2, 1, 64),
+                                               (45, None, 2, 2, 128), (333, 100, 2, 1, 128)])
+def test_any_length_forward_and_backward(t, window, hq, hk, d):
+    torch.manual_seed(5)
+    b = 3
+    q, k, v = (torch.randn(b, t, h, w, device="cuda").bfloat16() for h, w in ((hq, d), (hk, d), (hk, 64)))
+    g = torch.randn(b, t, hq, 64, device="cuda").bfloat16()
+    for x in (q, k, v, g):
+        x[1] = float("nan")                       # a tile that reaches past a sequence's end must not see the next sequence
+    q, k, v = (x.requires_grad_() for x in (q, k, v))
+    before = cuda_ops.path_counts().get("attention:tcgen05", 0)
+    out = attention_cuda.attention(q, k, v, window=window)
+    assert cuda_ops.path_counts()["attention:tcgen05"] == before + 1
+    grads = torch.autograd.grad(out, (q, k, v), g)
+    keep = [0, 2]
+    want_in = [x.detach()[keep].float().requires_grad_() for x in (q, k, v)]
+    want = ref.attention(*want_in, causal=True, window=window)
+    want_grads = torch.autograd.grad(want, want_in, g[keep].float())
+    # bf16 probabilities and results: a rounding is 2^-9 / sqrt(3) = 1.1e-3 on average, two to three of them on the way to each output
+    assert rel(out[keep], want) < 6e-3
+    for got, exp in zip(grads, want_grads):
+        if exp.norm() > 1e-3:                     # a single row attends to itself alone: its score gradients vanish
+            assert rel(got[keep], exp) < 1e-2
+        else:
+            assert got[keep].float().norm() < 1e-1
+    cuda_ops.check_status()
+
+
+@pytest.mark.parametrize("t", [200, 300])
+def test_any_length_with_document_mask(t):
+    torch.manual_seed(6)
+    q, k, v = (torch.randn(2, t, 2, 64, device="cuda").bfloat16().requires_grad_() for _ in range(3))
+    g = torch.randn(2, t, 2, 64, device="cuda").bfloat16()
+    docs = (torch.rand(2, t, device="cuda") < 0.02).int().cumsum(1)
+    out = attention_cuda.attention(q, k, v, document_ids=docs)
+    grads = torch.autograd.grad(out, (q, k, v), g)
+    want_in = [x.detach().float().requires_grad_() for x in (q, k, v)]
+    want = ref.attention(*want_in, causal=True, document_ids=docs)
+    assert rel(out, want) < 6e-3
+    for got, exp in zip(grads, torch.autograd.grad(want, want_in, g.float())):
+        assert rel(got, exp) < 1e-2
+    cuda_ops.check_status()
