@@ -419,6 +419,34 @@ Tensor ce_fwd_bwd(Tensor& logits, const Tensor& targets, const Tensor& grad_scal
     return loss;
 }
 
+// fp32 [rows]: -log softmax(logits)[target], 0 for ignored rows; logits [rows, vocab] bf16 are only read
+Tensor row_nll(const Tensor& logits, const Tensor& targets, int64_t ignore_index) {
+    c10::cuda::CUDAGuard guard(logits.device());
+    GM_CHECK(logits.is_cuda() && logits.scalar_type() == torch::kBFloat16 && logits.dim() == 2 && logits.stride(1) == 1, "row_nll: logits [rows, vocab] bf16");
+    GM_CHECK(targets.is_cuda() && targets.scalar_type() == torch::kInt64 && targets.is_contiguous() && targets.numel() == logits.size(0), "row_nll: int64 targets");
+    Tensor loss = gm::out_empty({logits.size(0)}, logits.options().dtype(torch::kFloat32));
+    launch_row_nll(logits.data_ptr(), reinterpret_cast<const long long*>(targets.data_ptr<int64_t>()), loss.data_ptr<float>(), logits.size(0), logits.size(1),
+                   logits.stride(0), ignore_index, status_word(logits.device().index()), stream());
+    return loss;
+}
+
+// fp32 [n, length - 1]: log-probabilities of the tokens prefix[i] <= position < end[i], 0 at other positions
+Tensor continuation_logprob(const Tensor& logits, const Tensor& tokens, const Tensor& prefix, const Tensor& end) {
+    c10::cuda::CUDAGuard guard(logits.device());
+    GM_CHECK(logits.is_cuda() && logits.scalar_type() == torch::kBFloat16 && logits.dim() == 3 && logits.stride(2) == 1, "continuation_logprob: logits [n, length, vocab] bf16");
+    const int n = logits.size(0), length = logits.size(1);
+    GM_CHECK(n >= 1 && n <= 65535 && length >= 2, "continuation_logprob: 1 to 65535 rows of at least two tokens");
+    GM_CHECK(tokens.is_cuda() && tokens.scalar_type() == torch::kInt64 && tokens.dim() == 2 && tokens.size(0) == n && tokens.size(1) == length && tokens.stride(1) == 1,
+             "continuation_logprob: int64 tokens [n, length]");
+    for (const Tensor* t : {&prefix, &end})
+        GM_CHECK(t->is_cuda() && t->scalar_type() == torch::kInt64 && t->is_contiguous() && t->numel() == n, "continuation_logprob: int64 bounds [n]");
+    Tensor lp = gm::out_empty({n, length - 1}, logits.options().dtype(torch::kFloat32));
+    auto ll = [](const Tensor& t) { return reinterpret_cast<const long long*>(t.data_ptr<int64_t>()); };
+    launch_continuation_logprob(logits.data_ptr(), ll(tokens), ll(prefix), ll(end), lp.data_ptr<float>(), n, length, logits.size(2), logits.stride(0),
+                                logits.stride(1), tokens.stride(0), status_word(logits.device().index()), stream());
+    return lp;
+}
+
 void adamw(Tensor& p, const Tensor& g, Tensor& m, Tensor& v, const OptTensor& p_bf16, double lr, double beta1, double beta2,
            double eps, double wd, int64_t step, double grad_scale) {
     c10::cuda::CUDAGuard guard(p.device());
@@ -680,6 +708,8 @@ void register_kernels(pybind11::module_& m) {
     m.def("activation_fwd", &activation_fwd, py::arg("pre"), py::arg("name"), py::arg("meta") = py::none(), py::arg("quantize") = false);
     m.def("activation_bwd", &activation_bwd, py::arg("dact"), py::arg("pre"), py::arg("name"), py::arg("meta") = py::none(), py::arg("quantize") = false);
     m.def("ce_fwd_bwd", &ce_fwd_bwd);
+    m.def("row_nll", &row_nll);
+    m.def("continuation_logprob", &continuation_logprob);
     m.def("adamw", &adamw);
     m.def("muon_prepare", &muon_prepare);
     m.def("muon_apply", &muon_apply);

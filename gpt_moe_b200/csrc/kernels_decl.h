@@ -72,6 +72,10 @@ bool launch_router_bwd(const void* logits, bool bf16, const long long* top_idx, 
                        void* dlogits, int tokens, int experts, int top_k, int renormalise, cudaStream_t s);
 
 // fused/loss_optim.cu
+void launch_row_nll(const void* logits, const long long* targets, float* loss, int rows, int vocab, long long row_stride, long long ignore_index,
+                    int* status, cudaStream_t s);
+void launch_continuation_logprob(const void* logits, const long long* tokens, const long long* prefix, const long long* end, float* lp, int n, int length,
+                                 int vocab, long long batch_stride, long long row_stride, long long token_stride, int* status, cudaStream_t s);
 void launch_ce_fwd_bwd(void* logits, const long long* targets, float* loss, const float* grad_scale, int rows, int vocab,
                        long long row_stride, long long ignore_index, int write_grad, cudaStream_t s);
 void launch_adamw(float* p, const float* g, void* m, void* v, bool moments_bf16, void* p_bf16, long long n, float lr, float beta1,

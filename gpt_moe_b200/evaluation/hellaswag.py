@@ -67,8 +67,15 @@ def one_shot_prefix(example: Dict) -> str:
 def continuation_scores(logits: torch.Tensor, input_ids: torch.Tensor, prefix_lengths: Sequence[int],
                         true_lengths: Sequence[int]) -> torch.Tensor:
     """Mean log-probability of tokens [prefix_len, true_len) of every row, predicted from the previous position."""
-    log_probs = F.log_softmax(logits.float(), dim=-1)
     n, t = input_ids.shape
+    if logits.is_cuda and len(prefix_lengths) == len(true_lengths) == n:
+        from ..ops import cuda_ops
+        bounds = torch.stack([torch.as_tensor(x, dtype=torch.int64) for x in (prefix_lengths, true_lengths)]).to(input_ids.device)
+        token_lp = cuda_ops.continuation_logprob(logits, input_ids, bounds[0], bounds[1])      # 0 outside the continuations
+        if token_lp is not None:
+            count = (bounds[1].clamp(max=t) - bounds[0].clamp(min=1)).clamp(min=1)              # positions 1 .. t - 1 have a prediction
+            return token_lp.sum(dim=1) / count
+    log_probs = F.log_softmax(logits.float(), dim=-1)
     token_lp = log_probs[:, :-1].gather(-1, input_ids[:, 1:, None]).squeeze(-1)          # [n, t-1]: log p(token j+1 | <= j)
     pos = torch.arange(1, t, device=input_ids.device)[None, :]
     pre = torch.as_tensor(prefix_lengths, device=input_ids.device)[:, None]

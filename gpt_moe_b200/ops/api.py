@@ -11,7 +11,7 @@ show that none did:
               (`ops/attention_cuda.py`)
   linear      row pitch not a multiple of 16 bytes (k or n not a multiple of 8)  -> torch `F.linear`
   rms_norm    widths other than 128*{1,2,4,6,8,12,16}, other dtypes               -> torch ops
-  cross_entropy on materialised logits (evaluation)                              -> torch ops
+  cross_entropy on materialised logits with gradients, or not in bf16           -> torch ops
 """
 from __future__ import annotations
 

@@ -1,0 +1,55 @@
+"""Losses and continuation scores from materialised logits against fp64."""
+import pytest
+import torch
+
+from gpt_moe_b200.evaluation.hellaswag import continuation_scores
+from gpt_moe_b200.ops import cuda_ops
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rows,vocab,pitch", [(1, 1, 1), (5, 7, 7), (3, 1000, 1003), (64, 8192, 8192), (33, 50304, 50304)])
+def test_row_losses(rows, vocab, pitch):
+    torch.manual_seed(1)
+    logits = (6 * torch.randn(rows, pitch, device="cuda")).bfloat16()[:, :vocab]
+    if vocab > 4:
+        logits[0, :3] = float("-inf")
+        logits[-1, 2] = 80.0                                   # one entry far above the rest
+    targets = torch.randint(min(3, vocab - 1), vocab, (rows,), device="cuda")
+    if rows > 4:
+        targets[2] = -100
+    got = cuda_ops.cross_entropy(logits, targets, -100)
+    want = torch.nn.functional.cross_entropy(logits.double(), targets, ignore_index=-100)
+    # fp32 sums of up to 50304 exponentials with 2-ulp exponentials: 1e-6 of a loss of a few units
+    assert abs(got.item() - want.item()) < 1e-5 * max(1.0, abs(want.item()))
+    assert torch.isnan(cuda_ops.cross_entropy(logits, torch.full_like(targets, -100), -100))      # nothing to average, as in torch
+    cuda_ops.check_status()
+
+
+def test_target_outside_the_vocabulary_is_reported():
+    logits = torch.randn(2, 64, device="cuda").bfloat16()
+    assert torch.isnan(cuda_ops.cross_entropy(logits, torch.tensor([3, 64], device="cuda"), -100))
+    with pytest.raises(RuntimeError):
+        cuda_ops.check_status()
+
+
+def test_gradients_still_run_through_torch():
+    logits = torch.randn(4, 64, device="cuda").bfloat16().requires_grad_()
+    cuda_ops.cross_entropy(logits, torch.tensor([1, 2, 3, 4], device="cuda"), -100).backward()
+    assert logits.grad is not None and logits.grad.abs().sum() > 0
+
+
+@pytest.mark.parametrize("n,t,vocab", [(1, 2, 9), (4, 17, 1000), (6, 33, 50304)])
+def test_continuation_scores(n, t, vocab):
+    torch.manual_seed(2)
+    logits = (3 * torch.randn(n, t, vocab, device="cuda")).bfloat16()
+    ids = torch.randint(0, vocab, (n, t), device="cuda")
+    prefix = [min(i, t) for i in range(n)]                     # from the very first position on, where there is no prediction
+    true = [min(prefix[i] + 4 * i + 1, t) for i in range(n)]
+    true[-1] = t + 5 if n > 1 else true[-1]                    # past the end
+    if n > 3:
+        true[1] = prefix[1]                                    # empty
+    got = continuation_scores(logits, ids, prefix, true)
+    want = continuation_scores(logits.cpu().float(), ids.cpu(), prefix, true)
+    assert torch.allclose(got.cpu(), want, rtol=2e-5, atol=2e-5)
+    cuda_ops.check_status()
