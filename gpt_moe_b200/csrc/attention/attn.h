@@ -31,6 +31,7 @@ struct AttnParams {
     void* dv;
     long long dkv_stride, dv_stride;
     int* status;
+    int long_first;                 // backward, set by launch_attn_bwd: key tiles run slowest through the grid, so that the longest start first
     int single_tile;                // 1 keeps the call on the basic kernel of its direction: one query tile per CTA (forward),
                                     // score and gradient products in program order (backward)
 };

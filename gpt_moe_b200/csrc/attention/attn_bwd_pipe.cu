@@ -105,7 +105,8 @@ attn_bwd_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_qdo + BP_STAGES);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int kv_tile = blockIdx.x, kv_head = blockIdx.y, batch = blockIdx.z;
+    const int kv_tile = p.long_first ? blockIdx.z : blockIdx.x, kv_head = p.long_first ? blockIdx.x : blockIdx.y;
+    const int batch = p.long_first ? blockIdx.y : blockIdx.z;
     const int kv0 = kv_tile * BP_TILE;
     const int window = p.window_ptr ? min(max(*p.window_ptr, 0), p.seq_len) : p.window;
     const int q_tiles_total = (p.seq_len + BP_TILE - 1) / BP_TILE;
@@ -344,7 +345,8 @@ static cudaError_t launch_pipe_variant(const CUtensorMap& tq, const CUtensorMap&
         if (e != cudaSuccess) return e;
         configured = true;
     }
-    dim3 grid((p.seq_len + BP_TILE - 1) / BP_TILE, p.heads / p.group, p.batch);
+    const int tiles = (p.seq_len + BP_TILE - 1) / BP_TILE, kv_heads = p.heads / p.group;
+    const dim3 grid = p.long_first ? dim3(kv_heads, p.batch, tiles) : dim3(tiles, kv_heads, p.batch);
     kernel<<<grid, BP_THREADS, smem, stream>>>(tq, tk, tv, tdo, tdq, p);
     return cudaGetLastError();
 }

@@ -120,7 +120,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     float* row_stat = reinterpret_cast<float*>(bars + 16);     // [2 halves][128 rows]
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int q_tile = blockIdx.x, head = blockIdx.y, batch = blockIdx.z;
+    // heads and sequences run fastest through the grid, tiles slowest and the longest first: without a window a tile's work grows with its
+    // position, and started last the longest would leave most SMs idle at the end
+    const int q_tile = gridDim.z - 1 - blockIdx.z, head = blockIdx.x, batch = blockIdx.y;
     const int q0 = q_tile * AT_BM;
     const int window = p.window_ptr ? min(max(*p.window_ptr, 0), p.seq_len) : p.window;
     const int row0 = batch * p.seq_len;
@@ -327,7 +329,7 @@ static cudaError_t launch_fwd_variant(const CUtensorMap& tq, const CUtensorMap& 
         if (e != cudaSuccess) return e;
         configured = true;
     }
-    dim3 grid((p.seq_len + AT_BM - 1) / AT_BM, p.heads, p.batch);
+    dim3 grid(p.heads, p.batch, (p.seq_len + AT_BM - 1) / AT_BM);
     kernel<<<grid, AT_THREADS, smem, stream>>>(tq, tk, tv, p);
     return cudaGetLastError();
 }

@@ -203,8 +203,10 @@ attn_fwd_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_free + DU_STAGES);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int head = blockIdx.y, batch = blockIdx.z;
-    const int q0 = blockIdx.x * 2 * DU_BM;
+    // heads and sequences run fastest through the grid, tiles slowest and the longest first: without a window a tile's work grows with its
+    // position, and started last the longest would leave most SMs idle at the end
+    const int head = blockIdx.x, batch = blockIdx.y;
+    const int q0 = (gridDim.z - 1 - blockIdx.z) * 2 * DU_BM;
     const int window = p.window_ptr ? min(max(*p.window_ptr, 0), p.seq_len) : p.window;
     const int row0 = batch * p.seq_len;
     // key tiles (units of 128 keys) of each query tile: from the tile holding the first key its first row sees to its diagonal tile
@@ -381,10 +383,13 @@ attn_fwd_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
 }
 
 bool attn_fwd_dual_supported(const AttnParams& p) {
-    // an odd number of query tiles leaves the second half of the last CTA idle.  Measured against the single-tile kernel: windowed, 9 tiles,
-    // 26.9 us against 31.7; without a window the last tile is also the longest: 13 tiles 57.8 against 52.9, 33 tiles 136 against 119
+    // Windowed calls, where two query tiles share most of their keys: 16 x 2048 tokens, window 1024 225 us against 238 for the single-tile
+    // kernel; also with an odd number of tiles, where half of the last CTA idles, once there are nine (26.9 against 31.7).  Without
+    // a window the single-tile kernel's finer grain fills the end of the grid better: 16384 tokens 955 us against 1060, 4 x 4096 285
+    // against 303, 13 tiles 52.9 against 57.8; up to 16 tiles an even number is equal or better here (2 tiles 51 against 63).
     const int tiles = (p.seq_len + DU_BM - 1) / DU_BM;
-    return p.qk_dim == 64 && p.doc_start == nullptr && (tiles % 2 == 0 || (tiles >= 9 && p.window <= p.seq_len / 2));
+    const bool windowed = p.window <= p.seq_len / 2;
+    return p.qk_dim == 64 && p.doc_start == nullptr && (windowed ? tiles % 2 == 0 || tiles >= 9 : tiles % 2 == 0 && tiles <= 16);
 }
 
 template <bool CAPPED>
@@ -397,7 +402,7 @@ static cudaError_t launch_dual_variant(const CUtensorMap& tq, const CUtensorMap&
         if (e != cudaSuccess) return e;
         configured = true;
     }
-    dim3 grid((p.seq_len + 2 * DU_BM - 1) / (2 * DU_BM), p.heads, p.batch);
+    dim3 grid(p.heads, p.batch, (p.seq_len + 2 * DU_BM - 1) / (2 * DU_BM));
     kernel<<<grid, DU_THREADS, smem, stream>>>(tq, tk, tv, p);
     return cudaGetLastError();
 }
