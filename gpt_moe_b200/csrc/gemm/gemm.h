@@ -38,8 +38,10 @@ bool make_tensor_map(CUtensorMap* out, const void* base, int elem_bytes, uint64_
                      uint64_t row_stride_bytes, uint64_t batch_stride_bytes, uint32_t box_cols, uint32_t box_rows,
                      int swizzle_bytes);
 
-cudaError_t launch_gemm_bf16(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const GemmParams& p, bool a_mn,
-                             bool b_mn, int sms, cudaStream_t stream);
+// `tc`: map of C in the layout of D (64 x 128 box) when the epilogue may fetch it by TMA (dense, bf16 output, K > 0, A K-major), else null;
+// `tmirror`: with it, for symmetric results, the map of D with a 64-row box.
+cudaError_t launch_gemm_bf16(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const CUtensorMap* tc, const CUtensorMap* tmirror,
+                             const GemmParams& p, bool a_mn, bool b_mn, int sms, cudaStream_t stream);
 
 // Block-scaled MXFP8 GEMM: D[M,N] (bf16) = alpha * A[M,K] B[N,K]^T, e4m3 operands, UE8M0 scales per 32 elements of K.
 // Scales are stored as 512-byte records [row block of 128][K block of 128]; byte (r % 32) * 16 + (r / 32) * 4 + g of a record

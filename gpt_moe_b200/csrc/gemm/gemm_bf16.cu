@@ -41,7 +41,8 @@ constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN_HALF * BK * 2, STAGE_BYTES = A
 constexpr int GEMM_THREADS = 320;           // warp 0 TMA, warp 1 MMA, warps 2-9 epilogue
 constexpr int GROUP_M = 4;               // in pair tiles (256 rows each)
 constexpr uint32_t TMEM_COLS = 512;
-constexpr int STAGING_BYTES = 2 * BM * 128;      // two slabs of [128 rows][128 bytes]; the staging area holds two such buffers
+constexpr int SLAB_BYTES = BM * 128;              // one slab of [128 rows][128 bytes]
+constexpr int STAGING_BYTES = 2 * SLAB_BYTES;    // two slabs; the staging area holds two such buffers
 
 struct TileCoord {
     int m0, n0;        // element offsets of the tile in the output
@@ -121,10 +122,11 @@ __device__ __forceinline__ TileCoord tile_coord(const GemmParams& p, int tile, i
     return t;
 }
 
-template <bool A_MN, bool B_MN>
+template <bool A_MN, bool B_MN, bool TMA_C>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                 const __grid_constant__ CUtensorMap tmap_d, const GemmParams p) {
+                 const __grid_constant__ CUtensorMap tmap_d, const __grid_constant__ CUtensorMap tmap_c,
+                 const __grid_constant__ CUtensorMap tmap_mirror, const GemmParams p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* staging = smem + STAGES * STAGE_BYTES;
@@ -132,7 +134,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     uint64_t* empty = full + STAGES;
     uint64_t* acc_full = empty + STAGES;
     uint64_t* acc_empty = acc_full + 2;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    uint64_t* c_full = acc_empty + 2;                              // TMA_C: [2] slab of C landed
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(c_full + 2);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int cta_rank = static_cast<int>(cluster_ctarank());     // 0 = leader of the pair
@@ -140,11 +143,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
         // acc_empty of the leader collects one arrival per epilogue warp of each of the two CTAs (a remote arrival per thread
         // would put 256 messages per tile on the cluster's shared-memory network)
-        for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 16); }
+        for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 16); mbar_init(&c_full[a], 1); }
         fence_barrier_init();
         tma_prefetch_desc(&tmap_a);
         tma_prefetch_desc(&tmap_b);
         tma_prefetch_desc(&tmap_d);
+        if (TMA_C) tma_prefetch_desc(&tmap_c);
     }
     if (warp == 1) { tmem_alloc_pair(tmem_slot, TMEM_COLS); tmem_relinquish_pair(); }
     tc_fence_before();
@@ -214,6 +218,111 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                 if (++acc == 2) { acc = 0; acc_ph ^= 1; }
             }
         }
+    } else if (TMA_C) {
+        // Epilogue of D = alpha * acc + beta * C for dense bf16 outputs.  C arrives by TMA in the slab the result is staged in: rounds of 64
+        // columns walk a ring of four slabs [128 rows][128 bytes], the slab of the next round is requested while this one is worked
+        // on, and every thread replaces the 16-byte pieces of its row in place.  (Read by the threads themselves, 64 bytes of a row
+        // each, C cost 32 cache lines per load in the chain between accumulator and store: 96 products of 768 x 6144 x 768 took 802 us,
+        // 629 now against 600 without C; 128 of 768 x 3072 x 768 627, 454 and 427; 128 symmetric ones of 768^3 134 and 103.)
+        const int quad = warp & 3;
+        const int half = (warp - 2) >> 2;                          // 32 of a round's 64 columns
+        const int row_in_tile = quad * 32 + lane;
+        const bool leader = threadIdx.x == 64;
+        const int sw = row_in_tile & 7;
+        int acc = 0; uint32_t acc_ph = 0;
+        uint32_t use = 0, fetched = 0;                             // slabs handed to a store so far; slabs of C consumed so far
+        auto fetch_c = [&](const TileCoord& t, int round, uint32_t slab, uint32_t k) {
+            mbar_expect_tx(&c_full[k & 1], SLAB_BYTES);
+            tma_load_3d(staging + (slab & 3) * SLAB_BYTES, &tmap_c, &c_full[k & 1], t.n0 + round * 64, t.m0, t.dz);
+        };
+        if (leader && first_tile < tiles) fetch_c(tile_coord(p, first_tile, cta_rank, m_tiles, n_tiles), 0, 0, 0);
+        for (int tile = first_tile; tile < tiles && ok; tile += tile_step) {
+            const TileCoord t = tile_coord(p, tile, cta_rank, m_tiles, n_tiles);
+            const int rounds = min(BN / 64, (t.n_limit - t.n0 + 63) / 64);
+            float alpha = p.alpha, beta = p.beta;
+            if (p.batch_sumsq != nullptr) {                   // an operand is an un-normalised Muon update: scale the result instead
+                const float inv = 1.f / (sqrtf(p.batch_sumsq[t.dz]) * 1.02f + 1e-6f);
+                if (p.scale_mode == 2) alpha *= inv * inv;
+                else { alpha *= inv; beta *= inv; }
+            }
+            const bool mirror = p.symmetric && t.n0 != t.m0 - cta_rank * BM;
+            if (!mbar_wait(&acc_full[acc], acc_ph)) { atomicExch(p.status, 104); ok = false; break; }
+            tc_fence_after();
+            for (int round = 0; round < rounds; ++round) {
+                if (leader) {
+                    // at most the latest store still reads its slab: the one before it, whose slab comes next at the earliest, is done
+                    asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+                    const uint32_t next = use + (mirror ? 2 : 1);
+                    if (round + 1 < rounds) fetch_c(t, round + 1, next, fetched + 1);
+                    else if (tile + tile_step < tiles) fetch_c(tile_coord(p, tile + tile_step, cta_rank, m_tiles, n_tiles), 0, next, fetched + 1);
+                }
+                uint32_t r[32];
+                tmem_ld_32x32b_x32(tmem_base + acc * BN + (round * 2 + half) * 32 + (static_cast<uint32_t>(quad * 32) << 16), r);
+                tmem_ld_wait();
+                if (round == rounds - 1) {                                    // accumulator fully read: release it early
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster(&acc_empty[acc], 0);
+                }
+                if (!mbar_wait(&c_full[fetched & 1], (fetched >> 1) & 1)) { atomicExch(p.status, 105); ok = false; break; }
+                uint8_t* slab = staging + (use & 3) * SLAB_BYTES;
+                uint8_t* slab_row = slab + row_in_tile * 128;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    uint4* piece = reinterpret_cast<uint4*>(slab_row + (((half * 4 + q) ^ sw) << 4));
+                    const uint4 cv = *piece;
+                    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&cv);
+                    float v[8];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float2 f = __bfloat1622float2(h[e]);
+                        v[2 * e] = __uint_as_float(r[8 * q + 2 * e]) * alpha + beta * f.x;
+                        v[2 * e + 1] = __uint_as_float(r[8 * q + 2 * e + 1]) * alpha + beta * f.y;
+                    }
+                    uint4 o;
+                    o.x = pack_bf16x2(v[0], v[1]); o.y = pack_bf16x2(v[2], v[3]); o.z = pack_bf16x2(v[4], v[5]); o.w = pack_bf16x2(v[6], v[7]);
+                    *piece = o;
+                    if (mirror) { r[4 * q] = o.x; r[4 * q + 1] = o.y; r[4 * q + 2] = o.z; r[4 * q + 3] = o.w; }      // kept packed for the transposed store
+                }
+                fence_proxy_async();
+                asm volatile("bar.sync 1, 256;" ::: "memory");                 // slab complete and visible to the async proxy
+                const int col = t.n0 + round * 64;
+                if (leader) {
+                    if (t.m0 < t.m_limit)
+                        asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
+                                     ::"l"(&tmap_d), "r"(smem_u32(slab)), "r"(col), "r"(t.m0), "r"(t.dz) : "memory");
+                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                }
+                ++use; ++fetched;
+                if (mirror) {
+                    // the 128 x 64 block goes out transposed: 64 rows of two 128-byte slab rows (this CTA's rows [m0, m0 + 64) and the next 64).
+                    // The slab was free before this round's first barrier (see above)
+                    uint8_t* tbuf = staging + (use & 3) * SLAB_BYTES;
+                    uint8_t* tcol = tbuf + (row_in_tile >> 6) * (SLAB_BYTES / 2) + (row_in_tile & 7) * 2;
+                    const int piece = (row_in_tile & 63) >> 3;
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) {
+                        const uint16_t bits = static_cast<uint16_t>(r[(i >> 3) * 4 + ((i & 7) >> 1)] >> ((i & 1) * 16));
+                        *reinterpret_cast<uint16_t*>(tcol + (half * 32 + i) * 128 + ((piece ^ (i & 7)) << 4)) = bits;
+                    }
+                    fence_proxy_async();
+                    asm volatile("bar.sync 1, 256;" ::: "memory");
+                    if (leader) {
+                        for (int sl = 0; sl < 2; ++sl) {
+                            const int tc = t.m0 + sl * 64;
+                            if (tc >= t.n_limit) break;
+                            asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
+                                         ::"l"(&tmap_mirror), "r"(smem_u32(tbuf + sl * (SLAB_BYTES / 2))), "r"(tc), "r"(col), "r"(t.dz) : "memory");
+                        }
+                        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                    }
+                    ++use;
+                }
+            }
+            if (!ok) break;
+            if (++acc == 2) { acc = 0; acc_ph ^= 1; }
+        }
+        if (leader) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     } else {
         // Eight epilogue warps: TMEM lanes 32*quad .. 32*quad+31 are readable by warps with warp % 4 == quad, so two warps share
         // a lane quadrant and split the columns of every round between them (half 0: first slab, half 1: second slab).
@@ -402,10 +511,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 
 constexpr int GEMM_SMEM_BYTES = STAGES * STAGE_BYTES + 2 * STAGING_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/;
 
-template <bool A_MN, bool B_MN>
-static cudaError_t launch_variant(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const GemmParams& p, int sms,
-                                  cudaStream_t stream) {
-    auto kernel = gemm_bf16_kernel<A_MN, B_MN>;
+template <bool A_MN, bool B_MN, bool TMA_C>
+static cudaError_t launch_variant(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const CUtensorMap& tc, const CUtensorMap& tm,
+                                  const GemmParams& p, int sms, cudaStream_t stream) {
+    auto kernel = gemm_bf16_kernel<A_MN, B_MN, TMA_C>;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM_BYTES);
@@ -424,13 +533,17 @@ static cudaError_t launch_variant(const CUtensorMap& ta, const CUtensorMap& tb, 
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, ta, tb, td, p);
+    return cudaLaunchKernelEx(&cfg, kernel, ta, tb, td, tc, tm, p);
 }
 
-cudaError_t launch_gemm_bf16(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const GemmParams& p, bool a_mn,
-                             bool b_mn, int sms, cudaStream_t stream) {
-    if (a_mn) return b_mn ? launch_variant<true, true>(ta, tb, td, p, sms, stream) : launch_variant<true, false>(ta, tb, td, p, sms, stream);
-    return b_mn ? launch_variant<false, true>(ta, tb, td, p, sms, stream) : launch_variant<false, false>(ta, tb, td, p, sms, stream);
+cudaError_t launch_gemm_bf16(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const CUtensorMap* tc, const CUtensorMap* tmirror,
+                             const GemmParams& p, bool a_mn, bool b_mn, int sms, cudaStream_t stream) {
+    if (tc != nullptr && !a_mn) {
+        const CUtensorMap& tm = tmirror != nullptr ? *tmirror : td;
+        return b_mn ? launch_variant<false, true, true>(ta, tb, td, *tc, tm, p, sms, stream) : launch_variant<false, false, true>(ta, tb, td, *tc, tm, p, sms, stream);
+    }
+    if (a_mn) return b_mn ? launch_variant<true, true, false>(ta, tb, td, td, td, p, sms, stream) : launch_variant<true, false, false>(ta, tb, td, td, td, p, sms, stream);
+    return b_mn ? launch_variant<false, true, false>(ta, tb, td, td, td, p, sms, stream) : launch_variant<false, false, false>(ta, tb, td, td, td, p, sms, stream);
 }
 
 }  // namespace gm
