@@ -202,8 +202,9 @@ std::vector<torch::Tensor> mxfp8_quantize(const torch::Tensor& x, const c10::opt
 }
 
 // w [.., rows, cols] bf16 contiguous -> (q [.., rows, cols], scales along cols, qt [.., cols, rows], scales along the original rows)
-std::vector<torch::Tensor> mxfp8_quantize_weight(const torch::Tensor& w) {
-    c10::cuda::CUDAGuard guard(w.device());
+std::vector<torch::Tensor> mxfp8_quantize_weight(const torch::Tensor& weight) {
+    c10::cuda::CUDAGuard guard(weight.device());
+    const torch::Tensor w = reinterpret_cast<uintptr_t>(weight.data_ptr()) % 16 == 0 ? weight : weight.clone();      // the kernel loads 16 bytes at a time
     GM_CHECK(w.is_cuda() && w.scalar_type() == torch::kBFloat16 && w.is_contiguous() && (w.dim() == 2 || w.dim() == 3), "mxfp8_quantize_weight wants a contiguous bf16 CUDA tensor");
     const int64_t batch = w.dim() == 3 ? w.size(0) : 1, rows = w.size(-2), cols = w.size(-1);
     GM_CHECK(rows % 32 == 0 && cols % 32 == 0, "mxfp8_quantize_weight: both dimensions must be multiples of 32");
