@@ -8,6 +8,7 @@
 #include <list>
 #include <unordered_map>
 
+#include "bindings_shared.h"
 #include "guarded_alloc.h"
 #include "gemm/gemm.h"
 #include "attention/attn.h"
@@ -376,6 +377,17 @@ torch::Tensor attn_bwd(const torch::Tensor& q, const torch::Tensor& k, const tor
 
 namespace gm {
 int* status_word(int device) { return status_tensor(device).data_ptr<int>(); }
+
+void gemm_plain(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d) {
+    gemm_bf16(a, b, d, false, false, 1.0, 0.0, c10::nullopt, false, GEMM_DENSE, c10::nullopt, c10::nullopt, c10::nullopt, false, c10::nullopt, 0);
+}
+void gemm_by_expert(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d, const torch::Tensor& tile_expert, const torch::Tensor& meta) {
+    gemm_bf16(a, b, d, false, false, 1.0, 0.0, c10::nullopt, false, GEMM_GROUPED_M, tile_expert, meta, c10::nullopt, false, c10::nullopt, 0);
+}
+torch::Tensor attention_out(const torch::Tensor& q, const torch::Tensor& k, const torch::Tensor& v, int64_t window, double scale, double softcap,
+                            const c10::optional<torch::Tensor>& doc_start) {
+    return attn_fwd(q, k, v, window, scale, softcap, doc_start, false, false, c10::nullopt)[0];
+}
 }  // namespace gm
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {

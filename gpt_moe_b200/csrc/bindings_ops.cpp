@@ -4,6 +4,7 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 
+#include "bindings_shared.h"
 #include "guarded_alloc.h"
 #include "kernels.h"
 #include "kernels_decl.h"
@@ -447,6 +448,58 @@ Tensor continuation_logprob(const Tensor& logits, const Tensor& tokens, const Te
     return lp;
 }
 
+// ---- whole branches of a block without gradients ---------------------------------------------------------------------------
+// With few tokens a forward pass without gradients was bound by the host: a binding call, its Python side and an autograd node cost
+// several times a launch.  These issue the same launches as the separate calls.
+
+// QKV projection -> RoPE + QK-norm -> attention -> output projection.  x [batch * seq, hidden] bf16; returns [batch * seq, hidden].
+Tensor attention_branch(const Tensor& x, const Tensor& w_qkv, const Tensor& w_out, const OptTensor& cos_t, const OptTensor& sin_t, const OptTensor& q_scale,
+                        const OptTensor& k_scale, int64_t batch, int64_t heads, int64_t kv_heads, int64_t head_dim, double eps, bool rms, double smin,
+                        double smax, int64_t window, double scale, double softcap, const OptTensor& doc_start) {
+    c10::cuda::CUDAGuard guard(x.device());
+    check_bf16(x, "x");
+    const int64_t tokens = x.size(0), seq = tokens / batch, width = (heads + 2 * kv_heads) * head_dim;
+    GM_CHECK(x.dim() == 2 && batch > 0 && tokens == batch * seq && w_qkv.size(0) == width, "attention_branch: x [batch * seq, hidden], w_qkv [(H + 2 Hkv) * D, hidden]");
+    for (const OptTensor* t : {&cos_t, &sin_t})
+        GM_CHECK(!t->has_value() || ((*t)->scalar_type() == torch::kFloat32 && (*t)->is_contiguous() && (*t)->size(0) >= seq && (*t)->size(1) == head_dim / 2),
+                 "attention_branch: fp32 rotary tables [>= seq, D / 2]");
+    GM_CHECK((!q_scale.has_value() || (q_scale->scalar_type() == torch::kFloat32 && q_scale->is_contiguous() && q_scale->numel() == heads)) &&
+             (!k_scale.has_value() || (k_scale->scalar_type() == torch::kFloat32 && k_scale->is_contiguous() && k_scale->numel() == kv_heads)),
+             "attention_branch: fp32 QK scales");
+    Tensor qkv = gm::out_empty({tokens, width}, x.options());
+    gemm_plain(x, w_qkv, qkv);
+    Tensor rotated = gm::out_empty({tokens, width}, x.options());
+    rope_qknorm_fwd(qkv, rotated, cos_t, sin_t, q_scale, k_scale, seq, heads, kv_heads, head_dim, eps, rms, smin, smax, kv_heads * head_dim);
+    auto part = [&](int64_t first, int64_t n) {
+        return rotated.as_strided({batch, seq, n, head_dim}, {seq * width, width, head_dim, 1}, rotated.storage_offset() + first * head_dim);
+    };
+    Tensor o = attention_out(part(0, heads), part(heads, kv_heads), part(heads + kv_heads, kv_heads), window, scale, softcap, doc_start);
+    Tensor y = gm::out_empty({tokens, w_out.size(0)}, x.options());
+    gemm_plain(o.view({tokens, heads * head_dim}), w_out, y);
+    return y;
+}
+
+// Router projection -> routing -> gather -> grouped up GEMM -> activation -> grouped down GEMM -> gated combine.
+Tensor moe_branch(const Tensor& x, const Tensor& w_router, int64_t top_k, bool renormalise, const Tensor& w_up, const Tensor& w_down,
+                  const std::string& activation) {
+    c10::cuda::CUDAGuard guard(x.device());
+    check_bf16(x, "x");
+    GM_CHECK(x.dim() == 2 && w_up.dim() == 3 && w_down.dim() == 3, "moe_branch: x [tokens, hidden], weights [E, N, K]");
+    const int64_t tokens = x.size(0), experts = w_up.size(0);
+    Tensor logits = gm::out_empty({tokens, w_router.size(0)}, x.options());
+    gemm_plain(x, w_router, logits);
+    auto routed = router_fwd(logits, top_k, renormalise, false);
+    auto plan = route(routed[0], experts);
+    const Tensor &dest = plan[0], &src = plan[1], &tiles = plan[4], &meta = plan[5];
+    Tensor packed = gather_rows(x, src, meta, top_k, false)[0];
+    Tensor pre = gm::out_empty({packed.size(0), w_up.size(1)}, x.options());
+    gemm_by_expert(packed, w_up, pre, tiles, meta);
+    Tensor act = activation_fwd(pre, activation, meta, false)[0];
+    Tensor y = gm::out_empty({packed.size(0), w_down.size(1)}, x.options());
+    gemm_by_expert(act, w_down, y, tiles, meta);
+    return combine_fwd(y, dest, routed[1], top_k);
+}
+
 void adamw(Tensor& p, const Tensor& g, Tensor& m, Tensor& v, const OptTensor& p_bf16, double lr, double beta1, double beta2,
            double eps, double wd, int64_t step, double grad_scale) {
     c10::cuda::CUDAGuard guard(p.device());
@@ -709,6 +762,8 @@ void register_kernels(pybind11::module_& m) {
     m.def("activation_bwd", &activation_bwd, py::arg("dact"), py::arg("pre"), py::arg("name"), py::arg("meta") = py::none(), py::arg("quantize") = false);
     m.def("ce_fwd_bwd", &ce_fwd_bwd);
     m.def("row_nll", &row_nll);
+    m.def("attention_branch", &attention_branch);
+    m.def("moe_branch", &moe_branch);
     m.def("continuation_logprob", &continuation_logprob);
     m.def("adamw", &adamw);
     m.def("muon_prepare", &muon_prepare);

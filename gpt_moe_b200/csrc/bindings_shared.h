@@ -1,0 +1,11 @@
+// Tensor-level functions of bindings.cpp that the composed calls of bindings_ops.cpp issue as well.
+#pragma once
+#include <torch/extension.h>
+
+namespace gm {
+// d = a b^T (bf16), dense; or grouped by expert: a [rows, K], b [E, N, K] with the tile table of `route`
+void gemm_plain(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d);
+void gemm_by_expert(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d, const torch::Tensor& tile_expert, const torch::Tensor& meta);
+torch::Tensor attention_out(const torch::Tensor& q, const torch::Tensor& k, const torch::Tensor& v, int64_t window, double scale, double softcap,
+                            const c10::optional<torch::Tensor>& doc_start);
+}  // namespace gm

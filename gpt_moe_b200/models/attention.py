@@ -8,7 +8,7 @@ the reference's `[B,H,T,D]` transposes (`self_attention.py:185-187, 265`) never 
 """
 from __future__ import annotations
 
-from typing import Optional
+from typing import Optional, Tuple
 
 import torch
 import torch.nn as nn
@@ -110,14 +110,14 @@ class SelfAttention(nn.Module):
             self.qk_eps, self.qk_norm_type == "rms", self.qk_scale_min, self.qk_scale_max)
         return q, k, v
 
-    def _fused_rope_attention(self, x: Tensor, ctx: AttentionContext) -> Optional[Tensor]:
-        """One QKV GEMM, then RoPE + QK-norm + causal / sliding-window attention as a single autograd node (CUDA, 64-wide heads,
-        optional logit soft-capping and document masking, no padding mask).  Returns None when the shapes or options call for the general path."""
+    def _fused_rope_attention(self, x: Tensor, ctx: AttentionContext) -> Tuple[Optional[Tensor], bool]:
+        """(output, whether the output projection is in it).  One QKV GEMM, then RoPE + QK-norm + causal / sliding-window attention as a single autograd node (CUDA, 64-wide heads,
+        optional logit soft-capping and document masking, no padding mask).  The output is None when the shapes or options call for the general path."""
         b, t, _ = x.shape
         d, hq, hk = self.head_size, self.n_heads, self.n_kv_heads
         if not (x.is_cuda and self.q_proj.bias is None and d == 64 and hq + hk <= 64 and hq % hk == 0 and (t % 128 == 0 or self.softcap == 0.0)
                 and self.is_causal and ctx.attn_mask is None):
-            return None
+            return None, False
         from ..ops import cuda_ops
         from ..ops.attention_cuda import _window_int
         cos = sin = None
@@ -140,15 +140,28 @@ class SelfAttention(nn.Module):
                 b, t, hq, hk, d, self.qk_eps, self.qk_norm_type == "rms", self.qk_scale_min, self.qk_scale_max, window, None,
                 self.softcap, doc_start, quantize_out=self.out_proj.precision in ("mxfp8", "fp8"))
             if y is not None:
-                return y
+                return y, False
+        out_proj = self.out_proj
+        if (cuda_ops.plain_call() and self.q_proj.precision == out_proj.precision == "default" and type(out_proj) is Linear and out_proj.bias is None
+                and not out_proj._forward_hooks and not out_proj._forward_pre_hooks and self.hidden_size % 8 == 0):
+            # without gradients: the whole branch, output projection included, as one call
+            cuda_ops.count_path("attention:tcgen05")
+            y = cuda_ops.ext().attention_branch(
+                cuda_ops._as_bf16_2d(x), cuda_ops.bf16_weight(weights), cuda_ops.bf16_weight((out_proj.weight,)), cos, sin,
+                cuda_ops.as_fp32(self.q_scale) if self.use_qk_norm else None, cuda_ops.as_fp32(self.k_scale) if self.use_qk_norm else None, b, hq, hk, d,
+                self.qk_eps, self.qk_norm_type == "rms", max(self.qk_scale_min, -3.0e38), min(self.qk_scale_max, 3.0e38), t if window is None else window,
+                d ** -0.5, self.softcap, doc_start)
+            return y.view(b, t, -1), True
         qkv = cuda_ops.linear_multi(x, weights, self.q_proj.precision)
         return cuda_ops.rope_attention_packed(
             qkv.view(b * t, -1), cos, sin, self.q_scale if self.use_qk_norm else None, self.k_scale if self.use_qk_norm else None,
-            b, t, hq, hk, d, self.qk_eps, self.qk_norm_type == "rms", self.qk_scale_min, self.qk_scale_max, window, None, self.softcap, doc_start)
+            b, t, hq, hk, d, self.qk_eps, self.qk_norm_type == "rms", self.qk_scale_min, self.qk_scale_max, window, None, self.softcap, doc_start), False
 
     def forward(self, x: Tensor, ctx: AttentionContext) -> Tensor:
         b, t, _ = x.shape
-        y = self._fused_rope_attention(x, ctx)
+        y, projected = self._fused_rope_attention(x, ctx)
+        if projected:
+            return y
         if y is not None:
             merged = y.reshape(b, t, self.attn_dim)
             if getattr(y, "mxq", None) is not None:           # MXFP8 copy written by the attention kernel's epilogue
