@@ -78,6 +78,8 @@ def linear(x: Tensor, weight: Tensor, bias: Optional[Tensor], precision: str = "
 
 
 def activate(x: Tensor, name: str) -> Tensor:
+    if x.is_cuda and x.dtype == torch.bfloat16:
+        return _cuda().activate(x, name)
     return ref.activate(x, name)
 
 
