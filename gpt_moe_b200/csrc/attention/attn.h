@@ -11,6 +11,7 @@ struct AttnParams {
     int group;                      // q heads per kv head
     int qk_dim;                     // width of a query / key head: 64 or 128
     int q_col0, k_col0, v_col0;     // first column of head 0 inside each tensor map
+    int v_head, dv_head;            // columns from one value head (of v; of dv) to the next: 64, or more when something lies between them
     int window;                     // inclusive look-back W (a query sees keys q-W..q); >= seq_len means plain causal
     const int* window_ptr;          // optional device-resident window (overrides `window`; clamped to [0, seq_len] by the kernels), so
                                     // that a window-schedule step is a write to that word and a captured launch stays valid

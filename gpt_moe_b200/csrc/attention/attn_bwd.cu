@@ -181,7 +181,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
             mbar_expect_tx(bar_kv, QK_BYTES + T_BYTES);
 #pragma unroll
             for (int sl = 0; sl < QK_SLABS; ++sl) tma_load_3d(sk + sl * T_BYTES, &tmap_k, bar_kv, kv_head * DQK + 64 * sl, kv0, batch);
-            tma_load_3d(sv, &tmap_v, bar_kv, kv_head * HD, kv0, batch);
+            tma_load_3d(sv, &tmap_v, bar_kv, kv_head * p.v_head, kv0, batch);
             for (int it = 0; it < QDO_STAGES && it < n_iter; ++it) load_qdo(it);
             if (!mbar_wait(bar_kv, 0)) { atomicExch(p.status, 301); ok = false; }
             auto issue_sdp = [&](int it) -> bool {               // S = Q K^T ; dP = dO V^T for iteration `it`
@@ -323,7 +323,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
             const bool live = kv0 + r < p.seq_len;
             const long long token = static_cast<long long>(row0) + kv0 + r;
             __nv_bfloat16* dk = reinterpret_cast<__nv_bfloat16*>(p.dk) + token * p.dkv_stride + kv_head * DQK + half * (DQK / 2);
-            __nv_bfloat16* dv = reinterpret_cast<__nv_bfloat16*>(p.dv) + token * p.dv_stride + kv_head * HD + half * 32;
+            __nv_bfloat16* dv = reinterpret_cast<__nv_bfloat16*>(p.dv) + token * p.dv_stride + kv_head * p.dv_head + half * 32;
             uint32_t vreg[32];
             tmem_ld_32x32b_x32(tmem_base + COL_DV + lane_off + half * 32, vreg);
             tmem_ld_wait();

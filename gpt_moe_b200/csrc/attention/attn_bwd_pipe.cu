@@ -140,7 +140,7 @@ attn_bwd_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
             };
             mbar_expect_tx(bar_kv, 2 * BP_T_BYTES);
             tma_load_3d(sk, &tmap_k, bar_kv, kv_head * BP_HD, kv0, batch);
-            tma_load_3d(sv, &tmap_v, bar_kv, kv_head * BP_HD, kv0, batch);
+            tma_load_3d(sv, &tmap_v, bar_kv, kv_head * p.v_head, kv0, batch);
             for (int it = 0; it < BP_STAGES && it < n_iter; ++it) load_qdo(it);
             for (int it = BP_STAGES; it < n_iter; ++it) {
                 // the stage was read by S/dP and by the gradient products of iteration it - BP_STAGES
@@ -298,7 +298,7 @@ attn_bwd_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
             const bool live = kv0 + r < p.seq_len;
             const long long token = static_cast<long long>(row0) + kv0 + r;
             __nv_bfloat16* dk = reinterpret_cast<__nv_bfloat16*>(p.dk) + token * p.dkv_stride + kv_head * BP_HD + half * 32;
-            __nv_bfloat16* dv = reinterpret_cast<__nv_bfloat16*>(p.dv) + token * p.dv_stride + kv_head * BP_HD + half * 32;
+            __nv_bfloat16* dv = reinterpret_cast<__nv_bfloat16*>(p.dv) + token * p.dv_stride + kv_head * p.dv_head + half * 32;
             uint32_t vreg[32], kreg[32];
             tmem_ld_32x32b_x32(tmem_base + BP_COL_DV + lane_off + half * 32, vreg);
             tmem_ld_32x32b_x32(tmem_base + BP_COL_DK + lane_off + half * 32, kreg);

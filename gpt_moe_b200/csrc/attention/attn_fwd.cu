@@ -139,7 +139,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     kv_lo &= ~(AT_BN - 1);
     const int n_tiles = (q0 + AT_BM - kv_lo) / AT_BN;
     const int kv_head = head / p.group;                       // grouped-query attention: several q heads share a kv head
-    const int q_col = p.q_col0 + head * DQK, k_col = p.k_col0 + kv_head * DQK, v_col = p.v_col0 + kv_head * AT_D;
+    const int q_col = p.q_col0 + head * DQK, k_col = p.k_col0 + kv_head * DQK, v_col = p.v_col0 + kv_head * p.v_head;
 
     if (threadIdx.x == 0) {
         mbar_init(bar_q, 1); mbar_init(bar_s, 1); mbar_init(bar_p, 256); mbar_init(bar_o, 1);

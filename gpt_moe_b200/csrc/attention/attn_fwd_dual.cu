@@ -214,7 +214,7 @@ attn_fwd_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     const int lo_a = first_a > 0 ? first_a / DU_BN : 0, lo_b = first_b > 0 ? first_b / DU_BN : 0;
     const int hi_a = q0 / DU_BN;                                // B's diagonal tile is hi_a + 1
     const int kv_head = head / p.group;                       // grouped-query attention: several q heads share a kv head
-    const int q_col = p.q_col0 + head * DU_D, k_col = p.k_col0 + kv_head * DU_D, v_col = p.v_col0 + kv_head * DU_D;
+    const int q_col = p.q_col0 + head * DU_D, k_col = p.k_col0 + kv_head * DU_D, v_col = p.v_col0 + kv_head * p.v_head;
 
     if (threadIdx.x == 0) {
         mbar_init(bar_q, 1);

@@ -265,17 +265,20 @@ void gemm_mxfp8(const torch::Tensor& a, const torch::Tensor& sfa, const torch::T
 // sequence], so that a tile past the end of a sequence reads zeros and a reduction into it is clipped
 // Elements from one token to the next of a [B, T, H, D] view.  Torch leaves the stride of a dimension of size one open: with one token
 // a sequence the sequence stride says it, with one token altogether there is nothing to say.
+int64_t head_pitch(const torch::Tensor& t) { return t.size(2) != 1 ? t.stride(2) : t.size(3); }
 int64_t token_pitch(const torch::Tensor& t) {
     if (t.size(1) != 1) return t.stride(1);
-    return t.size(0) != 1 ? t.stride(0) : t.size(2) * t.size(3);
+    return t.size(0) != 1 ? t.stride(0) : t.size(2) * head_pitch(t);
 }
 
-CUtensorMap head_map(const torch::Tensor& t, int box_rows) {
+// `values`: value heads may lie further apart than they are wide (by whole 16-byte pieces), as in a projection that interleaves them with keys.
+CUtensorMap head_map(const torch::Tensor& t, int box_rows, bool values = false) {
     GM_CHECK(t.is_cuda() && t.scalar_type() == torch::kBFloat16 && t.dim() == 4, "attention operands must be [B, T, H, D] bf16 CUDA tensors");
     const int64_t pitch = token_pitch(t);
-    GM_CHECK(t.stride(3) == 1 && t.stride(2) == t.size(3) && (t.size(0) == 1 || t.stride(0) == t.size(1) * pitch),
+    const int64_t head = head_pitch(t);
+    GM_CHECK(t.stride(3) == 1 && (values ? head >= 64 && head % 8 == 0 : head == t.size(3)) && (t.size(0) == 1 || t.stride(0) == t.size(1) * pitch),
              "attention operands must be token-major with contiguous heads");
-    return cached_map(t.data_ptr(), 2, t.size(2) * t.size(3), t.size(1), t.size(0), pitch * 2, t.size(1) * pitch * 2, 64, box_rows, 128);
+    return cached_map(t.data_ptr(), 2, (t.size(2) - 1) * head + t.size(3), t.size(1), t.size(0), pitch * 2, t.size(1) * pitch * 2, 64, box_rows, 128);
 }
 
 // Returns (out [B,T,H,64] bf16, lse [B,H,T] fp32).
@@ -308,6 +311,7 @@ std::vector<torch::Tensor> attn_fwd(const torch::Tensor& q, const torch::Tensor&
     gm::AttnParams p;
     std::memset(&p, 0, sizeof(p));
     p.batch = B; p.heads = H; p.seq_len = T; p.group = H / Hkv; p.qk_dim = D;
+    p.v_head = p.dv_head = static_cast<int>(head_pitch(v));
     p.window = static_cast<int>(std::min<int64_t>(window, T));
     p.scale = static_cast<float>(scale);
     p.scale_log2e = static_cast<float>(scale * 1.4426950408889634);
@@ -327,7 +331,7 @@ std::vector<torch::Tensor> attn_fwd(const torch::Tensor& q, const torch::Tensor&
     p.status = status_tensor(q.device().index()).data_ptr<int>();
     p.single_tile = single_tile ? 1 : 0;
     p.window_ptr = window_word(window_tensor);
-    cudaError_t e = gm::launch_attn_fwd(head_map(q, 128), head_map(k, 128), head_map(v, 128), p, current_stream());
+    cudaError_t e = gm::launch_attn_fwd(head_map(q, 128), head_map(k, 128), head_map(v, 128, true), p, current_stream());
     GM_CHECK(e == cudaSuccess, cudaGetErrorString(e));
     if (quantize) return {out, lse, oq, osf};
     return {out, lse};
@@ -344,12 +348,13 @@ torch::Tensor attn_bwd(const torch::Tensor& q, const torch::Tensor& k, const tor
     const int B = q.size(0), T = q.size(1), H = q.size(2), D = q.size(3), Hkv = k.size(2);
     GM_CHECK((D == 64 || D == 128) && k.size(3) == D && v.size(3) == 64 && T >= 1 && H % Hkv == 0,
              "attention kernel: query/key heads 64 or 128 wide, value heads 64 wide");
-    GM_CHECK(dk.stride(3) == 1 && dk.stride(2) == D && dv.stride(3) == 1 && dv.stride(2) == 64 && token_pitch(dk) % 8 == 0 && token_pitch(dv) % 8 == 0,
+    GM_CHECK(dk.stride(3) == 1 && dk.stride(2) == D && dv.stride(3) == 1 && head_pitch(dv) % 8 == 0 && head_pitch(dv) >= 64 && token_pitch(dk) % 8 == 0 && token_pitch(dv) % 8 == 0,
              "dk/dv must be token-major views with contiguous heads and 16-byte aligned rows");
     GM_CHECK(out.stride(3) == 1 && out.stride(2) == 64 && d_out.stride(3) == 1 && d_out.stride(2) == 64, "out/d_out layout");
     gm::AttnParams p;
     std::memset(&p, 0, sizeof(p));
     p.batch = B; p.heads = H; p.seq_len = T; p.group = H / Hkv; p.qk_dim = D;
+    p.v_head = p.dv_head = static_cast<int>(head_pitch(v));
     p.window = static_cast<int>(std::min<int64_t>(window, T));
     p.scale = static_cast<float>(scale);
     p.scale_log2e = static_cast<float>(scale * 1.4426950408889634);
@@ -360,13 +365,13 @@ torch::Tensor attn_bwd(const torch::Tensor& q, const torch::Tensor& k, const tor
     auto dq = gm::out_zeros({B, T, H, D}, lse.options());
     p.delta = delta.data_ptr<float>();
     p.dq_accum = dq.data_ptr<float>();
-    p.dk = dk.data_ptr(); p.dv = dv.data_ptr(); p.dkv_stride = token_pitch(dk); p.dv_stride = token_pitch(dv);
+    p.dk = dk.data_ptr(); p.dv = dv.data_ptr(); p.dv_head = static_cast<int>(head_pitch(dv)); p.dkv_stride = token_pitch(dk); p.dv_stride = token_pitch(dv);
     p.status = status_tensor(q.device().index()).data_ptr<int>();
     p.single_tile = unpipelined ? 1 : 0;
     p.window_ptr = window_word(window_tensor);
     const CUtensorMap& tdq = cached_map(dq.data_ptr(), 4, static_cast<uint64_t>(H) * D, T, B, static_cast<uint64_t>(H) * D * 4,
                                         static_cast<uint64_t>(T) * H * D * 4, 32, 128, 128);
-    cudaError_t e = gm::launch_attn_bwd(head_map(q, 128), head_map(k, 128), head_map(v, 128), head_map(d_out, 128), tdq, p,
+    cudaError_t e = gm::launch_attn_bwd(head_map(q, 128), head_map(k, 128), head_map(v, 128, true), head_map(d_out, 128), tdq, p,
                                         d_out.data_ptr(), out.data_ptr(), token_pitch(d_out), token_pitch(out), delta.data_ptr<float>(),
                                         current_stream());
     GM_CHECK(e == cudaSuccess, cudaGetErrorString(e));

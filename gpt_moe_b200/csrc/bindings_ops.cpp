@@ -147,6 +147,52 @@ std::vector<Tensor> rope_qknorm_bwd(const Tensor& x, const Tensor& dy, Tensor& d
     return {dscale};
 }
 
+// Latent attention, 128-wide heads (content + rotary columns), values 64 wide (see mla_rope_kernel).  q [tokens, H * 128], kv [tokens, Hk * (content +
+// 64)] (per head content | value), rope [tokens, rope_dim] (any row pitch of whole 16-byte pieces); cos / sin fp32 [>= seq, rope_dim / 2].
+void check_mla_rows(const Tensor& q, const Tensor& kv, const Tensor& rope, const Tensor& cos, const Tensor& sin, int64_t seq_len, int64_t q_heads, int64_t k_heads) {
+    const int64_t tokens = q.size(0), dr = rope.size(-1);
+    auto rows = [&](const Tensor& t, int64_t width) {
+        return t.is_cuda() && t.scalar_type() == torch::kBFloat16 && t.dim() == 2 && t.size(0) == tokens && t.size(1) == width && t.stride(1) == 1 && t.stride(0) % 8 == 0 &&
+               reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
+    };
+    GM_CHECK(rows(q, q_heads * 128) && dr % 8 == 0 && dr >= 8 && dr <= 120 && rows(kv, k_heads * (192 - dr)) && rows(rope, dr) && seq_len > 0 && tokens % seq_len == 0, "mla_rope: bf16 rows of 16-byte pieces");
+    for (const Tensor* t : {&cos, &sin})
+        GM_CHECK(t->is_cuda() && t->scalar_type() == torch::kFloat32 && t->is_contiguous() && t->dim() == 2 && t->size(0) >= seq_len && t->size(1) == dr / 2 &&
+                 reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 == 0, "mla_rope: rotary tables fp32 [>= seq, rope / 2]");
+}
+
+Tensor mla_rope_fwd(const Tensor& q, const Tensor& kv, const Tensor& rope, const Tensor& cos, const Tensor& sin, const OptTensor& q_scale, const OptTensor& k_scale,
+                    int64_t seq_len, int64_t q_heads, int64_t k_heads, double eps, bool rms, double smin, double smax) {
+    c10::cuda::CUDAGuard guard(q.device());
+    check_mla_rows(q, kv, rope, cos, sin, seq_len, q_heads, k_heads);
+    Tensor packed = gm::out_empty({q.size(0), (q_heads + k_heads) * 128}, q.options());
+    GM_CHECK(launch_mla_rope(false, q.data_ptr(), kv.data_ptr(), rope.data_ptr(), packed.data_ptr(), cos.data_ptr<float>(), sin.data_ptr<float>(), fptr(q_scale),
+                             fptr(k_scale), nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, q.size(0), seq_len, q_heads, k_heads, q.stride(0), kv.stride(0),
+                             rope.stride(0), rope.size(1), eps, rms, smin, smax, stream()), "mla_rope: at most 64 heads");
+    return packed;
+}
+
+// dq32 fp32 [tokens, H * 128], dk bf16 [tokens, Hk * 128] contiguous.  Writes the content columns of dkv [tokens, Hk * (content + 64)]; returns (dq, drope, dscale).
+std::vector<Tensor> mla_rope_bwd(const Tensor& q, const Tensor& kv, const Tensor& rope, const Tensor& cos, const Tensor& sin, const OptTensor& q_scale,
+                                 const OptTensor& k_scale, const Tensor& dq32, const Tensor& dk, Tensor& dkv, int64_t seq_len, int64_t q_heads, int64_t k_heads,
+                                 double eps, bool rms, double smin, double smax) {
+    c10::cuda::CUDAGuard guard(q.device());
+    check_mla_rows(q, kv, rope, cos, sin, seq_len, q_heads, k_heads);
+    const int64_t tokens = q.size(0);
+    GM_CHECK(dq32.scalar_type() == torch::kFloat32 && dq32.is_contiguous() && dq32.numel() == tokens * q_heads * 128, "mla_rope_bwd: dq32 fp32 [tokens, H * 128]");
+    check_bf16(dk, "dk");
+    check_bf16(dkv, "dkv");
+    GM_CHECK(dk.numel() == tokens * k_heads * 128 && dkv.numel() == tokens * kv.size(1), "mla_rope_bwd: dk [tokens, Hk * 128], dkv as kv");
+    Tensor dq = gm::out_empty({tokens, q_heads * 128}, q.options()), drope = gm::out_empty({tokens, rope.size(1)}, q.options());
+    const int blocks = mla_rope_blocks(tokens), heads = q_heads + k_heads;
+    Tensor partial = gm::out_empty({blocks, heads}, dq32.options()), dscale = gm::out_empty({heads}, dq32.options());
+    GM_CHECK(launch_mla_rope(true, q.data_ptr(), kv.data_ptr(), rope.data_ptr(), nullptr, cos.data_ptr<float>(), sin.data_ptr<float>(), fptr(q_scale), fptr(k_scale),
+                             dq32.data_ptr<float>(), dk.data_ptr(), dq.data_ptr(), dkv.data_ptr(), drope.data_ptr(), partial.data_ptr<float>(), tokens, seq_len,
+                             q_heads, k_heads, q.stride(0), kv.stride(0), rope.stride(0), rope.size(1), eps, rms, smin, smax, stream()), "mla_rope: at most 64 heads");
+    launch_column_sum(partial.data_ptr<float>(), dscale.data_ptr<float>(), blocks, heads, 0, stream());
+    return {dq, drope, dscale};
+}
+
 // Router after the logits GEMM: (top_idx int64 [T, k], gates fp32 [T, k]) and, with `want_balance`, (balance fp32 [1], counts fp32 [E]).
 // renormalise: gates = softmax over the selected logits; otherwise the full-softmax probability of each selected expert.
 std::vector<Tensor> router_fwd(const Tensor& logits, int64_t top_k, bool renormalise, bool want_balance) {
@@ -742,6 +788,8 @@ void register_kernels(pybind11::module_& m) {
     m.def("rope_qknorm_bwd", &rope_qknorm_bwd, py::arg("x"), py::arg("dy"), py::arg("dx"), py::arg("cos"), py::arg("sin"), py::arg("q_scale"),
           py::arg("k_scale"), py::arg("seq_len"), py::arg("q_heads"), py::arg("k_heads"), py::arg("head_dim"), py::arg("eps"), py::arg("rms"),
           py::arg("smin"), py::arg("smax"), py::arg("dq32") = py::none(), py::arg("quantize") = false);
+    m.def("mla_rope_fwd", &mla_rope_fwd);
+    m.def("mla_rope_bwd", &mla_rope_bwd);
     m.def("mla_decode", &mla_decode);
     m.def("mla_decode_ok", &mla_decode_ok);
     m.def("rows_linear", &rows_linear);

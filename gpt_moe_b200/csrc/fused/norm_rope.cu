@@ -473,6 +473,150 @@ rope_qknorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* dy,
     }
 }
 
+// ---- rotation and QK-norm of latent attention, straight from its projections -------------------------------------------------------
+// A 128-wide query head [content | rotary] is a row slice of the query projection; a key head is the content columns of its head in the
+// up-projection [content | value] followed by the token's one rotary key, shared by all heads.  Forward: packed rotated rows [query heads | key
+// heads] as the attention kernels read them (the concatenations that used to assemble them, their slices' gradients and the copies between took 1.5 ms of a three-layer step at 2 x 4096 tokens, 16
+// heads; this kernel takes 35 us forward and 84 us backward a layer).
+// Backward: gradients of the three inputs, written where the projections' gradient GEMMs read them; the rotary key's sums over the
+// heads, so a warp owns a token and walks its heads, two at a time (16 lanes of 8 columns each: content first, the last rope_dim / 8 rotary).
+template <bool BWD>
+__global__ void __launch_bounds__(256)
+mla_rope_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ kv, const __nv_bfloat16* __restrict__ rope, __nv_bfloat16* __restrict__ packed,
+                const float* __restrict__ cos_t, const float* __restrict__ sin_t, const float* __restrict__ q_scale, const float* __restrict__ k_scale,
+                const float* __restrict__ dq32, const __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dq, __nv_bfloat16* __restrict__ dkv,
+                __nv_bfloat16* __restrict__ drope, float* __restrict__ dscale_partial, int tokens, int seq_len, int q_heads, int k_heads,
+                long long q_pitch, long long kv_pitch, long long rope_pitch, int rope_dim, int kv_head, float eps, int rms, float smin, float smax) {
+    constexpr int D = 128;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane >> 4, li = lane & 15;
+    const int heads = q_heads + k_heads;
+    const int rl = li - (D - rope_dim) / 8;                       // this lane's 8 columns of the rotary part, if any
+    const bool has_norm = q_scale != nullptr, rotary = rl >= 0;
+    __shared__ float ds_smem[8][64];
+    if (BWD) {
+        for (int i = threadIdx.x; i < 8 * 64; i += blockDim.x) (&ds_smem[0][0])[i] = 0.f;
+        __syncthreads();
+    }
+    for (int t = blockIdx.x * 8 + warp; t < tokens; t += gridDim.x * 8) {
+        float c[4] = {1.f, 1.f, 1.f, 1.f}, sn[4] = {0.f, 0.f, 0.f, 0.f};
+        const uint4 rope_raw = rotary ? *reinterpret_cast<const uint4*>(rope + t * rope_pitch + rl * 8) : make_uint4(0, 0, 0, 0);
+        if (rotary) {                                              // tables [position, rope_dim / 2]
+            const long long pair = static_cast<long long>(t % seq_len) * (rope_dim / 2) + rl * 4;
+            const float4 cv = *reinterpret_cast<const float4*>(cos_t + pair), sv = *reinterpret_cast<const float4*>(sin_t + pair);
+            c[0] = cv.x; c[1] = cv.y; c[2] = cv.z; c[3] = cv.w;
+            sn[0] = sv.x; sn[1] = sv.y; sn[2] = sv.z; sn[3] = sv.w;
+        }
+        float rope_sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 2
+        for (int h0 = 0; h0 < heads; h0 += 2) {
+            const int h = h0 + sub;
+            const bool live = h < heads, is_q = h < q_heads;
+            const int kh = h - q_heads;
+            uint4 xraw = make_uint4(0, 0, 0, 0), graw = xraw;
+            float4 ga = make_float4(0.f, 0.f, 0.f, 0.f), gb = ga;
+            if (live) {
+                if (is_q) xraw = *reinterpret_cast<const uint4*>(q + t * q_pitch + h * D + li * 8);
+                else xraw = rotary ? rope_raw : *reinterpret_cast<const uint4*>(kv + t * kv_pitch + kh * kv_head + li * 8);
+                if (BWD) {
+                    if (is_q) {
+                        const float* src = dq32 + (static_cast<long long>(t) * q_heads + h) * D + li * 8;
+                        ga = *reinterpret_cast<const float4*>(src);
+                        gb = *reinterpret_cast<const float4*>(src + 4);
+                    } else {
+                        graw = *reinterpret_cast<const uint4*>(dk + (static_cast<long long>(t) * k_heads + kh) * D + li * 8);
+                    }
+                }
+            }
+            const __nv_bfloat162* xp = reinterpret_cast<const __nv_bfloat162*>(&xraw);
+            const __nv_bfloat162* gp = reinterpret_cast<const __nv_bfloat162*>(&graw);
+            const float gq[8] = {ga.x, ga.y, ga.z, ga.w, gb.x, gb.y, gb.z, gb.w};
+            float r1[4], r2[4], g1[4], g2[4], ss = 0.f, dot = 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float2 xf = __bfloat1622float2(xp[i]);
+                r1[i] = xf.x * c[i] - xf.y * sn[i];
+                r2[i] = xf.x * sn[i] + xf.y * c[i];
+                ss += r1[i] * r1[i] + r2[i] * r2[i];
+                if (BWD) {
+                    const float2 gf = __bfloat1622float2(gp[i]);
+                    g1[i] = is_q ? gq[2 * i] : gf.x;
+                    g2[i] = is_q ? gq[2 * i + 1] : gf.y;
+                    dot += g1[i] * r1[i] + g2[i] * r2[i];
+                }
+            }
+            const float raw = !live ? 1.f : is_q ? (q_scale ? q_scale[h] : 1.f) : (k_scale ? k_scale[kh] : 1.f);
+            float gain = 1.f, mult = 1.f;
+            if (has_norm) {
+                ss = head_sum<D>(ss);
+                gain = rsqrtf((rms ? ss / D : ss) + eps);
+                mult = gain * fminf(fmaxf(raw, smin), smax);
+            }
+            uint4 oraw;
+            __nv_bfloat162* op = reinterpret_cast<__nv_bfloat162*>(&oraw);
+            if (!BWD) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) op[i] = __floats2bfloat162_rn(r1[i] * mult, r2[i] * mult);
+                if (live) *reinterpret_cast<uint4*>(packed + (static_cast<long long>(t) * heads + h) * D + li * 8) = oraw;
+                continue;
+            }
+            dot = head_sum<D>(dot);
+            if (has_norm && live && li == 0 && raw >= smin && raw <= smax) ds_smem[warp][h] += dot * gain;
+            const float coef = has_norm ? gain * gain * (rms ? dot / D : dot) : 0.f;
+            float d[8];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float d1 = mult * (g1[i] - r1[i] * coef), d2 = mult * (g2[i] - r2[i] * coef);
+                d[2 * i] = d1 * c[i] + d2 * sn[i];
+                d[2 * i + 1] = -d1 * sn[i] + d2 * c[i];
+                op[i] = __floats2bfloat162_rn(d[2 * i], d[2 * i + 1]);
+            }
+            if (live && is_q) *reinterpret_cast<uint4*>(dq + (static_cast<long long>(t) * q_heads + h) * D + li * 8) = oraw;
+            if (live && !is_q) {
+                if (!rotary) {
+                    *reinterpret_cast<uint4*>(dkv + static_cast<long long>(t) * k_heads * kv_head + kh * kv_head + li * 8) = oraw;
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) rope_sum[i] += d[i];
+                }
+            }
+        }
+        if (BWD) {
+            uint4 oraw;
+            __nv_bfloat162* op = reinterpret_cast<__nv_bfloat162*>(&oraw);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) rope_sum[i] += __shfl_xor_sync(0xffffffffu, rope_sum[i], 16);      // even and odd heads
+#pragma unroll
+            for (int i = 0; i < 4; ++i) op[i] = __floats2bfloat162_rn(rope_sum[2 * i], rope_sum[2 * i + 1]);
+            if (rotary && sub == 0) *reinterpret_cast<uint4*>(drope + static_cast<long long>(t) * rope_dim + rl * 8) = oraw;
+        }
+    }
+    if (BWD) {
+        __syncthreads();
+        for (int h = threadIdx.x; h < heads; h += blockDim.x) {
+            float s = 0.f;
+#pragma unroll
+            for (int wi = 0; wi < 8; ++wi) s += ds_smem[wi][h];
+            dscale_partial[static_cast<long long>(blockIdx.x) * heads + h] = s;
+        }
+    }
+}
+
+int mla_rope_blocks(long long tokens) { return static_cast<int>((tokens + 7) / 8 < 1184 ? (tokens + 7) / 8 : 1184); }
+
+bool launch_mla_rope(bool bwd, const void* q, const void* kv, const void* rope, void* packed, const float* cos_t, const float* sin_t, const float* q_scale,
+                     const float* k_scale, const float* dq32, const void* dk, void* dq, void* dkv, void* drope, float* dscale_partial, long long tokens, int seq_len,
+                     int q_heads, int k_heads, long long q_pitch, long long kv_pitch, long long rope_pitch, int rope_dim, float eps, int rms, float smin,
+                     float smax, cudaStream_t s) {
+    if (q_heads + k_heads > 64 || rope_dim < 8 || rope_dim > 120 || rope_dim % 8 || tokens <= 0 || tokens >= (1LL << 31) - 1184 * 8) return false;
+    auto* kernel = bwd ? mla_rope_kernel<true> : mla_rope_kernel<false>;
+    using B = __nv_bfloat16;
+    kernel<<<mla_rope_blocks(tokens), 256, 0, s>>>(static_cast<const B*>(q), static_cast<const B*>(kv), static_cast<const B*>(rope), static_cast<B*>(packed), cos_t,
+                                                   sin_t, q_scale, k_scale, dq32, static_cast<const B*>(dk), static_cast<B*>(dq), static_cast<B*>(dkv),
+                                                   static_cast<B*>(drope), dscale_partial, static_cast<int>(tokens), seq_len, q_heads, k_heads, q_pitch, kv_pitch,
+                                                   rope_pitch, rope_dim, 128 - rope_dim + 64, eps, rms, smin, smax);
+    return true;
+}
+
 int rope_blocks(long long tokens, int heads) {
     const long long want = (tokens * ((heads + 3) / 4) + 7) / 8;      // at least 4 heads of a token per warp pass for every supported head size
     return static_cast<int>(want < 2368 ? want : 2368);

@@ -17,6 +17,11 @@ void launch_residual_bwd(const float* dxn, const void* branch, const float* beta
                          long long n, cudaStream_t s);
 void launch_column_sum(const float* partial, float* out, int rows, int cols, int accumulate, cudaStream_t s);
 int rope_blocks(long long tokens, int heads);
+int mla_rope_blocks(long long tokens);
+bool launch_mla_rope(bool bwd, const void* q, const void* kv, const void* rope, void* packed, const float* cos_t, const float* sin_t, const float* q_scale,
+                     const float* k_scale, const float* dq32, const void* dk, void* dq, void* dkv, void* drope, float* dscale_partial, long long tokens, int seq_len,
+                     int q_heads, int k_heads, long long q_pitch, long long kv_pitch, long long rope_pitch, int rope_dim, float eps, int rms, float smin,
+                     float smax, cudaStream_t s);
 bool launch_rope_qknorm(bool bwd, int D, const void* x, const void* dy, void* out, const float* cos_t, const float* sin_t,
                         const float* q_scale, const float* k_scale, float* dscale_partial, long long tokens, int seq_len,
                         int q_heads, int k_heads, long long x_stride, long long o_stride, float eps, int rms, float smin,

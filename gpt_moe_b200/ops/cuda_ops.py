@@ -540,6 +540,53 @@ def rope_attention_packed(qkv: Tensor, cos, sin, q_scale, k_scale, batch: int, s
                                   d ** -0.5 if scale is None else float(scale), float(softcap), doc_start)
 
 
+class _MLARopeAttentionFn(torch.autograd.Function):
+    """Latent attention from its projections to the attention output as one node: query [B, T, H * 128], kv [B, T, Hk * (content + 64 value)],
+    rope [B, T, 128 - content].  Forward: one kernel rotates, normalises and packs query and key heads, the attention kernel reads the values out of
+    kv.  Backward: dV lands in its columns of dkv, one kernel turns the fp32 dQ and dK into the gradients of all three inputs."""
+
+    @staticmethod
+    def forward(ctx, query: Tensor, kv: Tensor, rope: Tensor, cos, sin, q_scale, k_scale, hq, hk, eps, rms, smin, smax, window, scale):
+        c = ext()
+        b, t, _ = query.shape
+        q2, kv2, r2 = query.reshape(b * t, -1), kv.reshape(b * t, -1), rope.reshape(b * t, -1)
+        qs, ks = (None if s is None else as_fp32(s.detach()).reshape(-1) for s in (q_scale, k_scale))
+        packed = c.mla_rope_fwd(q2, kv2, r2, cos, sin, qs, ks, t, hq, hk, eps, rms, smin, smax).view(b, t, hq + hk, 128)
+        v = kv2.view(b, t, hk, -1)[..., -64:]
+        o, lse = c.attn_fwd(packed[:, :, :hq], packed[:, :, hq:], v, window, scale)
+        empty = query.new_empty(0)
+        ctx.save_for_backward(q2, kv2, r2, cos, sin, packed, o, lse, empty if qs is None else qs, empty if ks is None else ks)
+        ctx.cfg = (b, t, hq, hk, eps, rms, smin, smax, window, scale, qs is not None)
+        ctx.scale_shapes = None if qs is None else ((q_scale.shape, q_scale.dtype), (k_scale.shape, k_scale.dtype))
+        return o
+
+    @staticmethod
+    def backward(ctx, d_out: Tensor):
+        c = ext()
+        q2, kv2, r2, cos, sin, packed, o, lse, qs, ks = ctx.saved_tensors
+        b, t, hq, hk, eps, rms, smin, smax, window, scale, has_norm = ctx.cfg
+        d_out = d_out if (d_out.dtype == BF16 and d_out.is_contiguous()) else d_out.to(BF16).contiguous()
+        dkv = torch.empty_like(kv2, memory_format=torch.contiguous_format)
+        dk = torch.empty((b, t, hk, 128), dtype=BF16, device=d_out.device)
+        dq32 = c.attn_bwd(packed[:, :, :hq], packed[:, :, hq:], kv2.view(b, t, hk, -1)[..., -64:], o, d_out, lse, dk,
+                          dkv.view(b, t, hk, -1)[..., -64:], window, scale)
+        dq, drope, dscale = c.mla_rope_bwd(q2, kv2, r2, cos, sin, qs if has_norm else None, ks if has_norm else None, dq32, dk, dkv, t, hq, hk, eps, rms, smin, smax)
+        dqs = dks = None
+        if has_norm:
+            (qshape, qdt), (kshape, kdt) = ctx.scale_shapes
+            dqs, dks = dscale[:hq].reshape(qshape).to(qdt), dscale[hq:].reshape(kshape).to(kdt)
+        return (dq.view(b, t, -1), dkv.view(b, t, -1), drope.view(b, t, -1), None, None, dqs, dks) + (None,) * 8
+
+
+def mla_rope_attention(query: Tensor, kv: Tensor, rope: Tensor, cos: Tensor, sin: Tensor, q_scale, k_scale, hq: int, hk: int, eps: float, rms: bool, smin: float,
+                       smax: float, window: Optional[int], scale: float) -> Tensor:
+    """[B, T, H, 64] attention output of latent attention with 128-wide query / key heads and 64-wide values."""
+    t = query.shape[1]
+    count_path("attention:tcgen05")
+    return run_function(_MLARopeAttentionFn, query, kv, rope, cos, sin, q_scale, k_scale, hq, hk, eps, rms, max(smin, -3.0e38), min(smax, 3.0e38),
+                        t if window is None else min(int(window), t), scale)
+
+
 def rope_qk_norm(q, k, cos, sin, q_scale, k_scale, eps, rms, scale_min, scale_max):
     """Unpacked entry (separate q and k tensors [B,T,H,D]): pack, run the fused kernel, unpack."""
     b, t, hq, d = q.shape

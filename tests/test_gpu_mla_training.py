@@ -1,0 +1,74 @@
+"""Latent attention from its projections (one autograd node) and the shared expert's activation against fp32 definitions."""
+import pytest
+import torch
+
+from gpt_moe_b200.ops import api, cuda_ops
+from gpt_moe_b200.ops import reference as ref
+
+pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    return ((a.detach().double() - b.detach().double()).norm() / b.detach().double().norm().clamp_min(1e-30)).item()
+
+
+# rotary widths, odd head counts (a warp's second head is empty), grouped heads, ragged lengths, window, no QK-norm, clamped scales
+@pytest.mark.parametrize("b,t,hq,hk,dr,window,norm", [(2, 256, 4, 4, 64, None, True), (1, 200, 3, 3, 64, 50, True), (2, 45, 4, 2, 32, None, True),
+                                                      (1, 130, 2, 1, 8, None, False), (3, 1, 2, 2, 64, None, True)])
+def test_node_matches_reference(b, t, hq, hk, dr, window, norm):
+    torch.manual_seed(9)
+    content = 128 - dr
+    q = torch.randn(b, t, hq * 128, device="cuda").bfloat16().requires_grad_()
+    kv = torch.randn(b, t, hk * (content + 64), device="cuda").bfloat16().requires_grad_()
+    low = torch.randn(b, t, 16 + dr, device="cuda").bfloat16().requires_grad_()
+    qs = torch.tensor([0.8, 1.3, 6.0, 1.0][:hq], device="cuda").view(1, hq, 1, 1).requires_grad_() if norm else None       # 6 is clamped to 5
+    ks = torch.linspace(0.7, 1.2, hk, device="cuda").view(1, hk, 1, 1).requires_grad_() if norm else None
+    cos, sin = ref.rope_tables(dr, 10000, t + 3)
+    cos, sin = cos.cuda(), sin.cuda()
+    scale = 128 ** -0.5
+    out = cuda_ops.mla_rope_attention(q, kv, low[..., 16:], cos, sin, qs, ks, hq, hk, 1e-6, True, float("-inf"), 5.0, window, scale)
+    g = torch.randn_like(out)
+    leaves = [x for x in (q, kv, low, qs, ks) if x is not None]
+    grads = torch.autograd.grad(out, leaves, g)
+
+    want_leaves = [x.detach().float().requires_grad_() for x in leaves]
+    wq, wkv, wlow = want_leaves[:3]
+    wqs, wks = want_leaves[3:] if norm else (None, None)
+    query = wq.view(b, t, hq, 128)
+    kvh = wkv.view(b, t, hk, content + 64)
+    rope = ref.apply_rope(wlow[..., 16:].reshape(b, t, 1, dr), cos, sin)
+    query = torch.cat((query[..., :content], ref.apply_rope(query[..., content:], cos, sin)), dim=-1)
+    key = torch.cat((kvh[..., :content], rope.expand(-1, -1, hk, -1)), dim=-1)
+    if norm:
+        # one copy of a scale per token: their gradients are the terms of the scale's, and the terms cancel
+        tqs, tks = (w.clamp(max=5.0).view(1, 1, -1, 1).expand(b, t, -1, 1).clone() for w in (wqs, wks))
+        tqs.retain_grad(), tks.retain_grad()
+        query = query * torch.rsqrt(query.pow(2).mean(-1, keepdim=True) + 1e-6) * tqs
+        key = key * torch.rsqrt(key.pow(2).mean(-1, keepdim=True) + 1e-6) * tks
+    want = ref.attention(query, key, kvh[..., content:], causal=True, window=window, scale=scale)
+    want.backward(g.float())
+    want_grads = [x.grad for x in want_leaves]
+    # rotated heads, probabilities and results are rounded to bf16, 1.1e-3 on average each
+    assert rel(out, want) < 8e-3
+    for got, exp, name in zip(grads, want_grads, ("q", "kv", "low", "q_scale", "k_scale")):
+        # a scale's gradient is a sum of terms many times its size, each as exact as a gradient (rounding the rotated heads alone moves the
+        # sum by up to 3e-3 of the terms' norm)
+        size = exp.norm() if name not in ("q_scale", "k_scale") else (tqs if name == "q_scale" else tks).grad.norm()
+        if size > 1e-2:                       # one position: the scores have no gradient
+            assert (got.float() - exp).norm() < 1.5e-2 * size, name
+    cuda_ops.check_status()
+
+
+@pytest.mark.parametrize("name", ["gelu", "relu", "relu2", "silu", "swiglu"])
+@pytest.mark.parametrize("shape", [(3, 5, 16), (300, 1024), (7, 6)])
+def test_activation_entry_point(name, shape):
+    torch.manual_seed(4)
+    x = (3 * torch.randn(*shape, device="cuda")).bfloat16().requires_grad_()
+    y = api.activate(x, name)
+    g = torch.randn_like(y)
+    (dx,) = torch.autograd.grad(y, x, g)
+    xf = x.detach().float().requires_grad_()
+    want = ref.activate(xf, name)
+    (dwant,) = torch.autograd.grad(want, xf, g.float())
+    tol = 4e-3 if shape[-1] % 16 == 0 else 8e-3          # one rounding in the kernel; torch's ops round every intermediate
+    assert rel(y, want) < tol and rel(dx, dwant) < tol
