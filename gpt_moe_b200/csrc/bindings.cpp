@@ -389,6 +389,12 @@ void gemm_plain(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d
 void gemm_by_expert(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d, const torch::Tensor& tile_expert, const torch::Tensor& meta) {
     gemm_bf16(a, b, d, false, false, 1.0, 0.0, c10::nullopt, false, GEMM_GROUPED_M, tile_expert, meta, c10::nullopt, false, c10::nullopt, 0);
 }
+void gemm_fp32(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d, bool accumulate) {
+    gemm_bf16(a, b, d, false, false, 1.0, 0.0, c10::nullopt, accumulate, GEMM_DENSE, c10::nullopt, c10::nullopt, c10::nullopt, false, c10::nullopt, 0);
+}
+CUtensorMap rows_map(const void* base, uint64_t cols, uint64_t rows, uint64_t batch, uint64_t row_pitch, uint64_t batch_pitch) {
+    return cached_map(base, 2, cols, rows, batch, row_pitch * 2, batch_pitch * 2, 64, 128, 128);
+}
 torch::Tensor attention_out(const torch::Tensor& q, const torch::Tensor& k, const torch::Tensor& v, int64_t window, double scale, double softcap,
                             const c10::optional<torch::Tensor>& doc_start) {
     return attn_fwd(q, k, v, window, scale, softcap, doc_start, false, false, c10::nullopt)[0];

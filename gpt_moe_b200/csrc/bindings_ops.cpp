@@ -6,6 +6,7 @@
 
 #include "bindings_shared.h"
 #include "guarded_alloc.h"
+#include "attention/attn.h"
 #include "kernels.h"
 #include "kernels_decl.h"
 
@@ -275,11 +276,10 @@ Tensor rows_linear(const Tensor& x, const Tensor& w) {
 // Latent-cache attention of T new tokens per sequence from their projections (attention/mla_decode.cu): appends them to the cache and
 // returns bf16 [B * T, H * value].  query [B*T, H * (content + dr)] and low [B*T, r + dr] bf16 (any row pitch), w_up fp32
 // [Hkv * (content + value), r], cos / sin fp32 tables [>= start + T, dr / 2], caches bf16 [B, capacity, width] with packed rows.
-Tensor mla_cached(const Tensor& query, const Tensor& low, const Tensor& w_up, const OptTensor& norm_w, double norm_eps, const Tensor& cos,
-                  const Tensor& sin, const OptTensor& q_scale, const OptTensor& k_scale, double qk_eps, bool rms, double smin, double smax,
-                  Tensor& latent, Tensor& rope, Tensor& key_gain, int64_t start, int64_t heads, int64_t content, int64_t value, double scale,
-                  double softcap, int64_t window) {
-    c10::cuda::CUDAGuard guard(query.device());
+// `terms`: w_up as two bf16 terms [2, rows, rank] (split_terms), for calls that expand the cache (mla_prefill.cu).
+MlaCachedArgs mla_cached_args(const Tensor& query, const Tensor& low, const Tensor& w_up, const OptTensor& norm_w, double norm_eps, const Tensor& cos, const Tensor& sin,
+                            const OptTensor& q_scale, const OptTensor& k_scale, double qk_eps, bool rms, double smin, double smax, Tensor& latent, Tensor& rope,
+                            Tensor& key_gain, int64_t start, int64_t heads, int64_t content, int64_t value, double scale, double softcap, int64_t window) {
     MlaCachedArgs a;
     a.B = latent.size(0); a.H = heads; a.Hkv = key_gain.size(2); a.r = latent.size(2); a.dr = rope.size(2);
     a.content = content; a.value = value; a.start = start; a.window = static_cast<int>(std::max<int64_t>(-1, window));
@@ -311,6 +311,72 @@ Tensor mla_cached(const Tensor& query, const Tensor& low, const Tensor& w_up, co
     a.latent = latent.data_ptr(); a.rope = rope.data_ptr(); a.key_gain = key_gain.data_ptr();
     a.latent_bs = latent.stride(0); a.rope_bs = rope.stride(0); a.gain_bs = key_gain.stride(0);
     a.norm_eps = norm_eps; a.qk_eps = qk_eps; a.smin = smin; a.smax = smax; a.scale = scale; a.softcap = softcap; a.rms = rms;
+    return a;
+}
+
+// Whether a call expands the visible cache instead of running the absorbed form: heads of 64 + 64 columns with 64-wide values, no
+// soft-capping, and enough queries.  The absorbed form costs by (query, position) pair, the expansion by position and some 15 us more
+// of launches.  Measured, 16 heads, rank 512, absorbed against expanded in us: sequences x new tokens over positions 1 x 64 over 2064 144 : 147,
+// 1 x 96 over 2096 179 : 150, 1 x 64 over 7064 277 : 312, 1 x 96 over 7096 357 : 314, 2 x 48 over 1548 162 : 148, 4 x 34 over 4034 329 : 332, 4 x 48 over
+// 4048 563 : 331, 1 x 128 over 228 125 : 145, 1 x 256 over 356 190 : 145; 2 x 512 over 2012 1193 : 160.
+bool mla_prefill_wanted(int64_t B, int64_t T, int64_t end, int64_t window, int64_t r, int64_t dr, int64_t content, int64_t value, double softcap) {
+    const int64_t visible = window < 0 ? end : std::min(end, window + T);
+    return T >= 48 && B * T >= 96 && B * T * visible >= 90000 && r % 64 == 0 && dr == 64 && content == 64 && value == 64 && softcap <= 0.0;
+}
+
+Tensor mla_prefill(const MlaCachedArgs& args, const Tensor& latent, const Tensor& terms) {
+    MlaCachedArgs a = args;
+    const int end = a.start + a.T;
+    const int base = a.window < 0 ? 0 : std::max(0, a.start - a.window) / 128 * 128;      // first position any query sees, on a tile's edge
+    const int S = end - base, S_pad = (S + 127) / 128 * 128;
+    GM_CHECK(terms.is_cuda() && terms.scalar_type() == torch::kBFloat16 && terms.is_contiguous() && terms.dim() == 3 && terms.size(0) == 2 &&
+             terms.size(1) == static_cast<int64_t>(a.Hkv) * 128 && terms.size(2) == a.r, "mla_prefill: terms [2, Hkv * 128, rank] bf16");
+    GM_CHECK(reinterpret_cast<uintptr_t>(a.latent) % 16 == 0 && reinterpret_cast<uintptr_t>(a.rope) % 16 == 0 && a.latent_bs % 8 == 0 && a.rope_bs % 8 == 0 &&
+             reinterpret_cast<uintptr_t>(a.query) % 8 == 0 && a.q_pitch % 4 == 0, "mla_prefill: aligned cache and queries");
+    auto bf = latent.options();
+    Tensor q = gm::out_empty({a.B, a.T, a.H * 128}, bf);
+    launch_mla_prefill_prepare(a, q.data_ptr(), stream());
+    Tensor kv = gm::out_empty({a.B, S, a.Hkv * 128}, bf.dtype(torch::kFloat32));
+    const Tensor hi = terms.select(0, 0), lo = terms.select(0, 1);
+    const bool whole = a.B == 1 || (S == latent.size(1) && latent.stride(0) == static_cast<int64_t>(S) * a.r);
+    for (int b = 0; b < (whole ? 1 : a.B); ++b) {
+        const Tensor rows = whole ? latent.narrow(1, base, S).reshape({static_cast<int64_t>(a.B) * S, a.r}) : latent.select(0, b).narrow(0, base, S);
+        Tensor d = whole ? kv.view({static_cast<int64_t>(a.B) * S, a.Hkv * 128}) : kv.select(0, b);
+        gemm_fp32(rows, lo, d, false);
+        gemm_fp32(rows, hi, d, true);
+    }
+    Tensor split = gm::out_empty({4, a.B, S, a.Hkv * 64}, bf), gain = gm::out_empty({a.B, a.Hkv, S_pad}, kv.options());
+    void* parts[4];
+    for (int i = 0; i < 4; ++i) parts[i] = split.select(0, i).data_ptr();
+    launch_mla_prefill_split(a, base, kv.data_ptr<float>(), parts, gain.data_ptr<float>(), S, S_pad, stream());
+    Tensor out = gm::out_empty({static_cast<int64_t>(a.B) * a.T, a.H * 64}, bf);
+    a.out = out.data_ptr();
+    auto term_map = [&](int i) { return rows_map(parts[i], a.Hkv * 64, S, a.B, a.Hkv * 64, static_cast<uint64_t>(S) * a.Hkv * 64); };
+    const CUtensorMap tq = rows_map(q.data_ptr(), a.H * 128, a.T, a.B, a.H * 128, static_cast<uint64_t>(a.T) * a.H * 128);
+    const CUtensorMap tr = rows_map(static_cast<const uint16_t*>(a.rope) + static_cast<int64_t>(base) * 64, 64, S, a.B, 64, a.rope_bs);
+    cudaError_t e = launch_mla_prefill_attention(a, base, tq, term_map(0), term_map(1), tr, term_map(2), term_map(3), gain.data_ptr<float>(), S, S_pad,
+                                                 status_word(latent.device().index()), stream());
+    GM_CHECK(e == cudaSuccess, cudaGetErrorString(e));
+    return out;
+}
+
+// fp32 [rows, cols] as bf16 terms [2, rows, cols]
+Tensor split_terms(const Tensor& w) {
+    c10::cuda::CUDAGuard guard(w.device());
+    GM_CHECK(w.is_cuda() && w.scalar_type() == torch::kFloat32 && w.is_contiguous() && w.dim() == 2, "split_terms: contiguous fp32 matrix");
+    Tensor out = gm::out_empty({2, w.size(0), w.size(1)}, w.options().dtype(torch::kBFloat16));
+    launch_split_terms(w.data_ptr<float>(), out.select(0, 0).data_ptr(), out.select(0, 1).data_ptr(), w.numel(), stream());
+    return out;
+}
+
+Tensor mla_cached(const Tensor& query, const Tensor& low, const Tensor& w_up, const OptTensor& norm_w, double norm_eps, const Tensor& cos, const Tensor& sin,
+                  const OptTensor& q_scale, const OptTensor& k_scale, double qk_eps, bool rms, double smin, double smax, Tensor& latent, Tensor& rope,
+                  Tensor& key_gain, int64_t start, int64_t heads, int64_t content, int64_t value, double scale, double softcap, int64_t window,
+                  const OptTensor& terms) {
+    c10::cuda::CUDAGuard guard(query.device());
+    MlaCachedArgs a = mla_cached_args(query, low, w_up, norm_w, norm_eps, cos, sin, q_scale, k_scale, qk_eps, rms, smin, smax, latent, rope, key_gain, start, heads,
+                                      content, value, scale, softcap, window);
+    if (terms.has_value() && mla_prefill_wanted(a.B, a.T, start + a.T, window, a.r, a.dr, content, value, softcap)) return mla_prefill(a, latent, *terms);
     a.splits = mla_decode_splits(a.B, a.T, a.H, a.r, start + a.T);
     const int64_t rows = static_cast<int64_t>(a.B) * a.T * a.H;
     // one fp32 workspace: queries in latent space, rotary queries, partial contexts, partial maxima and sums
@@ -334,7 +400,7 @@ Tensor mla_step(const Tensor& x, const Tensor& w_in, const Tensor& w_out, const 
     const int64_t nq = heads * (content + rope.size(2));
     GM_CHECK(both.size(1) == nq + latent.size(2) + rope.size(2), "mla_step: w_in holds the query rows, then the latent and rotary rows");
     Tensor out = mla_cached(both.narrow(1, 0, nq), both.narrow(1, nq, both.size(1) - nq), w_up, norm_w, norm_eps, cos, sin, q_scale, k_scale, qk_eps, rms, smin,
-                            smax, latent, rope, key_gain, start, heads, content, value, scale, softcap, window);
+                            smax, latent, rope, key_gain, start, heads, content, value, scale, softcap, window, c10::nullopt);
     return rows_linear(out, w_out);
 }
 
@@ -794,6 +860,8 @@ void register_kernels(pybind11::module_& m) {
     m.def("mla_decode_ok", &mla_decode_ok);
     m.def("rows_linear", &rows_linear);
     m.def("mla_cached", &mla_cached);
+    m.def("mla_prefill_wanted", &mla_prefill_wanted);
+    m.def("split_terms", &split_terms);
     m.def("mla_step", &mla_step);
     m.def("mma_issue_bench", &mma_issue_bench, py::arg("shape"), py::arg("count") = 64);
     m.def("router_fwd", &router_fwd);

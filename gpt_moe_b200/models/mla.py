@@ -238,7 +238,13 @@ class MLAttention(nn.Module):
         if self.q_rank:
             query = api.rms_norm(self.q_down_proj(query), self.q_norm.weight, self.q_norm.eps)
         query = self.q_proj(query).reshape(b * t, -1)
-        out = c.mla_cached(query, self.kv_down_proj(x).reshape(b * t, -1), *rest)
+        terms = None
+        if c.mla_prefill_wanted(b, t, start + t, rest[-1], self.kv_rank, self.rope_dim, self.content_dim, self.value_dim, self.softcap) and all(
+                p.data_ptr() % 16 == 0 and p.stride(0) % 8 == 0 for p in caches[:2]):
+            # many new tokens: the visible cache is expanded (csrc/attention/mla_prefill.cu), with W as two bf16 terms laid out once
+            up = self.kv_up_proj.weight
+            terms = cuda_ops._cached(("terms", id(up)), (up,), lambda old: c.split_terms(up.detach()))
+        out = c.mla_cached(query, self.kv_down_proj(x).reshape(b * t, -1), *rest, terms)
         return self.out_proj(out.view(b, t, self.attn_dim))
 
 

@@ -25,6 +25,11 @@ CASES = [
     (2, 3, 32, 8, 256, 10, 54, 62, None, False, 0),          # 32 heads, rotary width no multiple of 8, no QK-norm
     (1, 70, 16, 16, 768, 32, 32, 5, None, True, 64),         # wide latent, low-rank queries, many tokens per weight pass
     (2, 1, 8, 2, 1024, 64, 64, 200, 64, True, 0),            # widest latent
+    (3, 256, 16, 16, 512, 64, 64, 0, None, True, 0),         # expanded keys and values from here on: an empty cache, whole tiles
+    (1, 200, 16, 4, 512, 64, 64, 333, None, True, 0),        # groups of heads, ragged queries and positions
+    (4, 129, 8, 8, 256, 64, 64, 500, 100, True, 0),          # a window shorter than a tile: expansion starts inside the cache
+    (4, 130, 16, 16, 768, 64, 64, 126, 300, False, 0),       # a window longer than a tile, no QK-norm
+    (1, 300, 16, 16, 512, 64, 64, 1, None, True, 64),        # low-rank queries
 ]
 
 
@@ -33,7 +38,7 @@ def test_cached_step_matches_the_plain_path(b, t, h, hkv, r, dr, c, start, windo
     torch.manual_seed(11)
     gc, tc = get_preset("mla")
     gc.hidden_size, gc.n_heads, gc.n_kv_heads, gc.use_qk_norm = 256, h, hkv, norm
-    gc.mla_kv_rank, gc.mla_qk_rope_dim, gc.mla_qk_content_dim, gc.mla_value_dim, gc.mla_q_rank = r, dr, c, 32, q_rank
+    gc.mla_kv_rank, gc.mla_qk_rope_dim, gc.mla_qk_content_dim, gc.mla_value_dim, gc.mla_q_rank = r, dr, c, 64 if t >= 128 else 32, q_rank
     tc.resolve(1)
     cpu = MLAttention(gc, tc).eval()
     for p in cpu.parameters():
@@ -57,6 +62,8 @@ def test_cached_step_matches_the_plain_path(b, t, h, hkv, r, dr, c, start, windo
     before = cuda_ops.path_counts().get("mla_decode:kernel", 0)
     got = gpu.forward_cached(x.cuda(), cache, window)
     assert cuda_ops.path_counts().get("mla_decode:kernel", 0) == before + 1
+    if t >= 128:
+        assert cuda_ops.ext().mla_prefill_wanted(b, t, start + t, -1 if window is None else window, r, dr, c, 64, 0.0)
     want = cpu.forward_cached(x.float(), plain, window)
     assert got.dtype == torch.bfloat16 and cache.length == plain.length == start + t
     new = slice(start, start + t)
