@@ -528,7 +528,8 @@ Tensor ce_fwd_bwd(Tensor& logits, const Tensor& targets, const Tensor& grad_scal
     const int rows = logits.size(0);
     Tensor loss = gm::out_empty({rows}, logits.options().dtype(torch::kFloat32));
     launch_ce_fwd_bwd(logits.data_ptr(), reinterpret_cast<const long long*>(targets.data_ptr<int64_t>()), loss.data_ptr<float>(),
-                      grad_scale.data_ptr<float>(), rows, logits.size(1), logits.stride(0), ignore_index, write_grad, stream());
+                      grad_scale.data_ptr<float>(), rows, logits.size(1), logits.stride(0), ignore_index, write_grad,
+                      status_word(logits.device().index()), stream());
     return loss;
 }
 

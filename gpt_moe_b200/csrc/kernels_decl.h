@@ -86,7 +86,7 @@ void launch_row_nll(const void* logits, const long long* targets, float* loss, i
 void launch_continuation_logprob(const void* logits, const long long* tokens, const long long* prefix, const long long* end, float* lp, int n, int length,
                                  int vocab, long long batch_stride, long long row_stride, long long token_stride, int* status, cudaStream_t s);
 void launch_ce_fwd_bwd(void* logits, const long long* targets, float* loss, const float* grad_scale, int rows, int vocab,
-                       long long row_stride, long long ignore_index, int write_grad, cudaStream_t s);
+                       long long row_stride, long long ignore_index, int write_grad, int* status, cudaStream_t s);
 void launch_adamw(float* p, const float* g, void* m, void* v, bool moments_bf16, void* p_bf16, long long n, float lr, float beta1,
                   float beta2, float eps, float wd, float bc1, float bc2_sqrt, float grad_scale, cudaStream_t s);
 void launch_muon_prepare(const float* const* grads, float* const* bufs, void* packed, float* sumsq, int n_mats, int rows, int cols,

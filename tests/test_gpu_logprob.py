@@ -53,3 +53,33 @@ def test_continuation_scores(n, t, vocab):
     want = continuation_scores(logits.cpu().float(), ids.cpu(), prefix, true)
     assert torch.allclose(got.cpu(), want, rtol=2e-5, atol=2e-5)
     cuda_ops.check_status()
+
+
+# one 16-byte unit, fewer units than pieces, units that do not divide into pieces, the training vocabulary, both sides of the shared-memory limit
+@pytest.mark.parametrize("vocab", [8, 24, 40, 4104, 50304, 56960, 56968, 50301])
+@pytest.mark.parametrize("write_grad", [True, False])
+def test_loss_and_gradient_in_place(vocab, write_grad):
+    torch.manual_seed(3)
+    pitch = (vocab + 15) // 8 * 8
+    store = torch.randn(9, pitch, device="cuda").mul_(4).bfloat16()
+    logits = store[:, :vocab]
+    logits[1, 0] = float("-inf")
+    logits[2, vocab - 1] = 90.0
+    targets = torch.randint(0, vocab, (9,), device="cuda")
+    targets[1], targets[3], targets[4] = vocab - 1, 0, -100
+    before, tail = logits.clone(), store[:, vocab:].clone()
+    scale = torch.tensor([0.25], device="cuda")
+    loss = cuda_ops.ext().ce_fwd_bwd(logits, targets, scale, -100, write_grad)
+    exact = before.double()
+    want = torch.nn.functional.cross_entropy(exact, targets, ignore_index=-100, reduction="none")
+    assert torch.allclose(loss.double(), want, rtol=1e-5, atol=1e-5)
+    if write_grad:
+        grad = torch.softmax(exact, dim=-1)
+        keep = targets != -100
+        grad[keep, targets[keep]] -= 1.0
+        grad[~keep] = 0.0
+        assert torch.allclose(logits.double(), grad * 0.25, rtol=2 ** -8, atol=1e-7)       # one rounding to bf16
+    else:
+        assert torch.equal(logits, before)
+    assert torch.equal(store[:, vocab:], tail)
+    cuda_ops.check_status()
