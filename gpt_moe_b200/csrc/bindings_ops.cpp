@@ -533,6 +533,21 @@ Tensor ce_fwd_bwd(Tensor& logits, const Tensor& targets, const Tensor& grad_scal
     return loss;
 }
 
+// grad[ids[i]] += dy[order[i]] for tokens sorted by id (int32 ids, int64 positions of a stable sort); fp32
+void embedding_grad(const Tensor& dy, const Tensor& ids, const Tensor& order, Tensor& grad) {
+    c10::cuda::CUDAGuard guard(dy.device());
+    GM_CHECK(dy.is_cuda() && dy.scalar_type() == torch::kFloat32 && dy.is_contiguous() && dy.dim() == 2 && dy.size(1) % 4 == 0 &&
+             reinterpret_cast<uintptr_t>(dy.data_ptr()) % 16 == 0, "embedding_grad: dy [tokens, d] fp32, d a multiple of 4");
+    GM_CHECK(grad.is_cuda() && grad.scalar_type() == torch::kFloat32 && grad.is_contiguous() && grad.dim() == 2 && grad.size(1) == dy.size(1) &&
+             reinterpret_cast<uintptr_t>(grad.data_ptr()) % 16 == 0, "embedding_grad: grad [vocab, d] fp32");
+    GM_CHECK(ids.is_cuda() && ids.scalar_type() == torch::kInt32 && ids.is_contiguous() && ids.numel() == dy.size(0) && order.is_cuda() &&
+             order.scalar_type() == torch::kInt64 && order.is_contiguous() && order.numel() == dy.size(0), "embedding_grad: sorted int32 ids and their int64 positions");
+    const int tokens = dy.size(0);
+    Tensor edge = gm::out_empty({2 * embedding_grad_windows(tokens), dy.size(1)}, dy.options());
+    launch_embedding_grad(dy.data_ptr<float>(), ids.data_ptr<int>(), reinterpret_cast<const long long*>(order.data_ptr<int64_t>()), grad.data_ptr<float>(),
+                          edge.data_ptr<float>(), tokens, dy.size(1), grad.size(0), stream());
+}
+
 // fp32 [rows]: -log softmax(logits)[target], 0 for ignored rows; logits [rows, vocab] bf16 are only read
 Tensor row_nll(const Tensor& logits, const Tensor& targets, int64_t ignore_index) {
     c10::cuda::CUDAGuard guard(logits.device());
@@ -879,6 +894,7 @@ void register_kernels(pybind11::module_& m) {
     m.def("activation_bwd", &activation_bwd, py::arg("dact"), py::arg("pre"), py::arg("name"), py::arg("meta") = py::none(), py::arg("quantize") = false);
     m.def("ce_fwd_bwd", &ce_fwd_bwd);
     m.def("row_nll", &row_nll);
+    m.def("embedding_grad", &embedding_grad);
     m.def("attention_branch", &attention_branch);
     m.def("moe_branch", &moe_branch);
     m.def("continuation_logprob", &continuation_logprob);

@@ -20,7 +20,7 @@ constexpr long long kWaitBudgetCycles = 2000000000LL;   // ~1 s at B200 clocks
 // A failing test records its code in the translation unit's word (first failure wins) and evaluates to false, so the caller
 // SKIPS the access: nothing traps, the context stays usable, and the host reads the code through `read_bounds_status`.  In the
 // normal build the macro is the constant `true` and costs nothing.  Codes: 901 expert id in routing, 902 gathered token,
-// 903 combined row, 904 combine-backward token, 905 cross-entropy target, 906 router-backward expert id.
+// 903 combined row, 904 combine-backward token, 905 cross-entropy target, 906 router-backward expert id, 907 embedding row.
 #ifdef GM_CHECK_BOUNDS
 static __device__ int gm_bounds_word = 0;
 #define GM_IN_BOUNDS(cond, code) ((cond) ? true : (atomicCAS(&gm_bounds_word, 0, (code)), false))

@@ -342,6 +342,90 @@ void launch_continuation_logprob(const void* logits, const long long* tokens, co
                                                                           batch_stride, row_stride, token_stride, vec16, status);
 }
 
+// ---- embedding gradient, added into the optimizer's buffer -----------------------------------------------------------------
+// The gradient of an embedding table touches as many rows as there are tokens.  Formed as a tensor of the table's size it was filled with
+// zeros, scattered into and added to the gradient buffer: three passes over 154 MB at 50304 x 768, whatever the number of tokens.  Here
+// the tokens come sorted by id (stable, so every sum has the order of the positions) and runs of one id are summed and added to
+// their row of the buffer: a CTA takes EMB_WINDOW sorted tokens, adds the runs that lie inside its window, and leaves the pieces of a
+// run that crosses windows (the first and the last run of a window) in `edge`; the second kernel adds those up in window order.
+// 32768 tokens of a 50304 x 768 table: 54 us and 36 for the sort, where torch's scatter, its sort, the fill and the addition took 560.
+constexpr int EMB_WINDOW = 32;
+
+__global__ void __launch_bounds__(256)
+embedding_grad_kernel(const float* __restrict__ dy, const int* __restrict__ ids, const long long* __restrict__ order, float* __restrict__ grad,
+                      float* __restrict__ edge, int tokens, int d, int vocab) {
+    const int w0 = blockIdx.x * EMB_WINDOW, w1 = min(w0 + EMB_WINDOW, tokens);
+    __shared__ int id_s[EMB_WINDOW + 2];
+    __shared__ long long row_s[EMB_WINDOW];
+    for (int i = threadIdx.x; i < EMB_WINDOW + 2; i += blockDim.x) {
+        const int at = w0 - 1 + i;                                     // one neighbour on each side
+        id_s[i] = at >= 0 && at < tokens ? ids[at] : -1;
+        if (i < EMB_WINDOW && w0 + i < tokens) row_s[i] = order[w0 + i];
+    }
+    __syncthreads();
+    const bool from_before = id_s[0] == id_s[1], goes_on = w1 < tokens && id_s[w1 - w0] == id_s[w1 - w0 + 1];
+    for (int c = threadIdx.x * 4; c < d; c += blockDim.x * 4) {
+        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+        bool first_run = true;
+        for (int i0 = 0; i0 < w1 - w0; i0 += 8) {
+            float4 v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u)                                 // eight rows in flight
+                v[u] = i0 + u < w1 - w0 ? __ldcs(reinterpret_cast<const float4*>(dy + row_s[i0 + u] * d + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int i = i0 + u;
+                if (i >= w1 - w0) break;
+                sum.x += v[u].x; sum.y += v[u].y; sum.z += v[u].z; sum.w += v[u].w;
+                if (i + 1 < w1 - w0 && id_s[i + 2] == id_s[i + 1]) continue;            // the run goes on inside the window
+                const long long id = id_s[i + 1];
+                const bool last = i + 1 == w1 - w0;
+                if (first_run && from_before) *reinterpret_cast<float4*>(edge + (2LL * blockIdx.x) * d + c) = sum;       // belongs to a run of earlier windows
+                else if (last && goes_on) *reinterpret_cast<float4*>(edge + (2LL * blockIdx.x + 1) * d + c) = sum;      // starts here, ends later
+                else if (GM_IN_BOUNDS(id >= 0 && id < vocab, 907) && id >= 0 && id < vocab) {
+                    float4* g = reinterpret_cast<float4*>(grad + id * d + c);
+                    float4 old = *g;
+                    old.x += sum.x; old.y += sum.y; old.z += sum.z; old.w += sum.w;
+                    *g = old;
+                }
+                sum = make_float4(0.f, 0.f, 0.f, 0.f);
+                first_run = false;
+            }
+        }
+    }
+}
+
+// one CTA per window in which a run starts that later windows continue
+__global__ void __launch_bounds__(256)
+embedding_grad_edges_kernel(const int* __restrict__ ids, const float* __restrict__ edge, float* __restrict__ grad, int tokens, int d, int vocab) {
+    const int w0 = blockIdx.x * EMB_WINDOW, w1 = w0 + EMB_WINDOW;
+    if (w1 >= tokens) return;
+    const long long id = ids[w1 - 1];
+    if (ids[w1] != id || id < 0 || id >= vocab) return;                 // the window's last run ends with it
+    if (w0 > 0 && ids[w0 - 1] == id && ids[w0] == id) return;           // the run starts in an earlier window (this one holds nothing else)
+    for (int c = threadIdx.x * 4; c < d; c += blockDim.x * 4) {
+        float4 sum = *reinterpret_cast<const float4*>(edge + (2LL * blockIdx.x + 1) * d + c);
+        for (int w = blockIdx.x + 1; static_cast<long long>(w) * EMB_WINDOW < tokens && ids[w * EMB_WINDOW] == id; ++w) {
+            const float4 v = *reinterpret_cast<const float4*>(edge + 2LL * w * d + c);
+            sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+            const long long end = static_cast<long long>(w + 1) * EMB_WINDOW;
+            if (end >= tokens || ids[end - 1] != id) break;
+        }
+        float4* g = reinterpret_cast<float4*>(grad + id * d + c);
+        float4 old = *g;
+        old.x += sum.x; old.y += sum.y; old.z += sum.z; old.w += sum.w;
+        *g = old;
+    }
+}
+
+void launch_embedding_grad(const float* dy, const int* ids, const long long* order, float* grad, float* edge, int tokens, int d, int vocab, cudaStream_t s) {
+    if (tokens == 0) return;
+    const int windows = (tokens + EMB_WINDOW - 1) / EMB_WINDOW, threads = d / 4 < 256 ? (d / 4 + 31) / 32 * 32 : 256;
+    embedding_grad_kernel<<<windows, threads, 0, s>>>(dy, ids, order, grad, edge, tokens, d, vocab);
+    embedding_grad_edges_kernel<<<windows, threads, 0, s>>>(ids, edge, grad, tokens, d, vocab);
+}
+int embedding_grad_windows(int tokens) { return (tokens + EMB_WINDOW - 1) / EMB_WINDOW; }
+
 // ---- AdamW ---------------------------------------------------------------------------------------------
 // p, g fp32; moments fp32 or bf16.  Decoupled weight decay; bias corrections passed in.  Optionally refreshes a
 // bf16 copy of the parameter (the GEMM operand) in the same pass.

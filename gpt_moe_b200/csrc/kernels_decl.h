@@ -81,6 +81,8 @@ bool launch_router_bwd(const void* logits, bool bf16, const long long* top_idx, 
                        void* dlogits, int tokens, int experts, int top_k, int renormalise, cudaStream_t s);
 
 // fused/loss_optim.cu
+void launch_embedding_grad(const float* dy, const int* ids, const long long* order, float* grad, float* edge, int tokens, int d, int vocab, cudaStream_t s);
+int embedding_grad_windows(int tokens);
 void launch_row_nll(const void* logits, const long long* targets, float* loss, int rows, int vocab, long long row_stride, long long ignore_index,
                     int* status, cudaStream_t s);
 void launch_continuation_logprob(const void* logits, const long long* tokens, const long long* prefix, const long long* end, float* lp, int n, int length,

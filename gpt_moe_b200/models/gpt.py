@@ -248,7 +248,7 @@ class GPT(nn.Module):
                 ) -> Union[Tensor, Tuple[Tensor, Optional[Tensor]], Tuple[Tensor, Tensor, Tensor]]:
         batch, seq_len = indices.shape[:2]
         if self.stage_index != 1:
-            x = self.transformer.wte(indices)
+            x = api.embedding(self.transformer.wte, indices)
             if "wpe" in self.transformer:
                 x = x + self.transformer.wpe(torch.arange(seq_len, dtype=torch.long, device=indices.device))
         else:

@@ -77,6 +77,10 @@ def linear(x: Tensor, weight: Tensor, bias: Optional[Tensor], precision: str = "
     return F.linear(x, weight.to(x.dtype), None if bias is None else bias.to(x.dtype))
 
 
+def embedding(module, indices: Tensor) -> Tensor:
+    return _cuda().embedding(module, indices) if indices.is_cuda else module(indices)
+
+
 def activate(x: Tensor, name: str) -> Tensor:
     if x.is_cuda and x.dtype == torch.bfloat16:
         return _cuda().activate(x, name)

@@ -266,6 +266,40 @@ def _take_accumulate_flag(weights: Sequence[Tensor]) -> bool:
     return acc
 
 
+# ---- embedding ----------------------------------------------------------------------------------------------
+class _EmbeddingFn(torch.autograd.Function):
+    """Table lookup whose gradient is added straight into the optimizer's buffer (`weight.main_grad`): only the rows of tokens that
+    occur are touched, each sum in the order of the positions."""
+
+    @staticmethod
+    def forward(ctx, indices: Tensor, weight: Tensor) -> Tensor:
+        ctx.save_for_backward(indices)
+        ctx.weight = weight
+        return F.embedding(indices, weight)
+
+    @staticmethod
+    def backward(ctx, dy: Tensor):
+        (indices,) = ctx.saved_tensors
+        weight = ctx.weight
+        if not _take_accumulate_flag((weight,)):
+            weight.main_grad.zero_()
+        ids, order = torch.sort(indices.reshape(-1).to(torch.int32), stable=True)
+        ext().embedding_grad(dy.reshape(-1, dy.shape[-1]).float().contiguous(), ids, order, weight.main_grad)
+        return None, None
+
+
+def embedding(module, indices: Tensor) -> Tensor:
+    """`module(indices)` for an nn.Embedding; with a gradient buffer of the engine on its weight, the gradient goes there."""
+    weight = module.weight
+    main = getattr(weight, "main_grad", None)
+    if (main is None or not torch.is_grad_enabled() or not weight.requires_grad or weight.dtype != torch.float32 or not main.is_contiguous()
+            or weight.shape[1] % 4 or main.data_ptr() % 16 or weight.shape[0] >= 2 ** 31 or module.padding_idx is not None
+            or module.max_norm is not None or module.scale_grad_by_freq or module.sparse or module._forward_hooks or module._forward_pre_hooks
+            or torch._C._are_functorch_transforms_active()):
+        return module(indices)
+    return _EmbeddingFn.apply(indices, weight)
+
+
 # ---- linear -------------------------------------------------------------------------------------------------
 class _LinearFn(torch.autograd.Function):
     """y = x @ cat(weights)^T in bf16 with fp32 accumulation; weight gradients in fp32."""
