@@ -596,12 +596,13 @@ Tensor attention_branch(const Tensor& x, const Tensor& w_qkv, const Tensor& w_ou
              "attention_branch: fp32 QK scales");
     Tensor qkv = gm::out_empty({tokens, width}, x.options());
     gemm_plain(x, w_qkv, qkv);
-    Tensor rotated = gm::out_empty({tokens, width}, x.options());
-    rope_qknorm_fwd(qkv, rotated, cos_t, sin_t, q_scale, k_scale, seq, heads, kv_heads, head_dim, eps, rms, smin, smax, kv_heads * head_dim);
-    auto part = [&](int64_t first, int64_t n) {
-        return rotated.as_strided({batch, seq, n, head_dim}, {seq * width, width, head_dim, 1}, rotated.storage_offset() + first * head_dim);
+    const int64_t turned = (heads + kv_heads) * head_dim;      // query and key heads; the values are read where the projection left them
+    Tensor rotated = gm::out_empty({tokens, turned}, x.options());
+    rope_qknorm_fwd(qkv, rotated, cos_t, sin_t, q_scale, k_scale, seq, heads, kv_heads, head_dim, eps, rms, smin, smax, 0);
+    auto part = [&](const Tensor& rows, int64_t first, int64_t n) {
+        return rows.as_strided({batch, seq, n, head_dim}, {seq * rows.size(1), rows.size(1), head_dim, 1}, rows.storage_offset() + first * head_dim);
     };
-    Tensor o = attention_out(part(0, heads), part(heads, kv_heads), part(heads + kv_heads, kv_heads), window, scale, softcap, doc_start);
+    Tensor o = attention_out(part(rotated, 0, heads), part(rotated, heads, kv_heads), part(qkv, heads + kv_heads, kv_heads), window, scale, softcap, doc_start);
     Tensor y = gm::out_empty({tokens, w_out.size(0)}, x.options());
     gemm_plain(o.view({tokens, heads * head_dim}), w_out, y);
     return y;

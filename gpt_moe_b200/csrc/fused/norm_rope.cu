@@ -323,7 +323,7 @@ __device__ __forceinline__ float head_sum(float v) {
 }
 
 template <int D, bool BWD>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 4)
 rope_qknorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* dy, __nv_bfloat16* out,
                    const float* __restrict__ cos_t, const float* __restrict__ sin_t, const float* __restrict__ q_scale,
                    const float* __restrict__ k_scale, float* __restrict__ dscale_partial, long long tokens, int seq_len,
@@ -337,96 +337,143 @@ rope_qknorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* dy,
     const int sub = lane / LANES, li = lane % LANES;
     const int heads = q_heads + k_heads;
     const int groups = (heads + HEADS_PER_WARP - 1) / HEADS_PER_WARP;
-    const long long total = tokens * groups;
     const bool has_norm = q_scale != nullptr;
     __shared__ float ds_smem[8][64];
     if (BWD) {
         for (int i = threadIdx.x; i < 8 * 64; i += blockDim.x) (&ds_smem[0][0])[i] = 0.f;
         __syncthreads();
     }
-    for (long long idx = static_cast<long long>(blockIdx.x) * 8 + warp; idx < total; idx += static_cast<long long>(gridDim.x) * 8) {
-        const long long t = idx / groups;
-        const int h = static_cast<int>(idx - t * groups) * HEADS_PER_WARP + sub;
-        const bool live = h < heads;
-        const int pos = static_cast<int>(t % seq_len);
+    // A warp owns a token: one position, one row of the rotary tables, and the loads of U head groups are issued before the first of them is
+    // worked on.  (With one group in flight per warp and two divisions to find it the kernel ran at two thirds of the copy rate.)
+    // 32768 tokens, 24 heads of 64: forward 41 us (69 with the copy of the value columns that the attention kernel no longer needs), backward with
+    // the MXFP8 copy 109 us (124).
+    constexpr int U = BWD ? 1 : 3;               // within 64 registers, four CTAs an SM; the backward's gradients and outputs leave no registers for more (2: 1895 us for 1495 over 12 layers)
+    for (long long t = static_cast<long long>(blockIdx.x) * 8 + warp; t < tokens; t += static_cast<long long>(gridDim.x) * 8) {
         float c[4] = {1.f, 1.f, 1.f, 1.f}, sn[4] = {0.f, 0.f, 0.f, 0.f};
         if (cos_t) {
+            const long long pos = t % seq_len;
             const float4 cv = *reinterpret_cast<const float4*>(cos_t + pos * PAIRS + li * 4);
             const float4 sv = *reinterpret_cast<const float4*>(sin_t + pos * PAIRS + li * 4);
             c[0] = cv.x; c[1] = cv.y; c[2] = cv.z; c[3] = cv.w;
             sn[0] = sv.x; sn[1] = sv.y; sn[2] = sv.z; sn[3] = sv.w;
         }
-        uint4 xraw = make_uint4(0, 0, 0, 0), graw = make_uint4(0, 0, 0, 0);
-        if (live) {
-            xraw = *reinterpret_cast<const uint4*>(x + t * x_stride + h * D + li * 8);
-            if (BWD && !(dq32 != nullptr && h < q_heads)) graw = *reinterpret_cast<const uint4*>(dy + t * o_stride + h * D + li * 8);
-        }
-        const __nv_bfloat162* xp = reinterpret_cast<const __nv_bfloat162*>(&xraw);
-        const __nv_bfloat162* gp = reinterpret_cast<const __nv_bfloat162*>(&graw);
-        float r1[4], r2[4], g1[4], g2[4];
-        float ss = 0.f, dot = 0.f;
-        // backward: query-head gradients may arrive as fp32 (the attention backward's dQ accumulator) instead of bf16 rows
-        const bool g_fp32 = BWD && dq32 != nullptr && live && h < q_heads;
-        float4 ga = make_float4(0.f, 0.f, 0.f, 0.f), gb = ga;
-        if (g_fp32) {
-            ga = *reinterpret_cast<const float4*>(dq32 + t * dq_stride + h * D + li * 8);
-            gb = *reinterpret_cast<const float4*>(dq32 + t * dq_stride + h * D + li * 8 + 4);
-        }
-        const float gq[8] = {ga.x, ga.y, ga.z, ga.w, gb.x, gb.y, gb.z, gb.w};
+#pragma unroll 1
+        for (int g0 = 0; g0 < groups; g0 += U) {
+            uint4 xr[U], gr[U];
+            float4 ga_[U], gb_[U];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float2 xf = __bfloat1622float2(xp[i]);
-            r1[i] = xf.x * c[i] - xf.y * sn[i];
-            r2[i] = xf.x * sn[i] + xf.y * c[i];
-            ss += r1[i] * r1[i] + r2[i] * r2[i];
-            if (BWD) {
-                const float2 gf = __bfloat1622float2(gp[i]);
-                g1[i] = g_fp32 ? gq[2 * i] : gf.x;
-                g2[i] = g_fp32 ? gq[2 * i + 1] : gf.y;
-                dot += g1[i] * r1[i] + g2[i] * r2[i];
+            for (int u = 0; u < U; ++u) {
+                const int h = (g0 + u) * HEADS_PER_WARP + sub;
+                xr[u] = gr[u] = make_uint4(0, 0, 0, 0);
+                ga_[u] = gb_[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (h < heads) {
+                    xr[u] = *reinterpret_cast<const uint4*>(x + t * x_stride + h * D + li * 8);
+                    if (BWD) {
+                        // query-head gradients may arrive as fp32 (the attention backward's dQ accumulator) instead of bf16 rows
+                        if (dq32 != nullptr && h < q_heads) {
+                            ga_[u] = *reinterpret_cast<const float4*>(dq32 + t * dq_stride + h * D + li * 8);
+                            gb_[u] = *reinterpret_cast<const float4*>(dq32 + t * dq_stride + h * D + li * 8 + 4);
+                        } else {
+                            gr[u] = *reinterpret_cast<const uint4*>(dy + t * o_stride + h * D + li * 8);
+                        }
+                    }
+                }
             }
-        }
-        const float raw = !live ? 1.f : h < q_heads ? (q_scale ? q_scale[h] : 1.f) : (k_scale ? k_scale[h - q_heads] : 1.f);
-        const float sc = fminf(fmaxf(raw, smin), smax);
-        float gain = 1.f, mult = 1.f;
-        if (has_norm) {
-            ss = head_sum<D>(ss);
-            gain = rsqrtf((rms ? ss / D : ss) + eps);
-            mult = gain * sc;
-        }
-        uint4 oraw;
-        __nv_bfloat162* op = reinterpret_cast<__nv_bfloat162*>(&oraw);
-        if (BWD) {
-            dot = head_sum<D>(dot);
-            if (has_norm && live && li == 0 && raw >= smin && raw <= smax) ds_smem[warp][h] += dot * gain;
-            const float coef = has_norm ? gain * gain * (rms ? dot / D : dot) : 0.f;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float d1 = mult * (g1[i] - r1[i] * coef), d2 = mult * (g2[i] - r2[i] * coef);
-                op[i] = __floats2bfloat162_rn(d1 * c[i] + d2 * sn[i], -d1 * sn[i] + d2 * c[i]);
-            }
-            if (live) *reinterpret_cast<uint4*>(out + t * x_stride + h * D + li * 8) = oraw;
-            if (mxq != nullptr) {
-                // MXFP8 copy of the packed gradient row (the operand of the projection's input-gradient GEMM): a lane's 8
-                // values are a quarter of a 32-column block, the 4 lanes of a block are adjacent
-                float v8[8];
+            for (int u = 0; u < U; ++u) {
+                if (g0 + u >= groups) break;                                  // the same for the whole warp
+                const int h = (g0 + u) * HEADS_PER_WARP + sub;
+                const bool live = h < heads;
+                const __nv_bfloat162* xp = reinterpret_cast<const __nv_bfloat162*>(&xr[u]);
+                const __nv_bfloat162* gp = reinterpret_cast<const __nv_bfloat162*>(&gr[u]);
+                float r1[4], r2[4], g1[4], g2[4];
+                float ss = 0.f, dot = 0.f;
+                const bool g_fp32 = BWD && dq32 != nullptr && live && h < q_heads;
+                const float gq[8] = {ga_[u].x, ga_[u].y, ga_[u].z, ga_[u].w, gb_[u].x, gb_[u].y, gb_[u].z, gb_[u].w};
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const float2 f = __bfloat1622float2(op[i]);
-                    v8[2 * i] = live ? f.x : 0.f; v8[2 * i + 1] = live ? f.y : 0.f;
+                    const float2 xf = __bfloat1622float2(xp[i]);
+                    r1[i] = xf.x * c[i] - xf.y * sn[i];
+                    r2[i] = xf.x * sn[i] + xf.y * c[i];
+                    ss += r1[i] * r1[i] + r2[i] * r2[i];
+                    if (BWD) {
+                        const float2 gf = __bfloat1622float2(gp[i]);
+                        g1[i] = g_fp32 ? gq[2 * i] : gf.x;
+                        g2[i] = g_fp32 ? gq[2 * i + 1] : gf.y;
+                        dot += g1[i] * r1[i] + g2[i] * r2[i];
+                    }
                 }
-                uint32_t o2[2];
-                const uint32_t e8 = quantize_block_lanes<8>(v8, o2);
-                if (live) {
-                    const int col = h * D + li * 8;
-                    *reinterpret_cast<uint2*>(mxq + t * mx_width + col) = make_uint2(o2[0], o2[1]);
-                    if ((lane & 3) == 0) mxsf[sf_offset(t, col >> 5, (mx_width + 127) >> 7)] = static_cast<uint8_t>(e8);
+                const float raw = !live ? 1.f : h < q_heads ? (q_scale ? q_scale[h] : 1.f) : (k_scale ? k_scale[h - q_heads] : 1.f);
+                const float sc = fminf(fmaxf(raw, smin), smax);
+                float gain = 1.f, mult = 1.f;
+                if (has_norm) {
+                    ss = head_sum<D>(ss);
+                    gain = rsqrtf((rms ? ss / D : ss) + eps);
+                    mult = gain * sc;
+                }
+                uint4 oraw;
+                __nv_bfloat162* op = reinterpret_cast<__nv_bfloat162*>(&oraw);
+                if (BWD) {
+                    dot = head_sum<D>(dot);
+                    if (has_norm && live && li == 0 && raw >= smin && raw <= smax) ds_smem[warp][h] += dot * gain;
+                    const float coef = has_norm ? gain * gain * (rms ? dot / D : dot) : 0.f;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float d1 = mult * (g1[i] - r1[i] * coef), d2 = mult * (g2[i] - r2[i] * coef);
+                        op[i] = __floats2bfloat162_rn(d1 * c[i] + d2 * sn[i], -d1 * sn[i] + d2 * c[i]);
+                    }
+                    if (live) *reinterpret_cast<uint4*>(out + t * x_stride + h * D + li * 8) = oraw;
+                    if (mxq != nullptr) {
+                        // MXFP8 copy of the packed gradient row (the operand of the projection's input-gradient GEMM): a lane's 8
+                        // values are a quarter of a 32-column block, the 4 lanes of a block are adjacent
+                        float v8[8];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const float2 f = __bfloat1622float2(op[i]);
+                            v8[2 * i] = live ? f.x : 0.f; v8[2 * i + 1] = live ? f.y : 0.f;
+                        }
+                        uint32_t o2[2];
+                        const uint32_t e8 = quantize_block_lanes<8>(v8, o2);
+                        if (live) {
+                            const int col = h * D + li * 8;
+                            *reinterpret_cast<uint2*>(mxq + t * mx_width + col) = make_uint2(o2[0], o2[1]);
+                            if ((lane & 3) == 0) mxsf[sf_offset(t, col >> 5, (mx_width + 127) >> 7)] = static_cast<uint8_t>(e8);
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) op[i] = __floats2bfloat162_rn(r1[i] * mult, r2[i] * mult);
+                    if (live) *reinterpret_cast<uint4*>(out + t * o_stride + h * D + li * 8) = oraw;
                 }
             }
-        } else {
+        }
+        if (BWD && mxq != nullptr) {
+            // the trailing (value) columns of the gradient row pass through unchanged: only their quantised copy is produced here
+#pragma unroll 1
+            for (int v0 = 0; v0 < copy_cols; v0 += 4 * 256) {
+                uint4 vr[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) op[i] = __floats2bfloat162_rn(r1[i] * mult, r2[i] * mult);
-            if (live) *reinterpret_cast<uint4*>(out + t * o_stride + h * D + li * 8) = oraw;
+                for (int u = 0; u < 4; ++u) {
+                    const int col = v0 + u * 256 + lane * 8;
+                    vr[u] = col < copy_cols ? *reinterpret_cast<const uint4*>(dy + t * o_stride + heads * D + col) : make_uint4(0, 0, 0, 0);
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    if (v0 + u * 256 >= copy_cols) break;              // the same for the whole warp
+                    const int col = v0 + u * 256 + lane * 8;
+                    const __nv_bfloat162* hp = reinterpret_cast<const __nv_bfloat162*>(&vr[u]);
+                    float v8[8];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) { const float2 f = __bfloat1622float2(hp[e]); v8[2 * e] = f.x; v8[2 * e + 1] = f.y; }
+                    uint32_t o2[2];
+                    const uint32_t e8 = quantize_block_lanes<8>(v8, o2);
+                    if (col < copy_cols) {
+                        const int at = heads * D + col;
+                        *reinterpret_cast<uint2*>(mxq + t * mx_width + at) = make_uint2(o2[0], o2[1]);
+                        if ((lane & 3) == 0) mxsf[sf_offset(t, at >> 5, (mx_width + 127) >> 7)] = static_cast<uint8_t>(e8);
+                    }
+                }
+            }
         }
     }
     if (!BWD && copy_cols > 0) {
@@ -436,30 +483,6 @@ rope_qknorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* dy,
             const long long t = i / vecs;
             const int v = static_cast<int>(i - t * vecs);
             *reinterpret_cast<uint4*>(out + t * o_stride + heads * D + v * 8) = *reinterpret_cast<const uint4*>(x + t * x_stride + heads * D + v * 8);
-        }
-    }
-    if (BWD && mxq != nullptr && copy_cols > 0) {
-        // the trailing (value) columns of the gradient row pass through unchanged: only their quantised copy is produced here
-        const int vecs = copy_cols / 8;
-        const long long n = tokens * vecs;
-        for (long long base = static_cast<long long>(blockIdx.x) * blockDim.x + (threadIdx.x & ~31); base < n; base += static_cast<long long>(gridDim.x) * blockDim.x) {
-            const long long i = base + lane;
-            const bool active = i < n;
-            const long long t = active ? i / vecs : 0;
-            const int col = heads * D + (active ? static_cast<int>(i - t * vecs) * 8 : 0);
-            float v8[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            if (active) {
-                const uint4 raw = *reinterpret_cast<const uint4*>(dy + t * o_stride + col);
-                const __nv_bfloat162* hp = reinterpret_cast<const __nv_bfloat162*>(&raw);
-#pragma unroll
-                for (int e = 0; e < 4; ++e) { const float2 f = __bfloat1622float2(hp[e]); v8[2 * e] = f.x; v8[2 * e + 1] = f.y; }
-            }
-            uint32_t o2[2];
-            const uint32_t e8 = quantize_block_lanes<8>(v8, o2);
-            if (active) {
-                *reinterpret_cast<uint2*>(mxq + t * mx_width + col) = make_uint2(o2[0], o2[1]);
-                if ((lane & 3) == 0) mxsf[sf_offset(t, col >> 5, (mx_width + 127) >> 7)] = static_cast<uint8_t>(e8);
-            }
         }
     }
     if (BWD && dscale_partial) {
@@ -618,8 +641,8 @@ bool launch_mla_rope(bool bwd, const void* q, const void* kv, const void* rope, 
 }
 
 int rope_blocks(long long tokens, int heads) {
-    const long long want = (tokens * ((heads + 3) / 4) + 7) / 8;      // at least 4 heads of a token per warp pass for every supported head size
-    return static_cast<int>(want < 2368 ? want : 2368);
+    const long long want = (tokens + 7) / 8;                          // a warp per token
+    return static_cast<int>(want < 1 ? 1 : (want < 2368 ? want : 2368));
 }
 
 bool launch_rope_qknorm(bool bwd, int D, const void* x, const void* dy, void* out, const float* cos_t, const float* sin_t,

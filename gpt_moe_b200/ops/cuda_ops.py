@@ -520,14 +520,15 @@ class _RopeAttentionFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, qkv: Tensor, cos, sin, q_scale, k_scale, batch, seq_len, hq, hk, d, eps, rms, smin, smax, window, scale, softcap, doc_start):
         c = ext()
-        out = torch.empty_like(qkv)
+        # rotated query and key heads; the value heads are read where the projection left them
+        out = torch.empty((qkv.shape[0], (hq + hk) * d), dtype=qkv.dtype, device=qkv.device)
         qs = None if q_scale is None else q_scale.detach().float().reshape(-1).contiguous()
         ks = None if k_scale is None else k_scale.detach().float().reshape(-1).contiguous()
-        c.rope_qknorm_fwd(qkv, out, cos, sin, qs, ks, seq_len, hq, hk, d, eps, rms, smin, smax, qkv.shape[-1] - (hq + hk) * d)
+        c.rope_qknorm_fwd(qkv, out, cos, sin, qs, ks, seq_len, hq, hk, d, eps, rms, smin, smax, 0)
         packed = out.view(batch, seq_len, -1)
         q = packed[..., : hq * d].unflatten(-1, (hq, d))
-        k = packed[..., hq * d: (hq + hk) * d].unflatten(-1, (hk, d))
-        v = packed[..., (hq + hk) * d:].unflatten(-1, (hk, d))
+        k = packed[..., hq * d:].unflatten(-1, (hk, d))
+        v = qkv.view(batch, seq_len, -1)[..., (hq + hk) * d:].unflatten(-1, (hk, d))
         o, lse = c.attn_fwd(q, k, v, window, scale, softcap, doc_start)
         ctx.doc_start = doc_start
         empty = qkv.new_empty(0)
@@ -545,10 +546,10 @@ class _RopeAttentionFn(torch.autograd.Function):
         batch, seq_len, hq, hk, d, eps, rms, smin, smax, window, scale, softcap, has_rope, has_norm = ctx.cfg
         packed = out.view(batch, seq_len, -1)
         q = packed[..., : hq * d].unflatten(-1, (hq, d))
-        k = packed[..., hq * d: (hq + hk) * d].unflatten(-1, (hk, d))
-        v = packed[..., (hq + hk) * d:].unflatten(-1, (hk, d))
+        k = packed[..., hq * d:].unflatten(-1, (hk, d))
+        v = qkv.view(batch, seq_len, -1)[..., (hq + hk) * d:].unflatten(-1, (hk, d))
         d_out = d_out if (d_out.dtype == BF16 and d_out.is_contiguous()) else d_out.to(BF16).contiguous()
-        grad = torch.empty_like(packed)                               # dq columns are produced by the rope backward from the fp32 dQ
+        grad = torch.empty_like(qkv).view(batch, seq_len, -1)          # dq columns are produced by the rope backward from the fp32 dQ
         dk = grad[..., hq * d: (hq + hk) * d].unflatten(-1, (hk, d))
         dv = grad[..., (hq + hk) * d:].unflatten(-1, (hk, d))
         dq32 = c.attn_bwd(q, k, v, o, d_out, lse, dk, dv, window, scale, softcap, ctx.doc_start)

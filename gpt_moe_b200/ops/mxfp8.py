@@ -161,14 +161,15 @@ class _MXFP8QKVAttentionFn(torch.autograd.Function):
             xq, xsf = c.mxfp8_quantize(x2)
         qkv = torch.empty((x2.shape[0], w.shape[0]), dtype=BF16, device=x.device)
         c.gemm_mxfp8(xq, xsf, wq, wsf, qkv)
-        out = torch.empty_like(qkv)
+        # rotated query and key heads; the value heads are read where the projection left them
+        out = torch.empty((qkv.shape[0], (hq + hk) * d), dtype=BF16, device=x.device)
         qs = None if q_scale is None else q_scale.detach().float().reshape(-1).contiguous()
         ks = None if k_scale is None else k_scale.detach().float().reshape(-1).contiguous()
-        c.rope_qknorm_fwd(qkv, out, cos, sin, qs, ks, seq_len, hq, hk, d, eps, rms, smin, smax, qkv.shape[-1] - (hq + hk) * d)
+        c.rope_qknorm_fwd(qkv, out, cos, sin, qs, ks, seq_len, hq, hk, d, eps, rms, smin, smax, 0)
         packed = out.view(batch, seq_len, -1)
         q = packed[..., : hq * d].unflatten(-1, (hq, d))
-        k = packed[..., hq * d: (hq + hk) * d].unflatten(-1, (hk, d))
-        v = packed[..., (hq + hk) * d:].unflatten(-1, (hk, d))
+        k = packed[..., hq * d:].unflatten(-1, (hk, d))
+        v = qkv.view(batch, seq_len, -1)[..., (hq + hk) * d:].unflatten(-1, (hk, d))
         res = c.attn_fwd(q, k, v, window, scale, softcap, doc_start, quant_out)
         o, lse = res[0], res[1]
         empty = qkv.new_empty(0)
@@ -193,10 +194,10 @@ class _MXFP8QKVAttentionFn(torch.autograd.Function):
         x_shape, x_dtype, w_shape = ctx.meta
         packed = out.view(batch, seq_len, -1)
         q = packed[..., : hq * d].unflatten(-1, (hq, d))
-        k = packed[..., hq * d: (hq + hk) * d].unflatten(-1, (hk, d))
-        v = packed[..., (hq + hk) * d:].unflatten(-1, (hk, d))
+        k = packed[..., hq * d:].unflatten(-1, (hk, d))
+        v = qkv.view(batch, seq_len, -1)[..., (hq + hk) * d:].unflatten(-1, (hk, d))
         d_out = d_out if (d_out.dtype == BF16 and d_out.is_contiguous()) else d_out.to(BF16).contiguous()
-        grad = torch.empty_like(packed)
+        grad = torch.empty_like(qkv).view(batch, seq_len, -1)
         dk = grad[..., hq * d: (hq + hk) * d].unflatten(-1, (hk, d))
         dv = grad[..., (hq + hk) * d:].unflatten(-1, (hk, d))
         dq32 = c.attn_bwd(q, k, v, o, d_out, lse, dk, dv, window, scale, softcap, ctx.doc_start)
