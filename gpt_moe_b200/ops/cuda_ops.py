@@ -132,6 +132,9 @@ class _NoGradContext:
     def mark_non_differentiable(self, *tensors) -> None:
         pass
 
+    def set_materialize_grads(self, value: bool) -> None:
+        pass
+
 
 def plain_call() -> bool:
     """No gradients are recorded and nothing intercepts autograd functions (functorch transforms, forward-mode tangents): a Function's
@@ -400,6 +403,7 @@ class _ResidualRMSNormFn(torch.autograd.Function):
         h, rstd, x_new = res[0], res[1], res[2]
         ctx.save_for_backward(x_new, w, rstd, br, b)
         ctx.meta = (beta.shape, beta.dtype, weight.dtype, beta.requires_grad)
+        ctx.set_materialize_grads(False)       # no zero-filled gradients for the quantised copies
         if quantize:                           # the MXFP8 copy of h (payload, scale records) for the projection that consumes it
             ctx.mark_non_differentiable(res[3], res[4])
             return x_new, h, res[3], res[4]
@@ -678,6 +682,7 @@ class _RouterFn(torch.autograd.Function):
         ctx.save_for_backward(lg, top_idx, counts if counts is not None else lg.new_empty(0))
         ctx.cfg = (renormalise, want_balance)
         ctx.mark_non_differentiable(top_idx)
+        ctx.set_materialize_grads(False)       # nor for the indices
         return top_idx, gates, (balance.reshape(()) if want_balance else None)
 
     @staticmethod

@@ -182,6 +182,7 @@ class _MXFP8QKVAttentionFn(torch.autograd.Function):
                             None if k_scale is None else (k_scale.shape, k_scale.dtype))
         if quant_out:                             # MXFP8 copy of the attention output, written by the kernel's epilogue
             ctx.mark_non_differentiable(res[2], res[3])
+            ctx.set_materialize_grads(False)      # no zero-filled gradients for them
             return o, res[2], res[3]
         return o, None, None
 
