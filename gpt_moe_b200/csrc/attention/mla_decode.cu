@@ -14,11 +14,12 @@
 //     registers) with its slice of the 32 latent rows, the eight partial score tiles are summed through shared memory together
 //     with the rotary part (one 16-wide slice each for the first warps), and the same slice of the tile is the value operand of
 //     its slice of the context, which stays in registers;
-//   * the queries and the probabilities are fp32 numbers and stay so: each is the sum of three bf16 numbers (8 + 8 + 8 bits of
-//     mantissa), one product each, accumulated in fp32.  The cache is bf16 and needs no splitting.
-// Measured (16 heads, rank 512): 8 sequences x 1 token over 4022 positions 20 us against 96 us for a kernel that formed the products
-// with fp32 multiply-adds and warp reductions (38 MB of cache; its merge took another 48 us, now 8 with W_v); 2 x 512 tokens over 2012
-// positions 0.80 ms against 4.84 ms.  Error of the layer's output against 64 bits: 3.8e-3 against 5.6e-3 (queries and rotation stay
+//   * queries and probabilities are fp32 numbers: each enters as two bf16 terms (16 bits of mantissa), one product each, accumulated
+//     in fp32.  The cache is bf16 and needs no splitting.  The products bound the kernel, so a third term, which moves no digit of the
+//     output's error, is left out.
+// Measured (16 heads, rank 512): 8 sequences x 1 token over 4022 positions 18 us against 96 us for a kernel that formed the products
+// with fp32 multiply-adds and warp reductions (38 MB of cache; its merge took another 48 us, now 9 with W_v); 32 x 1 over 8000 positions
+// 92 us, 3.3 TB/s.  Error of the layer's output against 64 bits: 3.8e-3 against 5.6e-3 (queries and rotation stay
 // fp32 between the projection and the scores).
 // The first kernel of the file turns projections into what the split kernel reads (and appends the new tokens to the cache); the
 // last one merges the splits by their log-sum-exp and, for the module's own use, expands the context with W_v.
@@ -30,9 +31,12 @@
 namespace gm {
 
 constexpr int MD_TILE = 32;          // cache positions per tile
+constexpr int MD_TERMS = 2;          // bf16 terms of a query or probability
 constexpr int MD_WARPS = 8;
-// ring depth by latent width (r = 128 KS): as many tiles as fit beside the score tiles
-constexpr int md_stages(int ks) { return ks <= 4 ? 4 : (ks <= 6 ? 3 : 2); }
+// One tile of rows of an up to 512-wide latent leaves room for two CTAs on an SM: every tile passes three barriers, and the other CTA's
+// products run meanwhile.  Wider latents and two tiles of rows take the SM to themselves.  Ring depth: as many tiles as fit beside the scores.
+constexpr int md_ctas(int ks, int mt) { return ks <= 4 && mt == 1 ? 2 : 1; }
+constexpr int md_stages(int ks, int mt) { return ks <= 2 ? 4 : md_ctas(ks, mt) == 2 ? 2 : ks <= 4 ? 4 : ks <= 6 ? 3 : 2; }
 constexpr int MD_ROPE_MAX = 64;
 constexpr int MD_MAX_SPLITS = 64;
 constexpr int MD_SP_PITCH = 40;      // floats per row of a partial score tile: two half-warps' rows fall on different banks
@@ -72,34 +76,24 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool v
     const int bytes = valid ? 16 : 0;
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
-// x = t0 + t1 + t2 with bf16 terms: each remainder is exact, so the sum carries the 24 bits of x
-__device__ __forceinline__ void split3(float x, float (&t)[3]) {
-    t[0] = __bfloat162float(__float2bfloat16(x));
-    const float r1 = x - t[0];
-    t[1] = __bfloat162float(__float2bfloat16(r1));
-    t[2] = r1 - t[1];
-}
-__device__ __forceinline__ void split3_pair(float x, float y, uint32_t& a, uint32_t& b, uint32_t& c) {
-    float tx[3], ty[3];
-    split3(x, tx);
-    split3(y, ty);
-    a = pack_bf16x2(tx[0], ty[0]);
-    b = pack_bf16x2(tx[1], ty[1]);
-    c = pack_bf16x2(tx[2], ty[2]);
+// x = high + low with bf16 terms, up to 2^-17 of x (the remainder after the first term is exact)
+__device__ __forceinline__ void split_pair(float x, float y, uint32_t& high, uint32_t& low) {
+    high = pack_bf16x2(x, y);
+    low = pack_bf16x2(x - __uint_as_float(high << 16), y - __uint_as_float(high & 0xffff0000u));
 }
 
 // KS = k-steps of 16 latent dimensions per warp (r = 128 * KS); MT = 16-row tiles per CTA
 template <int KS, int MT>
-__global__ void __launch_bounds__(MD_WARPS * 32, 1)
+__global__ void __launch_bounds__(MD_WARPS * 32, md_ctas(KS, MT))
 mla_decode_split_kernel(const MlaDecodeParams p) {
     extern __shared__ __align__(16) uint8_t md_smem[];
-    constexpr int r = KS * 128, MD_STAGES = md_stages(KS);
+    constexpr int r = KS * 128, MD_STAGES = md_stages(KS, MT);
     constexpr int LAT_PITCH = r * 2 + 16, ROPE_PITCH = MD_ROPE_MAX * 2 + 16;     // bytes; ldmatrix rows on different banks
     constexpr int STAGE = MD_TILE * (LAT_PITCH + ROPE_PITCH);
     constexpr int ROWS = MT * 16;
     float* sp = reinterpret_cast<float*>(md_smem + MD_STAGES * STAGE);                          // [8 warps][ROWS][MD_SP_PITCH]
-    __nv_bfloat16* pr = reinterpret_cast<__nv_bfloat16*>(sp + MD_WARPS * ROWS * MD_SP_PITCH);   // [3 terms][ROWS][MD_P_PITCH]
-    float* alpha_s = reinterpret_cast<float*>(pr + 3 * ROWS * MD_P_PITCH);                      // [ROWS]
+    __nv_bfloat16* pr = reinterpret_cast<__nv_bfloat16*>(sp + MD_WARPS * ROWS * MD_SP_PITCH);   // [MD_TERMS][ROWS][MD_P_PITCH]
+    float* alpha_s = reinterpret_cast<float*>(pr + MD_TERMS * ROWS * MD_P_PITCH);                      // [ROWS]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int split = blockIdx.x, row_group = blockIdx.y, b = blockIdx.z;
     const int total_rows = p.T * p.H;
@@ -163,8 +157,8 @@ mla_decode_split_kernel(const MlaDecodeParams p) {
     };
     for (int i = 0; i < MD_STAGES - 1; ++i) load_tile(i);
 
-    // this warp's slice of the queries as A fragments (three bf16 terms): rows g / g + 8, columns 2 tq, 2 tq + 1 and + 8
-    uint32_t qa[MT][KS][3][4], qr[MT][3][4];
+    // this warp's slice of the queries as A fragments (both terms): rows g / g + 8, columns 2 tq, 2 tq + 1 and + 8
+    uint32_t qa[MT][KS][MD_TERMS][4], qr[MT][MD_TERMS][4];
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt) {
 #pragma unroll
@@ -178,14 +172,14 @@ mla_decode_split_kernel(const MlaDecodeParams p) {
                 for (int cc = 0; cc < 2; ++cc) {
                     float2 v = *reinterpret_cast<const float2*>(p.q_latent + base * r + (warp * KS + ks) * 16 + cc * 8 + tq * 2);
                     if (!live) v = make_float2(0.f, 0.f);
-                    split3_pair(v.x, v.y, qa[mt][ks][0][cc * 2 + hf], qa[mt][ks][1][cc * 2 + hf], qa[mt][ks][2][cc * 2 + hf]);
+                    split_pair(v.x, v.y, qa[mt][ks][0][cc * 2 + hf], qa[mt][ks][1][cc * 2 + hf]);
                 }
 #pragma unroll
             for (int cc = 0; cc < 2; ++cc) {
                 const int c0 = warp * 16 + cc * 8 + tq * 2;                       // dr is even: a pair is in or out as a whole
                 float2 v = make_float2(0.f, 0.f);
                 if (live && has_rope && c0 < p.dr) v = *reinterpret_cast<const float2*>(p.q_rope + base * p.dr + c0);
-                split3_pair(v.x, v.y, qr[mt][0][cc * 2 + hf], qr[mt][1][cc * 2 + hf], qr[mt][2][cc * 2 + hf]);
+                split_pair(v.x, v.y, qr[mt][0][cc * 2 + hf], qr[mt][1][cc * 2 + hf]);
             }
         }
     }
@@ -247,7 +241,7 @@ mla_decode_split_kernel(const MlaDecodeParams p) {
 #pragma unroll
                 for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-                    for (int term = 2; term >= 0; --term) {
+                    for (int term = MD_TERMS - 1; term >= 0; --term) {
                         mma16816(sc[mt][np * 2], qa[mt][ks][term], bf[0], bf[1]);
                         mma16816(sc[mt][np * 2 + 1], qa[mt][ks][term], bf[2], bf[3]);
                     }
@@ -260,7 +254,7 @@ mla_decode_split_kernel(const MlaDecodeParams p) {
 #pragma unroll
                 for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-                    for (int term = 2; term >= 0; --term) {
+                    for (int term = MD_TERMS - 1; term >= 0; --term) {
                         mma16816(sc[mt][np * 2], qr[mt][term], bf[0], bf[1]);
                         mma16816(sc[mt][np * 2 + 1], qr[mt][term], bf[2], bf[3]);
                     }
@@ -299,11 +293,11 @@ mla_decode_split_kernel(const MlaDecodeParams p) {
             const float p0 = vis[0] ? expf(s[0] - m_new) : 0.f, p1 = vis[1] ? expf(s[1] - m_new) : 0.f;
             l[mt] = l[mt] * corr + (p0 + p1);
             m[mt] = m_new;
-            uint32_t t0, t1, t2;
-            split3_pair(p0, p1, t0, t1, t2);
+            uint32_t t0, t1;
+            split_pair(p0, p1, t0, t1);
             uint32_t* dst = reinterpret_cast<uint32_t*>(pr + (mt * 16 + srow) * MD_P_PITCH + skey);
             constexpr int term_words = ROWS * MD_P_PITCH / 2;
-            dst[0] = t0; dst[term_words] = t1; dst[2 * term_words] = t2;
+            dst[0] = t0; dst[term_words] = t1;
             if ((tid & 15) == 0) alpha_s[mt * 16 + srow] = corr;
         }
         __syncthreads();
@@ -317,11 +311,11 @@ mla_decode_split_kernel(const MlaDecodeParams p) {
         }
 #pragma unroll
         for (int ks = 0; ks < 2; ++ks) {                     // 16 positions each
-            uint32_t pa[MT][3][4];
+            uint32_t pa[MT][MD_TERMS][4];
 #pragma unroll
             for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-                for (int term = 0; term < 3; ++term)
+                for (int term = 0; term < MD_TERMS; ++term)
                     ldsm_x4(pa[mt][term], smem_u32(pr + (term * ROWS + mt * 16 + (lane & 15)) * MD_P_PITCH + ks * 16 + (lane >> 4) * 8));
 #pragma unroll
             for (int np = 0; np < KS; ++np) {                // 16 dimensions: two column tiles
@@ -330,7 +324,7 @@ mla_decode_split_kernel(const MlaDecodeParams p) {
 #pragma unroll
                 for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-                    for (int term = 2; term >= 0; --term) {
+                    for (int term = MD_TERMS - 1; term >= 0; --term) {
                         mma16816(acc[mt][np * 2], pa[mt][term], bf[0], bf[1]);
                         mma16816(acc[mt][np * 2 + 1], pa[mt][term], bf[2], bf[3]);
                     }
@@ -671,8 +665,8 @@ bool launch_rows_linear(const void* x, const void* w, void* y, int rows, int N, 
 template <int KS, int MT>
 static void launch_split(const MlaDecodeParams& p, cudaStream_t s) {
     constexpr int rows = MT * 16;
-    constexpr int smem = md_stages(KS) * MD_TILE * (KS * 256 + 16 + MD_ROPE_MAX * 2 + 16) + MD_WARPS * rows * MD_SP_PITCH * 4 + 3 * rows * MD_P_PITCH * 2 + rows * 4;
-    static_assert(smem <= 232448, "shared memory of the decode kernel");
+    constexpr int smem = md_stages(KS, MT) * MD_TILE * (KS * 256 + 16 + MD_ROPE_MAX * 2 + 16) + MD_WARPS * rows * MD_SP_PITCH * 4 + MD_TERMS * rows * MD_P_PITCH * 2 + rows * 4;
+    static_assert((smem + 1024) * md_ctas(KS, MT) <= 233472, "shared memory of the decode kernel");
     auto k = mla_decode_split_kernel<KS, MT>;
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     k<<<dim3(p.splits, (p.T * p.H + rows - 1) / rows, p.B), MD_WARPS * 32, smem, s>>>(p);
@@ -686,7 +680,10 @@ int mla_decode_splits(int B, int T, int H, int r, int S) {
     const int rows = 16 * decode_row_tiles(T, H, r);
     const int ctas = B * ((T * H + rows - 1) / rows);
     const int tiles = (S + MD_TILE - 1) / MD_TILE;
-    int want = 148 / ctas;                                  // one CTA fits an SM; a second wave would cost as much as the first
+    // one wave of CTAs, since a second would cost as much as the first: two CTAs an SM where they fit and have six tiles each, else one (8 x
+    // 4022 positions: 18 splits of 7 tiles 18.1 + 8.7 us with the merge, 37 of 4 tiles 17.2 + 11.9; 32 x 8000: 4 splits 146 us, 9 splits 92)
+    const int both = 148 * md_ctas(r / 128, rows / 16) / ctas;
+    int want = both > 0 && tiles / both >= 6 ? both : 148 / ctas;
     want = want < 1 ? 1 : (want > MD_MAX_SPLITS ? MD_MAX_SPLITS : want);
     return want < tiles ? want : (tiles < 1 ? 1 : tiles);
 }
