@@ -318,10 +318,11 @@ MlaCachedArgs mla_cached_args(const Tensor& query, const Tensor& low, const Tens
 // soft-capping, and enough queries.  The absorbed form costs by (query, position) pair, the expansion by position and some 15 us more
 // of launches.  Measured, 16 heads, rank 512, absorbed against expanded in us: sequences x new tokens over positions 1 x 64 over 2064 144 : 147,
 // 1 x 96 over 2096 179 : 150, 1 x 64 over 7064 277 : 312, 1 x 96 over 7096 357 : 314, 2 x 48 over 1548 162 : 148, 4 x 34 over 4034 329 : 332, 4 x 48 over
-// 4048 563 : 331, 1 x 128 over 228 125 : 145, 1 x 256 over 356 190 : 145; 2 x 512 over 2012 1193 : 160.
+// 4048 563 : 331, 1 x 128 over 228 125 : 145, 1 x 256 over 356 190 : 145; 2 x 512 over 2012 1193 : 160.  The expansion holds 1 KB per position and
+// kv head (4 GB at the limit for 16 heads); longer calls stay absorbed.
 bool mla_prefill_wanted(int64_t B, int64_t T, int64_t end, int64_t window, int64_t r, int64_t dr, int64_t content, int64_t value, double softcap) {
     const int64_t visible = window < 0 ? end : std::min(end, window + T);
-    return T >= 48 && B * T >= 96 && B * T * visible >= 90000 && r % 64 == 0 && dr == 64 && content == 64 && value == 64 && softcap <= 0.0;
+    return T >= 48 && B * T >= 96 && B * T * visible >= 90000 && B * visible <= 262144 && r % 64 == 0 && dr == 64 && content == 64 && value == 64 && softcap <= 0.0;
 }
 
 Tensor mla_prefill(const MlaCachedArgs& args, const Tensor& latent, const Tensor& terms) {

@@ -211,7 +211,7 @@ class MLAttention(nn.Module):
         b, t, hidden = x.shape
         caches = (cache.latent, cache.rope, cache.key_gain)
         w_up = self.kv_up_proj.weight
-        if not (x.is_cuda and self.rotary is not None and t > 0 and all(c.dtype == torch.bfloat16 and c.is_cuda and c.stride(2) == 1
+        if not (x.is_cuda and self.rotary is not None and 0 < b * t <= 131072 and all(c.dtype == torch.bfloat16 and c.is_cuda and c.stride(2) == 1
                 and c.stride(1) == c.size(2) for c in caches) and all(m.bias is None for m in (self.q_proj, self.kv_down_proj, self.kv_up_proj))
                 and w_up.dtype == torch.float32 and w_up.is_contiguous() and w_up.data_ptr() % 16 == 0 and self.content_dim <= 256
                 and (self.softcap <= 0.0 or self.tanh_backend == "exact") and start + t <= self.rotary.cos_cached.shape[0]
