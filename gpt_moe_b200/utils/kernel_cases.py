@@ -25,7 +25,7 @@ def _timed(fn, iters):
 
 def main() -> None:
     ap = argparse.ArgumentParser()
-    ap.add_argument("case", choices=["gemm", "gemm_mxfp8", "quantize", "gemm_wgrad", "grouped", "attn_fwd", "attn_fwd_full", "attn_bwd", "attn_bwd_full", "rs_muon", "ce", "rmsnorm", "rope", "rope_bwd", "ep_dispatch", "ep_combine", "rmsnorm_bwd", "attn_fwd_mla", "attn_bwd_mla", "gemm_xxt", "gemm_xxt_full", "polar", "gemm_big", "gemm_mxfp8_big", "gemm_mxfp8_down", "quantize_weight", "mma_issue"])
+    ap.add_argument("case", choices=["gemm", "gemm_mxfp8", "quantize", "gemm_wgrad", "grouped", "attn_fwd", "attn_fwd_full", "attn_bwd", "attn_bwd_full", "rs_muon", "ce", "rmsnorm", "rope", "rope_bwd", "ep_dispatch", "ep_combine", "rmsnorm_bwd", "attn_fwd_mla", "attn_bwd_mla", "gemm_xxt", "gemm_xxt_full", "polar", "gemm_big", "gemm_mxfp8_big", "gemm_mxfp8_down", "quantize_weight", "gemm_addend", "mla_decode", "mma_issue"])
     ap.add_argument("--iters", type=int, default=3)
     ap.add_argument("--single-tile", action="store_true", help="attention: the basic kernels (one query tile per CTA forward, unpipelined backward)")
     args = ap.parse_args()
@@ -123,6 +123,18 @@ def main() -> None:
         a = torch.empty(96, 768, 768, device=dev, dtype=torch.bfloat16)
         fn = lambda: c.gemm_bf16(x, x, a, symmetric=args.case == "gemm_xxt")
         flops = 2 * 96 * 768 * 768 * 6144                 # of the full product: the symmetric form does two thirds of it
+    elif args.case == "gemm_addend":             # Polar Express' B X + a X for 96 matrices [768, 6144], the addend fetched by TMA
+        b = torch.randn(96, 768, 768, device=dev).mul_(0.03).bfloat16()
+        x = torch.randn(96, 768, 6144, device=dev).bfloat16()
+        y = torch.empty_like(x)
+        fn = lambda: c.gemm_bf16(b, x, y, False, True, 1.0, 0.3, x)
+        flops = 2 * 96 * 768 * 768 * 6144
+    elif args.case == "mla_decode":              # one token for 32 sequences over 8000 latent positions, 16 heads, rank 512
+        q, qr = torch.randn(32, 1, 16, 512, device=dev) * 0.05, torch.randn(32, 1, 16, 64, device=dev)
+        latent, rope = (torch.randn(32, 8000, n, device=dev).bfloat16() for n in (512, 64))
+        gain = torch.rand(32, 8000, 16, device=dev).bfloat16()
+        fn = lambda: c.mla_decode(q, qr, latent, rope, gain, 7999, 0.09, 0.0, -1)
+        bytes_ = 32 * 8000 * (512 + 64 + 16) * 2
     elif args.case == "polar":                   # five Polar Express iterations on the same batch
         x = torch.randn(96, 768, 6144, device=dev)
         x = (x / (x.norm(dim=(-2, -1), keepdim=True) * 1.02 + 1e-6)).bfloat16()
