@@ -19,10 +19,15 @@ __device__ __forceinline__ float ex2_approx(float x) {
 }
 
 // One block per row.  loss[row] = logsumexp(logits) - logits[target]; logits are overwritten by
-// (softmax - onehot) * (*grad_scale) in bf16, zeros for ignored rows.  64-bit row offsets.
+// (softmax - onehot) * (*grad_scale) in bf16, zeros for ignored rows.  64-bit row offsets.  A target that is neither a class nor
+// `ignore_index` is no address: the row's loss becomes NaN, its gradient zero, and the status word says so.
+__device__ __forceinline__ bool outside(long long tgt, int vocab, long long ignore_index) {
+    return tgt != ignore_index && (tgt < 0 || tgt >= vocab);
+}
+
 __global__ void __launch_bounds__(512)
 ce_fwd_bwd_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ targets, float* __restrict__ loss,
-                  const float* __restrict__ grad_scale, int vocab, long long row_stride, long long ignore_index, int write_grad) {
+                  const float* __restrict__ grad_scale, int vocab, long long row_stride, long long ignore_index, int write_grad, int* status) {
     __shared__ float red_m[16], red_s[16];
     const long long row = blockIdx.x;
     __nv_bfloat16* p = logits + row * row_stride;
@@ -30,8 +35,12 @@ ce_fwd_bwd_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restric
     if (!GM_IN_BOUNDS(tgt == ignore_index || (tgt >= 0 && tgt < vocab), 905)) tgt = ignore_index;      // checked build: the row is ignored
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     const int vec = vocab / 8;
-    if (tgt == ignore_index) {
-        if (threadIdx.x == 0) loss[row] = 0.f;
+    const bool bad = outside(tgt, vocab, ignore_index);
+    if (tgt == ignore_index || bad) {
+        if (threadIdx.x == 0) {
+            loss[row] = bad ? __int_as_float(0x7fc00000) : 0.f;
+            if (bad) atomicExch(status, 701);
+        }
         if (write_grad) {
             for (int i = threadIdx.x; i < vec; i += blockDim.x) reinterpret_cast<uint4*>(p)[i] = make_uint4(0, 0, 0, 0);
             for (int i = vec * 8 + threadIdx.x; i < vocab; i += blockDim.x) p[i] = __float2bfloat16(0.f);
@@ -108,8 +117,12 @@ ce_fwd_bwd_bulk_kernel(__nv_bfloat16* __restrict__ logits, const long long* __re
     if (!GM_IN_BOUNDS(tgt == ignore_index || (tgt >= 0 && tgt < vocab), 905)) tgt = ignore_index;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int vec = vocab / 8;
-    if (tgt == ignore_index) {
-        if (threadIdx.x == 0) loss[row] = 0.f;
+    const bool bad = outside(tgt, vocab, ignore_index);
+    if (tgt == ignore_index || bad) {
+        if (threadIdx.x == 0) {
+            loss[row] = bad ? __int_as_float(0x7fc00000) : 0.f;
+            if (bad) atomicExch(status, 701);
+        }
         if (write_grad)
             for (int i = threadIdx.x; i < vec; i += CE_THREADS) reinterpret_cast<uint4*>(p)[i] = make_uint4(0, 0, 0, 0);
         return;
@@ -221,7 +234,7 @@ void launch_ce_fwd_bwd(void* logits, const long long* targets, float* loss, cons
         return;
     }
     ce_fwd_bwd_kernel<<<rows, 512, 0, s>>>(static_cast<__nv_bfloat16*>(logits), targets, loss, grad_scale, vocab, row_stride,
-                                           ignore_index, write_grad);
+                                           ignore_index, write_grad, status);
 }
 
 // ---- log-probabilities of given tokens from logits that somebody else keeps ------------------------------------------------
@@ -293,10 +306,11 @@ row_nll_kernel(const __nv_bfloat16* __restrict__ logits, const long long* __rest
                long long row_stride, int vec16, long long ignore_index, int* status) {
     const long long row = blockIdx.x;
     const long long tgt = targets[row];
-    if (tgt == ignore_index || tgt < 0 || tgt >= vocab) {
+    const bool bad = outside(tgt, vocab, ignore_index);
+    if (tgt == ignore_index || bad) {
         if (threadIdx.x == 0) {
-            loss[row] = tgt == ignore_index ? 0.f : __int_as_float(0x7fc00000);
-            if (tgt != ignore_index) atomicExch(status, 701);
+            loss[row] = bad ? __int_as_float(0x7fc00000) : 0.f;
+            if (bad) atomicExch(status, 701);
         }
         return;
     }

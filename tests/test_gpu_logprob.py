@@ -33,6 +33,25 @@ def test_target_outside_the_vocabulary_is_reported():
         cuda_ops.check_status()
 
 
+@pytest.mark.parametrize("vocab", [64, 56960, 60000, 1003])           # rows in shared memory up to 56960 columns, streamed beyond and for odd widths
+@pytest.mark.parametrize("bad", [-1, 0, 7, 1 << 20, -(1 << 40), (1 << 62)])          # distance from the vocabulary's end; negative: from its start
+def test_target_outside_the_vocabulary_in_the_training_loss(vocab, bad):
+    if cuda_ops.ext().bounds_checked():
+        pytest.skip("the bounds-checked build ignores such a row and records code 905")
+    torch.manual_seed(6)
+    logits = torch.randn(4, (vocab + 7) // 8 * 8, device="cuda").bfloat16()[:, :vocab]
+    targets = torch.randint(0, vocab, (4,), device="cuda")
+    targets[1] = bad if bad < 0 else vocab + bad
+    before = logits.double()
+    loss = cuda_ops.ext().ce_fwd_bwd(logits, targets, torch.ones(1, device="cuda"), -100, True)
+    keep = torch.tensor([0, 2, 3], device="cuda")
+    want = torch.nn.functional.cross_entropy(before[keep], targets[keep], reduction="none")
+    assert torch.isnan(loss[1]) and torch.allclose(loss[keep].double(), want, rtol=1e-5, atol=1e-5)
+    assert (logits[1] == 0).all() and (logits[keep] != 0).any(dim=1).all()
+    with pytest.raises(RuntimeError, match="701"):
+        cuda_ops.check_status()
+
+
 def test_gradients_still_run_through_torch():
     logits = torch.randn(4, 64, device="cuda").bfloat16().requires_grad_()
     cuda_ops.cross_entropy(logits, torch.tensor([1, 2, 3, 4], device="cuda"), -100).backward()
