@@ -249,7 +249,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         const float c = p.scale_log2e;
         constexpr bool capped = CAPPED;
         const float cap_a = capped ? p.softcap / p.scale : 0.f, cap_b = capped ? p.scale / p.softcap : 0.f;
-        for (int it = 0; it < n_iter && ok; ++it) {
+        for (int it = 0; it < n_iter; ++it) {
             const uint32_t ph = it & 1;
             const int head = kv_head * p.group + it / n_q;
             const int q0 = (kv_tile + it % n_q) * TILE;
@@ -266,7 +266,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
                 w_last = min(window, last - p.doc_start[row0 + last]);
             }
             const bool need_mask = (q0 == kv0) || (q0 + TILE - 1 - kv0 > w_last);
-            if (!mbar_wait(bar_sdp, ph)) { atomicExch(p.status, 305); ok = false; break; }
+            if (ok && !mbar_wait(bar_sdp, ph)) { atomicExch(p.status, 305); ok = false; }
             tc_fence_after();
             if (WIDE) {                      // the previous dQ reduce-add must have finished reading the P / dS tiles it was staged in
                 if (leader) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
@@ -283,7 +283,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
             tc_fence_before();
             fence_proxy_async();
             mbar_arrive(bar_pds);
-            if (!mbar_wait(bar_mma, ph)) { atomicExch(p.status, 306); ok = false; break; }
+            if (ok && !mbar_wait(bar_mma, ph)) { atomicExch(p.status, 306); ok = false; }
             tc_fence_after();
             // dQ tile: this thread's row, half of the DQK columns; scaled, staged, then one TMA reduce-add per 32-column slab
             uint32_t qreg[DQK / 64][32];

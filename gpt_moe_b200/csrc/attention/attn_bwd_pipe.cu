@@ -216,8 +216,8 @@ attn_bwd_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         const float cap_a = capped ? p.softcap / p.scale : 0.f, cap_b = capped ? p.scale / p.softcap : 0.f;
         const uint32_t s_addr = tmem_base + BP_COL_S + lane_off + half * 64, dp_addr = tmem_base + BP_COL_DP + lane_off + half * 64;
         // dQ of iteration `jt`: this thread's row, 32 of the 64 columns; scaled, staged, then one TMA reduce-add per 32-column slab
-        auto drain_dq = [&](int jt) -> bool {
-            if (!mbar_wait(bar_mma, jt & 1)) return false;
+        auto drain_dq = [&](int jt) {
+            if (ok && !mbar_wait(bar_mma, jt & 1)) { atomicExch(p.status, 306); ok = false; }
             tc_fence_after();
             uint32_t qreg[32];
             tmem_ld_32x32b_x32(tmem_base + BP_COL_DQ + lane_off + half * 32, qreg);
@@ -243,7 +243,6 @@ attn_bwd_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
                 }
                 asm volatile("cp.async.bulk.commit_group;" ::: "memory");
             }
-            return true;
         };
         // statistics of this thread's query row of iteration `jt`, [batch, head, seq].  Rows past the sequence end are zeros; an
         // infinite log-sum-exp makes their probabilities 0
@@ -257,7 +256,7 @@ attn_bwd_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
             delta_next = live ? p.delta[stat] : 0.f;
         };
         if (n_iter > 0) fetch_stats(0);
-        for (int it = 0; it < n_iter && ok; ++it) {
+        for (int it = 0; it < n_iter; ++it) {
             const uint32_t ph = it & 1;
             const int head = kv_head * p.group + it / n_q;
             const int q0 = (kv_tile + it % n_q) * BP_TILE;
@@ -274,7 +273,7 @@ attn_bwd_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
                 w_last = min(window, last - p.doc_start[row0 + last]);
             }
             const bool need_mask = (q0 == kv0) || (q0 + BP_TILE - 1 - kv0 > w_last);
-            if (!mbar_wait(bar_sdp, ph)) { atomicExch(p.status, 305); ok = false; break; }
+            if (ok && !mbar_wait(bar_sdp, ph)) { atomicExch(p.status, 305); ok = false; }
             tc_fence_after();
             uint4 wp[8], wd[8];
             if (need_mask) bp_tile_math<true, capped>(s_addr, dp_addr, wp, wd, kv0 + half * 64, qpos, w_row, c, lse2, delta, cap_a, cap_b);
@@ -282,7 +281,7 @@ attn_bwd_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
             tc_fence_before();
             mbar_arrive(bar_sread);                                       // S / dP of the next iteration may be written
             // the gradient products of the previous iteration read the P / dS tiles: wait for them, and drain their dQ
-            if (it > 0 && !drain_dq(it - 1)) { atomicExch(p.status, 306); ok = false; break; }
+            if (it > 0) drain_dq(it - 1);
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const int piece = (j ^ sw) << 4;
@@ -292,7 +291,7 @@ attn_bwd_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
             fence_proxy_async();
             mbar_arrive(bar_pds);
         }
-        if (ok && n_iter > 0 && !drain_dq(n_iter - 1)) { atomicExch(p.status, 306); ok = false; }
+        if (n_iter > 0) drain_dq(n_iter - 1);
         if (ok && n_iter > 0) {
             // dK, dV: TMEM lanes are the 128 keys of this CTA; each thread writes half of the columns of its key row
             const bool live = kv0 + r < p.seq_len;

@@ -226,10 +226,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 #pragma unroll
         for (int i = 0; i < AT_D / 2; ++i) o[i] = 0.f;
         const int bar_id = 1 + quad;                             // pairs (w, w+4) meet on their own named barrier
-        for (int j = 0; j < n_tiles && ok; ++j) {
+        for (int j = 0; j < n_tiles; ++j) {
             const uint32_t ph = j & 1;
             const int kv0 = kv_lo + j * AT_BN + half * 64;
-            if (!mbar_wait(bar_s, ph)) { atomicExch(p.status, 206); ok = false; break; }
+            if (ok && !mbar_wait(bar_s, ph)) { atomicExch(p.status, 206); ok = false; }
             tc_fence_after();
             // tiles strictly inside the band need no mask; the diagonal tile and the tile(s) at the window edge do
             const int tile0 = kv_lo + j * AT_BN;
@@ -249,7 +249,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
             m = m_new;
             tc_fence_before();
             mbar_arrive(bar_p);
-            if (!mbar_wait(bar_o, ph)) { atomicExch(p.status, 207); ok = false; break; }
+            if (ok && !mbar_wait(bar_o, ph)) { atomicExch(p.status, 207); ok = false; }
             tc_fence_after();
             {
                 uint32_t oreg[32];
@@ -261,11 +261,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
             tc_fence_before();
             asm volatile("bar.sync %0, 64;" ::"r"(bar_id) : "memory");     // partner has read this tile's maximum
         }
-        if (ok) {
-            row_stat[half * AT_BM + r] = l;
-            asm volatile("bar.sync %0, 64;" ::"r"(bar_id) : "memory");
-            l += row_stat[(half ^ 1) * AT_BM + r];
-        }
+        row_stat[half * AT_BM + r] = l;
+        asm volatile("bar.sync %0, 64;" ::"r"(bar_id) : "memory");
+        l += row_stat[(half ^ 1) * AT_BM + r];
         if (ok && live) {
             const float inv = 1.f / l;
             const long long token = static_cast<long long>(row0) + qpos;

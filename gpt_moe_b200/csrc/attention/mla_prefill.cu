@@ -265,11 +265,11 @@ mla_prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const _
         float m = -INFINITY, l = 0.f, o[32];
 #pragma unroll
         for (int i = 0; i < 32; ++i) o[i] = 0.f;
-        for (int j = 0; j < n_tiles && ok; ++j) {
+        for (int j = 0; j < n_tiles; ++j) {
             const uint32_t ph = j & 1;
             const int tile0 = lo + j * PF_N, kv0 = tile0 + half * 64;
             const float* gain = p.gain + (static_cast<long long>(batch) * (p.H / p.group) + kv_head) * p.S_pad + kv0;
-            if (!mbar_wait(bar_s, ph)) { atomicExch(p.status, 236); ok = false; break; }
+            if (ok && !mbar_wait(bar_s, ph)) { atomicExch(p.status, 236); ok = false; }
             tc_fence_after();
             const bool need_mask = tile0 + PF_N - 1 > first_pos || first_pos + PF_M - 1 - tile0 > window;
             float v[64];
@@ -325,7 +325,7 @@ mla_prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const _
             m = m_new;
             tc_fence_before();
             mbar_arrive(bar_p);
-            if (!mbar_wait(bar_o, ph)) { atomicExch(p.status, 237); ok = false; break; }
+            if (ok && !mbar_wait(bar_o, ph)) { atomicExch(p.status, 237); ok = false; }
             tc_fence_after();
             {
                 uint32_t oreg[32];
@@ -337,11 +337,9 @@ mla_prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const _
             tc_fence_before();
             asm volatile("bar.sync %0, 64;" ::"r"(bar_id) : "memory");         // partner has read this tile's maximum
         }
-        if (ok) {
-            row_stat[half * PF_M + r] = l;
-            asm volatile("bar.sync %0, 64;" ::"r"(bar_id) : "memory");
-            l += row_stat[(half ^ 1) * PF_M + r];
-        }
+        row_stat[half * PF_M + r] = l;
+        asm volatile("bar.sync %0, 64;" ::"r"(bar_id) : "memory");
+        l += row_stat[(half ^ 1) * PF_M + r];
         if (ok && live) {
             const float inv = 1.f / l;
             __nv_bfloat16* out = p.out + (static_cast<long long>(batch) * p.T + q0 + r) * p.H * 64 + head * 64 + half * 32;

@@ -4,6 +4,9 @@
 // Waiting policy: no wait in this code base is unbounded.  `mbar_wait` polls with a cycle budget
 // and returns false when it runs out; the caller records a code in the kernel's status word,
 // stops issuing work and falls through to the common teardown (TMEM is always freed).
+// Threads that meet at a barrier (`bar.sync`, __syncthreads) do not leave their loop when a wait gives up, since the budget of
+// each starts when it begins to wait and one may give up where another is still served: they go on without waiting
+// (`if (ok && !mbar_wait(..)) ok = false;`), so that every one of them passes every barrier, and the results are void.
 #pragma once
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>

@@ -229,6 +229,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         const int row_in_tile = quad * 32 + lane;
         const bool leader = threadIdx.x == 64;
         const int sw = row_in_tile & 7;
+        // A thread whose wait gives up goes on through the loops without waiting (see mbar_wait in ptx.cuh): the 256 threads meet at named
+        // barriers, and one that left would keep the others there for good
         int acc = 0; uint32_t acc_ph = 0;
         uint32_t use = 0, fetched = 0;                             // slabs handed to a store so far; slabs of C consumed so far
         auto fetch_c = [&](const TileCoord& t, int round, uint32_t slab, uint32_t k) {
@@ -236,7 +238,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             tma_load_3d(staging + (slab & 3) * SLAB_BYTES, &tmap_c, &c_full[k & 1], t.n0 + round * 64, t.m0, t.dz);
         };
         if (leader && first_tile < tiles) fetch_c(tile_coord(p, first_tile, cta_rank, m_tiles, n_tiles), 0, 0, 0);
-        for (int tile = first_tile; tile < tiles && ok; tile += tile_step) {
+        for (int tile = first_tile; tile < tiles; tile += tile_step) {
             const TileCoord t = tile_coord(p, tile, cta_rank, m_tiles, n_tiles);
             const int rounds = min(BN / 64, (t.n_limit - t.n0 + 63) / 64);
             float alpha = p.alpha, beta = p.beta;
@@ -246,10 +248,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                 else { alpha *= inv; beta *= inv; }
             }
             const bool mirror = p.symmetric && t.n0 != t.m0 - cta_rank * BM;
-            if (!mbar_wait(&acc_full[acc], acc_ph)) { atomicExch(p.status, 104); ok = false; break; }
+            if (ok && !mbar_wait(&acc_full[acc], acc_ph)) { atomicExch(p.status, 104); ok = false; }
             tc_fence_after();
             for (int round = 0; round < rounds; ++round) {
-                if (leader) {
+                if (leader && ok) {                                    // a barrier that was given up is not armed again
                     // at most the latest store still reads its slab: the one before it, whose slab comes next at the earliest, is done
                     asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
                     const uint32_t next = use + (mirror ? 2 : 1);
@@ -264,7 +266,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                     __syncwarp();
                     if (lane == 0) mbar_arrive_cluster(&acc_empty[acc], 0);
                 }
-                if (!mbar_wait(&c_full[fetched & 1], (fetched >> 1) & 1)) { atomicExch(p.status, 105); ok = false; break; }
+                if (ok && !mbar_wait(&c_full[fetched & 1], (fetched >> 1) & 1)) { atomicExch(p.status, 105); ok = false; }
                 uint8_t* slab = staging + (use & 3) * SLAB_BYTES;
                 uint8_t* slab_row = slab + row_in_tile * 128;
 #pragma unroll
@@ -319,7 +321,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                     ++use;
                 }
             }
-            if (!ok) break;
             if (++acc == 2) { acc = 0; acc_ph ^= 1; }
         }
         if (leader) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
@@ -339,7 +340,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         const int sw = row_in_tile & 7;
         int acc = 0; uint32_t acc_ph = 0;
         uint32_t stores = 0;                                       // committed store groups: selects the staging buffer
-        for (int tile = first_tile; tile < tiles && ok; tile += tile_step) {
+        for (int tile = first_tile; tile < tiles; tile += tile_step) {
             const TileCoord t = tile_coord(p, tile, cta_rank, m_tiles, n_tiles);
             const bool have_acc = t.k_blocks != 0;
             if (!have_acc && !(t.store_zeros && !p.accumulate)) continue;      // nothing to add, nothing to clear
@@ -353,7 +354,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             }
             const bool mirror = p.symmetric && t.n0 != t.m0 - cta_rank * BM;      // off-diagonal pair tile (uniform across the pair)
             if (have_acc) {
-                if (!mbar_wait(&acc_full[acc], acc_ph)) { atomicExch(p.status, 104); ok = false; break; }
+                if (ok && !mbar_wait(&acc_full[acc], acc_ph)) { atomicExch(p.status, 104); ok = false; }
                 tc_fence_after();
             }
             for (int round = 0; round < rounds; ++round) {

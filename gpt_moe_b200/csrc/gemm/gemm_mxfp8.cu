@@ -185,9 +185,9 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         const int sw = row_in_tile & 7;
         uint32_t acc_ph = 0;
         uint32_t stores = 0;
-        for (int tile = first_tile; tile < tiles && ok; tile += tile_step) {
+        for (int tile = first_tile; tile < tiles; tile += tile_step) {
             const FTile t = f_tile(p, tile, cta_rank, m_pairs, n_tiles);
-            if (!mbar_wait(acc_full, acc_ph)) { atomicExch(p.status, 404); ok = false; break; }
+            if (ok && !mbar_wait(acc_full, acc_ph)) { atomicExch(p.status, 404); ok = false; }
             tc_fence_after();
             acc_ph ^= 1;
             uint32_t r[2][2][32];                                  // [round][chunk of this half][column]

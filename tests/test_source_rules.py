@@ -74,6 +74,35 @@ def test_every_open_ended_loop_in_a_kernel_has_a_budget():
     assert not bad, bad
 
 
+def _roles(text):
+    """(first line, text) of every branch that directly follows `if (warp ...` or an `else` of it in the body of a kernel."""
+    for m in re.finditer(r"^ {4}(?:if \(warp[^\n]*|\} else[^\n]*)\{\n", text, re.M):
+        end = re.search(r"^ {4}\}", text[m.end():], re.M)
+        yield text.count("\n", 0, m.end()) + 1, text[m.end(): m.end() + end.start()]
+
+
+def _leaves_waiting_threads(role):
+    """Lines on which a thread of a role that meets at named barriers leaves a loop or a function because a wait gave up."""
+    if "bar.sync" not in role and not re.search(r"bar_id", role):
+        return []
+    return [n for n, line in enumerate(role.splitlines())
+            if ("mbar_wait" in line and re.search(r"\bbreak\b|\breturn\b", line)) or re.search(r"for \([^\n]*&& ok;|if \(!ok\) (break|return)|if \(ok\) \{", line)]
+
+
+def test_threads_that_meet_at_a_barrier_stay_when_a_wait_gives_up():
+    """The budget of a wait starts when the thread begins to wait, so one thread can give up where its neighbour is still served.  If it left,
+    the neighbour would stand at the next `bar.sync` for good: roles with named barriers go on without waiting instead."""
+    assert _leaves_waiting_threads('for (int i = 0; i < n && ok; ++i) {\nif (!mbar_wait(b, 0)) { ok = false; break; }\nasm("bar.sync 1, 256;");\n}') == [0, 1]
+    bad, seen = [], 0
+    for path in _native_sources():
+        if not path.endswith(".cu"):
+            continue
+        for first, role in _roles(open(path).read()):
+            seen += "bar.sync" in role
+            bad += [f"{path}:{first + n}" for n in _leaves_waiting_threads(role)]
+    assert seen >= 6 and not bad, (seen, bad)
+
+
 def test_profile_commands_leave_the_clocks_alone():
     folder = os.path.join(ROOT, "profiles")
     bad = []
