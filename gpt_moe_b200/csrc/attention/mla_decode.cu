@@ -7,8 +7,8 @@
 // Every head of a token reads the same latent rows (keys and values are both the latent cache), so one token's heads are the
 // rows of a 16-row matrix product and the kernel should be bound by reading the cache once.  tcgen05 has no tile with fewer than
 // 64 rows (48 of them would be padding), so the products are warp-level m16n8k16 instructions:
-//   * grid = (splits of the cache, groups of MT * 16 rows, batch); a row is a (token, head) pair, token-major, so 16 heads make
-//     one token a tile of rows;
+//   * a CTA per split of the cache (fastest), group of MT * 16 rows and sequence; a row is a (token, head) pair, token-major, so 16
+//     heads make one token a tile of rows.  All grids of the file are one-dimensional: rows and sequences may number more than 65535;
 //   * a CTA walks its share of the cache in tiles of 32 positions that arrive through a cp.async ring;
 //   * warp w owns the latent dimensions [w r/8, (w+1) r/8) for both products: it multiplies its slice of the queries (held in
 //     registers) with its slice of the 32 latent rows, the eight partial score tiles are summed through shared memory together
@@ -95,8 +95,9 @@ mla_decode_split_kernel(const MlaDecodeParams p) {
     __nv_bfloat16* pr = reinterpret_cast<__nv_bfloat16*>(sp + MD_WARPS * ROWS * MD_SP_PITCH);   // [MD_TERMS][ROWS][MD_P_PITCH]
     float* alpha_s = reinterpret_cast<float*>(pr + MD_TERMS * ROWS * MD_P_PITCH);                      // [ROWS]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int split = blockIdx.x, row_group = blockIdx.y, b = blockIdx.z;
-    const int total_rows = p.T * p.H;
+    const int total_rows = p.T * p.H, row_groups = (total_rows + ROWS - 1) / ROWS;
+    const int split = blockIdx.x % p.splits, group_of_all = blockIdx.x / p.splits;
+    const int b = group_of_all / row_groups, row_group = group_of_all - b * row_groups;
     const int row_base = row_group * ROWS;
     const int t_first = row_base / p.H, t_last = min(row_base + ROWS - 1, total_rows - 1) / p.H;
     const int hi_max = min(p.S - 1, p.start + t_last);                                          // last position any row sees
@@ -397,7 +398,7 @@ mla_decode_values_kernel(const float* __restrict__ part_ctx, const float* __rest
     constexpr int r = NV * 128;
     __shared__ float factor[TB][MD_MAX_SPLITS];
     __shared__ __align__(16) float ctx_s[TB][r];
-    const int h = blockIdx.x, tok0 = blockIdx.y * TB;
+    const int h = blockIdx.x % H, tok0 = blockIdx.x / H * TB;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int tb = warp; tb < TB; tb += 8)
         if (tok0 + tb < tokens) merge_factors(part_ml + (static_cast<long long>(tok0 + tb) * H + h) * splits * 2, splits, factor[tb], lane);
@@ -474,7 +475,7 @@ mla_prepare_kernel(const MlaPrepareParams p) {
     float* red_s = lat_s + TB * r;                            // [8 warps][TB][r]
     float* q_s = red_s + 8 * TB * r;                          // [TB][content]
     __shared__ float ksq_s[8][TB], rsq_s[TB];
-    const int kvh = blockIdx.x, tok0 = blockIdx.y * TB;
+    const int kvh = blockIdx.x % p.Hkv, tok0 = blockIdx.x / p.Hkv * TB;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int group = p.H / p.Hkv, head_w = p.content + p.dr;
 
@@ -669,7 +670,7 @@ static void launch_split(const MlaDecodeParams& p, cudaStream_t s) {
     static_assert((smem + 1024) * md_ctas(KS, MT) <= 233472, "shared memory of the decode kernel");
     auto k = mla_decode_split_kernel<KS, MT>;
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    k<<<dim3(p.splits, (p.T * p.H + rows - 1) / rows, p.B), MD_WARPS * 32, smem, s>>>(p);
+    k<<<static_cast<unsigned>(p.splits) * ((p.T * p.H + rows - 1) / rows) * p.B, MD_WARPS * 32, smem, s>>>(p);
 }
 
 // 16-row tiles per CTA: two when there are tiles to share a pass over the cache (a CTA then does twice the products per byte), but
@@ -697,6 +698,7 @@ static bool launch_decode_split(const float* q_latent, const float* q_rope, cons
                                 long long latent_bs, long long rope_bs, long long gain_bs, float* part_ctx, float* part_ml, int B, int T, int H, int Hkv,
                                 int r, int dr, int S, int splits, int start, int window, float scale, float softcap, cudaStream_t s) {
     if (!mla_decode_supported(H, Hkv, r, dr) || B <= 0 || T <= 0 || S <= 0 || splits < 1 || splits > MD_MAX_SPLITS) return false;
+    if (static_cast<long long>(B) * T * H * splits >= (1LL << 31)) return false;            // an upper bound of every grid of a call
     MlaDecodeParams p;
     p.q_latent = q_latent; p.q_rope = q_rope;
     p.latent = static_cast<const __nv_bfloat16*>(latent); p.rope = static_cast<const __nv_bfloat16*>(rope);
@@ -730,7 +732,7 @@ static void launch_prepare(const MlaPrepareParams& p, cudaStream_t s) {
     const size_t smem = (static_cast<size_t>(9) * TB * NV * 128 + static_cast<size_t>(TB) * p.content) * 4;
     auto k = mla_prepare_kernel<NV, TB>;
     if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    k<<<dim3(p.Hkv, (p.tokens + TB - 1) / TB), 256, smem, s>>>(p);
+    k<<<static_cast<unsigned>(p.Hkv) * ((p.tokens + TB - 1) / TB), 256, smem, s>>>(p);
 }
 
 template <int NV>
@@ -743,9 +745,9 @@ static void launch_cached(const MlaPrepareParams& p, bool many, const float* par
     }
     const int group = p.H / p.Hkv;
     if (many)
-        mla_decode_values_kernel<NV, TB><<<dim3(p.H, (p.tokens + TB - 1) / TB), 256, 0, s>>>(part_ctx, part_ml, p.w_up, out, p.tokens, p.H, group, p.content, p.value, splits);
+        mla_decode_values_kernel<NV, TB><<<static_cast<unsigned>(p.H) * ((p.tokens + TB - 1) / TB), 256, 0, s>>>(part_ctx, part_ml, p.w_up, out, p.tokens, p.H, group, p.content, p.value, splits);
     else
-        mla_decode_values_kernel<NV, 1><<<dim3(p.H, p.tokens), 256, 0, s>>>(part_ctx, part_ml, p.w_up, out, p.tokens, p.H, group, p.content, p.value, splits);
+        mla_decode_values_kernel<NV, 1><<<static_cast<unsigned>(p.H) * p.tokens, 256, 0, s>>>(part_ctx, part_ml, p.w_up, out, p.tokens, p.H, group, p.content, p.value, splits);
 }
 
 bool launch_mla_cached(const MlaCachedArgs& a, cudaStream_t s) {

@@ -22,6 +22,10 @@ const float* fptr(const OptTensor& t) { return t.has_value() ? t->data_ptr<float
 void check_bf16(const Tensor& t, const char* name) {
     GM_CHECK(t.is_cuda() && t.scalar_type() == torch::kBFloat16 && t.is_contiguous(), std::string(name) + " must be a contiguous CUDA bf16 tensor");
 }
+void check_launch(const char* what) {
+    const cudaError_t e = cudaGetLastError();
+    GM_CHECK(e == cudaSuccess, std::string(what) + ": " + cudaGetErrorString(e));
+}
 // MXFP8 copy of a [rows, cols] matrix: e4m3 payload (uint8 [rows, cols]) and scale records (uint8 [ceil(rows/128) * ceil(cols/128) * 512]).
 // The scale array is not cleared: every byte that belongs to a row the producer writes is written by it, the others belong to
 // rows the GEMM clips.
@@ -257,6 +261,7 @@ Tensor mla_decode(const Tensor& q_latent, const Tensor& q_rope, const Tensor& la
                                latent.stride(0), rope.stride(0), key_gain.stride(0), part_ctx.data_ptr<float>(), part_ml.data_ptr<float>(),
                                context.data_ptr<float>(), B, T, H, Hkv, r, dr, S, splits, start, window, static_cast<float>(scale),
                                static_cast<float>(softcap), stream()), "mla_decode: unsupported shape");
+    check_launch("mla_decode");
     return context;
 }
 
@@ -270,6 +275,7 @@ Tensor rows_linear(const Tensor& x, const Tensor& w) {
     Tensor y = gm::out_empty({x.size(0), w.size(0)}, x.options());
     GM_CHECK(launch_rows_linear(x.data_ptr(), w.data_ptr(), y.data_ptr(), x.size(0), w.size(0), w.size(1), x.stride(0), w.size(0), stream()),
              "rows_linear: at most 32 rows, K a multiple of 32");
+    check_launch("rows_linear");
     return y;
 }
 
@@ -389,6 +395,7 @@ Tensor mla_cached(const Tensor& query, const Tensor& low, const Tensor& w_up, co
     Tensor out = gm::out_empty({query.size(0), heads * value}, query.options());
     a.out = out.data_ptr();
     GM_CHECK(launch_mla_cached(a, stream()), "mla_cached: unsupported shape");
+    check_launch("mla_cached");
     return out;
 }
 

@@ -76,6 +76,34 @@ def test_cached_step_matches_the_plain_path(b, t, h, hkv, r, dr, c, start, windo
     cuda_ops.check_status()
 
 
+# grids of more than 65535 groups of rows or sequences; a window of zero positions keeps the work small
+@pytest.mark.parametrize("b,t,h,r", [(1, 131072, 16, 768), (1, 65600, 32, 256), (65600, 1, 8, 256)])
+def test_more_rows_than_a_grid_dimension_holds(b, t, h, r):
+    torch.manual_seed(12)
+    gc, tc = get_preset("mla")
+    gc.hidden_size, gc.n_heads, gc.n_kv_heads = 128, h, h
+    gc.mla_kv_rank, gc.mla_qk_rope_dim, gc.mla_qk_content_dim, gc.mla_value_dim, gc.mla_q_rank = r, 32, 32, 32, 0
+    tc.seq_len_train = tc.seq_len_val = t + 64
+    tc.resolve(1)
+    attn = MLAttention(gc, tc).cuda().eval()
+    x = torch.randn(b, t, 128, device="cuda").bfloat16()
+    whole = attn.allocate_cache(b, t + 2, device="cuda", dtype=torch.bfloat16)
+    got = attn.forward_cached(x, whole, 0)
+    parts = attn.allocate_cache(b, t + 2, device="cuda", dtype=torch.bfloat16)
+    if t > 1:                                                # the same tokens in calls of 32768
+        want = torch.cat([attn.forward_cached(x[:, i: i + 32768], parts, 0) for i in range(0, t, 32768)], dim=1)
+    else:
+        want = torch.empty_like(got)
+        for i in range(0, b, 32768):
+            part = attn.allocate_cache(min(32768, b - i), t + 2, device="cuda", dtype=torch.bfloat16)
+            want[i: i + 32768] = attn.forward_cached(x[i: i + 32768], part, 0)
+            parts.latent[i: i + 32768] = part.latent
+    assert whole.latent[:, :t].abs().sum(dim=-1).min() > 0 and torch.equal(whole.latent, parts.latent)
+    assert torch.equal(got, want)
+    from gpt_moe_b200.ops import cuda_ops
+    cuda_ops.check_status()
+
+
 @pytest.mark.parametrize("rows,n,k", [(1, 16, 32), (8, 576, 1024), (9, 8, 96), (17, 2624, 1024), (32, 24, 64)])
 def test_rows_linear_matches_matmul(rows, n, k):
     from gpt_moe_b200.ops import cuda_ops
