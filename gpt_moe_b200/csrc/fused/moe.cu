@@ -263,20 +263,20 @@ void launch_combine_bwd(const void* dout, const void* y, const int* src_of_row, 
 }
 
 // ---- activations ---------------------------------------------------------------------------------------
-// kind: 0 gelu (erf), 1 relu, 2 relu^2, 3 silu, 4 swiglu (pre = [gate | up], gate first).
+// kind: 0 gelu (erf), 1 relu, 2 relu^2, 3 silu, 4 swiglu (pre = [gate | up], gate first).  A NaN stays one: the tests read `x <= 0`.
 __device__ __forceinline__ float act_fwd(int kind, float x) {
     switch (kind) {
         case 0: return 0.5f * x * (1.f + erff(x * 0.70710678118f));
-        case 1: return fmaxf(x, 0.f);
-        case 2: { const float r = fmaxf(x, 0.f); return r * r; }
+        case 1: return x <= 0.f ? 0.f : x;
+        case 2: { const float r = x <= 0.f ? 0.f : x; return r * r; }
         default: return x / (1.f + __expf(-x));
     }
 }
 __device__ __forceinline__ float act_grad(int kind, float x) {
     switch (kind) {
         case 0: return 0.5f * (1.f + erff(x * 0.70710678118f)) + x * 0.3989422804f * __expf(-0.5f * x * x);
-        case 1: return x > 0.f ? 1.f : 0.f;
-        case 2: return 2.f * fmaxf(x, 0.f);
+        case 1: return x <= 0.f ? 0.f : 1.f;
+        case 2: return x <= 0.f ? 0.f : 2.f * x;
         default: { const float s = 1.f / (1.f + __expf(-x)); return s * (1.f + x * (1.f - s)); }
     }
 }

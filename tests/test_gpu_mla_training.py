@@ -72,3 +72,17 @@ def test_activation_entry_point(name, shape):
     (dwant,) = torch.autograd.grad(want, xf, g.float())
     tol = 4e-3 if shape[-1] % 16 == 0 else 8e-3          # one rounding in the kernel; torch's ops round every intermediate
     assert rel(y, want) < tol and rel(dx, dwant) < tol
+
+
+@pytest.mark.parametrize("name", ["gelu", "relu", "relu2", "silu", "swiglu"])
+def test_activation_keeps_nan_and_infinities(name):
+    x = torch.tensor([float("nan"), float("inf"), -float("inf"), 0.0, -0.0, 1.0, -1.0, 3.0e38] * 4, device="cuda").bfloat16()
+    x = torch.stack((x, x.flip(0))).requires_grad_()
+    y = api.activate(x, name)
+    (dx,) = torch.autograd.grad(y, x, torch.ones_like(y))
+    xf = x.detach().float().requires_grad_()
+    want = ref.activate(xf, name)
+    (dwant,) = torch.autograd.grad(want, xf, torch.ones_like(want))
+    assert torch.equal(torch.isnan(y), torch.isnan(want))
+    if name in ("relu", "relu2"):
+        assert torch.allclose(y.float(), want.bfloat16().float(), equal_nan=True) and torch.allclose(dx.float(), dwant.bfloat16().float(), equal_nan=True)
