@@ -499,9 +499,10 @@ std::vector<Tensor> activation_fwd(const Tensor& pre, const std::string& name, c
     c10::cuda::CUDAGuard guard(pre.device());
     check_bf16(pre, "pre");
     const int kind = act_kind(name);
-    const int in_w = pre.size(-1), h = kind == 4 ? in_w / 2 : in_w;
+    const int in_w = pre.dim() > 0 ? pre.size(-1) : 0, h = kind == 4 ? in_w / 2 : in_w;
+    GM_CHECK(in_w > 0 && (kind != 4 || in_w % 2 == 0), "activation: rows of at least one value, an even number of them for swiglu");
     const int rows = pre.numel() / in_w;
-    GM_CHECK(h % 8 == 0 && pre.is_contiguous(), "activation width must be a multiple of 8 (16-byte vectors) and rows contiguous");
+    GM_CHECK(h % 8 == 0 && reinterpret_cast<uintptr_t>(pre.data_ptr()) % 16 == 0, "activation width must be a multiple of 8 (16-byte vectors) and rows aligned to 16 bytes");
     auto sizes = pre.sizes().vec();
     sizes.back() = h;
     Tensor act = gm::out_empty(sizes, pre.options());
@@ -516,9 +517,12 @@ std::vector<Tensor> activation_bwd(const Tensor& dact, const Tensor& pre, const 
     c10::cuda::CUDAGuard guard(pre.device());
     check_bf16(dact, "dact");
     const int kind = act_kind(name);
-    const int in_w = pre.size(-1), h = kind == 4 ? in_w / 2 : in_w;
+    const int in_w = pre.dim() > 0 ? pre.size(-1) : 0, h = kind == 4 ? in_w / 2 : in_w;
+    GM_CHECK(in_w > 0 && (kind != 4 || in_w % 2 == 0), "activation: rows of at least one value, an even number of them for swiglu");
     const int rows = pre.numel() / in_w;
-    GM_CHECK(h % 8 == 0 && pre.is_contiguous() && dact.is_contiguous(), "activation width must be a multiple of 8 (16-byte vectors) and rows contiguous");
+    GM_CHECK(h % 8 == 0 && pre.is_contiguous() && reinterpret_cast<uintptr_t>(pre.data_ptr()) % 16 == 0 && reinterpret_cast<uintptr_t>(dact.data_ptr()) % 16 == 0,
+             "activation width must be a multiple of 8 (16-byte vectors) and rows contiguous and aligned to 16 bytes");
+    GM_CHECK(dact.numel() == static_cast<int64_t>(rows) * h, "activation_bwd: the gradient does not match the activation");
     Tensor dpre = gm::out_empty_like(pre);
     GM_CHECK(!quantize || h % 32 == 0, "activation with an MXFP8 copy: width must be a multiple of 32");
     QuantOut qo = alloc_quant(quantize, rows, in_w, pre);

@@ -647,10 +647,16 @@ def attention(q, k, v, *, causal=True, window=None, scale=None, softcap_value=0.
 
 
 # ---- activation ------------------------------------------------------------------------------------------------------------
+def _vector_rows(t: Tensor) -> Tensor:
+    """bf16, contiguous and on a 16-byte boundary (a slice of a buffer may be contiguous and start anywhere)."""
+    t = t if (t.dtype == BF16 and t.is_contiguous()) else t.to(BF16).contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 class _ActivationFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, pre: Tensor, name: str) -> Tensor:
-        pre = pre if (pre.dtype == BF16 and pre.is_contiguous()) else pre.to(BF16).contiguous()
+        pre = _vector_rows(pre)
         ctx.save_for_backward(pre)
         ctx.name = name
         return ext().activation_fwd(pre, name)[0]
@@ -658,13 +664,13 @@ class _ActivationFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dact: Tensor):
         (pre,) = ctx.saved_tensors
-        dact = dact if (dact.dtype == BF16 and dact.is_contiguous()) else dact.to(BF16).contiguous()
+        dact = _vector_rows(dact)
         return ext().activation_bwd(dact, pre, ctx.name)[0], None
 
 
 def activate(x: Tensor, name: str) -> Tensor:
-    width = x.shape[-1] // 2 if name == "swiglu" else x.shape[-1]
-    if width % 8:                               # the kernels move 16-byte vectors
+    # the kernels move 16-byte vectors of rows that are whole vectors; an odd SwiGLU width is an error that torch's ops raise
+    if name not in ("gelu", "relu", "relu2", "silu", "swiglu") or x.dim() == 0 or x.numel() == 0 or x.shape[-1] % (16 if name == "swiglu" else 8):
         return ref.activate(x, name)
     return run_function(_ActivationFn, x, name)
 

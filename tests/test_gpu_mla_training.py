@@ -86,3 +86,29 @@ def test_activation_keeps_nan_and_infinities(name):
     assert torch.equal(torch.isnan(y), torch.isnan(want))
     if name in ("relu", "relu2"):
         assert torch.allclose(y.float(), want.bfloat16().float(), equal_nan=True) and torch.allclose(dx.float(), dwant.bfloat16().float(), equal_nan=True)
+
+
+@pytest.mark.parametrize("shape,name", [((3, 17), "swiglu"), ((2, 15), "swiglu"), ((4, 8), "unknown")])
+def test_activation_refuses_what_torch_refuses(shape, name):
+    x = torch.randn(*shape, device="cuda").bfloat16()
+    with pytest.raises((RuntimeError, ValueError)):
+        ref.activate(x, name)
+    with pytest.raises((RuntimeError, ValueError)):
+        api.activate(x, name)
+
+
+@pytest.mark.parametrize("name", ["gelu", "relu2", "swiglu"])
+def test_activation_of_empty_scalar_and_unaligned_tensors(name):
+    for shape in ((0, 16), (3, 0), (0,)):
+        assert api.activate(torch.empty(*shape, device="cuda", dtype=torch.bfloat16), name).shape == ref.activate(torch.empty(*shape), name).shape
+    if name != "swiglu":
+        assert api.activate(torch.tensor(2.0, device="cuda", dtype=torch.bfloat16), name).dim() == 0
+    base = torch.randn(1 + 5 * 32, device="cuda").bfloat16()
+    x = base[1:].view(5, 32).requires_grad_()                 # contiguous, on no 16-byte boundary
+    y = api.activate(x, name)
+    g = torch.randn(1 + y.numel(), device="cuda").bfloat16()[1:].view(y.shape)
+    (dx,) = torch.autograd.grad(y, x, g)
+    xf = x.detach().float().requires_grad_()
+    want = ref.activate(xf, name)
+    (dwant,) = torch.autograd.grad(want, xf, g.float())
+    assert rel(y, want) < 4e-3 and rel(dx, dwant) < 4e-3
