@@ -136,10 +136,17 @@ class _NoGradContext:
         pass
 
 
+def intercepted() -> bool:
+    """Something wants the torch ops of a call and not only their results: a functorch transform, forward-mode tangents, a TorchScript trace
+    (it would take the result of a native call for a constant) or a dispatch mode.  Calls that torch's ops can serve go to them then."""
+    return (torch._C._are_functorch_transforms_active() or forward_ad._current_level >= 0 or torch._C._get_tracing_state() is not None
+            or torch._C._len_torch_dispatch_stack() > 0)
+
+
 def plain_call() -> bool:
-    """No gradients are recorded and nothing intercepts autograd functions (functorch transforms, forward-mode tangents): a Function's
-    forward can be called as it is, which saves the node (about 10 us of host time per call)."""
-    return not torch.is_grad_enabled() and not torch._C._are_functorch_transforms_active() and forward_ad._current_level < 0
+    """No gradients are recorded and nothing intercepts autograd functions: a Function's forward can be called as it is, which saves the
+    node (about 10 us of host time per call)."""
+    return not torch.is_grad_enabled() and not intercepted()
 
 
 def run_function(fn, *args):
