@@ -143,7 +143,7 @@ class SelfAttention(nn.Module):
                 return y, False
         out_proj = self.out_proj
         if (cuda_ops.plain_call() and self.q_proj.precision == out_proj.precision == "default" and type(out_proj) is Linear and out_proj.bias is None
-                and not out_proj._forward_hooks and not out_proj._forward_pre_hooks and self.hidden_size % 8 == 0):
+                and cuda_ops.bypassable(out_proj) and self.hidden_size % 8 == 0):
             # without gradients: the whole branch, output projection included, as one call
             cuda_ops.count_path("attention:tcgen05")
             y = cuda_ops.ext().attention_branch(

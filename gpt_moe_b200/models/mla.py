@@ -231,7 +231,7 @@ class MLAttention(nn.Module):
                 self.softmax_scale, max(self.softcap, 0.0), -1 if (self.is_full_attention or window is None) else int(window))
         plain = (self.q_proj, self.kv_down_proj, self.out_proj)
         if (b * t <= 32 and not self.q_rank and hidden % 32 == 0 and self.attn_dim % 32 == 0 and self.out_proj.bias is None
-                and all(type(m) is Linear and m.precision == "default" and not m._forward_hooks and not m._forward_pre_hooks for m in plain)):
+                and all(type(m) is Linear and m.precision == "default" for m in plain) and cuda_ops.bypassable(*plain)):
             return c.mla_step(cuda_ops._as_bf16_2d(x), cuda_ops.bf16_weight((self.q_proj.weight, self.kv_down_proj.weight)),
                               cuda_ops.bf16_weight((self.out_proj.weight,)), *rest).view(b, t, -1)
         query = x

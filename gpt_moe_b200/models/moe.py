@@ -65,7 +65,7 @@ class MoE(nn.Module):
                 return None
         w_up, w_down = [m._parameters.get("weight") for m in ups], [m._parameters.get("weight") for m in downs]
         d, up_n = w_up[0].shape[1] if w_up[0] is not None else 0, w_up[0].shape[0] if w_up[0] is not None else 0
-        if (any(w is None for w in w_up) or any(w is None for w in w_down) or router._forward_hooks or router._forward_pre_hooks
+        if (any(w is None for w in w_up) or any(w is None for w in w_down) or not cuda_ops.bypassable(router)
                 or self.num_experts % 8 or self.num_experts > 128 or self.top_k > 8 or d % 8 or up_n % 16 or w_down[0].shape[0] % 8):
             return None
         renormalise = not (self.top_k == 1 or self.full_softmax_gating)

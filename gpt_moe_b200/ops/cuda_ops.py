@@ -19,6 +19,7 @@ import torch
 import torch.nn.functional as F
 from torch import Tensor
 from torch.autograd import forward_ad
+from torch.nn.modules import module as _nn_module
 
 from . import _ext
 from . import reference as ref
@@ -147,6 +148,13 @@ def plain_call() -> bool:
     """No gradients are recorded and nothing intercepts autograd functions: a Function's forward can be called as it is, which saves the
     node (about 10 us of host time per call)."""
     return not torch.is_grad_enabled() and not intercepted()
+
+
+def bypassable(*modules) -> bool:
+    """Calling these modules does nothing but run their class's forward: no hooks (a process may also have global ones) and no forward
+    of an instance's own.  Only then may a composed call stand in for them."""
+    return not _nn_module._has_any_global_hook() and not any(
+        m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or "forward" in m.__dict__ for m in modules)
 
 
 def run_function(fn, *args):
@@ -304,7 +312,7 @@ def embedding(module, indices: Tensor) -> Tensor:
     main = getattr(weight, "main_grad", None)
     if (main is None or not torch.is_grad_enabled() or not weight.requires_grad or weight.dtype != torch.float32 or not main.is_contiguous()
             or weight.shape[1] % 4 or main.data_ptr() % 16 or weight.shape[0] >= 2 ** 31 or module.padding_idx is not None
-            or module.max_norm is not None or module.scale_grad_by_freq or module.sparse or module._forward_hooks or module._forward_pre_hooks
+            or module.max_norm is not None or module.scale_grad_by_freq or module.sparse or not bypassable(module)
             or torch._C._are_functorch_transforms_active()):
         return module(indices)
     return _EmbeddingFn.apply(indices, weight)

@@ -29,6 +29,20 @@ def test_a_trace_records_the_call_and_not_its_result():
         assert torch.equal(traced(torch.full((3,), 5.0)), torch.full((3,), 11.0))
 
 
+def test_modules_with_hooks_or_a_forward_of_their_own_are_called():
+    a, b = torch.nn.Linear(2, 2), torch.nn.Embedding(3, 2)
+    assert cuda_ops.bypassable(a, b)
+    for register in (a.register_forward_hook, a.register_forward_pre_hook, a.register_full_backward_hook, a.register_full_backward_pre_hook,
+                     lambda f: torch.nn.modules.module.register_module_forward_hook(f),
+                     lambda f: torch.nn.modules.module.register_module_full_backward_hook(f)):
+        handle = register(lambda *args: None)
+        assert not cuda_ops.bypassable(b, a)
+        handle.remove()
+        assert cuda_ops.bypassable(a, b)
+    b.forward = lambda ids: torch.zeros(1)
+    assert not cuda_ops.bypassable(a, b)
+
+
 def test_plain_call_is_off_under_transforms_tangents_traces_and_modes():
     seen = []
     assert not cuda_ops.plain_call()                       # gradients are recorded

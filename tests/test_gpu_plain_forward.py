@@ -39,4 +39,12 @@ def test_no_grad_forward_equals_the_recorded_one(preset, t):
         with torch.no_grad():
             assert torch.equal(model(ids, document_ids=docs), masked)
         assert seen == ["out", "router"]
+        from torch.nn.modules.module import register_module_forward_hook
+        handle = register_module_forward_hook(lambda m, *a: seen.append(type(m).__name__))
+        try:
+            with torch.no_grad():
+                assert torch.equal(model(ids, document_ids=docs), masked)
+        finally:
+            handle.remove()
+        assert sum(name == "Linear" for name in seen) >= 2 * 2                  # out_proj and router of both layers
     cuda_ops.check_status()
