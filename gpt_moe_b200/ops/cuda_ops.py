@@ -671,21 +671,21 @@ def _vector_rows(t: Tensor) -> Tensor:
 class _ActivationFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, pre: Tensor, name: str) -> Tensor:
-        pre = _vector_rows(pre)
         ctx.save_for_backward(pre)
         ctx.name = name
-        return ext().activation_fwd(pre, name)[0]
+        return ext().activation_fwd(_vector_rows(pre), name)[0]
 
     @staticmethod
     def backward(ctx, dact: Tensor):
         (pre,) = ctx.saved_tensors
-        dact = _vector_rows(dact)
-        return ext().activation_bwd(dact, pre, ctx.name)[0], None
+        if torch.is_grad_enabled():              # the gradient is itself to be differentiated: torch's ops have a graph
+            return torch.autograd.grad(ref.activate(pre, ctx.name), pre, dact, create_graph=True)[0], None
+        return ext().activation_bwd(_vector_rows(dact), _vector_rows(pre), ctx.name)[0].view(pre.shape), None
 
 
 def activate(x: Tensor, name: str) -> Tensor:
     # the kernels move 16-byte vectors of rows that are whole vectors; an odd SwiGLU width is an error that torch's ops raise
-    if name not in ("gelu", "relu", "relu2", "silu", "swiglu") or x.dim() == 0 or x.numel() == 0 or x.shape[-1] % (16 if name == "swiglu" else 8):
+    if intercepted() or name not in ("gelu", "relu", "relu2", "silu", "swiglu") or x.dim() == 0 or x.numel() == 0 or x.shape[-1] % (16 if name == "swiglu" else 8):
         return ref.activate(x, name)
     return run_function(_ActivationFn, x, name)
 

@@ -112,3 +112,24 @@ def test_activation_of_empty_scalar_and_unaligned_tensors(name):
     want = ref.activate(xf, name)
     (dwant,) = torch.autograd.grad(want, xf, g.float())
     assert rel(y, want) < 4e-3 and rel(dx, dwant) < 4e-3
+
+
+@pytest.mark.parametrize("name", ["gelu", "relu2", "silu", "swiglu"])
+def test_activation_second_derivatives_tangents_and_vmap(name):
+    torch.manual_seed(8)
+    x = torch.randn(6, 64, device="cuda").bfloat16()
+    v = torch.randn(6, 64, device="cuda").bfloat16()
+
+    def second(leaf, f):
+        (g,) = torch.autograd.grad((f(leaf, name).float() ** 2).sum(), leaf, create_graph=True)
+        return torch.autograd.grad((g.float() * v.to(g.dtype).float()).sum(), leaf)[0]
+
+    want = second(x.float().requires_grad_(), ref.activate)
+    assert rel(second(x.clone().requires_grad_(), api.activate), want) < 2e-2                        # bf16 steps of torch's own derivatives
+    t = x.t().contiguous().t().requires_grad_()                                                     # the gradient reaches the strided input itself
+    assert rel(second(t, api.activate), want) < 2e-2
+    out, tangent = torch.func.jvp(lambda y: api.activate(y, name), (x,), (v,))
+    assert rel(tangent, torch.func.jvp(lambda y: ref.activate(y, name), (x.float(),), (v.float(),))[1]) < 2e-2
+    assert torch.equal(torch.func.vmap(lambda y: api.activate(y, name))(x), ref.activate(x, name))
+    traced = torch.jit.trace(lambda y: api.activate(y, name), x, check_trace=False)
+    assert torch.equal(traced(v), ref.activate(v, name))
