@@ -52,6 +52,24 @@ def test_target_outside_the_vocabulary_in_the_training_loss(vocab, bad):
         cuda_ops.check_status()
 
 
+def test_tangents_and_vmap_run_through_torch():
+    torch.manual_seed(7)
+    logits, v = torch.randn(4, 6, 64, device="cuda").bfloat16(), torch.randn(4, 6, 64, device="cuda").bfloat16()
+    ids = torch.randint(0, 64, (4, 6), device="cuda")
+    plain = torch.nn.functional.cross_entropy
+    with torch.no_grad():
+        out, tangent = torch.func.jvp(lambda x: cuda_ops.cross_entropy(x, ids[0], -100), (logits[0],), (v[0],))
+        want = torch.func.jvp(lambda x: plain(x.double(), ids[0]), (logits[0],), (v[0],))
+        assert abs(out.item() - want[0].item()) < 1e-4 and abs(tangent.item() - want[1].item()) < 1e-2
+        rows = torch.func.vmap(lambda x, t: cuda_ops.cross_entropy(x, t, -100))(logits, ids)
+        assert torch.allclose(rows.double(), torch.stack([plain(x.double(), t) for x, t in zip(logits, ids)]), atol=1e-4)
+        tangent = torch.func.jvp(lambda x: continuation_scores(x, ids, [1, 2, 3, 1], [6, 5, 4, 2]), (logits,), (v,))[1]
+        want = torch.func.jvp(lambda x: continuation_scores(x, ids.cpu(), [1, 2, 3, 1], [6, 5, 4, 2]), (logits.cpu().float(),), (v.cpu().float(),))[1]
+        assert torch.allclose(tangent.cpu().float(), want, atol=2e-2)
+        traced = torch.jit.trace(lambda x: cuda_ops.cross_entropy(x, ids[0], -100), logits[0], check_trace=False)
+        assert abs(traced(v[0]).item() - plain(v[0].double(), ids[0]).item()) < 1e-4
+
+
 def test_gradients_still_run_through_torch():
     logits = torch.randn(4, 64, device="cuda").bfloat16().requires_grad_()
     cuda_ops.cross_entropy(logits, torch.tensor([1, 2, 3, 4], device="cuda"), -100).backward()
