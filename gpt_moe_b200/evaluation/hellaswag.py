@@ -70,7 +70,10 @@ def continuation_scores(logits: torch.Tensor, input_ids: torch.Tensor, prefix_le
     n, t = input_ids.shape
     if logits.is_cuda and len(prefix_lengths) == len(true_lengths) == n:
         from ..ops import cuda_ops
-        bounds = torch.stack([torch.as_tensor(x, dtype=torch.int64) for x in (prefix_lengths, true_lengths)]).to(input_ids.device)
+        bounds = [torch.as_tensor(x, dtype=torch.int64) for x in (prefix_lengths, true_lengths)]
+        if bounds[0].device != bounds[1].device:                # lists and tensors may be mixed
+            bounds = [b.to(input_ids.device) for b in bounds]
+        bounds = torch.stack(bounds).to(input_ids.device)
         token_lp = cuda_ops.continuation_logprob(logits, input_ids, bounds[0], bounds[1])      # 0 outside the continuations
         if token_lp is not None:
             count = (bounds[1].clamp(max=t) - bounds[0].clamp(min=1)).clamp(min=1)              # positions 1 .. t - 1 have a prediction

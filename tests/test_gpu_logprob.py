@@ -92,6 +92,18 @@ def test_continuation_scores(n, t, vocab):
     cuda_ops.check_status()
 
 
+def test_continuation_bounds_of_any_kind():
+    torch.manual_seed(5)
+    logits, ids = torch.randn(3, 9, 128, device="cuda").bfloat16(), torch.randint(0, 128, (3, 9), device="cuda")
+    prefix, true = [2, 1, 4], [9, 3, 8]
+    want = continuation_scores(logits, ids, prefix, true)
+    for p in (prefix, torch.tensor(prefix), torch.tensor(prefix, device="cuda"), torch.tensor(prefix, dtype=torch.int32)):
+        for t in (true, torch.tensor(true, device="cuda")):
+            assert torch.equal(continuation_scores(logits, ids, p, t), want)
+    with pytest.raises(RuntimeError):                           # ids that lie elsewhere than the logits are refused, as by torch's ops
+        continuation_scores(logits, ids.cpu(), prefix, true)
+
+
 # one 16-byte unit, fewer units than pieces, units that do not divide into pieces, the training vocabulary, both sides of the shared-memory limit
 @pytest.mark.parametrize("vocab", [8, 24, 40, 4104, 50304, 56960, 56968, 50301])
 @pytest.mark.parametrize("write_grad", [True, False])
