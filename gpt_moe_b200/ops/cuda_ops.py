@@ -285,9 +285,21 @@ def _take_accumulate_flag(weights: Sequence[Tensor]) -> bool:
 
 
 # ---- embedding ----------------------------------------------------------------------------------------------
+def _wanted_as_tensor(ctx, weight: Tensor, index: int) -> bool:
+    """In a backward: the gradient of input `index` has a reader of its own.  Hooks on the parameter want it, a second derivative is being
+    recorded, or `torch.autograd.grad` asks for it (there is then no accumulation to stand in for, which the engine reports as an error)."""
+    if torch.is_grad_enabled() or weight._backward_hooks or weight._post_accumulate_grad_hooks:
+        return True
+    try:
+        torch._C._will_engine_execute_node(ctx.next_functions[index][0])
+        return False
+    except RuntimeError:
+        return True
+
+
 class _EmbeddingFn(torch.autograd.Function):
     """Table lookup whose gradient is added straight into the optimizer's buffer (`weight.main_grad`): only the rows of tokens that
-    occur are touched, each sum in the order of the positions."""
+    occur are touched, each sum in the order of the positions.  Where the gradient itself is wanted it is formed as a tensor."""
 
     @staticmethod
     def forward(ctx, indices: Tensor, weight: Tensor) -> Tensor:
@@ -299,10 +311,13 @@ class _EmbeddingFn(torch.autograd.Function):
     def backward(ctx, dy: Tensor):
         (indices,) = ctx.saved_tensors
         weight = ctx.weight
+        if _wanted_as_tensor(ctx, weight, 1):
+            return None, torch.ops.aten.embedding_dense_backward(dy, indices, weight.shape[0], -1, False)
         if not _take_accumulate_flag((weight,)):
             weight.main_grad.zero_()
         ids, order = torch.sort(indices.reshape(-1).to(torch.int32), stable=True)
-        ext().embedding_grad(dy.reshape(-1, dy.shape[-1]).float().contiguous(), ids, order, weight.main_grad)
+        rows = dy.reshape(-1, dy.shape[-1]).float().contiguous()
+        ext().embedding_grad(rows if rows.data_ptr() % 16 == 0 else rows.clone(), ids, order, weight.main_grad)
         return None, None
 
 

@@ -37,3 +37,33 @@ def test_gradient_is_added_row_by_row(tokens, vocab, d):
     weight.main_grad, weight.grad_ready = torch.full((vocab, d), float("nan"), device="cuda"), False
     cuda_ops.embedding(module, ids).backward(dy)         # a buffer that has not been written in this step is overwritten
     assert (weight.main_grad.double() - (want - before.double())).abs().max().item() < 4e-6 + count ** 1.5 * 6e-8
+
+
+def test_a_gradient_that_is_read_is_formed():
+    torch.manual_seed(2)
+    module = torch.nn.Embedding(11, 16, device="cuda")
+    weight = module.weight
+    ids = torch.randint(0, 11, (2, 9), device="cuda")
+    dy = torch.randn(2, 9, 16, device="cuda")
+    want = torch.zeros(11, 16, device="cuda").index_add_(0, ids.view(-1), dy.view(-1, 16))
+    weight.grad = torch.zeros(11, 16, device="cuda")                  # as the fused engine lays it out: one buffer for both
+    weight.main_grad, weight.grad_ready = weight.grad, True
+    buffer = weight.main_grad
+    (got,) = torch.autograd.grad(cuda_ops.embedding(module, ids), weight, dy)
+    assert torch.allclose(got, want, atol=1e-5) and (buffer == 0).all()
+    leaf = dy.clone().requires_grad_()
+    (got,) = torch.autograd.grad(cuda_ops.embedding(module, ids), weight, leaf, create_graph=True)
+    (back,) = torch.autograd.grad((got ** 2).sum(), leaf)             # 2 g, gathered at the positions
+    assert torch.allclose(back, 2 * want[ids], atol=1e-4)
+    seen = []
+    hook = weight.register_hook(lambda g: seen.append(g.clone()))
+    after = weight.register_post_accumulate_grad_hook(lambda p: seen.append(p.grad.clone()))
+    cuda_ops.embedding(module, ids).backward(dy)
+    hook.remove(), after.remove()
+    assert len(seen) == 2 and all(torch.allclose(g, want, atol=1e-5) for g in seen)
+    assert weight.grad.data_ptr() == buffer.data_ptr() and torch.allclose(buffer, want, atol=1e-5)
+    cuda_ops.embedding(module, ids).backward(dy)                      # and without them straight into the buffer again
+    assert weight.grad.data_ptr() == buffer.data_ptr() and torch.allclose(buffer, 2 * want, atol=2e-5)
+    base = torch.randn(1 + dy.numel(), device="cuda")
+    cuda_ops.embedding(module, ids).backward(base[1:].view(dy.shape))  # a gradient on no 16-byte boundary
+    assert torch.allclose(buffer, 2 * want + torch.zeros_like(want).index_add_(0, ids.view(-1), base[1:].view(-1, 16)), atol=2e-5)
