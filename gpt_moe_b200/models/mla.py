@@ -19,6 +19,7 @@ from typing import Optional, Tuple
 
 import torch
 import torch.nn as nn
+import torch.nn.functional as F
 from torch import Tensor
 
 from ..ops import api
@@ -126,13 +127,13 @@ class MLAttention(nn.Module):
     def _fused_forward(self, x: Tensor, ctx: AttentionContext) -> Optional[Tensor]:
         """CUDA training path: from the projections to the attention output as one autograd node (`cuda_ops.mla_rope_attention`): the rotary
         rotation of the rope parts, the per-head QK-norm over the whole 128-wide head and the learned clamped scales run as one kernel
-        that reads the projections where they are, followed by the 128/64-wide tcgen05 attention kernels.  Returns None when shapes or
-        options need the general path."""
+        that reads the projections where they are, followed by the 128/64-wide tcgen05 attention kernels.  That kernel takes rotary parts of
+        whole 16-byte pieces; other widths are packed first (`_packed_attention`).  Returns None when shapes or options need the general path."""
         b, t, _ = x.shape
         h, hk, d = self.n_heads, self.n_kv_heads, self.head_size
-        if not (x.is_cuda and d == 128 and self.value_dim == 64 and self.rope_dim >= 8 and self.rope_dim % 8 == 0 and self.rotary is not None and h + hk <= 64
+        if not (x.is_cuda and d == 128 and self.value_dim == 64 and self.rotary is not None and h + hk <= 64
                 and self.is_causal and self.softcap == 0.0 and ctx.attn_mask is None and ctx.document_ids is None
-                and self.q_proj.bias is None and b * t > 0 and t <= self.rotary.cos_cached.shape[0] and self.rotary.cos_cached.dtype == torch.float32):
+                and self.q_proj.bias is None and b * t > 0 and t <= self.rotary.cos_cached.shape[0]):
             return None
         from ..ops import cuda_ops
         from ..ops.attention_cuda import _window_int
@@ -147,10 +148,31 @@ class MLAttention(nn.Module):
         if not all(p.dtype == torch.bfloat16 for p in (query, kv, rope)) or self.kv_rank % 8:
             rope, query, kv = rope.to(torch.bfloat16).contiguous(), query.to(torch.bfloat16), kv.to(torch.bfloat16)
         window = None if (self.is_full_attention or not self.use_flex_attention) else _window_int(ctx.window)
+        cos, sin = self.rotary.cos_cached, self.rotary.sin_cached
+        if cos.dtype != torch.float32:                     # a model cast as a whole takes its tables along
+            cos, sin = cos[:t].float(), sin[:t].float()
+        if self.rope_dim % 8:
+            return self._packed_attention(query, kv, rope, cos[:t], sin[:t], window)
         return cuda_ops.mla_rope_attention(
-            query, kv, rope, self.rotary.cos_cached, self.rotary.sin_cached, self.q_scale if self.use_qk_norm else None,
+            query, kv, rope, cos, sin, self.q_scale if self.use_qk_norm else None,
             self.k_scale if self.use_qk_norm else None, h, hk, self.qk_eps, self.qk_norm_type == "rms", self.qk_scale_min, self.qk_scale_max, window,
             self.softmax_scale)
+
+    def _packed_attention(self, query: Tensor, kv: Tensor, rope: Tensor, cos: Tensor, sin: Tensor, window: Optional[int]) -> Tensor:
+        """The fused path for rotary widths that are no multiple of 8: query and key heads are assembled, then turned and normalised by the
+        kernel of ordinary attention, given tables that are the identity rotation (cos 1, sin 0) on the content half of a head."""
+        from ..ops import cuda_ops
+        b, t, _ = query.shape
+        h, hk, d = self.n_heads, self.n_kv_heads, self.head_size
+        k_content, value = kv.view(b, t, hk, -1).split((self.content_dim, self.value_dim), dim=-1)
+        key = torch.cat((k_content, rope.reshape(b, t, 1, self.rope_dim).expand(-1, -1, hk, -1)), dim=-1)
+        packed = torch.cat((query.view(b, t, h, d), key), dim=2)
+        pad = self.content_dim // 2
+        rotated = cuda_ops.rope_qk_norm_packed(
+            packed.view(b * t, -1), F.pad(cos, (pad, 0), value=1.0), F.pad(sin, (pad, 0)), self.q_scale if self.use_qk_norm else None,
+            self.k_scale if self.use_qk_norm else None, t, h, hk, d, self.qk_eps, self.qk_norm_type == "rms", self.qk_scale_min,
+            self.qk_scale_max).view(b, t, h + hk, d)
+        return api.attention(rotated[:, :, :h], rotated[:, :, h:], value.contiguous(), causal=True, window=window, scale=self.softmax_scale)
 
     def forward(self, x: Tensor, ctx: AttentionContext) -> Tensor:
         b, t, _ = x.shape

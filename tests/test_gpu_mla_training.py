@@ -1,7 +1,12 @@
 """Latent attention from its projections (one autograd node) and the shared expert's activation against fp32 definitions."""
+import copy
+
 import pytest
 import torch
 
+from gpt_moe_b200.config import get_preset
+from gpt_moe_b200.models.attention import AttentionContext
+from gpt_moe_b200.models.mla import MLAttention
 from gpt_moe_b200.ops import api, cuda_ops
 from gpt_moe_b200.ops import reference as ref
 
@@ -133,3 +138,37 @@ def test_activation_second_derivatives_tangents_and_vmap(name):
     assert torch.equal(torch.func.vmap(lambda y: api.activate(y, name))(x), ref.activate(x, name))
     traced = torch.jit.trace(lambda y: api.activate(y, name), x, check_trace=False)
     assert torch.equal(traced(v), ref.activate(v, name))
+
+
+# rotary widths that are no whole 16-byte pieces; tables that were cast with the model
+@pytest.mark.parametrize("dr,hk,t,cast", [(36, 4, 128, False), (4, 2, 75, False), (64, 4, 128, True), (20, 4, 130, True)])
+def test_every_128_wide_head_takes_the_fused_path(dr, hk, t, cast, monkeypatch):
+    torch.manual_seed(10)
+    gc, tc = get_preset("mla")
+    gc.hidden_size, gc.n_heads, gc.n_kv_heads = 256, 4, hk
+    gc.mla_kv_rank, gc.mla_qk_rope_dim, gc.mla_qk_content_dim, gc.mla_value_dim, gc.mla_q_rank = 128, dr, 128 - dr, 64, 0
+    tc.seq_len_train = tc.seq_len_val = 256
+    tc.resolve(1)
+    cpu = MLAttention(gc, tc)
+    for p in cpu.parameters():
+        if p.dim() == 2:
+            torch.nn.init.normal_(p, std=0.05)
+            p.data = p.data.bfloat16().float()
+    gpu = copy.deepcopy(cpu).cuda()
+    if cast:
+        for m in (cpu, gpu):
+            m.rotary.cos_cached, m.rotary.sin_cached = m.rotary.cos_cached.bfloat16(), m.rotary.sin_cached.bfloat16()
+        cpu.rotary.float()                                   # the same rounded values
+    monkeypatch.setattr(gpu, "_project", lambda *a: pytest.fail("general path"))
+    x = torch.randn(2, t, 256).bfloat16()
+    ctx = AttentionContext(40, None, None)
+    xg, xc = x.cuda().requires_grad_(), x.float().requires_grad_()
+    got, want = gpu(xg, ctx), cpu(xc, ctx)
+    g = torch.randn_like(want).bfloat16()
+    got.backward(g.cuda()), want.backward(g.float())
+    # one rounding to bf16 for each of projections, rotated heads, probabilities, output and their gradients, 1.1e-3 on average
+    assert rel(got.cpu(), want) < 1.2e-2 and rel(xg.grad.cpu(), xc.grad) < 2e-2
+    for (name, a), (_, b) in zip(gpu.named_parameters(), cpu.named_parameters()):
+        if a.dim() == 2:
+            assert rel(a.grad.cpu(), b.grad) < 2e-2, name
+    cuda_ops.check_status()
