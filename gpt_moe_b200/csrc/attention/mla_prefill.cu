@@ -8,7 +8,7 @@
 // expansion, whose fp32 sums are split into two bf16 terms per key and value, probabilities as two terms; products of a high and a low
 // part are kept, fp32 accumulation throughout.  Queries are rounded to bf16 once, after rotation and gain (the latent and the
 // rotary key are bf16 in the cache).
-// Launches: mla_prefill_prepare (latent norm, rotations, query gains, cache rows of the new tokens), two GEMMs (gemm_bf16.cu: W's high and
+// Launches: split_terms (W's two terms, formed in every call: nothing of a weight is kept), mla_prefill_prepare (latent norm, rotations, query gains, cache rows of the new tokens), two GEMMs (gemm_bf16.cu: W's high and
 // low term, the second accumulating), mla_prefill_split (key gains of the new tokens, terms of keys and values), mla_prefill_attention.
 // Measured (16 heads, rank 512, 2 x 512 tokens after 1500), layer with its projections: 160 us, 152 of them kernels (attention 55, GEMMs 74, split 14,
 // prepare 10), against 1193 us for the absorbed kernels; error of the output against 64 bits 4.6e-3 (absorbed 4.1e-3, the fp32
@@ -365,20 +365,22 @@ mla_prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const _
     }
 }
 
-// w = hi + lo + (at most 2^-17 of w), element-wise
+// w = hi + lo + (at most 2^-17 of w), four elements a thread (n is a multiple of 4, w on a 16-byte boundary)
 __global__ void __launch_bounds__(256)
 split_terms_kernel(const float* __restrict__ w, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo, long long n) {
-    for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n; i += gridDim.x * 256LL) {
-        const __nv_bfloat16 h = __float2bfloat16(w[i]);
-        hi[i] = h;
-        lo[i] = __float2bfloat16(w[i] - __bfloat162float(h));
+    for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n / 4; i += gridDim.x * 256LL) {
+        const float4 x = reinterpret_cast<const float4*>(w)[i];
+        const uint32_t h0 = pack_bf16x2(x.x, x.y), h1 = pack_bf16x2(x.z, x.w);
+        reinterpret_cast<uint2*>(hi)[i] = make_uint2(h0, h1);
+        reinterpret_cast<uint2*>(lo)[i] = make_uint2(pack_bf16x2(x.x - __uint_as_float(h0 << 16), x.y - __uint_as_float(h0 & 0xffff0000u)),
+                                                     pack_bf16x2(x.z - __uint_as_float(h1 << 16), x.w - __uint_as_float(h1 & 0xffff0000u)));
     }
 }
 
 }  // namespace
 
 void launch_split_terms(const float* w, void* hi, void* lo, long long n, cudaStream_t s) {
-    const long long blocks = (n + 255) / 256;
+    const long long blocks = (n / 4 + 255) / 256;
     split_terms_kernel<<<static_cast<unsigned>(blocks < 1184 ? (blocks < 1 ? 1 : blocks) : 1184), 256, 0, s>>>(w, static_cast<__nv_bfloat16*>(hi), static_cast<__nv_bfloat16*>(lo), n);
 }
 

@@ -282,7 +282,6 @@ Tensor rows_linear(const Tensor& x, const Tensor& w) {
 // Latent-cache attention of T new tokens per sequence from their projections (attention/mla_decode.cu): appends them to the cache and
 // returns bf16 [B * T, H * value].  query [B*T, H * (content + dr)] and low [B*T, r + dr] bf16 (any row pitch), w_up fp32
 // [Hkv * (content + value), r], cos / sin fp32 tables [>= start + T, dr / 2], caches bf16 [B, capacity, width] with packed rows.
-// `terms`: w_up as two bf16 terms [2, rows, rank] (split_terms), for calls that expand the cache (mla_prefill.cu).
 MlaCachedArgs mla_cached_args(const Tensor& query, const Tensor& low, const Tensor& w_up, const OptTensor& norm_w, double norm_eps, const Tensor& cos, const Tensor& sin,
                             const OptTensor& q_scale, const OptTensor& k_scale, double qk_eps, bool rms, double smin, double smax, Tensor& latent, Tensor& rope,
                             Tensor& key_gain, int64_t start, int64_t heads, int64_t content, int64_t value, double scale, double softcap, int64_t window) {
@@ -331,20 +330,24 @@ bool mla_prefill_wanted(int64_t B, int64_t T, int64_t end, int64_t window, int64
     return T >= 48 && B * T >= 96 && B * T * visible >= 90000 && B * visible <= 262144 && r % 64 == 0 && dr == 64 && content == 64 && value == 64 && softcap <= 0.0;
 }
 
-Tensor mla_prefill(const MlaCachedArgs& args, const Tensor& latent, const Tensor& terms) {
+bool mla_prefill_aligned(const MlaCachedArgs& a) {
+    return reinterpret_cast<uintptr_t>(a.latent) % 16 == 0 && reinterpret_cast<uintptr_t>(a.rope) % 16 == 0 && a.latent_bs % 8 == 0 && a.rope_bs % 8 == 0 &&
+           reinterpret_cast<uintptr_t>(a.query) % 8 == 0 && a.q_pitch % 4 == 0;
+}
+
+Tensor mla_prefill(const MlaCachedArgs& args, const Tensor& latent) {
     MlaCachedArgs a = args;
     const int end = a.start + a.T;
     const int base = a.window < 0 ? 0 : std::max(0, a.start - a.window) / 128 * 128;      // first position any query sees, on a tile's edge
     const int S = end - base, S_pad = (S + 127) / 128 * 128;
-    GM_CHECK(terms.is_cuda() && terms.scalar_type() == torch::kBFloat16 && terms.is_contiguous() && terms.dim() == 3 && terms.size(0) == 2 &&
-             terms.size(1) == static_cast<int64_t>(a.Hkv) * 128 && terms.size(2) == a.r, "mla_prefill: terms [2, Hkv * 128, rank] bf16");
-    GM_CHECK(reinterpret_cast<uintptr_t>(a.latent) % 16 == 0 && reinterpret_cast<uintptr_t>(a.rope) % 16 == 0 && a.latent_bs % 8 == 0 && a.rope_bs % 8 == 0 &&
-             reinterpret_cast<uintptr_t>(a.query) % 8 == 0 && a.q_pitch % 4 == 0, "mla_prefill: aligned cache and queries");
     auto bf = latent.options();
     Tensor q = gm::out_empty({a.B, a.T, a.H * 128}, bf);
     launch_mla_prefill_prepare(a, q.data_ptr(), stream());
     Tensor kv = gm::out_empty({a.B, S, a.Hkv * 128}, bf.dtype(torch::kFloat32));
+    // W as two bf16 terms: 8 MB moved in a call that expands thousands of positions with them, so nothing of the weight is kept between calls
+    Tensor terms = gm::out_empty({2, static_cast<int64_t>(a.Hkv) * 128, a.r}, bf);
     const Tensor hi = terms.select(0, 0), lo = terms.select(0, 1);
+    launch_split_terms(a.w_up, hi.data_ptr(), lo.data_ptr(), hi.numel(), stream());
     const bool whole = a.B == 1 || (S == latent.size(1) && latent.stride(0) == static_cast<int64_t>(S) * a.r);
     for (int b = 0; b < (whole ? 1 : a.B); ++b) {
         const Tensor rows = whole ? latent.narrow(1, base, S).reshape({static_cast<int64_t>(a.B) * S, a.r}) : latent.select(0, b).narrow(0, base, S);
@@ -367,23 +370,13 @@ Tensor mla_prefill(const MlaCachedArgs& args, const Tensor& latent, const Tensor
     return out;
 }
 
-// fp32 [rows, cols] as bf16 terms [2, rows, cols]
-Tensor split_terms(const Tensor& w) {
-    c10::cuda::CUDAGuard guard(w.device());
-    GM_CHECK(w.is_cuda() && w.scalar_type() == torch::kFloat32 && w.is_contiguous() && w.dim() == 2, "split_terms: contiguous fp32 matrix");
-    Tensor out = gm::out_empty({2, w.size(0), w.size(1)}, w.options().dtype(torch::kBFloat16));
-    launch_split_terms(w.data_ptr<float>(), out.select(0, 0).data_ptr(), out.select(0, 1).data_ptr(), w.numel(), stream());
-    return out;
-}
-
 Tensor mla_cached(const Tensor& query, const Tensor& low, const Tensor& w_up, const OptTensor& norm_w, double norm_eps, const Tensor& cos, const Tensor& sin,
                   const OptTensor& q_scale, const OptTensor& k_scale, double qk_eps, bool rms, double smin, double smax, Tensor& latent, Tensor& rope,
-                  Tensor& key_gain, int64_t start, int64_t heads, int64_t content, int64_t value, double scale, double softcap, int64_t window,
-                  const OptTensor& terms) {
+                  Tensor& key_gain, int64_t start, int64_t heads, int64_t content, int64_t value, double scale, double softcap, int64_t window) {
     c10::cuda::CUDAGuard guard(query.device());
     MlaCachedArgs a = mla_cached_args(query, low, w_up, norm_w, norm_eps, cos, sin, q_scale, k_scale, qk_eps, rms, smin, smax, latent, rope, key_gain, start, heads,
                                       content, value, scale, softcap, window);
-    if (terms.has_value() && mla_prefill_wanted(a.B, a.T, start + a.T, window, a.r, a.dr, content, value, softcap)) return mla_prefill(a, latent, *terms);
+    if (mla_prefill_wanted(a.B, a.T, start + a.T, window, a.r, a.dr, content, value, softcap) && mla_prefill_aligned(a)) return mla_prefill(a, latent);
     a.splits = mla_decode_splits(a.B, a.T, a.H, a.r, start + a.T);
     const int64_t rows = static_cast<int64_t>(a.B) * a.T * a.H;
     // one fp32 workspace: queries in latent space, rotary queries, partial contexts, partial maxima and sums
@@ -408,7 +401,7 @@ Tensor mla_step(const Tensor& x, const Tensor& w_in, const Tensor& w_out, const 
     const int64_t nq = heads * (content + rope.size(2));
     GM_CHECK(both.size(1) == nq + latent.size(2) + rope.size(2), "mla_step: w_in holds the query rows, then the latent and rotary rows");
     Tensor out = mla_cached(both.narrow(1, 0, nq), both.narrow(1, nq, both.size(1) - nq), w_up, norm_w, norm_eps, cos, sin, q_scale, k_scale, qk_eps, rms, smin,
-                            smax, latent, rope, key_gain, start, heads, content, value, scale, softcap, window, c10::nullopt);
+                            smax, latent, rope, key_gain, start, heads, content, value, scale, softcap, window);
     return rows_linear(out, w_out);
 }
 
@@ -890,7 +883,6 @@ void register_kernels(pybind11::module_& m) {
     m.def("rows_linear", &rows_linear);
     m.def("mla_cached", &mla_cached);
     m.def("mla_prefill_wanted", &mla_prefill_wanted);
-    m.def("split_terms", &split_terms);
     m.def("mla_step", &mla_step);
     m.def("mma_issue_bench", &mma_issue_bench, py::arg("shape"), py::arg("count") = 64);
     m.def("router_fwd", &router_fwd);

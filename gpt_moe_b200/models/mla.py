@@ -190,7 +190,9 @@ class MLAttention(nn.Module):
 
     @torch.no_grad()
     def forward_cached(self, x: Tensor, cache: MLACache, window: Optional[int] = None) -> Tensor:
-        """Append x's tokens to the cache and attend over the whole cache with absorbed weights."""
+        """Append x's tokens to the cache and attend over the whole cache with absorbed weights.  On the GPU the projections use bf16 copies
+        of their weights, kept while torch's version counters (and `mark_parameters_updated`) say that nothing changed, as everywhere in
+        `ops.cuda_ops`; steps of up to 32 rows hold q_proj and kv_down_proj as one copy of their own.  kv_up_proj is read as it is."""
         if self.training or not self.is_causal:
             raise ValueError("MLA cached forward requires causal attention in eval mode")
         b, t, _ = x.shape
@@ -260,13 +262,7 @@ class MLAttention(nn.Module):
         if self.q_rank:
             query = api.rms_norm(self.q_down_proj(query), self.q_norm.weight, self.q_norm.eps)
         query = self.q_proj(query).reshape(b * t, -1)
-        terms = None
-        if c.mla_prefill_wanted(b, t, start + t, rest[-1], self.kv_rank, self.rope_dim, self.content_dim, self.value_dim, self.softcap) and all(
-                p.data_ptr() % 16 == 0 and p.stride(0) % 8 == 0 for p in caches[:2]):
-            # many new tokens: the visible cache is expanded (csrc/attention/mla_prefill.cu), with W as two bf16 terms laid out once
-            up = self.kv_up_proj.weight
-            terms = cuda_ops._cached(("terms", id(up)), (up,), lambda old: c.split_terms(up.detach()))
-        out = c.mla_cached(query, self.kv_down_proj(x).reshape(b * t, -1), *rest, terms)
+        out = c.mla_cached(query, self.kv_down_proj(x).reshape(b * t, -1), *rest)      # many new tokens: csrc/attention/mla_prefill.cu
         return self.out_proj(out.view(b, t, self.attn_dim))
 
 

@@ -76,6 +76,25 @@ def test_cached_step_matches_the_plain_path(b, t, h, hkv, r, dr, c, start, windo
     cuda_ops.check_status()
 
 
+@pytest.mark.parametrize("t", [1, 40, 256])                    # one native call; absorbed; expanded
+def test_a_weight_written_behind_torchs_back_is_seen(t):
+    torch.manual_seed(13)
+    gc, tc = get_preset("mla")
+    gc.hidden_size, gc.n_heads, gc.n_kv_heads = 256, 8, 8
+    tc.resolve(1)
+    attn = MLAttention(gc, tc).cuda().eval()
+    x = torch.randn(1, t, 256, device="cuda").bfloat16()
+
+    def call(module):
+        return module.forward_cached(x, module.allocate_cache(1, 300, device="cuda", dtype=torch.bfloat16))
+
+    first = call(attn)
+    attn.kv_up_proj.weight.data.mul_(-0.5)                     # bumps no version counter
+    second = call(attn)
+    assert not torch.equal(first, second)
+    assert torch.equal(second, call(copy.deepcopy(attn)))
+
+
 # grids of more than 65535 groups of rows or sequences; a window of zero positions keeps the work small
 @pytest.mark.parametrize("b,t,h,r", [(1, 131072, 16, 768), (1, 65600, 32, 256), (65600, 1, 8, 256)])
 def test_more_rows_than_a_grid_dimension_holds(b, t, h, r):
