@@ -91,6 +91,7 @@ CUtensorMap operand_map(const torch::Tensor& t, bool mn_major, int tile_rows_k_m
 
 // D[.., M, N] = alpha * op(A) op(B)^T + beta * C, optionally accumulated into an fp32 D.
 //   a_mn = false: a is [.., M, K];  a_mn = true: a is [.., K, M]   (same for b with N)
+//   mode 0 (dense): a, b and d with the same batch, or one 2-D b for a whole batch
 //   mode 1 (grouped M): a [rows, K], b [E, N, K] or [E, K, N], d [rows, N]; tile_expert/num_m_tiles on device
 //   mode 2 (grouped K): a [rows, M] (a_mn), b [rows, N] (b_mn), d [E, M, N]; seg_ends on device
 void gemm_bf16(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d, bool a_mn, bool b_mn, double alpha,
@@ -124,6 +125,9 @@ void gemm_bf16(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d,
             p.num_m_tiles = num_m_tiles->data_ptr<int>();
         } else {
             GM_CHECK((a_mn ? a.size(-1) : a.size(-2)) == p.M, "GEMM: A does not match the output height");
+            GM_CHECK(p.batch == 1 || (a.dim() == 3 && a.size(0) == p.batch && (b.dim() == 2 || b.size(0) == p.batch)),
+                     "GEMM: a batch of outputs takes as many A and as many B, or one B for all");
+            p.b_shared = b.dim() == 2;
         }
     }
     p.D = d.data_ptr();

@@ -348,13 +348,9 @@ Tensor mla_prefill(const MlaCachedArgs& args, const Tensor& latent) {
     Tensor terms = gm::out_empty({2, static_cast<int64_t>(a.Hkv) * 128, a.r}, bf);
     const Tensor hi = terms.select(0, 0), lo = terms.select(0, 1);
     launch_split_terms(a.w_up, hi.data_ptr(), lo.data_ptr(), hi.numel(), stream());
-    const bool whole = a.B == 1 || (S == latent.size(1) && latent.stride(0) == static_cast<int64_t>(S) * a.r);
-    for (int b = 0; b < (whole ? 1 : a.B); ++b) {
-        const Tensor rows = whole ? latent.narrow(1, base, S).reshape({static_cast<int64_t>(a.B) * S, a.r}) : latent.select(0, b).narrow(0, base, S);
-        Tensor d = whole ? kv.view({static_cast<int64_t>(a.B) * S, a.Hkv * 128}) : kv.select(0, b);
-        gemm_fp32(rows, lo, d, false);
-        gemm_fp32(rows, hi, d, true);
-    }
+    const Tensor rows = latent.narrow(1, base, S);          // [B, S, rank] with the cache's own batch stride
+    gemm_fp32(rows, lo, kv, false);
+    gemm_fp32(rows, hi, kv, true);
     Tensor split = gm::out_empty({4, a.B, S, a.Hkv * 64}, bf), gain = gm::out_empty({a.B, a.Hkv, S_pad}, kv.options());
     void* parts[4];
     for (int i = 0; i < 4; ++i) parts[i] = split.select(0, i).data_ptr();

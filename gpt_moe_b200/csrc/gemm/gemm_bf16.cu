@@ -98,7 +98,8 @@ __device__ __forceinline__ TileCoord tile_coord(const GemmParams& p, int tile, i
     t.n_limit = p.N;
     t.k_begin = 0;
     t.k_blocks = (p.K + BK - 1) / BK;
-    t.az = t.bz = t.dz = z;
+    t.az = t.dz = z;
+    t.bz = p.b_shared ? 0 : z;
     if (p.mode == GEMM_GROUPED_M) {
         t.az = 0;
         t.dz = 0;

@@ -76,6 +76,34 @@ def test_cached_step_matches_the_plain_path(b, t, h, hkv, r, dr, c, start, windo
     cuda_ops.check_status()
 
 
+# an exactly full cache, one with room; a window that starts inside it; a rank whose expansion splits its contraction
+@pytest.mark.parametrize("start,t,r,window", [(200, 130, 512, None), (333, 256, 256, 70), (1000, 128, 1024, None)])
+def test_a_batch_expands_as_its_sequences_do(start, t, r, window):
+    torch.manual_seed(14)
+    gc, tc = get_preset("mla")
+    gc.hidden_size, gc.n_heads, gc.n_kv_heads, gc.mla_kv_rank = 256, 8, 4, r
+    tc.resolve(1)
+    attn = MLAttention(gc, tc).cuda().eval()
+    x = torch.randn(3, t, 256, device="cuda").bfloat16()
+    old = [torch.randn(3, start, n, device="cuda").bfloat16() for n in (r, 64)] + [torch.rand(3, start, 4, device="cuda").bfloat16() + 0.5]
+
+    def call(rows, spare):
+        cache = attn.allocate_cache(rows.stop - rows.start, start + t + spare, device="cuda", dtype=torch.bfloat16)
+        for part, past in zip((cache.latent, cache.rope, cache.key_gain), old):
+            part[:, :start] = past[rows]
+            part[:, start + t:] = float("nan")
+        cache.length = start
+        return attn.forward_cached(x[rows], cache, window)
+
+    from gpt_moe_b200.ops import cuda_ops
+    assert cuda_ops.ext().mla_prefill_wanted(1, t, start + t, -1 if window is None else window, r, 64, 64, 64, 0.0)
+    full, roomy = call(slice(0, 3), 0), call(slice(0, 3), 77)
+    alone = torch.cat([call(slice(i, i + 1), 5) for i in range(3)])
+    assert torch.equal(full, roomy)
+    assert rel(full, alone) < (1e-3 if r == 1024 else 1e-12)       # split contractions meet in the order of arrival, in fp32
+    cuda_ops.check_status()
+
+
 @pytest.mark.parametrize("t", [1, 40, 256])                    # one native call; absorbed; expanded
 def test_a_weight_written_behind_torchs_back_is_seen(t):
     torch.manual_seed(13)
