@@ -29,6 +29,9 @@ def test_addend(batch, m, n, k, b_mn):
     assert torch.equal(again, d)
     ext.gemm_bf16(a, b.transpose(1, 2).contiguous() if b_mn else b, again, False, b_mn, 0.7, -1.3, c[0])      # broadcast: read by the threads
     assert rel(again, 0.7 * (a.double() @ b.double().transpose(1, 2)) - 1.3 * c[:1].double()) < 3e-3
+    for spread in (c[:1].expand_as(c), c[:, :1].expand_as(c)):                                     # the same by a stride of zero
+        ext.gemm_bf16(a, b.transpose(1, 2).contiguous() if b_mn else b, again, False, b_mn, 0.7, -1.3, spread)
+        assert rel(again, 0.7 * (a.double() @ b.double().transpose(1, 2)) - 1.3 * spread.double()) < 3e-3
     cuda_ops.check_status()
 
 
