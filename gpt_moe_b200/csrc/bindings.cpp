@@ -143,6 +143,7 @@ void gemm_bf16(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d,
         p.C = c->data_ptr();
         p.ldc = c->stride(-2);
         p.c_batch_stride = c->dim() == 3 ? c->stride(0) : 0;
+        GM_CHECK(reinterpret_cast<uintptr_t>(p.C) % 16 == 0 && p.c_batch_stride % 8 == 0, "C must lie on 16-byte boundaries");      // read 16 bytes at a time
     }
     GM_CHECK(p.ldd % 8 == 0 && (p.C == nullptr || p.ldc % 8 == 0), "output row pitch must be a multiple of 8 elements");
     if (symmetric) {      // the caller vouches that alpha * A B^T + beta * C is symmetric; only the upper triangle of tiles is computed
@@ -171,10 +172,10 @@ void gemm_bf16(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d,
     const int eb = p.out_fp32 ? 4 : 2;
     const CUtensorMap& td = cached_map(d.data_ptr(), eb, p.N, p.M, d.dim() == 3 ? d.size(0) : 1, p.ldd * eb,
                                        d.dim() == 3 ? d.stride(0) * eb : 0, 128 / eb, 128, 128);
-    // C of the output's shape comes through TMA; any other (broadcast over the batch or over rows, unaligned, beside an fp32 output) is read by the threads
+    // C of the output's shape comes through TMA; any other (broadcast over the batch or over rows, beside an fp32 output) is read by the threads
     CUtensorMap tc, tmirror;
     const bool tma_c = p.C != nullptr && mode == gm::GEMM_DENSE && !p.out_fp32 && !a_mn && p.K > 0 && c->dim() == d.dim() && c->sizes() == d.sizes() &&
-                       reinterpret_cast<uintptr_t>(p.C) % 16 == 0 && p.ldc > 0 && (p.batch == 1 || (p.c_batch_stride % 8 == 0 && p.c_batch_stride > 0));
+                       p.ldc > 0 && (p.batch == 1 || p.c_batch_stride > 0);
     if (tma_c) {
         tc = cached_map(p.C, 2, p.N, p.M, p.batch, p.ldc * 2, d.dim() == 3 ? p.c_batch_stride * 2 : 0, 64, 128, 128);
         if (p.symmetric) tmirror = cached_map(p.D, 2, p.N, p.M, p.batch, p.ldd * 2, d.dim() == 3 ? p.d_batch_stride * 2 : 0, 64, 64, 128);

@@ -35,6 +35,13 @@ def test_addend(batch, m, n, k, b_mn):
     cuda_ops.check_status()
 
 
+def test_an_unaligned_addend_is_refused():
+    a, b = torch.randn(16, 64, device="cuda").bfloat16(), torch.randn(24, 64, device="cuda").bfloat16()
+    c = torch.randn(16 * 24 + 1, device="cuda").bfloat16()[1:].view(16, 24)
+    with pytest.raises(RuntimeError, match="16-byte"):
+        cuda_ops.ext().gemm_bf16(a, b, torch.empty(16, 24, device="cuda", dtype=torch.bfloat16), False, False, 1.0, 1.0, c)
+
+
 @pytest.mark.parametrize("batch,m", [(1, 8), (3, 200), (2, 264), (30, 768), (1, 1096)])
 def test_symmetric_addend(batch, m):
     torch.manual_seed(4)
