@@ -3,7 +3,7 @@ import torch
 from torch.autograd import forward_ad
 from torch.utils._python_dispatch import TorchDispatchMode
 
-from gpt_moe_b200.ops import cuda_ops
+from gpt_moe_b200.ops import attention_tc, cuda_ops
 
 
 class _Double(torch.autograd.Function):
@@ -27,6 +27,17 @@ def test_a_trace_records_the_call_and_not_its_result():
     with torch.no_grad():
         traced = torch.jit.trace(lambda x: cuda_ops.run_function(_Double, x) + 1, torch.ones(3), check_trace=False)
         assert torch.equal(traced(torch.full((3,), 5.0)), torch.full((3,), 11.0))
+
+
+def test_what_the_attention_kernels_take():
+    def qkv(b, t, s=None):
+        return [torch.empty(b, n, 1, 64, dtype=torch.bfloat16) for n in (t, s or t, s or t)]
+
+    assert attention_tc.supported(*qkv(1, 100), 0.0) and attention_tc.supported(*qkv(65535, 1), 0.0)
+    assert not attention_tc.supported(*qkv(65536, 1), 0.0)          # sequences are a grid dimension
+    assert not attention_tc.supported(*qkv(1, 100, 200), 0.0) and not attention_tc.supported(*qkv(2, 100, 50), 0.0)
+    with forward_ad.dual_level():
+        assert not attention_tc.supported(*qkv(1, 100), 0.0) and attention_tc.supported(*qkv(1, 128), 0.0)
 
 
 def test_modules_with_hooks_or_a_forward_of_their_own_are_called():
