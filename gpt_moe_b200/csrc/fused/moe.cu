@@ -296,12 +296,9 @@ __device__ __forceinline__ void emit_quantized8(const uint4& stored, bool active
     }
 }
 
-// 1 / (1 + exp(-x)) with the approximate reciprocal (1 ulp of fp32; the results are rounded to bf16)
-__device__ __forceinline__ float sigmoid_fast(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
-
 // IDX: type of the flat piece index.  Both kernels move 6 to 12 bytes per element and were short of issue slots, not of bandwidth: a 64-bit
-// division per piece and an IEEE division per element cost more instructions than the rest (34816 rows, h = 3072, with the MXFP8
-// copy: forward 162 -> 125 us, 6.0 TB/s; backward 237 -> 212 us, 6.1 TB/s).
+// division per piece cost more instructions than much of the rest.  The sigmoid keeps its IEEE division: the approximate one is faster
+// still, and loses bits (and everything of a gate below -87).
 template <bool SWIGLU, typename IDX>
 __global__ void __launch_bounds__(256)
 activation_fwd_kernel(const __nv_bfloat16* __restrict__ pre, __nv_bfloat16* __restrict__ act, const int* __restrict__ meta,
@@ -326,7 +323,7 @@ activation_fwd_kernel(const __nv_bfloat16* __restrict__ pre, __nv_bfloat16* __re
                 float u[8];
                 unpack8(*reinterpret_cast<const uint4*>(pre + r * in_w + h + c), u);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) o[j] = a[j] * sigmoid_fast(a[j]) * u[j];
+                for (int j = 0; j < 8; ++j) o[j] = a[j] / (1.f + __expf(-a[j])) * u[j];
             } else {
 #pragma unroll
                 for (int j = 0; j < 8; ++j) o[j] = act_fwd(kind, a[j]);
@@ -363,7 +360,7 @@ activation_bwd_kernel(const __nv_bfloat16* __restrict__ dact, const __nv_bfloat1
                 unpack8(*reinterpret_cast<const uint4*>(pre + r * in_w + h + c), u);
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
-                    const float sg = sigmoid_fast(a[j]);
+                    const float sg = 1.f / (1.f + __expf(-a[j]));
                     d0[j] = g[j] * u[j] * sg * (1.f + a[j] * (1.f - sg));      // d/d(gate): up * silu'(gate)
                     d1[j] = g[j] * a[j] * sg;                                    // d/d(up):   silu(gate)
                 }

@@ -172,3 +172,16 @@ def test_every_128_wide_head_takes_the_fused_path(dr, hk, t, cast, monkeypatch):
         if a.dim() == 2:
             assert rel(a.grad.cpu(), b.grad) < 2e-2, name
     cuda_ops.check_status()
+
+
+def test_swiglu_of_a_gate_far_below_zero():
+    """exp(88) is a float and its reciprocal is not a normal one; the products are within bf16's range all the same."""
+    x = torch.zeros(2, 32, device="cuda").bfloat16()
+    x[0, :16], x[1, :16], x[:, 16:] = -87.5, -88.0, 1.0
+    x.requires_grad_()
+    y = api.activate(x, "swiglu")
+    (dx,) = torch.autograd.grad(y, x, torch.ones_like(y))
+    xd = x.detach().double().requires_grad_()
+    want = ref.activate(xd, "swiglu")
+    (dwant,) = torch.autograd.grad(want, xd, torch.ones_like(want))
+    assert rel(y, want) < 1e-2 and rel(dx, dwant) < 1e-2
