@@ -184,4 +184,4 @@ def test_swiglu_of_a_gate_far_below_zero():
     xd = x.detach().double().requires_grad_()
     want = ref.activate(xd, "swiglu")
     (dwant,) = torch.autograd.grad(want, xd, torch.ones_like(want))
-    assert rel(y, want) < 1e-2 and rel(dx, dwant) < 1e-2
+    assert (y.double() / want - 1).abs().max() < 1e-2 and (dx.double() / dwant - 1).abs().max() < 1e-2       # single values: 2^-8 and exp's share
