@@ -243,7 +243,9 @@ void launch_ce_fwd_bwd(void* logits, const long long* targets, float* loss, cons
 
 // ---- log-probabilities of given tokens from logits that somebody else keeps ------------------------------------------------
 // Read-only: the row is streamed once, 64 bytes of it per thread and step; the maximum of a step is found on packed bf16 pairs, the
-// sum is only rescaled when that maximum grows.  Bound by reading the logits: 32768 x 50304 take 0.575 ms (5.7 TB/s), where a cast to
+// sum is only rescaled when that maximum grows.  Exponents are differences of two logits times log2(e) and the target's logit meets the
+// maximum before the logarithm joins, so that no rounding grows with the size of the logits (the difference of two bf16 numbers is exact
+// or nearly so).  Bound by reading the logits: 32768 x 50304 take 0.575 ms (5.7 TB/s), where a cast to
 // fp32, a log-softmax and a gather took 7.5 ms; 64 x 184 rows of which one in eight is scored 0.04 ms against 2.6 ms.
 constexpr int LP_THREADS = 256, LP_UNROLL = 4;
 
@@ -269,7 +271,7 @@ __device__ __forceinline__ void row_statistics(const __nv_bfloat16* __restrict__
         }
         const float mx = fmaxf(__bfloat162float(mx2.x), __bfloat162float(mx2.y));
         if (mx > m) { s *= ex2_approx((m - mx) * kLog2e); m = mx; }
-        const float shift = m == -INFINITY ? 0.f : m * kLog2e;
+        const float top = m == -INFINITY ? 0.f : m;
         float part[2] = {0.f, 0.f};
 #pragma unroll
         for (int u = 0; u < LP_UNROLL; ++u) {
@@ -277,8 +279,8 @@ __device__ __forceinline__ void row_statistics(const __nv_bfloat16* __restrict__
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const float2 f = __bfloat1622float2(h[e]);
-                part[0] += ex2_approx(fmaf(f.x, kLog2e, -shift));
-                part[1] += ex2_approx(fmaf(f.y, kLog2e, -shift));
+                part[0] += ex2_approx((f.x - top) * kLog2e);
+                part[1] += ex2_approx((f.y - top) * kLog2e);
             }
         }
         s += part[0] + part[1];
@@ -321,7 +323,7 @@ row_nll_kernel(const __nv_bfloat16* __restrict__ logits, const long long* __rest
     const __nv_bfloat16* p = logits + row * row_stride;
     float m, s;
     row_statistics(p, vocab, vec16 != 0, m, s);
-    if (threadIdx.x == 0) loss[row] = m + logf(s) - __bfloat162float(p[tgt]);
+    if (threadIdx.x == 0) loss[row] = logf(s) + (m - __bfloat162float(p[tgt]));
 }
 
 // lp[i, j] = log p(tokens[i, j + 1] | row i up to j) for prefix[i] <= j + 1 < end[i], 0 elsewhere (those rows of the logits are not read)
@@ -343,7 +345,7 @@ continuation_logprob_kernel(const __nv_bfloat16* __restrict__ logits, const long
     const __nv_bfloat16* p = logits + i * batch_stride + j * row_stride;
     float m, s;
     row_statistics(p, vocab, vec16 != 0, m, s);
-    if (threadIdx.x == 0) *dst = __bfloat162float(p[tok]) - (m + logf(s));
+    if (threadIdx.x == 0) *dst = (__bfloat162float(p[tok]) - m) - logf(s);
 }
 
 void launch_row_nll(const void* logits, const long long* targets, float* loss, int rows, int vocab, long long row_stride, long long ignore_index,

@@ -26,6 +26,18 @@ def test_row_losses(rows, vocab, pitch):
     cuda_ops.check_status()
 
 
+@pytest.mark.parametrize("spread,offset", [(0.5, 20.0), (3.0, -40.0), (10.0, 20.0), (30.0, 0.0)])
+@pytest.mark.parametrize("vocab", [1003, 50304])
+def test_row_losses_are_as_exact_as_torchs(spread, offset, vocab):
+    torch.manual_seed(9)
+    logits = (spread * torch.randn(512, vocab, device="cuda") + offset).bfloat16()
+    targets = torch.randint(0, vocab, (512,), device="cuda")
+    exact = torch.nn.functional.cross_entropy(logits.double(), targets, reduction="none")
+    mine = cuda_ops.ext().row_nll(logits, targets, -100).double() - exact
+    torchs = torch.nn.functional.cross_entropy(logits.float(), targets, reduction="none").double() - exact
+    assert mine.norm() < 1.25 * torchs.norm() and mine.norm() < 1e-7 * exact.norm()
+
+
 def test_target_outside_the_vocabulary_is_reported():
     logits = torch.randn(2, 64, device="cuda").bfloat16()
     assert torch.isnan(cuda_ops.cross_entropy(logits, torch.tensor([3, 64], device="cuda"), -100))
