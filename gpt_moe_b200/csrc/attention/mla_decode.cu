@@ -14,9 +14,10 @@
 //     registers) with its slice of the 32 latent rows, the eight partial score tiles are summed through shared memory together
 //     with the rotary part (one 16-wide slice each for the first warps), and the same slice of the tile is the value operand of
 //     its slice of the context, which stays in registers;
-//   * queries and probabilities are fp32 numbers: each enters as two bf16 terms (16 bits of mantissa), one product each, accumulated
-//     in fp32.  The cache is bf16 and needs no splitting.  A third term would lengthen the chain of products of every tile and moves no
-//     digit of the output's error.
+//   * queries and probabilities are fp32 numbers: each enters as bf16 terms, one product each, accumulated in fp32; the cache is bf16 and
+//     needs no splitting.  Three terms hold all bits, and a context that is returned in fp32 gets them (`mla_decode`).  The layer's own
+//     call rounds the context's expansion to bf16: two terms (16 bits) leave its error as it is (3.9e-3 against 64 bits either way)
+//     and shorten the chain of products of every tile.
 // Measured (16 heads, rank 512): 8 sequences x 1 token over 4022 positions 18 us against 96 us for a kernel that formed the products
 // with fp32 multiply-adds and warp reductions (38 MB of cache; its merge took another 48 us, now 9 with W_v); 32 x 1 over 8000 positions
 // 92 us, 3.3 TB/s, the tensor pipe 38 % busy: a tile's chain of products, sums and softmax is the limit.  Error of the layer's output against 64 bits: 3.8e-3 against 5.6e-3 (queries and rotation stay
@@ -31,12 +32,12 @@
 namespace gm {
 
 constexpr int MD_TILE = 32;          // cache positions per tile
-constexpr int MD_TERMS = 2;          // bf16 terms of a query or probability
 constexpr int MD_WARPS = 8;
 // One tile of rows of an up to 512-wide latent leaves room for two CTAs on an SM: every tile passes three barriers, and the other CTA's
-// products run meanwhile.  Wider latents and two tiles of rows take the SM to themselves.  Ring depth: as many tiles as fit beside the scores.
-constexpr int md_ctas(int ks, int mt) { return ks <= 4 && mt == 1 ? 2 : 1; }
-constexpr int md_stages(int ks, int mt) { return ks <= 2 ? 4 : md_ctas(ks, mt) == 2 ? 2 : ks <= 4 ? 4 : ks <= 6 ? 3 : 2; }
+// products run meanwhile.  Wider latents, two tiles of rows and three terms take the SM to themselves.  Ring depth: as many tiles as fit beside
+// the scores.
+constexpr int md_ctas(int ks, int mt, int terms) { return ks <= 4 && mt == 1 && terms == 2 ? 2 : 1; }
+constexpr int md_stages(int ks, int mt, int terms) { return ks <= 2 ? 4 : md_ctas(ks, mt, terms) == 2 ? 2 : ks <= 4 ? 4 : ks <= 6 ? 3 : 2; }
 constexpr int MD_ROPE_MAX = 64;
 constexpr int MD_MAX_SPLITS = 64;
 constexpr int MD_SP_PITCH = 40;      // floats per row of a partial score tile: two half-warps' rows fall on different banks
@@ -76,18 +77,23 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool v
     const int bytes = valid ? 16 : 0;
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
-// x = high + low with bf16 terms, up to 2^-17 of x (the remainder after the first term is exact)
-__device__ __forceinline__ void split_pair(float x, float y, uint32_t& high, uint32_t& low) {
-    high = pack_bf16x2(x, y);
-    low = pack_bf16x2(x - __uint_as_float(high << 16), y - __uint_as_float(high & 0xffff0000u));
+// x as a sum of bf16 terms, largest first (the remainder after each is exact): up to 2^-17 of x with two, all of it with three
+template <int TERMS>
+__device__ __forceinline__ void split_pair(float x, float y, uint32_t (&term)[TERMS]) {
+#pragma unroll
+    for (int i = 0; i < TERMS; ++i) {
+        term[i] = pack_bf16x2(x, y);
+        x -= __uint_as_float(term[i] << 16);
+        y -= __uint_as_float(term[i] & 0xffff0000u);
+    }
 }
 
-// KS = k-steps of 16 latent dimensions per warp (r = 128 * KS); MT = 16-row tiles per CTA
-template <int KS, int MT>
-__global__ void __launch_bounds__(MD_WARPS * 32, md_ctas(KS, MT))
+// KS = k-steps of 16 latent dimensions per warp (r = 128 * KS); MT = 16-row tiles per CTA; MD_TERMS = bf16 terms of a query or probability
+template <int KS, int MT, int MD_TERMS>
+__global__ void __launch_bounds__(MD_WARPS * 32, md_ctas(KS, MT, MD_TERMS))
 mla_decode_split_kernel(const MlaDecodeParams p) {
     extern __shared__ __align__(16) uint8_t md_smem[];
-    constexpr int r = KS * 128, MD_STAGES = md_stages(KS, MT);
+    constexpr int r = KS * 128, MD_STAGES = md_stages(KS, MT, MD_TERMS);
     constexpr int LAT_PITCH = r * 2 + 16, ROPE_PITCH = MD_ROPE_MAX * 2 + 16;     // bytes; ldmatrix rows on different banks
     constexpr int STAGE = MD_TILE * (LAT_PITCH + ROPE_PITCH);
     constexpr int ROWS = MT * 16;
@@ -158,7 +164,7 @@ mla_decode_split_kernel(const MlaDecodeParams p) {
     };
     for (int i = 0; i < MD_STAGES - 1; ++i) load_tile(i);
 
-    // this warp's slice of the queries as A fragments (both terms): rows g / g + 8, columns 2 tq, 2 tq + 1 and + 8
+    // this warp's slice of the queries as A fragments (all terms): rows g / g + 8, columns 2 tq, 2 tq + 1 and + 8
     uint32_t qa[MT][KS][MD_TERMS][4], qr[MT][MD_TERMS][4];
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt) {
@@ -173,14 +179,20 @@ mla_decode_split_kernel(const MlaDecodeParams p) {
                 for (int cc = 0; cc < 2; ++cc) {
                     float2 v = *reinterpret_cast<const float2*>(p.q_latent + base * r + (warp * KS + ks) * 16 + cc * 8 + tq * 2);
                     if (!live) v = make_float2(0.f, 0.f);
-                    split_pair(v.x, v.y, qa[mt][ks][0][cc * 2 + hf], qa[mt][ks][1][cc * 2 + hf]);
+                    uint32_t term[MD_TERMS];
+                    split_pair(v.x, v.y, term);
+#pragma unroll
+                    for (int i = 0; i < MD_TERMS; ++i) qa[mt][ks][i][cc * 2 + hf] = term[i];
                 }
 #pragma unroll
             for (int cc = 0; cc < 2; ++cc) {
                 const int c0 = warp * 16 + cc * 8 + tq * 2;                       // dr is even: a pair is in or out as a whole
                 float2 v = make_float2(0.f, 0.f);
                 if (live && has_rope && c0 < p.dr) v = *reinterpret_cast<const float2*>(p.q_rope + base * p.dr + c0);
-                split_pair(v.x, v.y, qr[mt][0][cc * 2 + hf], qr[mt][1][cc * 2 + hf]);
+                uint32_t term[MD_TERMS];
+                split_pair(v.x, v.y, term);
+#pragma unroll
+                for (int i = 0; i < MD_TERMS; ++i) qr[mt][i][cc * 2 + hf] = term[i];
             }
         }
     }
@@ -294,11 +306,12 @@ mla_decode_split_kernel(const MlaDecodeParams p) {
             const float p0 = vis[0] ? expf(s[0] - m_new) : 0.f, p1 = vis[1] ? expf(s[1] - m_new) : 0.f;
             l[mt] = l[mt] * corr + (p0 + p1);
             m[mt] = m_new;
-            uint32_t t0, t1;
-            split_pair(p0, p1, t0, t1);
+            uint32_t prob[MD_TERMS];
+            split_pair(p0, p1, prob);
             uint32_t* dst = reinterpret_cast<uint32_t*>(pr + (mt * 16 + srow) * MD_P_PITCH + skey);
             constexpr int term_words = ROWS * MD_P_PITCH / 2;
-            dst[0] = t0; dst[term_words] = t1;
+#pragma unroll
+            for (int i = 0; i < MD_TERMS; ++i) dst[i * term_words] = prob[i];
             if ((tid & 15) == 0) alpha_s[mt * 16 + srow] = corr;
         }
         __syncthreads();
@@ -663,12 +676,12 @@ bool launch_rows_linear(const void* x, const void* w, void* y, int rows, int N, 
     return true;
 }
 
-template <int KS, int MT>
+template <int KS, int MT, int TERMS>
 static void launch_split(const MlaDecodeParams& p, cudaStream_t s) {
     constexpr int rows = MT * 16;
-    constexpr int smem = md_stages(KS, MT) * MD_TILE * (KS * 256 + 16 + MD_ROPE_MAX * 2 + 16) + MD_WARPS * rows * MD_SP_PITCH * 4 + MD_TERMS * rows * MD_P_PITCH * 2 + rows * 4;
-    static_assert((smem + 1024) * md_ctas(KS, MT) <= 233472, "shared memory of the decode kernel");
-    auto k = mla_decode_split_kernel<KS, MT>;
+    constexpr int smem = md_stages(KS, MT, TERMS) * MD_TILE * (KS * 256 + 16 + MD_ROPE_MAX * 2 + 16) + MD_WARPS * rows * MD_SP_PITCH * 4 + TERMS * rows * MD_P_PITCH * 2 + rows * 4;
+    static_assert((smem + 1024) * md_ctas(KS, MT, TERMS) <= 233472, "shared memory of the decode kernel");
+    auto k = mla_decode_split_kernel<KS, MT, TERMS>;
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     k<<<static_cast<unsigned>(p.splits) * ((p.T * p.H + rows - 1) / rows) * p.B, MD_WARPS * 32, smem, s>>>(p);
 }
@@ -677,13 +690,13 @@ static void launch_split(const MlaDecodeParams& p, cudaStream_t s) {
 // the fragments of 1024-wide queries fill the registers
 static int decode_row_tiles(int T, int H, int r) { return T * H > 16 && r <= 512 ? 2 : 1; }
 
-int mla_decode_splits(int B, int T, int H, int r, int S) {
+int mla_decode_splits(int B, int T, int H, int r, int S, int terms) {
     const int rows = 16 * decode_row_tiles(T, H, r);
     const int ctas = B * ((T * H + rows - 1) / rows);
     const int tiles = (S + MD_TILE - 1) / MD_TILE;
     // one wave of CTAs, since a second would cost as much as the first: two CTAs an SM where they fit and have six tiles each, else one (8 x
     // 4022 positions: 18 splits of 7 tiles 18.1 + 8.7 us with the merge, 37 of 4 tiles 17.2 + 11.9; 32 x 8000: 4 splits 146 us, 9 splits 92)
-    const int both = 148 * md_ctas(r / 128, rows / 16) / ctas;
+    const int both = 148 * md_ctas(r / 128, rows / 16, terms) / ctas;
     int want = both > 0 && tiles / both >= 6 ? both : 148 / ctas;
     want = want < 1 ? 1 : (want > MD_MAX_SPLITS ? MD_MAX_SPLITS : want);
     return want < tiles ? want : (tiles < 1 ? 1 : tiles);
@@ -694,6 +707,7 @@ bool mla_decode_supported(int H, int Hkv, int r, int dr) {
            H % Hkv == 0 && dr % 2 == 0 && dr <= MD_ROPE_MAX && dr >= 2;
 }
 
+template <int TERMS>
 static bool launch_decode_split(const float* q_latent, const float* q_rope, const void* latent, const void* rope, const void* key_gain,
                                 long long latent_bs, long long rope_bs, long long gain_bs, float* part_ctx, float* part_ml, int B, int T, int H, int Hkv,
                                 int r, int dr, int S, int splits, int start, int window, float scale, float softcap, cudaStream_t s) {
@@ -710,17 +724,17 @@ static bool launch_decode_split(const float* q_latent, const float* q_rope, cons
     p.rope_vec = reinterpret_cast<uintptr_t>(rope) % 16 == 0 && rope_bs % 8 == 0 && dr % 8 == 0;
     p.scale = scale; p.softcap = softcap;
     const bool two = decode_row_tiles(T, H, r) == 2;
-    if (r == 256) { if (two) launch_split<2, 2>(p, s); else launch_split<2, 1>(p, s); }
-    else if (r == 512) { if (two) launch_split<4, 2>(p, s); else launch_split<4, 1>(p, s); }
-    else if (r == 768) launch_split<6, 1>(p, s);
-    else launch_split<8, 1>(p, s);
+    if (r == 256) { if (two) launch_split<2, 2, TERMS>(p, s); else launch_split<2, 1, TERMS>(p, s); }
+    else if (r == 512) { if (two) launch_split<4, 2, TERMS>(p, s); else launch_split<4, 1, TERMS>(p, s); }
+    else if (r == 768) launch_split<6, 1, TERMS>(p, s);
+    else launch_split<8, 1, TERMS>(p, s);
     return true;
 }
 
 bool launch_mla_decode(const float* q_latent, const float* q_rope, const void* latent, const void* rope, const void* key_gain,
                        long long latent_bs, long long rope_bs, long long gain_bs, float* part_ctx, float* part_ml, float* context, int B, int T,
                        int H, int Hkv, int r, int dr, int S, int splits, int start, int window, float scale, float softcap, cudaStream_t s) {
-    if (!launch_decode_split(q_latent, q_rope, latent, rope, key_gain, latent_bs, rope_bs, gain_bs, part_ctx, part_ml, B, T, H, Hkv, r, dr, S, splits,
+    if (!launch_decode_split<3>(q_latent, q_rope, latent, rope, key_gain, latent_bs, rope_bs, gain_bs, part_ctx, part_ml, B, T, H, Hkv, r, dr, S, splits,
                              start, window, scale, softcap, s))
         return false;
     mla_decode_merge_kernel<<<static_cast<unsigned>(B) * T * H, 128, 0, s>>>(part_ctx, part_ml, context, splits, r);
@@ -776,7 +790,7 @@ bool launch_mla_cached(const MlaCachedArgs& a, cudaStream_t s) {
         else launch_cached<8>(p, many, a.part_ctx, a.part_ml, out, a.splits, values, s);
     };
     stage(false);
-    if (!launch_decode_split(a.q_latent, a.q_rope, latent, rope, gain, a.latent_bs, a.rope_bs, a.gain_bs, a.part_ctx, a.part_ml, a.B, a.T, a.H, a.Hkv, a.r,
+    if (!launch_decode_split<2>(a.q_latent, a.q_rope, latent, rope, gain, a.latent_bs, a.rope_bs, a.gain_bs, a.part_ctx, a.part_ml, a.B, a.T, a.H, a.Hkv, a.r,
                              a.dr, a.start + a.T, a.splits, a.start, a.window, a.scale, a.softcap, s))
         return false;
     stage(true);

@@ -253,7 +253,7 @@ Tensor mla_decode(const Tensor& q_latent, const Tensor& q_rope, const Tensor& la
                  c->stride(1) == c->size(2), "mla_decode: bf16 cache tensors [B, S, width] with packed rows");
     GM_CHECK(latent.size(2) == r && rope.size(2) == dr && mla_decode_supported(H, Hkv, r, dr),
              "mla_decode: latent rank 256/512/768/1024, 8/16/32 heads (rank/32 * heads/8 <= 64), rope width even and <= 64");
-    const int splits = mla_decode_splits(B, T, H, r, S);
+    const int splits = mla_decode_splits(B, T, H, r, S, 3);
     Tensor part_ctx = gm::out_empty({B, T, H, splits, r}, q_latent.options());
     Tensor part_ml = gm::out_empty({B, T, H, splits, 2}, q_latent.options());
     Tensor context = gm::out_empty({B, T, H, r}, q_latent.options());
@@ -373,7 +373,7 @@ Tensor mla_cached(const Tensor& query, const Tensor& low, const Tensor& w_up, co
     MlaCachedArgs a = mla_cached_args(query, low, w_up, norm_w, norm_eps, cos, sin, q_scale, k_scale, qk_eps, rms, smin, smax, latent, rope, key_gain, start, heads,
                                       content, value, scale, softcap, window);
     if (mla_prefill_wanted(a.B, a.T, start + a.T, window, a.r, a.dr, content, value, softcap) && mla_prefill_aligned(a)) return mla_prefill(a, latent);
-    a.splits = mla_decode_splits(a.B, a.T, a.H, a.r, start + a.T);
+    a.splits = mla_decode_splits(a.B, a.T, a.H, a.r, start + a.T, 2);
     const int64_t rows = static_cast<int64_t>(a.B) * a.T * a.H;
     // one fp32 workspace: queries in latent space, rotary queries, partial contexts, partial maxima and sums
     Tensor ws = gm::out_empty({rows * (a.r + 64) + rows * a.splits * (a.r + 2)}, query.options().dtype(torch::kFloat32));

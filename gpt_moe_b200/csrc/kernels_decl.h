@@ -47,7 +47,7 @@ void launch_activation_bwd(const void* dact, const void* pre, void* dpre, const 
                            cudaStream_t s);
 
 // attention/mla_decode.cu
-int mla_decode_splits(int B, int T, int H, int r, int S);
+int mla_decode_splits(int B, int T, int H, int r, int S, int terms);      // terms: 3 for launch_mla_decode, 2 for launch_mla_cached
 bool mla_decode_supported(int H, int Hkv, int r, int dr);
 bool launch_mla_decode(const float* q_latent, const float* q_rope, const void* latent, const void* rope, const void* key_gain,
                        long long latent_bs, long long rope_bs, long long gain_bs, float* part_ctx, float* part_ml, float* context, int B, int T,

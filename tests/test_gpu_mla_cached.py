@@ -151,6 +151,22 @@ def test_more_rows_than_a_grid_dimension_holds(b, t, h, r):
     cuda_ops.check_status()
 
 
+# one and two tiles of rows, every rank
+@pytest.mark.parametrize("b,t,h,hkv,r,dr,s", [(2, 1, 16, 16, 512, 64, 777), (1, 5, 8, 2, 256, 32, 300), (2, 1, 32, 32, 512, 64, 130), (1, 2, 16, 4, 768, 64, 500), (1, 1, 8, 8, 1024, 10, 90)])
+def test_a_context_in_fp32_has_the_bits_of_fp32(b, t, h, hkv, r, dr, s):
+    from gpt_moe_b200.models.mla import api_mla_decode
+    torch.manual_seed(15)
+    q, qr = 0.3 * torch.randn(b, t, h, r, device="cuda"), torch.randn(b, t, h, dr, device="cuda")
+    lat, rope = torch.randn(b, s, r, device="cuda").bfloat16(), torch.randn(b, s, dr, device="cuda").bfloat16()
+    gain = (torch.rand(b, s, hkv, device="cuda") + 0.5).bfloat16()
+    got = api_mla_decode(q, qr, lat, rope, gain, s - t, 0.08, 0.0, "exact", None)
+    score = torch.einsum("bthr,bsr->bhts", q.double(), lat.double()) + torch.einsum("bthd,bsd->bhts", qr.double(), rope.double())
+    score = score * gain.double().permute(0, 2, 1).repeat_interleave(h // hkv, dim=1)[:, :, None, :] * 0.08
+    keep = torch.arange(s, device="cuda")[None, :] <= torch.arange(s - t, s, device="cuda")[:, None]
+    want = torch.einsum("bhts,bsr->bthr", torch.softmax(score.masked_fill(~keep, float("-inf")), dim=-1), lat.double())
+    assert rel(got, want) < 1e-6                                  # sums of a few hundred fp32 products; 3e-7 when every product is an fp32 one
+
+
 @pytest.mark.parametrize("rows,n,k", [(1, 16, 32), (8, 576, 1024), (9, 8, 96), (17, 2624, 1024), (32, 24, 64)])
 def test_rows_linear_matches_matmul(rows, n, k):
     from gpt_moe_b200.ops import cuda_ops
