@@ -53,7 +53,7 @@ cudaError_t launch_attn_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const 
                             const CUtensorMap& tdq, const AttnParams& p, const void* d_out, const void* out, long long do_stride,
                             long long o_stride, float* delta, cudaStream_t stream);
 
-// Prefill over expanded latent keys (mla_prefill.cu): maps with 64 x 128 boxes of the queries [B, T, H * 128], the key and value terms
+// Prefill over expanded latent keys (mla_prefill.cu): maps with 64 x 128 boxes of the queries [2 terms x B, T, H * 128], the key and value terms
 // [B, S, Hk * 64] and the rotary keys [B, S, 64]; positions count from `base`.
 struct MlaCachedArgs;
 cudaError_t launch_mla_prefill_attention(const MlaCachedArgs& a, int base, const CUtensorMap& tq, const CUtensorMap& tkh, const CUtensorMap& tkl, const CUtensorMap& trope,

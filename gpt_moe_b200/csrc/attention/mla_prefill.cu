@@ -5,9 +5,8 @@
 //   k_content[s, h] = W_k[h] latent[s],  v[s, h] = W_v[h] latent[s]          (2 x 64 columns per head),
 // and attend with 64 + 64-wide keys and 64-wide values: at rank 512 an eighth of the operations, on 128-row tcgen05 tiles.
 // The numbers that are fp32 in the absorbed form keep more than its precision: W as two bf16 terms (16 bits of mantissa) in the
-// expansion, whose fp32 sums are split into two bf16 terms per key and value, probabilities as two terms; products of a high and a low
-// part are kept, fp32 accumulation throughout.  Queries are rounded to bf16 once, after rotation and gain (the latent and the
-// rotary key are bf16 in the cache).
+// expansion, whose fp32 sums are split into two bf16 terms per key and value, queries (after rotation and gain) and probabilities as two
+// terms; products of a high and a low part are kept, fp32 accumulation throughout.  The latent and the rotary key are bf16 in the cache.
 // Launches: split_terms (W's two terms, formed in every call: nothing of a weight is kept), mla_prefill_prepare (latent norm, rotations, query gains, cache rows of the new tokens), two GEMMs (gemm_bf16.cu: W's high and
 // low term, the second accumulating), mla_prefill_split (key gains of the new tokens, terms of keys and values), mla_prefill_attention.
 // Measured (16 heads, rank 512, 2 x 512 tokens after 1500), layer with its projections: 160 us, 152 of them kernels (attention 55, GEMMs 74, split 14,
@@ -34,8 +33,8 @@ struct PrefillPrepareParams {
     const float *norm_w, *cos, *sin, *q_scale;   // tables: row of the first new position
     __nv_bfloat16 *latent, *rope;                // cache rows of the first new position
     long long latent_bs, rope_bs;
-    __nv_bfloat16* q_out;                        // [tokens, H * 128]
-    int T, H, r, rms;
+    __nv_bfloat16* q_out;                        // [2 terms, tokens, H * 128]
+    int tokens, T, H, r, rms;
     float norm_eps, qk_eps, smin, smax;
 };
 
@@ -74,10 +73,14 @@ mla_prefill_prepare_kernel(const PrefillPrepareParams p) {
             const float sq = pf_warp_sum(a.x * a.x + a.y * a.y + d.x * d.x + d.y * d.y);       // a rotation keeps the norm
             gain = rsqrtf((p.rms ? sq / 128.f : sq) + p.qk_eps) * fminf(fmaxf(p.q_scale[h], p.smin), p.smax);
         }
-        uint2 o;
-        o.x = pack_bf16x2((a.x * c0 - a.y * s0) * gain, (a.x * s0 + a.y * c0) * gain);
-        o.y = pack_bf16x2((d.x * c1 - d.y * s1) * gain, (d.x * s1 + d.y * c1) * gain);
-        *reinterpret_cast<uint2*>(p.q_out + static_cast<long long>(tok) * p.H * 128 + h * 128 + lane * 4) = o;
+        const float x0 = (a.x * c0 - a.y * s0) * gain, x1 = (a.x * s0 + a.y * c0) * gain;
+        const float x2 = (d.x * c1 - d.y * s1) * gain, x3 = (d.x * s1 + d.y * c1) * gain;
+        const uint32_t hi0 = pack_bf16x2(x0, x1), hi1 = pack_bf16x2(x2, x3);
+        __nv_bfloat16* out = p.q_out + static_cast<long long>(tok) * p.H * 128 + h * 128 + lane * 4;
+        *reinterpret_cast<uint2*>(out) = make_uint2(hi0, hi1);
+        *reinterpret_cast<uint2*>(out + static_cast<long long>(p.tokens) * p.H * 128) =
+            make_uint2(pack_bf16x2(x0 - __uint_as_float(hi0 << 16), x1 - __uint_as_float(hi0 & 0xffff0000u)),
+                       pack_bf16x2(x2 - __uint_as_float(hi1 << 16), x3 - __uint_as_float(hi1 & 0xffff0000u)));
     }
 }
 
@@ -140,9 +143,10 @@ mla_prefill_split_kernel(const PrefillSplitParams p) {
 constexpr int PF_M = 128, PF_N = 128, PF_THREADS = 288;
 constexpr int PF_SLAB = 128 * 64 * 2;            // 128 rows x 64 bf16 columns
 constexpr int PF_STAGES = 2;
+constexpr int PF_Q_BYTES = 4 * PF_SLAB;          // content and rotary columns, high terms then low
 constexpr int PF_K_BYTES = 3 * PF_SLAB, PF_V_BYTES = 2 * PF_SLAB;      // content high, low and rotary; value high, low
 constexpr uint32_t PF_TMEM_COLS = 512;
-constexpr int PF_SMEM = 2 * PF_SLAB + PF_STAGES * (PF_K_BYTES + PF_V_BYTES) + 1024 + 128 + 2 * PF_M * 4;
+constexpr int PF_SMEM = PF_Q_BYTES + PF_STAGES * (PF_K_BYTES + PF_V_BYTES) + 1024 + 128 + 2 * PF_M * 4;
 static_assert(PF_SMEM <= 232448, "shared memory of the prefill attention");
 
 struct PrefillAttnParams {
@@ -153,8 +157,8 @@ struct PrefillAttnParams {
 };
 
 // The roles, barriers and the running softmax are those of attn_fwd_kernel (attn_fwd.cu): warp 8 loads and issues, warps 0-7 are the
-// softmax warps, w and w + 4 sharing the rows of a TMEM quadrant.  Different here: a score is the sum of three products (query content with
-// both terms of the key, query rotary with the shared rotary key) times the key's gain, which every thread reads as it goes (all
+// softmax warps, w and w + 4 sharing the rows of a TMEM quadrant.  Different here: a score is the sum of five products (query content with
+// both terms of the key, the low term of the query with the high one, both terms of the query's rotary part with the shared rotary key) times the key's gain, which every thread reads as it goes (all
 // rows read the same one: one cache line per 32 keys); probabilities leave as two terms; P V is lo*hi + hi*lo + hi*hi.
 __global__ void __launch_bounds__(PF_THREADS, 1)
 mla_prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_kh, const __grid_constant__ CUtensorMap tmap_kl,
@@ -163,7 +167,7 @@ mla_prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const _
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sq = smem;
-    uint8_t* sk = sq + 2 * PF_SLAB;
+    uint8_t* sk = sq + PF_Q_BYTES;
     uint8_t* sv = sk + PF_STAGES * PF_K_BYTES;
     uint64_t* bars = reinterpret_cast<uint64_t*>(sv + PF_STAGES * PF_V_BYTES);
     uint64_t *bar_q = bars, *bar_s = bars + 1, *bar_p = bars + 2, *bar_o = bars + 3, *bar_k = bars + 4, *bar_v = bar_k + PF_STAGES;
@@ -201,11 +205,12 @@ mla_prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const _
             auto issue_s = [&](int st) {
                 const uint64_t kd = k_desc + st * (PF_K_BYTES >> 4);
 #pragma unroll
-                for (int part = 0; part < 3; ++part)                 // content x low term, content x high term, rotary
+                for (int part = 0; part < 5; ++part) {               // small ones first: Q K low, Q low K, Q low rotary; Q K, Q rotary
+                    constexpr int q_slab[5] = {0, 2, 3, 0, 1}, k_slab[5] = {1, 0, 2, 0, 2};
 #pragma unroll
                     for (int k4 = 0; k4 < 4; ++k4)
-                        umma_f16(tmem_s, q_desc + (part == 2 ? (PF_SLAB >> 4) : 0) + k4 * 2,
-                                 kd + (part == 0 ? (PF_SLAB >> 4) : part == 1 ? 0 : 2 * (PF_SLAB >> 4)) + k4 * 2, idesc_s, (part | k4) != 0);
+                        umma_f16(tmem_s, q_desc + q_slab[part] * (PF_SLAB >> 4) + k4 * 2, kd + k_slab[part] * (PF_SLAB >> 4) + k4 * 2, idesc_s, (part | k4) != 0);
+                }
                 umma_commit(bar_s);
             };
             auto load_k = [&](int tile) {
@@ -223,9 +228,10 @@ mla_prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const _
                 tma_load_3d(dst, &tmap_vh, &bar_v[st], kv_head * 64, lo + tile * PF_N, batch);
                 tma_load_3d(dst + PF_SLAB, &tmap_vl, &bar_v[st], kv_head * 64, lo + tile * PF_N, batch);
             };
-            mbar_expect_tx(bar_q, 2 * PF_SLAB);
-            tma_load_3d(sq, &tmap_q, bar_q, head * 128, q0, batch);
-            tma_load_3d(sq + PF_SLAB, &tmap_q, bar_q, head * 128 + 64, q0, batch);
+            mbar_expect_tx(bar_q, PF_Q_BYTES);
+#pragma unroll
+            for (int sl = 0; sl < 4; ++sl)
+                tma_load_3d(sq + sl * PF_SLAB, &tmap_q, bar_q, head * 128 + (sl & 1) * 64, q0, batch + (sl >> 1) * gridDim.y);
             for (int t = 0; t < PF_STAGES && t < n_tiles; ++t) { load_k(t); load_v(t); }
             if (!mbar_wait(bar_q, 0) || !mbar_wait(&bar_k[0], 0)) { atomicExch(p.status, 231); ok = false; }
             if (ok) { tc_fence_after(); issue_s(0); }
@@ -393,7 +399,7 @@ void launch_mla_prefill_prepare(const MlaCachedArgs& a, void* q_out, cudaStream_
     p.rope = static_cast<__nv_bfloat16*>(a.rope) + static_cast<long long>(a.start) * 64;
     p.latent_bs = a.latent_bs; p.rope_bs = a.rope_bs;
     p.q_out = static_cast<__nv_bfloat16*>(q_out);
-    p.T = a.T; p.H = a.H; p.r = a.r; p.rms = a.rms; p.norm_eps = a.norm_eps; p.qk_eps = a.qk_eps; p.smin = a.smin; p.smax = a.smax;
+    p.tokens = a.B * a.T; p.T = a.T; p.H = a.H; p.r = a.r; p.rms = a.rms; p.norm_eps = a.norm_eps; p.qk_eps = a.qk_eps; p.smin = a.smin; p.smax = a.smax;
     mla_prefill_prepare_kernel<<<a.B * a.T, 256, 0, s>>>(p);
 }
 

@@ -341,7 +341,7 @@ Tensor mla_prefill(const MlaCachedArgs& args, const Tensor& latent) {
     const int base = a.window < 0 ? 0 : std::max(0, a.start - a.window) / 128 * 128;      // first position any query sees, on a tile's edge
     const int S = end - base, S_pad = (S + 127) / 128 * 128;
     auto bf = latent.options();
-    Tensor q = gm::out_empty({a.B, a.T, a.H * 128}, bf);
+    Tensor q = gm::out_empty({2 * a.B, a.T, a.H * 128}, bf);              // high terms, then low ones
     launch_mla_prefill_prepare(a, q.data_ptr(), stream());
     Tensor kv = gm::out_empty({a.B, S, a.Hkv * 128}, bf.dtype(torch::kFloat32));
     // W as two bf16 terms: 8 MB moved in a call that expands thousands of positions with them, so nothing of the weight is kept between calls
@@ -358,7 +358,7 @@ Tensor mla_prefill(const MlaCachedArgs& args, const Tensor& latent) {
     Tensor out = gm::out_empty({static_cast<int64_t>(a.B) * a.T, a.H * 64}, bf);
     a.out = out.data_ptr();
     auto term_map = [&](int i) { return rows_map(parts[i], a.Hkv * 64, S, a.B, a.Hkv * 64, static_cast<uint64_t>(S) * a.Hkv * 64); };
-    const CUtensorMap tq = rows_map(q.data_ptr(), a.H * 128, a.T, a.B, a.H * 128, static_cast<uint64_t>(a.T) * a.H * 128);
+    const CUtensorMap tq = rows_map(q.data_ptr(), a.H * 128, a.T, 2 * a.B, a.H * 128, static_cast<uint64_t>(a.T) * a.H * 128);
     const CUtensorMap tr = rows_map(static_cast<const uint16_t*>(a.rope) + static_cast<int64_t>(base) * 64, 64, S, a.B, 64, a.rope_bs);
     cudaError_t e = launch_mla_prefill_attention(a, base, tq, term_map(0), term_map(1), tr, term_map(2), term_map(3), gain.data_ptr<float>(), S, S_pad,
                                                  status_word(latent.device().index()), stream());

@@ -167,6 +167,37 @@ def test_a_context_in_fp32_has_the_bits_of_fp32(b, t, h, hkv, r, dr, s):
     assert rel(got, want) < 1e-6                                  # sums of a few hundred fp32 products; 3e-7 when every product is an fp32 one
 
 
+@pytest.mark.parametrize("expanded", [True, False])
+@pytest.mark.parametrize("b,t,h,hkv,r,start", [(1, 200, 8, 8, 256, 300), (2, 130, 16, 4, 512, 60)])
+def test_only_the_output_is_rounded_to_bf16(b, t, h, hkv, r, start, expanded):
+    """Against 64 bits on what lies in the cache afterwards: queries, keys, probabilities and values keep more bits than bf16 in both forms."""
+    from gpt_moe_b200.ops import cuda_ops
+    torch.manual_seed(16)
+    end = start + t
+    width = h * 128 + (0 if expanded else 2)                        # rows on no 8-byte boundary stay with the absorbed form
+    query = (2 * torch.randn(b * t, width, device="cuda")).bfloat16()[:, :h * 128]
+    low = torch.randn(b * t, r + 64, device="cuda").bfloat16()
+    w = torch.randn(hkv * 128, r, device="cuda") * r ** -0.5
+    cos, sin = torch.rand(end, 32, device="cuda"), torch.rand(end, 32, device="cuda")
+    qs, ks = torch.linspace(0.5, 3.0, h, device="cuda"), torch.linspace(0.5, 2.0, hkv, device="cuda")
+    lat, rope = torch.randn(b, end, r, device="cuda").bfloat16(), torch.randn(b, end, 64, device="cuda").bfloat16()
+    gain = (torch.rand(b, end, hkv, device="cuda") + 0.5).bfloat16()
+    assert cuda_ops.ext().mla_prefill_wanted(b, t, end, -1, r, 64, 64, 64, 0.0)
+    got = cuda_ops.ext().mla_cached(query, low, w, None, 1e-6, cos, sin, qs, ks, 1e-6, True, -3e38, 3e38, lat, rope, gain, start, h, 64, 64, 128 ** -0.5, 0.0, -1)
+    q = query.double().view(b, t, h, 128)
+    norm = torch.rsqrt(q.pow(2).mean(-1, keepdim=True) + 1e-6) * qs.double().view(1, 1, -1, 1)
+    x0, x1 = q[..., 64::2], q[..., 65::2]
+    c, s = (m[start:].double()[None, :, None] for m in (cos, sin))
+    q = torch.cat((q[..., :64], torch.stack((x0 * c - x1 * s, x0 * s + x1 * c), dim=-1).flatten(-2)), dim=-1) * norm
+    kv = torch.einsum("bsr,hdr->bshd", lat.double(), w.double().view(hkv, 128, r))
+    key = torch.cat((kv[..., :64], rope.double()[:, :, None].expand(-1, -1, hkv, -1)), dim=-1) * gain.double()[..., None]
+    score = torch.einsum("bthd,bshd->bhts", q, key.repeat_interleave(h // hkv, dim=2)) * 128 ** -0.5
+    keep = torch.arange(end, device="cuda")[None, :] <= torch.arange(start, end, device="cuda")[:, None]
+    want = torch.einsum("bhts,bshd->bthd", torch.softmax(score.masked_fill(~keep, float("-inf")), dim=-1), kv[..., 64:].repeat_interleave(h // hkv, dim=2))
+    assert rel(got.view(b, t, h, 64), want) < 1.8e-3                # the rounding itself: 1.65e-3 of the norm; one of the queries alone adds as much
+    cuda_ops.check_status()
+
+
 @pytest.mark.parametrize("rows,n,k", [(1, 16, 32), (8, 576, 1024), (9, 8, 96), (17, 2624, 1024), (32, 24, 64)])
 def test_rows_linear_matches_matmul(rows, n, k):
     from gpt_moe_b200.ops import cuda_ops
