@@ -383,13 +383,14 @@ attn_fwd_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
 }
 
 bool attn_fwd_dual_supported(const AttnParams& p) {
-    // Windowed calls, where two query tiles share most of their keys: 16 x 2048 tokens, window 1024 225 us against 238 for the single-tile
-    // kernel; also with an odd number of tiles, where half of the last CTA idles, once there are nine (26.9 against 31.7).  Without
-    // a window the single-tile kernel's finer grain fills the end of the grid better: 16384 tokens 955 us against 1060, 4 x 4096 285
-    // against 303, 13 tiles 52.9 against 57.8; up to 16 tiles an even number is equal or better here (2 tiles 51 against 63).
-    const int tiles = (p.seq_len + DU_BM - 1) / DU_BM;
+    // Whole pairs of tiles.  Windowed calls, where two query tiles share most of their keys: 16 x 2048 tokens, window 1024 225 us against 238
+    // for the single-tile kernel.  Without a window the single-tile kernel's finer grain fills the end of the grid better: 16384 tokens
+    // 955 us against 1060, 4 x 4096 285 against 303; up to 16 tiles this one is equal or better (2 tiles 51 against 63).
+    // Other lengths run the single-tile kernel, whose row maximum is exact in every tile: here it may lag by up to 2^8, the largest
+    // probabilities are then no longer 1 (which bf16 holds exactly), and windowed outputs lie 1.5 to 4 % further from 64 bits (5 x 1000 tokens,
+    // window 256: 2.10e-3 against 2.05e-3, which is also what the library kernel had that used to serve these lengths).
     const bool windowed = p.window <= p.seq_len / 2;
-    return p.qk_dim == 64 && p.doc_start == nullptr && (windowed ? tiles % 2 == 0 || tiles >= 9 : tiles % 2 == 0 && tiles <= 16);
+    return p.qk_dim == 64 && p.doc_start == nullptr && p.seq_len % (2 * DU_BM) == 0 && (windowed || p.seq_len <= 16 * DU_BM);
 }
 
 template <bool CAPPED>

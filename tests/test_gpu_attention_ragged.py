@@ -13,7 +13,7 @@ def rel(a, b):
     return ((a - b).norm() / b.norm().clamp_min(1e-30)).item()
 
 
-# one row, inside a tile, edges of one and two tiles, an odd number of tiles on both sides of the two-tile kernel's rule
+# one row, inside a tile, edges of one and two tiles, odd and even numbers of tiles
 @pytest.mark.parametrize("t,window,hq,hk,d", [(1, None, 2, 2, 64), (45, None, 4, 4, 64), (127, 20, 2, 1, 64), (129, None, 4, 2, 64),
                                                (184, 64, 2, 2, 64), (300, None, 2, 2, 64), (1000, 256, 3, 3, 64), (1100, None, 2, 1, 64),
                                                (45, None, 2, 2, 128), (333, 100, 2, 1, 128)])
@@ -57,3 +57,17 @@ def test_any_length_with_document_mask(t):
     for got, exp in zip(grads, torch.autograd.grad(want, want_in, g.float())):
         assert rel(got, exp) < 1e-2
     cuda_ops.check_status()
+
+
+@pytest.mark.parametrize("t,window,pairs", [(200, 50, False), (1000, 256, False), (1152, 256, False), (250, None, False), (1280, 256, True), (512, None, True)])
+def test_lengths_without_whole_pairs_of_tiles_keep_the_exact_maximum(t, window, pairs):
+    torch.manual_seed(7)
+    q, k, v = (torch.nn.functional.rms_norm(torch.randn(2, t, 4, 64, device="cuda"), (64,)).bfloat16() for _ in range(3))
+    w = t if window is None else window
+    out, lse = cuda_ops.ext().attn_fwd(q, k, v, w, 0.125)
+    single, lse1 = cuda_ops.ext().attn_fwd(q, k, v, w, 0.125, single_tile=True)
+    assert torch.equal(out, single) == (not pairs)
+    want = ref.attention(q.double(), k.double(), v.double(), causal=True, window=window)
+    library = torch.nn.functional.scaled_dot_product_attention(*(x.transpose(1, 2) for x in (q, k, v)), attn_mask=ref.attention_mask(t, q.device, True, window)).transpose(1, 2)
+    if not pairs:
+        assert rel(out, want) < 1.02 * max(rel(library, want), 2.03e-3)
