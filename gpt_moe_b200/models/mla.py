@@ -227,21 +227,20 @@ class MLAttention(nn.Module):
         out = torch.einsum("bthgr,hdr->bthgd", context, w_v).reshape(b, t, self.attn_dim)
         return self.out_proj(out.to(x.dtype))
 
-
     def _cached_on_gpu(self, x: Tensor, cache: MLACache, start: int, window: Optional[int]) -> Optional[Tensor]:
         """The cached step as five launches (`csrc/attention/mla_decode.cu`): projections; norm, rotation, QK gains, absorbed
         queries and the cache entries; attention over the cache in splits; merge and W_v; output projection.  The general path
         of `forward_cached` issues some sixty.  None when a shape, type or option needs that path."""
+        from ..ops import cuda_ops
         b, t, hidden = x.shape
         caches = (cache.latent, cache.rope, cache.key_gain)
         w_up = self.kv_up_proj.weight
-        if not (x.is_cuda and self.rotary is not None and 0 < b * t <= 131072 and all(c.dtype == torch.bfloat16 and c.is_cuda and c.stride(2) == 1
+        if not (x.is_cuda and cuda_ops.plain_call() and self.rotary is not None and 0 < b * t <= 131072 and all(c.dtype == torch.bfloat16 and c.is_cuda and c.stride(2) == 1
                 and c.stride(1) == c.size(2) for c in caches) and all(m.bias is None for m in (self.q_proj, self.kv_down_proj, self.kv_up_proj))
                 and w_up.dtype == torch.float32 and w_up.is_contiguous() and w_up.data_ptr() % 16 == 0 and self.content_dim <= 256
                 and (self.softcap <= 0.0 or self.tanh_backend == "exact") and start + t <= self.rotary.cos_cached.shape[0]
                 and cache.rope.size(1) == cache.latent.size(1) == cache.key_gain.size(1) and self.rotary.cos_cached.dtype == torch.float32):
             return None
-        from ..ops import cuda_ops
         c = cuda_ops.ext()
         if not c.mla_decode_ok(self.n_heads, self.n_kv_heads, self.kv_rank, self.rope_dim):
             return None

@@ -123,6 +123,16 @@ def test_a_weight_written_behind_torchs_back_is_seen(t):
     assert torch.equal(second, call(copy.deepcopy(attn)))
 
 
+def test_a_tangent_is_not_dropped():
+    gc, tc = get_preset("mla")
+    gc.hidden_size, gc.n_heads, gc.n_kv_heads = 256, 8, 8
+    tc.resolve(1)
+    attn = MLAttention(gc, tc).cuda().eval()
+    x = torch.randn(1, 4, 256, device="cuda").bfloat16()
+    with torch.no_grad(), pytest.raises(RuntimeError):          # the projections have no rule for forward mode and say so
+        torch.func.jvp(lambda y: attn.forward_cached(y, attn.allocate_cache(1, 8, device="cuda", dtype=torch.bfloat16)), (x,), (x,))
+
+
 # grids of more than 65535 groups of rows or sequences; a window of zero positions keeps the work small
 @pytest.mark.parametrize("b,t,h,r", [(1, 131072, 16, 768), (1, 65600, 32, 256), (65600, 1, 8, 256)])
 def test_more_rows_than_a_grid_dimension_holds(b, t, h, r):
