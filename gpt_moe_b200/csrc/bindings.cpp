@@ -94,11 +94,12 @@ CUtensorMap operand_map(const torch::Tensor& t, bool mn_major, int tile_rows_k_m
 //   mode 0 (dense): a, b and d with the same batch, or one 2-D b for a whole batch
 //   mode 1 (grouped M): a [rows, K], b [E, N, K] or [E, K, N], d [rows, N]; tile_expert/num_m_tiles on device
 //   mode 2 (grouped K): a [rows, M] (a_mn), b [rows, N] (b_mn), d [E, M, N]; seg_ends on device
-void gemm_bf16(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d, bool a_mn, bool b_mn, double alpha,
-               double beta, const c10::optional<torch::Tensor>& c, bool accumulate, int64_t mode,
-               const c10::optional<torch::Tensor>& tile_expert, const c10::optional<torch::Tensor>& num_m_tiles,
-               const c10::optional<torch::Tensor>& seg_ends, bool symmetric, const c10::optional<torch::Tensor>& batch_sumsq,
-               int64_t scale_mode) {
+//   may_split: a long contraction with few output tiles may be shared by several CTAs, whose partial results meet in the order of arrival
+void gemm_run(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d, bool a_mn, bool b_mn, double alpha,
+              double beta, const c10::optional<torch::Tensor>& c, bool accumulate, int64_t mode,
+              const c10::optional<torch::Tensor>& tile_expert, const c10::optional<torch::Tensor>& num_m_tiles,
+              const c10::optional<torch::Tensor>& seg_ends, bool symmetric, const c10::optional<torch::Tensor>& batch_sumsq,
+              int64_t scale_mode, bool may_split) {
     c10::cuda::CUDAGuard guard(a.device());
     gm::GemmParams p;
     std::memset(&p, 0, sizeof(p));
@@ -160,7 +161,7 @@ void gemm_bf16(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d,
     p.status = status_tensor(a.device().index()).data_ptr<int>();
     // split-K: a long contraction with too few output tiles to fill the GPU (weight gradients) is shared by several CTAs per tile
     p.split_k = 1;
-    if (mode == gm::GEMM_DENSE && p.out_fp32) {
+    if (mode == gm::GEMM_DENSE && p.out_fp32 && may_split) {
         const int64_t tiles = ((p.M + 255) / 256) * 2 * ((p.N + 255) / 256) * p.batch;      // CTA pairs own 256-row tiles
         const int64_t k_blocks = (p.K + 63) / 64;
         if (tiles * 2 <= sm_count() && k_blocks >= 16)
@@ -183,6 +184,12 @@ void gemm_bf16(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d,
     cudaError_t e = gm::launch_gemm_bf16(ta, tb, td, tma_c ? &tc : nullptr, tma_c && p.symmetric ? &tmirror : nullptr, p, a_mn, b_mn, sm_count(),
                                          current_stream());
     GM_CHECK(e == cudaSuccess, cudaGetErrorString(e));
+}
+void gemm_bf16(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d, bool a_mn, bool b_mn, double alpha, double beta,
+               const c10::optional<torch::Tensor>& c, bool accumulate, int64_t mode, const c10::optional<torch::Tensor>& tile_expert,
+               const c10::optional<torch::Tensor>& num_m_tiles, const c10::optional<torch::Tensor>& seg_ends, bool symmetric,
+               const c10::optional<torch::Tensor>& batch_sumsq, int64_t scale_mode) {
+    gemm_run(a, b, d, a_mn, b_mn, alpha, beta, c, accumulate, mode, tile_expert, num_m_tiles, seg_ends, symmetric, batch_sumsq, scale_mode, true);
 }
 
 // ---- MXFP8 ----------------------------------------------------------------------------------------
@@ -395,7 +402,7 @@ void gemm_by_expert(const torch::Tensor& a, const torch::Tensor& b, torch::Tenso
     gemm_bf16(a, b, d, false, false, 1.0, 0.0, c10::nullopt, false, GEMM_GROUPED_M, tile_expert, meta, c10::nullopt, false, c10::nullopt, 0);
 }
 void gemm_fp32(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d, bool accumulate) {
-    gemm_bf16(a, b, d, false, false, 1.0, 0.0, c10::nullopt, accumulate, GEMM_DENSE, c10::nullopt, c10::nullopt, c10::nullopt, false, c10::nullopt, 0);
+    gemm_run(a, b, d, false, false, 1.0, 0.0, c10::nullopt, accumulate, GEMM_DENSE, c10::nullopt, c10::nullopt, c10::nullopt, false, c10::nullopt, 0, false);
 }
 CUtensorMap rows_map(const void* base, uint64_t cols, uint64_t rows, uint64_t batch, uint64_t row_pitch, uint64_t batch_pitch) {
     return cached_map(base, 2, cols, rows, batch, row_pitch * 2, batch_pitch * 2, 64, 128, 128);

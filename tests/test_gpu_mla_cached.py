@@ -76,8 +76,8 @@ def test_cached_step_matches_the_plain_path(b, t, h, hkv, r, dr, c, start, windo
     cuda_ops.check_status()
 
 
-# an exactly full cache, one with room; a window that starts inside it; a rank whose expansion splits its contraction
-@pytest.mark.parametrize("start,t,r,window", [(200, 130, 512, None), (333, 256, 256, 70), (1000, 128, 1024, None)])
+# an exactly full cache, one with room; a window that starts inside it; a rank whose contraction is long for its few tiles
+@pytest.mark.parametrize("start,t,r,window", [(1000, 130, 512, None), (633, 512, 256, 200), (1000, 128, 1024, None)])
 def test_a_batch_expands_as_its_sequences_do(start, t, r, window):
     torch.manual_seed(14)
     gc, tc = get_preset("mla")
@@ -99,8 +99,7 @@ def test_a_batch_expands_as_its_sequences_do(start, t, r, window):
     assert cuda_ops.ext().mla_prefill_wanted(1, t, start + t, -1 if window is None else window, r, 64, 64, 64, 0.0)
     full, roomy = call(slice(0, 3), 0), call(slice(0, 3), 77)
     alone = torch.cat([call(slice(i, i + 1), 5) for i in range(3)])
-    assert torch.equal(full, roomy)
-    assert rel(full, alone) < (1e-3 if r == 1024 else 1e-12)       # split contractions meet in the order of arrival, in fp32
+    assert torch.equal(full, roomy) and torch.equal(full, alone)
     cuda_ops.check_status()
 
 
@@ -178,7 +177,7 @@ def test_a_context_in_fp32_has_the_bits_of_fp32(b, t, h, hkv, r, dr, s):
 
 
 @pytest.mark.parametrize("expanded", [True, False])
-@pytest.mark.parametrize("b,t,h,hkv,r,start", [(1, 200, 8, 8, 256, 300), (2, 130, 16, 4, 512, 60)])
+@pytest.mark.parametrize("b,t,h,hkv,r,start", [(1, 500, 8, 8, 256, 300), (2, 130, 16, 4, 512, 360)])
 def test_only_the_output_is_rounded_to_bf16(b, t, h, hkv, r, start, expanded):
     """Against 64 bits on what lies in the cache afterwards: queries, keys, probabilities and values keep more bits than bf16 in both forms."""
     from gpt_moe_b200.ops import cuda_ops
