@@ -73,6 +73,27 @@ __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], 
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+// Two neighbouring column tiles: d += sum over the terms of a * b, smallest first.  The tensor core cuts a sum off instead of rounding it, which adds up over a long chain:
+// three terms, which are there for the last bits, form each step's sum from zero and add it in fp32.
+template <int TERMS>
+__device__ __forceinline__ void mma_terms(float (&d0)[4], float (&d1)[4], const uint32_t (&a)[TERMS][4], const uint32_t (&b)[4]) {
+    if constexpr (TERMS == 3) {
+        float p0[4] = {0.f, 0.f, 0.f, 0.f}, p1[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int t = TERMS - 1; t >= 0; --t) {
+            mma16816(p0, a[t], b[0], b[1]);
+            mma16816(p1, a[t], b[2], b[3]);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { d0[e] += p0[e]; d1[e] += p1[e]; }
+    } else {
+#pragma unroll
+        for (int t = TERMS - 1; t >= 0; --t) {
+            mma16816(d0, a[t], b[0], b[1]);
+            mma16816(d1, a[t], b[2], b[3]);
+        }
+    }
+}
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {      // zeros when not valid
     const int bytes = valid ? 16 : 0;
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
@@ -252,12 +273,7 @@ mla_decode_split_kernel(const MlaDecodeParams p) {
                 uint32_t bf[4];
                 ldsm_x4(bf, lat_a + (np * 16 + key_l) * LAT_PITCH + ks * 32 + col_l);
 #pragma unroll
-                for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-                    for (int term = MD_TERMS - 1; term >= 0; --term) {
-                        mma16816(sc[mt][np * 2], qa[mt][ks][term], bf[0], bf[1]);
-                        mma16816(sc[mt][np * 2 + 1], qa[mt][ks][term], bf[2], bf[3]);
-                    }
+                for (int mt = 0; mt < MT; ++mt) mma_terms(sc[mt][np * 2], sc[mt][np * 2 + 1], qa[mt][ks], bf);
             }
         if (has_rope) {
 #pragma unroll
@@ -265,12 +281,7 @@ mla_decode_split_kernel(const MlaDecodeParams p) {
                 uint32_t bf[4];
                 ldsm_x4(bf, rope_a + (np * 16 + key_l) * ROPE_PITCH + col_l);
 #pragma unroll
-                for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-                    for (int term = MD_TERMS - 1; term >= 0; --term) {
-                        mma16816(sc[mt][np * 2], qr[mt][term], bf[0], bf[1]);
-                        mma16816(sc[mt][np * 2 + 1], qr[mt][term], bf[2], bf[3]);
-                    }
+                for (int mt = 0; mt < MT; ++mt) mma_terms(sc[mt][np * 2], sc[mt][np * 2 + 1], qr[mt], bf);
             }
         }
 #pragma unroll
@@ -336,12 +347,7 @@ mla_decode_split_kernel(const MlaDecodeParams p) {
                 uint32_t bf[4];
                 ldsm_x4_t(bf, lat_a + (ks * 16 + (lane & 15)) * LAT_PITCH + np * 32 + (lane >> 4) * 16);
 #pragma unroll
-                for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-                    for (int term = MD_TERMS - 1; term >= 0; --term) {
-                        mma16816(acc[mt][np * 2], pa[mt][term], bf[0], bf[1]);
-                        mma16816(acc[mt][np * 2 + 1], pa[mt][term], bf[2], bf[3]);
-                    }
+                for (int mt = 0; mt < MT; ++mt) mma_terms(acc[mt][np * 2], acc[mt][np * 2 + 1], pa[mt], bf);
             }
         }
     }

@@ -161,7 +161,7 @@ def test_more_rows_than_a_grid_dimension_holds(b, t, h, r):
 
 
 # one and two tiles of rows, every rank
-@pytest.mark.parametrize("b,t,h,hkv,r,dr,s", [(2, 1, 16, 16, 512, 64, 777), (1, 5, 8, 2, 256, 32, 300), (2, 1, 32, 32, 512, 64, 130), (1, 2, 16, 4, 768, 64, 500), (1, 1, 8, 8, 1024, 10, 90)])
+@pytest.mark.parametrize("b,t,h,hkv,r,dr,s", [(2, 1, 16, 16, 512, 64, 777), (4, 1, 16, 16, 512, 64, 4022), (1, 5, 8, 2, 256, 32, 300), (2, 1, 32, 32, 512, 64, 130), (1, 2, 16, 4, 768, 64, 500), (1, 1, 8, 8, 1024, 10, 90)])
 def test_a_context_in_fp32_has_the_bits_of_fp32(b, t, h, hkv, r, dr, s):
     from gpt_moe_b200.models.mla import api_mla_decode
     torch.manual_seed(15)
@@ -173,7 +173,7 @@ def test_a_context_in_fp32_has_the_bits_of_fp32(b, t, h, hkv, r, dr, s):
     score = score * gain.double().permute(0, 2, 1).repeat_interleave(h // hkv, dim=1)[:, :, None, :] * 0.08
     keep = torch.arange(s, device="cuda")[None, :] <= torch.arange(s - t, s, device="cuda")[:, None]
     want = torch.einsum("bhts,bsr->bthr", torch.softmax(score.masked_fill(~keep, float("-inf")), dim=-1), lat.double())
-    assert rel(got, want) < 1e-6                                  # sums of a few hundred fp32 products; 3e-7 when every product is an fp32 one
+    assert rel(got, want) < 6e-7                                  # 2e-7 to 4e-7 with fp32 products and sums throughout
 
 
 @pytest.mark.parametrize("expanded", [True, False])
