@@ -1,8 +1,8 @@
 // Causal sliding-window attention backward for sm_100a, 64-wide heads, with the score products of the next query tile issued
 // ahead of the gradient products of the current one.
 //
-// Same tiling and products as attn_bwd.cu (sequences of any length: the tensor maps end at the sequence's last row; one CTA owns 128 keys of one (batch, kv head) and walks the query tiles that see
-// them; S = Q K^T and dP = dO V^T into TMEM, P and dS to shared memory, dV += P^T dO, dK += dS^T Q, dQ = dS K reduced into a
+// Same tiling and products as attn_bwd.cu (sequences of any length: the tensor maps end at the sequence's last row; one CTA owns 128 keys
+// of one (batch, kv head) and walks the query tiles that see them; S = Q K^T and dP = dO V^T into TMEM, P and dS to shared memory, dV += P^T dO, dK += dS^T Q, dQ = dS K reduced into a
 // fp32 buffer by TMA).  What differs is the order.  In attn_bwd.cu one iteration is a chain: S/dP -> softmax warps -> three
 // gradient products -> dQ read-out, and the S/dP of the next iteration queue behind the gradient products, so the tensor
 // core idles while the softmax warps work and the other way round (a tcgen05.mma with N = 64 takes about 56 clocks to issue

@@ -329,7 +329,7 @@ attn_fwd_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
                 const float inv = 1.f / l;
                 const long long token = static_cast<long long>(row0) + qpos;
                 __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.out) + token * p.out_stride + head * DU_D;
-    #pragma unroll
+#pragma unroll
                 for (int q = 0; q < 8; ++q) {
                     uint4 w;
                     w.x = pack_bf16x2(o[8 * q] * inv, o[8 * q + 1] * inv);
@@ -342,17 +342,17 @@ attn_fwd_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
                     // the thread's 64 output columns are two MXFP8 blocks of the token-major row: quantise the bf16 values just stored
                     // (reference: attention output quantised straight from its own layout, model/linear/fp8/custom/output_projection.py:16-49)
                     const int width = p.heads * DU_D;
-    #pragma unroll
+#pragma unroll
                     for (int blk = 0; blk < 2; ++blk) {
                         float amax = 0.f;
-    #pragma unroll
+#pragma unroll
                         for (int i = 0; i < 32; ++i) { o[32 * blk + i] = round_bf16(o[32 * blk + i] * inv); amax = fmaxf(amax, fabsf(o[32 * blk + i])); }
                         const uint32_t e8 = e8m0_from_amax(amax);
                         const float qs = inv_scale_from_e8m0(e8);
                         const int col = head * DU_D + 32 * blk;
                         uint8_t* dst = p.out_q + token * width + col;
                         const float* ob = o + 32 * blk;
-    #pragma unroll
+#pragma unroll
                         for (int q = 0; q < 2; ++q) {
                             uint4 w;
                             w.x = pack_e4m3x4(ob[16 * q] * qs, ob[16 * q + 1] * qs, ob[16 * q + 2] * qs, ob[16 * q + 3] * qs);

@@ -7,8 +7,9 @@
 // The numbers that are fp32 in the absorbed form keep more than its precision: W as two bf16 terms (16 bits of mantissa) in the
 // expansion, whose fp32 sums are split into two bf16 terms per key and value, queries (after rotation and gain) and probabilities as two
 // terms; products of a high and a low part are kept, fp32 accumulation throughout.  The latent and the rotary key are bf16 in the cache.
-// Launches: split_terms (W's two terms, formed in every call: nothing of a weight is kept), mla_prefill_prepare (latent norm, rotations, query gains, cache rows of the new tokens), two GEMMs (gemm_bf16.cu: W's high and
-// low term, the second accumulating), mla_prefill_split (key gains of the new tokens, terms of keys and values), mla_prefill_attention.
+// Launches: mla_prefill_prepare (latent norm, rotations, query gains, cache rows of the new tokens), split_terms (W's two terms, formed in
+// every call: nothing of a weight is kept), two GEMMs (gemm_bf16.cu: W's low and high term, the second accumulating), mla_prefill_split
+// (key gains of the new tokens, terms of keys and values), mla_prefill_attention.
 // Measured (16 heads, rank 512, 2 x 512 tokens after 1500), layer with its projections: 160 us, 152 of them kernels (attention 55, GEMMs 74, split 14,
 // prepare 10), against 1193 us for the absorbed kernels; error of the output against 64 bits 4.6e-3 (absorbed 4.1e-3, the fp32
 // formulation both replaced, whose W products ran in TF32, 5.9e-3).  mla_prefill_wanted in bindings_ops.cpp says which calls come here.
@@ -158,11 +159,11 @@ struct PrefillAttnParams {
 
 // The roles, barriers and the running softmax are those of attn_fwd_kernel (attn_fwd.cu): warp 8 loads and issues, warps 0-7 are the
 // softmax warps, w and w + 4 sharing the rows of a TMEM quadrant.  Different here: a score is the sum of five products (query content with
-// both terms of the key, the low term of the query with the high one, both terms of the query's rotary part with the shared rotary key) times the key's gain, which every thread reads as it goes (all
-// rows read the same one: one cache line per 32 keys); probabilities leave as two terms; P V is lo*hi + hi*lo + hi*hi.
+// both terms of the key, the low term of the query with the high one, both terms of the query's rotary part with the shared rotary key)
+// times the key's gain, which every thread reads as it goes (all rows read the same one: one cache line per 32 keys); probabilities leave as two terms; P V is lo*hi + hi*lo + hi*hi.
 __global__ void __launch_bounds__(PF_THREADS, 1)
-mla_prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_kh, const __grid_constant__ CUtensorMap tmap_kl,
-                             const __grid_constant__ CUtensorMap tmap_rope, const __grid_constant__ CUtensorMap tmap_vh,
+mla_prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_kh,
+                             const __grid_constant__ CUtensorMap tmap_kl, const __grid_constant__ CUtensorMap tmap_rope, const __grid_constant__ CUtensorMap tmap_vh,
                              const __grid_constant__ CUtensorMap tmap_vl, const PrefillAttnParams p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));

@@ -347,7 +347,8 @@ rope_qknorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* dy,
     // worked on.  (With one group in flight per warp and two divisions to find it the kernel ran at two thirds of the copy rate.)
     // 32768 tokens, 24 heads of 64: forward 41 us (69 with the copy of the value columns that the attention kernel no longer needs), backward with
     // the MXFP8 copy 109 us (124).
-    constexpr int U = BWD ? 1 : 3;               // within 64 registers, four CTAs an SM; the backward's gradients and outputs leave no registers for more (2: 1895 us for 1495 over 12 layers)
+    // within 64 registers, four CTAs an SM; the backward's gradients and outputs leave no registers for more (2: 1895 us for 1495 over 12 layers)
+    constexpr int U = BWD ? 1 : 3;
     for (long long t = static_cast<long long>(blockIdx.x) * 8 + warp; t < tokens; t += static_cast<long long>(gridDim.x) * 8) {
         float c[4] = {1.f, 1.f, 1.f, 1.f}, sn[4] = {0.f, 0.f, 0.f, 0.f};
         if (cos_t) {
@@ -499,8 +500,8 @@ rope_qknorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* dy,
 // ---- rotation and QK-norm of latent attention, straight from its projections -------------------------------------------------------
 // A 128-wide query head [content | rotary] is a row slice of the query projection; a key head is the content columns of its head in the
 // up-projection [content | value] followed by the token's one rotary key, shared by all heads.  Forward: packed rotated rows [query heads | key
-// heads] as the attention kernels read them (the concatenations that used to assemble them, their slices' gradients and the copies between took 1.5 ms of a three-layer step at 2 x 4096 tokens, 16
-// heads; this kernel takes 35 us forward and 84 us backward a layer).
+// heads] as the attention kernels read them (the concatenations that used to assemble them, their slices' gradients and the copies between
+// took 1.5 ms of a three-layer step at 2 x 4096 tokens, 16 heads; this kernel takes 35 us forward and 84 us backward a layer).
 // Backward: gradients of the three inputs, written where the projections' gradient GEMMs read them; the rotary key's sums over the
 // heads, so a warp owns a token and walks its heads, two at a time (16 lanes of 8 columns each: content first, the last rope_dim / 8 rotary).
 template <bool BWD>

@@ -111,8 +111,9 @@ class SelfAttention(nn.Module):
         return q, k, v
 
     def _fused_rope_attention(self, x: Tensor, ctx: AttentionContext) -> Tuple[Optional[Tensor], bool]:
-        """(output, whether the output projection is in it).  One QKV GEMM, then RoPE + QK-norm + causal / sliding-window attention as a single autograd node (CUDA, 64-wide heads,
-        optional logit soft-capping and document masking, no padding mask).  The output is None when the shapes or options call for the general path."""
+        """(output, whether the output projection is in it).  One QKV GEMM, then RoPE + QK-norm + causal / sliding-window attention as a single
+        autograd node (CUDA, 64-wide heads, optional logit soft-capping and document masking, no padding mask).  The output is None when the
+        shapes or options call for the general path."""
         b, t, _ = x.shape
         d, hq, hk = self.head_size, self.n_heads, self.n_kv_heads
         if not (x.is_cuda and self.q_proj.bias is None and d == 64 and hq + hk <= 64 and hq % hk == 0 and (t % 128 == 0 or self.softcap == 0.0)

@@ -15,8 +15,9 @@ def supported(q: Tensor, k: Tensor, v: Tensor, softcap_value: float) -> bool:
     lengths keep the backend that the caller names).  Batches end where a grid dimension does; a length that is no multiple of 128 under a
     transform or a trace stays with the library's ops, which have rules for them."""
     b, t, h, d = q.shape
-    return (0 < b <= 65535 and (t % 128 == 0 or not intercepted()) and q.dtype == torch.bfloat16 and k.dtype == torch.bfloat16 and v.dtype == torch.bfloat16 and d in (64, 128) and k.shape[-1] == d
-            and v.shape[-1] == 64 and t > 0 and (softcap_value == 0.0 or (softcap_value > 0.0 and t % 128 == 0)) and h % k.shape[2] == 0 and k.shape[:2] == v.shape[:2] == q.shape[:2]
+    return (0 < b <= 65535 and (t % 128 == 0 or not intercepted()) and all(x.dtype == torch.bfloat16 for x in (q, k, v))
+            and d in (64, 128) and k.shape[-1] == d and v.shape[-1] == 64 and t > 0 and h % k.shape[2] == 0
+            and (softcap_value == 0.0 or (softcap_value > 0.0 and t % 128 == 0)) and k.shape[:2] == v.shape[:2] == q.shape[:2]
             and all(x.stride(3) == 1 and x.stride(2) == x.shape[3] and x.stride(0) == t * x.stride(1) and x.stride(1) % 8 == 0 and x.data_ptr() % 16 == 0
                     for x in (q, k, v)))
 

@@ -25,7 +25,7 @@ def _timed(fn, iters):
 
 def main() -> None:
     ap = argparse.ArgumentParser()
-    ap.add_argument("case", choices=["gemm", "gemm_mxfp8", "quantize", "gemm_wgrad", "grouped", "attn_fwd", "attn_fwd_full", "attn_bwd", "attn_bwd_full", "rs_muon", "ce", "rmsnorm", "rope", "rope_bwd", "ep_dispatch", "ep_combine", "rmsnorm_bwd", "attn_fwd_mla", "attn_bwd_mla", "gemm_xxt", "gemm_xxt_full", "polar", "gemm_big", "gemm_mxfp8_big", "gemm_mxfp8_down", "quantize_weight", "gemm_addend", "mla_decode", "mma_issue"])
+    ap.add_argument("case", choices=["gemm", "gemm_mxfp8", "quantize", "gemm_wgrad", "grouped", "attn_fwd", "attn_fwd_full", "attn_bwd", "attn_bwd_full", "rs_muon", "ce", "rmsnorm", "rope", "rope_bwd", "ep_dispatch", "ep_combine", "rmsnorm_bwd", "attn_fwd_mla", "attn_bwd_mla", "gemm_xxt", "gemm_xxt_full", "polar", "gemm_big", "gemm_mxfp8_big", "gemm_mxfp8_down", "quantize_weight", "gemm_addend", "mla_decode", "mla_prefill", "mla_rope", "mla_rope_bwd", "row_nll", "mma_issue"])
     ap.add_argument("--iters", type=int, default=3)
     ap.add_argument("--single-tile", action="store_true", help="attention: the basic kernels (one query tile per CTA forward, unpipelined backward)")
     args = ap.parse_args()
@@ -129,12 +129,34 @@ def main() -> None:
         y = torch.empty_like(x)
         fn = lambda: c.gemm_bf16(b, x, y, False, True, 1.0, 0.3, x)
         flops = 2 * 96 * 768 * 768 * 6144
-    elif args.case == "mla_decode":              # one token for 32 sequences over 8000 latent positions, 16 heads, rank 512
-        q, qr = torch.randn(32, 1, 16, 512, device=dev) * 0.05, torch.randn(32, 1, 16, 64, device=dev)
-        latent, rope = (torch.randn(32, 8000, n, device=dev).bfloat16() for n in (512, 64))
-        gain = torch.rand(32, 8000, 16, device=dev).bfloat16()
-        fn = lambda: c.mla_decode(q, qr, latent, rope, gain, 7999, 0.09, 0.0, -1)
-        bytes_ = 32 * 8000 * (512 + 64 + 16) * 2
+    elif args.case in ("mla_decode", "mla_prefill"):   # attention of new tokens over a latent cache with room left, 16 heads, rank 512, from the
+        b_, new, seen = (32, 1, 8000) if args.case == "mla_decode" else (2, 512, 2012)      # projections to the attention output
+        latent, rope = (torch.randn(b_, seen + 100, n, device=dev).bfloat16() for n in (512, 64))
+        gain = torch.rand(b_, seen + 100, 16, device=dev).bfloat16()
+        query, low = (torch.randn(b_ * new, n, device=dev).bfloat16() for n in (16 * 128, 576))
+        w_up = torch.randn(16 * 128, 512, device=dev) * 0.05
+        cos, sin, norm, qs, ks = torch.ones(seen, 32, device=dev), torch.zeros(seen, 32, device=dev), *(torch.ones(n, device=dev) for n in (512, 16, 16))
+        fn = lambda: c.mla_cached(query, low, w_up, norm, 1e-6, cos, sin, qs, ks, 1e-6, True, -3e38, 3e38, latent, rope, gain, seen - new, 16, 64, 64,
+                                  128 ** -0.5, 0.0, -1)
+        bytes_ = b_ * seen * (512 + 64 + 16) * 2
+        if new > 1:                                    # in the expanded form: W times every position, 128-wide scores, 64-wide values
+            flops = 2 * b_ * seen * 512 * 16 * 128 + 2 * b_ * 16 * (128 + 64) * sum(seen - new + i + 1 for i in range(new))
+    elif args.case in ("mla_rope", "mla_rope_bwd"):    # latent-attention training, 2 x 4096 tokens, 16 heads of 64 + 64 columns
+        tokens, h = 8192, 16
+        q, kv, low = (torch.randn(tokens, n, device=dev).bfloat16() for n in (h * 128, h * 128, 64))
+        cos, sin, qs, ks = torch.ones(4096, 32, device=dev), torch.zeros(4096, 32, device=dev), torch.ones(h, device=dev), torch.ones(h, device=dev)
+        if args.case == "mla_rope":
+            fn = lambda: c.mla_rope_fwd(q, kv, low, cos, sin, qs, ks, 4096, h, h, 1e-6, True, -3e38, 5.0)
+            bytes_ = tokens * (h * (128 + 64) + 64 + 2 * h * 128) * 2
+        else:
+            dq32, dk, dkv = torch.randn(tokens, h * 128, device=dev), torch.randn(tokens, h * 128, device=dev).bfloat16(), torch.empty_like(kv)
+            fn = lambda: c.mla_rope_bwd(q, kv, low, cos, sin, qs, ks, dq32, dk, dkv, 4096, h, h, 1e-6, True, -3e38, 5.0)
+            bytes_ = tokens * (h * (128 + 64) + 64 + 3 * h * 128 + h * (128 + 64) + 64) * 2
+    elif args.case == "row_nll":
+        logits = torch.randn(8192, 50304, device=dev).bfloat16()
+        targets = torch.randint(0, 50304, (8192,), device=dev)
+        fn = lambda: c.row_nll(logits, targets, -100)
+        bytes_ = 8192 * 50304 * 2
     elif args.case == "polar":                   # five Polar Express iterations on the same batch
         x = torch.randn(96, 768, 6144, device=dev)
         x = (x / (x.norm(dim=(-2, -1), keepdim=True) * 1.02 + 1e-6)).bfloat16()
@@ -153,21 +175,21 @@ def main() -> None:
         targets = torch.randint(0, 50304, (4096,), device=dev)
         scale = torch.ones(1, device=dev)
         fn = lambda: c.ce_fwd_bwd(logits, targets, scale, -100, True)
-        bytes_ = 4096 * 50304 * 2 * 3
+        bytes_ = 4096 * 50304 * 2 * 2
     elif args.case == "rmsnorm_bwd":            # backward of the fused residual + RMSNorm: fp32 residual stream, bf16 dy, residual gradient added
         x = torch.randn(32768, 768, device=dev); dy = torch.randn(32768, 768, device=dev).bfloat16()
         w = torch.ones(768, device=dev); rstd = torch.ones(32768, device=dev); res = torch.randn(32768, 768, device=dev)
         fn = lambda: c.rmsnorm_bwd(dy, x, w, rstd, res)
         bytes_ = 32768 * 768 * 14
-    elif args.case in ("rope", "rope_bwd"):     # packed QKV rows of 32768 tokens: 12 q + 12 k heads rotated and normalised, 12 v heads passed through
+    elif args.case in ("rope", "rope_bwd"):     # packed QKV rows of 32768 tokens: 12 q + 12 k heads rotated and normalised, the 12 v heads stay
         qkv = torch.randn(32768, 2304, device=dev).bfloat16()
-        out = torch.empty_like(qkv)
+        out = torch.empty(32768, 1536, device=dev, dtype=torch.bfloat16)
         pos = torch.arange(2048, device=dev).float()[:, None] * (10000.0 ** (-torch.arange(32, device=dev).float() / 32))[None, :]
         cos, sin = pos.cos().contiguous(), pos.sin().contiguous()
         qs, ks = torch.ones(12, device=dev), torch.ones(12, device=dev)
         if args.case == "rope":
-            fn = lambda: c.rope_qknorm_fwd(qkv, out, cos, sin, qs, ks, 2048, 12, 12, 64, 1e-6, True, -3e38, 5.0, 768)
-            bytes_ = 32768 * 2304 * 2 * 2
+            fn = lambda: c.rope_qknorm_fwd(qkv, out, cos, sin, qs, ks, 2048, 12, 12, 64, 1e-6, True, -3e38, 5.0, 0)
+            bytes_ = 32768 * 1536 * 2 * 2
         else:
             dy = torch.randn_like(qkv)
             fn = lambda: c.rope_qknorm_bwd(qkv, dy, dy, cos, sin, qs, ks, 2048, 12, 12, 64, 1e-6, True, -3e38, 5.0)
