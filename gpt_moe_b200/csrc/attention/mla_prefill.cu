@@ -7,9 +7,9 @@
 // The numbers that are fp32 in the absorbed form keep more than its precision: W as two bf16 terms (16 bits of mantissa) in the
 // expansion, whose fp32 sums are split into two bf16 terms per key and value, queries (after rotation and gain) and probabilities as two
 // terms; products of a high and a low part are kept, fp32 accumulation throughout.  The latent and the rotary key are bf16 in the cache.
-// Launches: mla_prefill_prepare (latent norm, rotations, query gains, cache rows of the new tokens), split_terms (W's two terms, formed in
-// every call: nothing of a weight is kept), two GEMMs (gemm_bf16.cu: W's low and high term, the second accumulating), mla_prefill_split
-// (key gains of the new tokens, terms of keys and values), mla_prefill_attention.
+// Launches: mla_prefill_prepare (latent norm, rotations, query gains, cache rows of the new tokens; W's two terms, formed in every call:
+// nothing of a weight is kept), two GEMMs (gemm_bf16.cu: W's low and high term, the second accumulating), mla_prefill_split (key gains of
+// the new tokens, terms of keys and values), mla_prefill_attention.
 // Measured (16 heads, rank 512, 2 x 512 tokens after 1500), layer with its projections: 160 us, 152 of them kernels (attention 55, GEMMs 74, split 14,
 // prepare 10), against 1193 us for the absorbed kernels; error of the output against 64 bits 4.6e-3 (absorbed 4.1e-3, the fp32
 // formulation both replaced, whose W products ran in TF32, 5.9e-3).  mla_prefill_wanted in bindings_ops.cpp says which calls come here.
@@ -37,12 +37,25 @@ struct PrefillPrepareParams {
     __nv_bfloat16* q_out;                        // [2 terms, tokens, H * 128]
     int tokens, T, H, r, rms;
     float norm_eps, qk_eps, smin, smax;
+    const float* w;                              // W [Hk * 128, r]: its two bf16 terms are formed by the first blocks
+    __nv_bfloat16 *w_hi, *w_lo;
+    int w_pieces, w_blocks;                      // pieces of four values
 };
 
-// one CTA per token: warp 0 also does the latent and the rotary key; every warp takes query heads, a lane four columns
+// W = high + low term + (at most 2^-17 of it) in the first `w_blocks` CTAs; then one CTA per token: warp 0 also does the latent and the rotary key; every warp takes query heads, a lane four columns
 __global__ void __launch_bounds__(256)
 mla_prefill_prepare_kernel(const PrefillPrepareParams p) {
-    const int tok = blockIdx.x, b = tok / p.T, t = tok - b * p.T;
+    if (static_cast<int>(blockIdx.x) < p.w_blocks) {
+        for (int i = blockIdx.x * 256 + threadIdx.x; i < p.w_pieces; i += p.w_blocks * 256) {
+            const float4 x = reinterpret_cast<const float4*>(p.w)[i];
+            const uint32_t h0 = pack_bf16x2(x.x, x.y), h1 = pack_bf16x2(x.z, x.w);
+            reinterpret_cast<uint2*>(p.w_hi)[i] = make_uint2(h0, h1);
+            reinterpret_cast<uint2*>(p.w_lo)[i] = make_uint2(pack_bf16x2(x.x - __uint_as_float(h0 << 16), x.y - __uint_as_float(h0 & 0xffff0000u)),
+                                                             pack_bf16x2(x.z - __uint_as_float(h1 << 16), x.w - __uint_as_float(h1 & 0xffff0000u)));
+        }
+        return;
+    }
+    const int tok = blockIdx.x - p.w_blocks, b = tok / p.T, t = tok - b * p.T;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool rot = lane >= 16;                                     // columns 64 .. 127 of a head: pairs 2 (lane - 16), + 1
     float c0 = 1.f, s0 = 0.f, c1 = 1.f, s1 = 0.f;
@@ -372,26 +385,9 @@ mla_prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const _
     }
 }
 
-// w = hi + lo + (at most 2^-17 of w), four elements a thread (n is a multiple of 4, w on a 16-byte boundary)
-__global__ void __launch_bounds__(256)
-split_terms_kernel(const float* __restrict__ w, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo, long long n) {
-    for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n / 4; i += gridDim.x * 256LL) {
-        const float4 x = reinterpret_cast<const float4*>(w)[i];
-        const uint32_t h0 = pack_bf16x2(x.x, x.y), h1 = pack_bf16x2(x.z, x.w);
-        reinterpret_cast<uint2*>(hi)[i] = make_uint2(h0, h1);
-        reinterpret_cast<uint2*>(lo)[i] = make_uint2(pack_bf16x2(x.x - __uint_as_float(h0 << 16), x.y - __uint_as_float(h0 & 0xffff0000u)),
-                                                     pack_bf16x2(x.z - __uint_as_float(h1 << 16), x.w - __uint_as_float(h1 & 0xffff0000u)));
-    }
-}
-
 }  // namespace
 
-void launch_split_terms(const float* w, void* hi, void* lo, long long n, cudaStream_t s) {
-    const long long blocks = (n / 4 + 255) / 256;
-    split_terms_kernel<<<static_cast<unsigned>(blocks < 1184 ? (blocks < 1 ? 1 : blocks) : 1184), 256, 0, s>>>(w, static_cast<__nv_bfloat16*>(hi), static_cast<__nv_bfloat16*>(lo), n);
-}
-
-void launch_mla_prefill_prepare(const MlaCachedArgs& a, void* q_out, cudaStream_t s) {
+void launch_mla_prefill_prepare(const MlaCachedArgs& a, void* q_out, void* w_hi, void* w_lo, cudaStream_t s) {
     PrefillPrepareParams p;
     p.query = static_cast<const __nv_bfloat16*>(a.query); p.low = static_cast<const __nv_bfloat16*>(a.low);
     p.q_pitch = a.q_pitch; p.low_pitch = a.low_pitch;
@@ -401,7 +397,10 @@ void launch_mla_prefill_prepare(const MlaCachedArgs& a, void* q_out, cudaStream_
     p.latent_bs = a.latent_bs; p.rope_bs = a.rope_bs;
     p.q_out = static_cast<__nv_bfloat16*>(q_out);
     p.tokens = a.B * a.T; p.T = a.T; p.H = a.H; p.r = a.r; p.rms = a.rms; p.norm_eps = a.norm_eps; p.qk_eps = a.qk_eps; p.smin = a.smin; p.smax = a.smax;
-    mla_prefill_prepare_kernel<<<a.B * a.T, 256, 0, s>>>(p);
+    p.w = a.w_up; p.w_hi = static_cast<__nv_bfloat16*>(w_hi); p.w_lo = static_cast<__nv_bfloat16*>(w_lo);
+    p.w_pieces = a.Hkv * 128 * a.r / 4;                                 // at most 32 heads and rank 1024
+    p.w_blocks = (p.w_pieces + 255) / 256 < 592 ? (p.w_pieces + 255) / 256 : 592;
+    mla_prefill_prepare_kernel<<<p.w_blocks + a.B * a.T, 256, 0, s>>>(p);
 }
 
 void launch_mla_prefill_split(const MlaCachedArgs& a, int base, const float* kv, void* const* terms, float* gain, int S, int S_pad, cudaStream_t s) {

@@ -342,12 +342,11 @@ Tensor mla_prefill(const MlaCachedArgs& args, const Tensor& latent) {
     const int S = end - base, S_pad = (S + 127) / 128 * 128;
     auto bf = latent.options();
     Tensor q = gm::out_empty({2 * a.B, a.T, a.H * 128}, bf);              // high terms, then low ones
-    launch_mla_prefill_prepare(a, q.data_ptr(), stream());
     Tensor kv = gm::out_empty({a.B, S, a.Hkv * 128}, bf.dtype(torch::kFloat32));
-    // W as two bf16 terms: 8 MB moved in a call that expands thousands of positions with them, so nothing of the weight is kept between calls
+    // W as two bf16 terms: 8 MB moved in a call that expands thousands of positions with them, so nothing of a weight is kept between calls
     Tensor terms = gm::out_empty({2, static_cast<int64_t>(a.Hkv) * 128, a.r}, bf);
     const Tensor hi = terms.select(0, 0), lo = terms.select(0, 1);
-    launch_split_terms(a.w_up, hi.data_ptr(), lo.data_ptr(), hi.numel(), stream());
+    launch_mla_prefill_prepare(a, q.data_ptr(), hi.data_ptr(), lo.data_ptr(), stream());
     const Tensor rows = latent.narrow(1, base, S);          // [B, S, rank] with the cache's own batch stride
     gemm_fp32(rows, lo, kv, false);
     gemm_fp32(rows, hi, kv, true);

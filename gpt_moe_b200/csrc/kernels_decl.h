@@ -67,8 +67,7 @@ struct MlaCachedArgs {
 };
 bool launch_mla_cached(const MlaCachedArgs& a, cudaStream_t s);
 // attention/mla_prefill.cu (its attention launcher takes tensor maps and is declared where it is called)
-void launch_split_terms(const float* w, void* hi, void* lo, long long n, cudaStream_t s);
-void launch_mla_prefill_prepare(const MlaCachedArgs& a, void* q_out, cudaStream_t s);
+void launch_mla_prefill_prepare(const MlaCachedArgs& a, void* q_out, void* w_hi, void* w_lo, cudaStream_t s);
 void launch_mla_prefill_split(const MlaCachedArgs& a, int base, const float* kv, void* const* terms, float* gain, int S, int S_pad, cudaStream_t s);
 bool rows_linear_supported(int rows, int N, int K);
 bool launch_rows_linear(const void* x, const void* w, void* y, int rows, int N, int K, long long x_pitch, long long y_pitch, cudaStream_t s);
