@@ -320,14 +320,22 @@ MlaCachedArgs mla_cached_args(const Tensor& query, const Tensor& low, const Tens
 }
 
 // Whether a call expands the visible cache instead of running the absorbed form: heads of 64 + 64 columns with 64-wide values, no
-// soft-capping, and enough queries.  The absorbed form costs by (query, position) pair, the expansion by position and some 15 us more
-// of launches.  Measured, 16 heads, rank 512, absorbed against expanded in us: sequences x new tokens over positions 1 x 64 over 2064 144 : 147,
-// 1 x 96 over 2096 179 : 150, 1 x 64 over 7064 277 : 312, 1 x 96 over 7096 357 : 314, 2 x 48 over 1548 162 : 148, 4 x 34 over 4034 329 : 332, 4 x 48 over
-// 4048 563 : 331, 1 x 128 over 228 125 : 145, 1 x 256 over 356 190 : 145; 2 x 512 over 2012 1193 : 160.  The expansion holds 1 KB per position and
-// kv head (4 GB at the limit for 16 heads); longer calls stay absorbed.
-bool mla_prefill_wanted(int64_t B, int64_t T, int64_t end, int64_t window, int64_t r, int64_t dr, int64_t content, int64_t value, double softcap) {
-    const int64_t visible = window < 0 ? end : std::min(end, window + T);
-    return T >= 48 && B * T >= 96 && B * T * visible >= 90000 && B * visible <= 262144 && r % 64 == 0 && dr == 64 && content == 64 && value == 64 && softcap <= 0.0;
+// soft-capping, at least 8 new tokens a sequence (fewer were not measured), and the cheaper of the two by an estimate of their kernels in us:
+//   absorbed   its (query row, position) products, 2 rank + rope wide, and W_k and W_v once per (token, head);
+//   expanded   the positions that one CTA of the attention walks, times the waves of CTAs, and every position's kv heads (product, split).
+// The constants are a fit to 266 calls of each form (8, 16 and 32 heads on 1 to 32 kv heads, ranks 256 to 1024, 1 to 32 sequences of 8 to 512
+// new tokens over 192 to 8000 positions, with room left in the cache): it is 9 % off on average, and taking the form it names costs 0.5 %
+// over taking the better one each time (at worst 25 %, one call of 60 against 48 us).  For 16 heads, rank 512, 2 x 512 over 2012 it says
+// 1091 : 133.  The expansion holds 1 KB per position and kv head, 4 GB at the limit; longer calls stay absorbed.
+bool mla_prefill_wanted(int64_t B, int64_t T, int64_t heads, int64_t kv_heads, int64_t end, int64_t window, int64_t r, int64_t dr, int64_t content,
+                        int64_t value, double softcap) {
+    if (T < 8 || r % 64 != 0 || dr != 64 || content != 64 || value != 64 || softcap > 0.0) return false;
+    const double visible = static_cast<double>(window < 0 ? end : std::min(end, window + T));
+    if (B * visible * kv_heads > 4194304.0) return false;
+    const double rows = static_cast<double>(B * T * heads), waves = std::max(1.0, heads * B * ((T + 127) / 128) / 148.0);
+    const double absorbed = 26.0 + 21.5e-9 * rows * visible * (2 * r + dr) + 3.5e-5 * rows * r;
+    const double expanded = 45.0 + 0.0235 * visible * waves + 6.3e-4 * B * visible * kv_heads;
+    return absorbed > expanded;
 }
 
 bool mla_prefill_aligned(const MlaCachedArgs& a) {
@@ -371,7 +379,7 @@ Tensor mla_cached(const Tensor& query, const Tensor& low, const Tensor& w_up, co
     c10::cuda::CUDAGuard guard(query.device());
     MlaCachedArgs a = mla_cached_args(query, low, w_up, norm_w, norm_eps, cos, sin, q_scale, k_scale, qk_eps, rms, smin, smax, latent, rope, key_gain, start, heads,
                                       content, value, scale, softcap, window);
-    if (mla_prefill_wanted(a.B, a.T, start + a.T, window, a.r, a.dr, content, value, softcap) && mla_prefill_aligned(a)) return mla_prefill(a, latent);
+    if (mla_prefill_wanted(a.B, a.T, heads, a.Hkv, start + a.T, window, a.r, a.dr, content, value, softcap) && mla_prefill_aligned(a)) return mla_prefill(a, latent);
     a.splits = mla_decode_splits(a.B, a.T, a.H, a.r, start + a.T, 2);
     const int64_t rows = static_cast<int64_t>(a.B) * a.T * a.H;
     // one fp32 workspace: queries in latent space, rotary queries, partial contexts, partial maxima and sums

@@ -63,7 +63,7 @@ def test_cached_step_matches_the_plain_path(b, t, h, hkv, r, dr, c, start, windo
     got = gpu.forward_cached(x.cuda(), cache, window)
     assert cuda_ops.path_counts().get("mla_decode:kernel", 0) == before + 1
     if t >= 128:
-        assert cuda_ops.ext().mla_prefill_wanted(b, t, start + t, -1 if window is None else window, r, dr, c, 64, 0.0)
+        assert cuda_ops.ext().mla_prefill_wanted(b, t, h, hkv, start + t, -1 if window is None else window, r, dr, c, 64, 0.0)
     want = cpu.forward_cached(x.float(), plain, window)
     assert got.dtype == torch.bfloat16 and cache.length == plain.length == start + t
     new = slice(start, start + t)
@@ -77,7 +77,7 @@ def test_cached_step_matches_the_plain_path(b, t, h, hkv, r, dr, c, start, windo
 
 
 # an exactly full cache, one with room; a window that starts inside it; a rank whose contraction is long for its few tiles
-@pytest.mark.parametrize("start,t,r,window", [(1000, 130, 512, None), (633, 512, 256, 200), (1000, 128, 1024, None)])
+@pytest.mark.parametrize("start,t,r,window", [(1000, 200, 512, None), (633, 512, 256, 200), (1000, 128, 1024, None)])
 def test_a_batch_expands_as_its_sequences_do(start, t, r, window):
     torch.manual_seed(14)
     gc, tc = get_preset("mla")
@@ -96,7 +96,7 @@ def test_a_batch_expands_as_its_sequences_do(start, t, r, window):
         return attn.forward_cached(x[rows], cache, window)
 
     from gpt_moe_b200.ops import cuda_ops
-    assert cuda_ops.ext().mla_prefill_wanted(1, t, start + t, -1 if window is None else window, r, 64, 64, 64, 0.0)
+    assert cuda_ops.ext().mla_prefill_wanted(1, t, 8, 4, start + t, -1 if window is None else window, r, 64, 64, 64, 0.0)
     full, roomy = call(slice(0, 3), 0), call(slice(0, 3), 77)
     alone = torch.cat([call(slice(i, i + 1), 5) for i in range(3)])
     assert torch.equal(full, roomy) and torch.equal(full, alone)
@@ -120,6 +120,17 @@ def test_a_weight_written_behind_torchs_back_is_seen(t):
     second = call(attn)
     assert not torch.equal(first, second)
     assert torch.equal(second, call(copy.deepcopy(attn)))
+
+
+# sequences, new tokens, heads, kv heads, positions, rank: where one form was measured to be at least 1.3 times as fast as the other
+@pytest.mark.parametrize("b,t,h,hkv,end,r,expanded", [(1, 64, 16, 16, 7000, 512, False), (2, 96, 16, 16, 1500, 512, True), (4, 48, 16, 16, 300, 512, True),
+                                                      (16, 16, 16, 16, 4000, 512, False), (16, 16, 16, 2, 4000, 512, True), (4, 32, 16, 2, 4000, 512, True),
+                                                      (2, 48, 8, 8, 1500, 256, False), (4, 48, 8, 8, 4000, 256, False), (1, 128, 8, 8, 7000, 256, False),
+                                                      (2, 48, 32, 32, 1500, 512, True), (32, 8, 16, 4, 1000, 768, True), (1, 48, 16, 16, 2000, 512, False),
+                                                      (16, 8, 16, 16, 4000, 1024, False), (16, 32, 16, 16, 500, 1024, True)])
+def test_the_form_follows_heads_and_rank(b, t, h, hkv, end, r, expanded):
+    from gpt_moe_b200.ops import cuda_ops
+    assert cuda_ops.ext().mla_prefill_wanted(b, t, h, hkv, end, -1, r, 64, 64, 64, 0.0) == expanded
 
 
 def test_a_tangent_is_not_dropped():
@@ -191,7 +202,7 @@ def test_only_the_output_is_rounded_to_bf16(b, t, h, hkv, r, start, expanded):
     qs, ks = torch.linspace(0.5, 3.0, h, device="cuda"), torch.linspace(0.5, 2.0, hkv, device="cuda")
     lat, rope = torch.randn(b, end, r, device="cuda").bfloat16(), torch.randn(b, end, 64, device="cuda").bfloat16()
     gain = (torch.rand(b, end, hkv, device="cuda") + 0.5).bfloat16()
-    assert cuda_ops.ext().mla_prefill_wanted(b, t, end, -1, r, 64, 64, 64, 0.0)
+    assert cuda_ops.ext().mla_prefill_wanted(b, t, h, hkv, end, -1, r, 64, 64, 64, 0.0)
     got = cuda_ops.ext().mla_cached(query, low, w, None, 1e-6, cos, sin, qs, ks, 1e-6, True, -3e38, 3e38, lat, rope, gain, start, h, 64, 64, 128 ** -0.5, 0.0, -1)
     q = query.double().view(b, t, h, 128)
     norm = torch.rsqrt(q.pow(2).mean(-1, keepdim=True) + 1e-6) * qs.double().view(1, 1, -1, 1)
