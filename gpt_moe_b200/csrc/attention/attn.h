@@ -39,7 +39,7 @@ struct AttnParams {
 
 cudaError_t launch_attn_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnParams& p, cudaStream_t stream);
 
-// Forward with two query tiles per CTA (attn_fwd_dual.cu): 64-wide heads, no document masking, lengths of whole pairs of query tiles.
+// Forward with two query tiles per CTA (attn_fwd_dual.cu): 64-wide heads, no document masking, an even number of query tiles or many.
 // launch_attn_fwd picks it when it applies and `single_tile` is 0.
 bool attn_fwd_dual_supported(const AttnParams& p);
 cudaError_t launch_attn_fwd_dual(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnParams& p, cudaStream_t stream);

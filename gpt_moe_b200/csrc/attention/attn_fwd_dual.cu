@@ -112,7 +112,7 @@ __device__ __forceinline__ void dual_zero16(uint32_t p_addr) {
 
 template <bool CAP>
 __device__ __forceinline__ void dual_softmax_tile(uint32_t s_addr, uint32_t p_addr, uint32_t o_addr, int kv0, int qpos, int warp_q0, int window,
-                                                  bool edge_tile, float c, float& m_ref, float& l, bool first, float cap_a, float cap_b) {
+                                                  bool edge_tile, float c, float step, float& m_ref, float& l, bool first, float cap_a, float cap_b) {
     int cls[4] = {CHUNK_FULL, CHUNK_FULL, CHUNK_FULL, CHUNK_FULL};
     if (edge_tile) {
 #pragma unroll
@@ -138,7 +138,7 @@ __device__ __forceinline__ void dual_softmax_tile(uint32_t s_addr, uint32_t p_ad
         if (cls[3] != CHUNK_EMPTY) { dual_prepare_chunk<CAP>(s3, cls[3], kv0 + 96, qpos, window, cap_a, cap_b); dual_max32(s3, mx); }
     }
     const float m_tile = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * c;
-    const bool grow = m_tile > m_ref + DU_RESCALE_STEP;       // also true for the first finite maximum (m_ref = -inf)
+    const bool grow = m_tile > m_ref + step;       // also true for the first finite maximum (m_ref = -inf)
     if (__any_sync(0xffffffffu, grow)) {
         const float alpha = grow ? exp2f(m_ref - m_tile) : 1.f;
         if (!first) {                 // the previous PV product is complete: the commit that announced this S came after it
@@ -297,6 +297,10 @@ attn_fwd_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         const float c = p.scale_log2e;
         constexpr bool capped = CAPPED;
         const float cap_a = capped ? p.softcap / p.scale : 0.f, cap_b = capped ? p.scale / p.softcap : 0.f;
+        // With a reference that lags, the largest probabilities are no longer 1, which bf16 holds exactly, and windowed outputs lie up to 4 %
+        // further from 64 bits than with the exact maximum of the library kernel that lengths outside whole pairs of tiles used to run:
+        // those rescale whenever the maximum grows (5 x 1000 tokens, window 256: 2.04e-3 instead of 2.10e-3, 28.4 us instead of 27)
+        const float step = p.seq_len % (2 * DU_BM) == 0 ? DU_RESCALE_STEP : 0.f;
         float m_ref = -INFINITY, l = 0.f;
         for (int i = 0; i < n_x && ok; ++i) {
             const int tile = lo_x + i;
@@ -313,7 +317,7 @@ attn_fwd_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
             }
             // tiles strictly inside the band need no mask; the diagonal tile and the tile at the window edge do
             const bool need_mask = (kv0 + DU_BN - 1 > q0x) || (q0x + DU_BM - 1 - kv0 > window);
-            dual_softmax_tile<capped>(s_addr, p_addr, o_addr, kv0, qpos, q0x + quad * 32, window, need_mask, c, m_ref, l, i == 0, cap_a, cap_b);
+            dual_softmax_tile<capped>(s_addr, p_addr, o_addr, kv0, qpos, q0x + quad * 32, window, need_mask, c, step, m_ref, l, i == 0, cap_a, cap_b);
             tmem_st_wait();
             tc_fence_before();
             mbar_arrive(&bar_p[x]);
@@ -383,14 +387,14 @@ attn_fwd_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
 }
 
 bool attn_fwd_dual_supported(const AttnParams& p) {
-    // Whole pairs of tiles.  Windowed calls, where two query tiles share most of their keys: 16 x 2048 tokens, window 1024 225 us against 238
-    // for the single-tile kernel.  Without a window the single-tile kernel's finer grain fills the end of the grid better: 16384 tokens
-    // 955 us against 1060, 4 x 4096 285 against 303; up to 16 tiles this one is equal or better (2 tiles 51 against 63).
-    // Other lengths run the single-tile kernel, whose row maximum is exact in every tile: here it may lag by up to 2^8, the largest
-    // probabilities are then no longer 1 (which bf16 holds exactly), and windowed outputs lie 1.5 to 4 % further from 64 bits (5 x 1000 tokens,
-    // window 256: 2.10e-3 against 2.05e-3, which is also what the library kernel had that used to serve these lengths).
+    // Windowed calls, where two query tiles share most of their keys: 16 x 2048 tokens, window 1024 225 us against 238 for the single-tile
+    // kernel, 16 x 1000, window 256 70 against 81; also with an odd number of tiles, where half of the last CTA idles, once there are
+    // nine (16 x 1152, window 256 84 against 91).  Without a window the single-tile kernel's finer grain fills the end of the grid better:
+    // 16384 tokens 955 us against 1060, 4 x 4096 285 against 303, 8 x 1100 57 against 65; up to 16 tiles an even number is better here
+    // (64 x 184 tokens 51 against 60, 5 x 1000 33 against 35).
+    const int tiles = (p.seq_len + DU_BM - 1) / DU_BM;
     const bool windowed = p.window <= p.seq_len / 2;
-    return p.qk_dim == 64 && p.doc_start == nullptr && p.seq_len % (2 * DU_BM) == 0 && (windowed || p.seq_len <= 16 * DU_BM);
+    return p.qk_dim == 64 && p.doc_start == nullptr && (windowed ? tiles % 2 == 0 || tiles >= 9 : tiles % 2 == 0 && tiles <= 16);
 }
 
 template <bool CAPPED>

@@ -59,15 +59,16 @@ def test_any_length_with_document_mask(t):
     cuda_ops.check_status()
 
 
-@pytest.mark.parametrize("t,window,pairs", [(200, 50, False), (1000, 256, False), (1152, 256, False), (250, None, False), (1280, 256, True), (512, None, True)])
-def test_lengths_without_whole_pairs_of_tiles_keep_the_exact_maximum(t, window, pairs):
+# lengths outside whole pairs of tiles: both forward kernels follow the row maximum exactly
+@pytest.mark.parametrize("t,window", [(184, 50), (184, None), (1000, 256), (1152, 256), (1500, None), (300, None), (1100, None)])
+def test_ragged_outputs_are_as_exact_as_the_single_tile_kernels(t, window):
     torch.manual_seed(7)
-    q, k, v = (torch.nn.functional.rms_norm(torch.randn(2, t, 4, 64, device="cuda"), (64,)).bfloat16() for _ in range(3))
+    q, k = (torch.nn.functional.rms_norm(torch.randn(2, t, 4, 64, device="cuda"), (64,)).bfloat16() for _ in range(2))
+    v = torch.randn(2, t, 4, 64, device="cuda").bfloat16()
     w = t if window is None else window
-    out, lse = cuda_ops.ext().attn_fwd(q, k, v, w, 0.125)
-    single, lse1 = cuda_ops.ext().attn_fwd(q, k, v, w, 0.125, single_tile=True)
-    assert torch.equal(out, single) == (not pairs)
+    out = cuda_ops.ext().attn_fwd(q, k, v, w, 0.125)[0]
+    single = cuda_ops.ext().attn_fwd(q, k, v, w, 0.125, single_tile=True)[0]
     want = ref.attention(q.double(), k.double(), v.double(), causal=True, window=window)
-    library = torch.nn.functional.scaled_dot_product_attention(*(x.transpose(1, 2) for x in (q, k, v)), attn_mask=ref.attention_mask(t, q.device, True, window)).transpose(1, 2)
-    if not pairs:
-        assert rel(out, want) < 1.02 * max(rel(library, want), 2.03e-3)
+    # the same probabilities in bf16; another order of the sums moves the error's fourth digit, a lagging maximum its second
+    assert rel(out, want) < 1.003 * rel(single, want)
+    cuda_ops.check_status()
