@@ -137,24 +137,31 @@ class _NoGradContext:
         pass
 
 
+# asked several times per block and call: bound once
+_grad_enabled, _functorch_active = torch.is_grad_enabled, torch._C._are_functorch_transforms_active
+_tracing_state, _dispatch_modes = torch._C._get_tracing_state, torch._C._len_torch_dispatch_stack
+
+
 def intercepted() -> bool:
     """Something wants the torch ops of a call and not only their results: a functorch transform, forward-mode tangents, a TorchScript trace
     (it would take the result of a native call for a constant) or a dispatch mode.  Calls that torch's ops can serve go to them then."""
-    return (torch._C._are_functorch_transforms_active() or forward_ad._current_level >= 0 or torch._C._get_tracing_state() is not None
-            or torch._C._len_torch_dispatch_stack() > 0)
+    return _functorch_active() or forward_ad._current_level >= 0 or _tracing_state() is not None or _dispatch_modes() > 0
 
 
 def plain_call() -> bool:
     """No gradients are recorded and nothing intercepts autograd functions: a Function's forward can be called as it is, which saves the
     node (about 10 us of host time per call)."""
-    return not torch.is_grad_enabled() and not intercepted()
+    return not (_grad_enabled() or _functorch_active() or forward_ad._current_level >= 0 or _tracing_state() is not None or _dispatch_modes() > 0)
 
 
 def bypassable(*modules) -> bool:
     """Calling these modules does nothing but run their class's forward: no hooks (a process may also have global ones) and no forward
     of an instance's own.  Only then may a composed call stand in for them."""
-    return not _nn_module._has_any_global_hook() and not any(
-        m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or "forward" in m.__dict__ for m in modules)
+    for m in modules:
+        own = m.__dict__
+        if own["_forward_hooks"] or own["_forward_pre_hooks"] or own["_backward_hooks"] or own["_backward_pre_hooks"] or "forward" in own:
+            return False
+    return not _nn_module._has_any_global_hook()
 
 
 def run_function(fn, *args):
