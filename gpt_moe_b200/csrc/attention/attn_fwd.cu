@@ -215,8 +215,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         const int quad = warp & 3, half = warp >> 2;         // TMEM lanes 32*quad..+31; key / output columns of this half
         const int r = quad * 32 + lane;
         const int qpos = q0 + r;
-        const bool live = qpos < p.seq_len;                     // rows past the sequence end are computed on zeros and not stored
-        const int w_row = p.doc_start && live ? min(window, qpos - p.doc_start[row0 + qpos]) : window;     // this row's look-back
+        // 1: a row of the sequence; 0: past its end, computed on zeros and not stored; -1: a wait gave up (one word: as two truth
+        // values it costs the 64-wide variant more spilled registers, 988 us for 960 at 16384 tokens, 16 heads of 4)
+        int state = qpos < p.seq_len ? 1 : 0;
+        const int w_row = p.doc_start && state ? min(window, qpos - p.doc_start[row0 + qpos]) : window;     // this row's look-back
         const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
         const float c = p.scale_log2e;
         constexpr bool capped = CAPPED;
@@ -229,7 +231,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         for (int j = 0; j < n_tiles; ++j) {
             const uint32_t ph = j & 1;
             const int kv0 = kv_lo + j * AT_BN + half * 64;
-            if (ok && !mbar_wait(bar_s, ph)) { atomicExch(p.status, 206); ok = false; }
+            if (state >= 0 && !mbar_wait(bar_s, ph)) { atomicExch(p.status, 206); state = -1; }
             tc_fence_after();
             // tiles strictly inside the band need no mask; the diagonal tile and the tile(s) at the window edge do
             const int tile0 = kv_lo + j * AT_BN;
@@ -249,7 +251,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
             m = m_new;
             tc_fence_before();
             mbar_arrive(bar_p);
-            if (ok && !mbar_wait(bar_o, ph)) { atomicExch(p.status, 207); ok = false; }
+            if (state >= 0 && !mbar_wait(bar_o, ph)) { atomicExch(p.status, 207); state = -1; }
             tc_fence_after();
             {
                 uint32_t oreg[32];
@@ -264,7 +266,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         row_stat[half * AT_BM + r] = l;
         asm volatile("bar.sync %0, 64;" ::"r"(bar_id) : "memory");
         l += row_stat[(half ^ 1) * AT_BM + r];
-        if (ok && live) {
+        if (state > 0) {
             const float inv = 1.f / l;
             const long long token = static_cast<long long>(row0) + qpos;
             __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.out) + token * p.out_stride + head * AT_D + half * 32;
