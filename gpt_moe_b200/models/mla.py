@@ -245,11 +245,8 @@ class MLAttention(nn.Module):
         if not c.mla_decode_ok(self.n_heads, self.n_kv_heads, self.kv_rank, self.rope_dim):
             return None
         cuda_ops.count_path("mla_decode:kernel")
-        qs = ks = None
-        if self.use_qk_norm:
-            qs, ks = self.q_scale.detach().float().reshape(-1), self.k_scale.detach().float().reshape(-1)
-        norm_w = None if self.kv_norm.weight is None else self.kv_norm.weight.detach().float()
-        rest = (w_up.detach(), norm_w, self.kv_norm.eps, self.rotary.cos_cached, self.rotary.sin_cached, qs, ks, self.qk_eps, self.qk_norm_type == "rms",
+        qs, ks = (cuda_ops.as_fp32(self.q_scale), cuda_ops.as_fp32(self.k_scale)) if self.use_qk_norm else (None, None)
+        rest = (w_up, cuda_ops.as_fp32(self.kv_norm.weight), self.kv_norm.eps, self.rotary.cos_cached, self.rotary.sin_cached, qs, ks, self.qk_eps, self.qk_norm_type == "rms",
                 max(self.qk_scale_min, -3.0e38), min(self.qk_scale_max, 3.0e38), *caches, start, self.n_heads, self.content_dim, self.value_dim,
                 self.softmax_scale, max(self.softcap, 0.0), -1 if (self.is_full_attention or window is None) else int(window))
         plain = (self.q_proj, self.kv_down_proj, self.out_proj)
