@@ -20,8 +20,9 @@
 //     and shorten the chain of products of every tile.
 // Measured (16 heads, rank 512): 8 sequences x 1 token over 4022 positions 18 us against 96 us for a kernel that formed the products
 // with fp32 multiply-adds and warp reductions (38 MB of cache; its merge took another 48 us, now 9 with W_v); 32 x 1 over 8000 positions
-// 92 us, 3.3 TB/s, the tensor pipe 38 % busy: a tile's chain of products, sums and softmax is the limit.  Error of the layer's output against 64 bits: 3.8e-3 against 5.6e-3 (queries and rotation stay
-// fp32 between the projection and the scores).
+// 97 us, 3.1 TB/s, the tensor pipe 37 % busy: a tile's chain of products, sums and softmax is the limit.  Error of the layer's output (of
+// the output alone, without the cache entries) against 64 bits: 3.8e-3 against 5.7e-3 (queries and rotation stay fp32 between the
+// projection and the scores, and the W products are fp32 instead of TF32).
 // The first kernel of the file turns projections into what the split kernel reads (and appends the new tokens to the cache); the
 // last one merges the splits by their log-sum-exp and, for the module's own use, expands the context with W_v.
 // Reference: the Triton kernels `_mla_decode_kernel` / `_mla_decode_merge_kernel` (experiments/073-mla-current-kv768.patch:456-673)
@@ -701,7 +702,7 @@ int mla_decode_splits(int B, int T, int H, int r, int S, int terms) {
     const int ctas = B * ((T * H + rows - 1) / rows);
     const int tiles = (S + MD_TILE - 1) / MD_TILE;
     // one wave of CTAs, since a second would cost as much as the first: two CTAs an SM where they fit and have six tiles each, else one (8 x
-    // 4022 positions: 18 splits of 7 tiles 18.1 + 8.7 us with the merge, 37 of 4 tiles 17.2 + 11.9; 32 x 8000: 4 splits 146 us, 9 splits 92)
+    // 4022 positions: 18 splits of 7 tiles 18.1 + 8.7 us with the merge, 37 of 4 tiles 17.2 + 11.9; 32 x 8000: 4 splits 146 us, 9 splits 97)
     const int both = 148 * md_ctas(r / 128, rows / 16, terms) / ctas;
     int want = both > 0 && tiles / both >= 6 ? both : 148 / ctas;
     want = want < 1 ? 1 : (want > MD_MAX_SPLITS ? MD_MAX_SPLITS : want);

@@ -10,9 +10,10 @@
 // Launches: mla_prefill_prepare (latent norm, rotations, query gains, cache rows of the new tokens; W's two terms, formed in every call:
 // nothing of a weight is kept), two GEMMs (gemm_bf16.cu: W's low and high term, the second accumulating), mla_prefill_split (key gains of
 // the new tokens, terms of keys and values), mla_prefill_attention.
-// Measured (16 heads, rank 512, 2 x 512 tokens after 1500), layer with its projections: 160 us, 152 of them kernels (attention 55, GEMMs 74, split 14,
-// prepare 10), against 1193 us for the absorbed kernels; error of the output against 64 bits 4.6e-3 (absorbed 4.1e-3, the fp32
-// formulation both replaced, whose W products ran in TF32, 5.9e-3).  mla_prefill_wanted in bindings_ops.cpp says which calls come here.
+// Measured (16 heads, rank 512, 2 x 512 tokens after 1500), layer with its projections: 170 us, 160 of them kernels (GEMMs 73, attention 61, split
+// 14, prepare with W's terms 13), against 1193 us for the absorbed kernels; error of the layer's output against 64 bits 4.1e-3 (the fp32
+// formulation that both forms replaced, whose W products ran in TF32, 5.9e-3; with the queries as one term 4.5e-3 and 162 us).
+// mla_prefill_wanted in bindings_ops.cpp says which calls come here.
 #include "../common/ptx.cuh"
 #include "../kernels_decl.h"
 #include "attn.h"
@@ -42,7 +43,8 @@ struct PrefillPrepareParams {
     int w_pieces, w_blocks;                      // pieces of four values
 };
 
-// W = high + low term + (at most 2^-17 of it) in the first `w_blocks` CTAs; then one CTA per token: warp 0 also does the latent and the rotary key; every warp takes query heads, a lane four columns
+// W = high + low term + (at most 2^-17 of it) in the first `w_blocks` CTAs; then one CTA per token: warp 0 also does the latent and the rotary
+// key; every warp takes query heads, a lane four columns
 __global__ void __launch_bounds__(256)
 mla_prefill_prepare_kernel(const PrefillPrepareParams p) {
     if (static_cast<int>(blockIdx.x) < p.w_blocks) {
