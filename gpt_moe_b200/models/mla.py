@@ -235,8 +235,8 @@ class MLAttention(nn.Module):
         b, t, hidden = x.shape
         caches = (cache.latent, cache.rope, cache.key_gain)
         w_up = self.kv_up_proj.weight
-        if not (x.is_cuda and cuda_ops.plain_call() and self.rotary is not None and 0 < b * t <= 131072 and all(c.dtype == torch.bfloat16 and c.is_cuda and c.stride(2) == 1
-                and c.stride(1) == c.size(2) for c in caches) and all(m.bias is None for m in (self.q_proj, self.kv_down_proj, self.kv_up_proj))
+        if not (x.is_cuda and cuda_ops.plain_call() and self.rotary is not None and 0 < b * t <= 131072
+                and all(c.dtype == torch.bfloat16 and c.is_cuda and c.stride(2) == 1 and c.stride(1) == c.size(2) for c in caches) and all(m.bias is None for m in (self.q_proj, self.kv_down_proj, self.kv_up_proj))
                 and w_up.dtype == torch.float32 and w_up.is_contiguous() and w_up.data_ptr() % 16 == 0 and self.content_dim <= 256
                 and (self.softcap <= 0.0 or self.tanh_backend == "exact") and start + t <= self.rotary.cos_cached.shape[0]
                 and cache.rope.size(1) == cache.latent.size(1) == cache.key_gain.size(1) and self.rotary.cos_cached.dtype == torch.float32):
@@ -246,8 +246,8 @@ class MLAttention(nn.Module):
             return None
         cuda_ops.count_path("mla_decode:kernel")
         qs, ks = (cuda_ops.as_fp32(self.q_scale), cuda_ops.as_fp32(self.k_scale)) if self.use_qk_norm else (None, None)
-        rest = (w_up, cuda_ops.as_fp32(self.kv_norm.weight), self.kv_norm.eps, self.rotary.cos_cached, self.rotary.sin_cached, qs, ks, self.qk_eps, self.qk_norm_type == "rms",
-                max(self.qk_scale_min, -3.0e38), min(self.qk_scale_max, 3.0e38), *caches, start, self.n_heads, self.content_dim, self.value_dim,
+        rest = (w_up, cuda_ops.as_fp32(self.kv_norm.weight), self.kv_norm.eps, self.rotary.cos_cached, self.rotary.sin_cached, qs, ks, self.qk_eps,
+                self.qk_norm_type == "rms", max(self.qk_scale_min, -3.0e38), min(self.qk_scale_max, 3.0e38), *caches, start, self.n_heads, self.content_dim, self.value_dim,
                 self.softmax_scale, max(self.softcap, 0.0), -1 if (self.is_full_attention or window is None) else int(window))
         plain = (self.q_proj, self.kv_down_proj, self.out_proj)
         if (b * t <= 32 and not self.q_rank and hidden % 32 == 0 and self.attn_dim % 32 == 0 and self.out_proj.bias is None

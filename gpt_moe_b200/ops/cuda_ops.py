@@ -335,7 +335,7 @@ def embedding(module, indices: Tensor) -> Tensor:
     if (main is None or not torch.is_grad_enabled() or not weight.requires_grad or weight.dtype != torch.float32 or not main.is_contiguous()
             or weight.shape[1] % 4 or main.data_ptr() % 16 or weight.shape[0] >= 2 ** 31 or module.padding_idx is not None
             or module.max_norm is not None or module.scale_grad_by_freq or module.sparse or not bypassable(module)
-            or torch._C._are_functorch_transforms_active()):
+            or intercepted()):
         return module(indices)
     return _EmbeddingFn.apply(indices, weight)
 
@@ -707,7 +707,8 @@ class _ActivationFn(torch.autograd.Function):
 
 def activate(x: Tensor, name: str) -> Tensor:
     # the kernels move 16-byte vectors of rows that are whole vectors; an odd SwiGLU width is an error that torch's ops raise
-    if intercepted() or name not in ("gelu", "relu", "relu2", "silu", "swiglu") or x.dim() == 0 or x.numel() == 0 or x.shape[-1] % (16 if name == "swiglu" else 8):
+    if (intercepted() or name not in ("gelu", "relu", "relu2", "silu", "swiglu") or x.dim() == 0 or x.numel() == 0
+            or x.shape[-1] % (16 if name == "swiglu" else 8)):
         return ref.activate(x, name)
     return run_function(_ActivationFn, x, name)
 
@@ -892,7 +893,8 @@ def cross_entropy(logits, targets, ignore_index=-100):
     """Mean fp32 cross-entropy of materialised logits.  Without gradients (validation) bf16 logits are read once, as they are; with
     them, or in another type, torch's ops run."""
     if (logits.dtype == BF16 and logits.dim() == 2 and logits.stride(1) == 1 and targets.dtype == torch.int64 and targets.dim() == 1
-            and targets.shape[0] == logits.shape[0] and targets.device == logits.device and not intercepted() and not (torch.is_grad_enabled() and logits.requires_grad)):
+            and targets.shape[0] == logits.shape[0] and targets.device == logits.device and not intercepted()
+            and not (torch.is_grad_enabled() and logits.requires_grad)):
         count_path("cross_entropy:kernel")
         return ext().row_nll(logits, targets.contiguous(), int(ignore_index)).sum() / (targets != ignore_index).sum()
     count_path("cross_entropy:torch")
@@ -902,7 +904,8 @@ def cross_entropy(logits, targets, ignore_index=-100):
 def continuation_logprob(logits: Tensor, tokens: Tensor, prefix: Tensor, end: Tensor) -> Optional[Tensor]:
     """log p of tokens[i, j] for prefix[i] <= j < end[i] (0 elsewhere) as fp32 [n, length - 1], column j - 1 for token j; None when the
     kernel does not cover the call (gradients, transforms, other types)."""
-    if (intercepted() or logits.dtype != BF16 or logits.dim() != 3 or logits.stride(2) != 1 or tokens.dtype != torch.int64 or tokens.device != logits.device
+    if (intercepted() or logits.dtype != BF16 or logits.dim() != 3 or logits.stride(2) != 1
+            or tokens.dtype != torch.int64 or tokens.device != logits.device
             or logits.shape[:2] != tokens.shape or not 1 <= tokens.shape[0] <= 65535 or tokens.shape[1] < 2 or tokens.stride(1) != 1
             or (torch.is_grad_enabled() and logits.requires_grad)):
         return None

@@ -67,3 +67,23 @@ def test_a_gradient_that_is_read_is_formed():
     base = torch.randn(1 + dy.numel(), device="cuda")
     cuda_ops.embedding(module, ids).backward(base[1:].view(dy.shape))  # a gradient on no 16-byte boundary
     assert torch.allclose(buffer, 2 * want + torch.zeros_like(want).index_add_(0, ids.view(-1), base[1:].view(-1, 16)), atol=2e-5)
+
+
+def test_tangents_and_traces_run_through_the_module():
+    module = torch.nn.Embedding(7, 8, device="cuda")
+    module.weight.main_grad, module.weight.grad_ready = torch.zeros(7, 8, device="cuda"), True
+    ids = torch.tensor([[1, 2, 6]], device="cuda")
+    from torch.autograd import forward_ad
+    with forward_ad.dual_level():
+        assert torch.equal(cuda_ops.embedding(module, ids), module(ids))
+
+    class Lookup(torch.nn.Module):
+        def __init__(self):
+            super().__init__()
+            self.table = module
+
+        def forward(self, i):
+            return cuda_ops.embedding(self.table, i)
+
+    traced = torch.jit.trace(Lookup(), ids, check_trace=False)
+    assert "PythonOp" not in str(traced.inlined_graph) and torch.equal(traced(ids.flip(1)), module(ids.flip(1)))
