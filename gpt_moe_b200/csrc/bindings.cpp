@@ -79,8 +79,8 @@ CUtensorMap cached_map(const void* ptr, int elem_bytes, uint64_t cols, uint64_t 
 }
 
 // operand map for the bf16 GEMM: `t` is [rows, cols] or [batch, rows, cols] with cols contiguous
-CUtensorMap operand_map(const torch::Tensor& t, bool mn_major, int tile_rows_k_major) {
-    GM_CHECK(t.is_cuda() && t.scalar_type() == torch::kBFloat16, "GEMM operands must be CUDA bf16 tensors");
+CUtensorMap operand_map(const torch::Tensor& t, bool mn_major, int tile_rows_k_major, torch::ScalarType type = torch::kBFloat16) {
+    GM_CHECK(t.is_cuda() && t.scalar_type() == type, "GEMM operands must be CUDA bf16 tensors");
     GM_CHECK(t.dim() == 2 || t.dim() == 3, "GEMM operands must be 2-D or 3-D");
     GM_CHECK(t.stride(-1) == 1, "GEMM operands must have a contiguous last dimension");
     const uint64_t batch = t.dim() == 3 ? t.size(0) : 1;
@@ -95,17 +95,23 @@ CUtensorMap operand_map(const torch::Tensor& t, bool mn_major, int tile_rows_k_m
 //   mode 1 (grouped M): a [rows, K], b [E, N, K] or [E, K, N], d [rows, N]; tile_expert/num_m_tiles on device
 //   mode 2 (grouped K): a [rows, M] (a_mn), b [rows, N] (b_mn), d [E, M, N]; seg_ends on device
 //   may_split: a long contraction with few output tiles may be shared by several CTAs, whose partial results meet in the order of arrival
+//   half_types: A, B and C may all be fp16 instead of bf16, and so may d (Polar Express; the calls from Python take bf16 and fp32)
+//   diag: added to the diagonal of a symmetric result alpha * A B^T + beta * C
 void gemm_run(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d, bool a_mn, bool b_mn, double alpha,
               double beta, const c10::optional<torch::Tensor>& c, bool accumulate, int64_t mode,
               const c10::optional<torch::Tensor>& tile_expert, const c10::optional<torch::Tensor>& num_m_tiles,
               const c10::optional<torch::Tensor>& seg_ends, bool symmetric, const c10::optional<torch::Tensor>& batch_sumsq,
-              int64_t scale_mode, bool may_split) {
+              int64_t scale_mode, bool may_split, bool half_types = false, double diag = 0.0) {
     c10::cuda::CUDAGuard guard(a.device());
     gm::GemmParams p;
     std::memset(&p, 0, sizeof(p));
     p.mode = static_cast<int>(mode);
     GM_CHECK(d.is_cuda() && d.stride(-1) == 1, "GEMM output must be a CUDA tensor with a contiguous last dimension");
-    GM_CHECK(d.scalar_type() == torch::kBFloat16 || d.scalar_type() == torch::kFloat32, "GEMM output must be bf16 or fp32");
+    GM_CHECK(d.scalar_type() == torch::kBFloat16 || d.scalar_type() == torch::kFloat32 || (half_types && d.scalar_type() == torch::kHalf),
+             "GEMM output must be bf16 or fp32");
+    const torch::ScalarType in_type = half_types && a.scalar_type() == torch::kHalf ? torch::kHalf : torch::kBFloat16;
+    p.in_f16 = in_type == torch::kHalf;
+    p.out_f16 = d.scalar_type() == torch::kHalf;
     p.M = d.size(-2);
     p.N = d.size(-1);
     p.batch = d.dim() == 3 ? d.size(0) : 1;
@@ -140,7 +146,7 @@ void gemm_run(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d, 
     p.alpha = static_cast<float>(alpha);
     p.beta = static_cast<float>(beta);
     if (c.has_value()) {
-        GM_CHECK(c->scalar_type() == torch::kBFloat16 && c->stride(-1) == 1, "C must be bf16 with a contiguous last dimension");
+        GM_CHECK(c->scalar_type() == in_type && c->stride(-1) == 1, "C must be bf16 with a contiguous last dimension");
         p.C = c->data_ptr();
         p.ldc = c->stride(-2);
         p.c_batch_stride = c->dim() == 3 ? c->stride(0) : 0;
@@ -168,8 +174,8 @@ void gemm_run(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d, 
             p.split_k = static_cast<int>(std::min<int64_t>(sm_count() / tiles, k_blocks / 8));
         if (p.split_k > 1 && !accumulate) d.zero_();
     }
-    const CUtensorMap& ta = operand_map(a, a_mn, 128);
-    const CUtensorMap& tb = operand_map(b, b_mn, 128);
+    const CUtensorMap& ta = operand_map(a, a_mn, 128, in_type);
+    const CUtensorMap& tb = operand_map(b, b_mn, 128, in_type);
     const int eb = p.out_fp32 ? 4 : 2;
     const CUtensorMap& td = cached_map(d.data_ptr(), eb, p.N, p.M, d.dim() == 3 ? d.size(0) : 1, p.ldd * eb,
                                        d.dim() == 3 ? d.stride(0) * eb : 0, 128 / eb, 128, 128);
@@ -177,6 +183,8 @@ void gemm_run(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d, 
     CUtensorMap tc, tmirror;
     const bool tma_c = p.C != nullptr && mode == gm::GEMM_DENSE && !p.out_fp32 && !a_mn && p.K > 0 && c->dim() == d.dim() && c->sizes() == d.sizes() &&
                        p.ldc > 0 && (p.batch == 1 || p.c_batch_stride > 0);
+    GM_CHECK((!p.in_f16 || p.C == nullptr || tma_c) && (diag == 0.0 || (tma_c && symmetric)), "GEMM: an fp16 C or a diagonal term needs C in the layout of the output");
+    p.diag = static_cast<float>(diag);
     if (tma_c) {
         tc = cached_map(p.C, 2, p.N, p.M, p.batch, p.ldc * 2, d.dim() == 3 ? p.c_batch_stride * 2 : 0, 64, 128, 128);
         if (p.symmetric) tmirror = cached_map(p.D, 2, p.N, p.M, p.batch, p.ldd * 2, d.dim() == 3 ? p.d_batch_stride * 2 : 0, 64, 64, 128);
@@ -190,6 +198,78 @@ void gemm_bf16(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d,
                const c10::optional<torch::Tensor>& num_m_tiles, const c10::optional<torch::Tensor>& seg_ends, bool symmetric,
                const c10::optional<torch::Tensor>& batch_sumsq, int64_t scale_mode) {
     gemm_run(a, b, d, a_mn, b_mn, alpha, beta, c, accumulate, mode, tile_expert, num_m_tiles, seg_ends, symmetric, batch_sumsq, scale_mode, true);
+}
+
+// ---- Polar Express ------------------------------------------------------------------------------------
+// Five steps X <- (a I + b A + c A^2) X, A = X X^T, on a batch of wide bf16 matrices x [n, m, k], m <= k; the result is bf16, and x is scratch.
+// The polynomials of consecutive steps commute, so a run of steps is carried out on the small m x m side: with Q = a I + b A + c A^2
+// the next Gram matrix is Q A Q, and the product of the run's Q goes to X once.  A run costs one X X^T and one Q X whatever its length,
+// where every step paid for both.  Runs of two and three steps are 18 products, 14 of them small, single steps 15 with 5 small ones.
+// us, single steps with bf16 Gram matrices / here: 96 of 768 x 6144 5060 / 2870, 96 of 768 x 3072 3050 / 2060, 128 of 768 x 1536 2490 / 2310,
+// 16 of 768 x 6144 990 / 657, 16 of 768 x 3072 607 / 505, in runs; where a run's fourteen small products are launches of a few waves they
+// cost what the large ones save (24 of 1024 x 2048 1075 / 1113, 3 of 512 x 2048 286 / 308): runs are taken for X at least three times as wide
+// as high with two tiles of Q X for every CTA pair, or twice as wide with six tiles of a small product.
+// Rounding noise of A grows by a^2 a step against the smallest singular values.  Error against 64 bits (2-norm; matrices 768 x 3072:
+// Gaussian / rank 8 plus noise / singular values 1/i / exp(-12 i / m)): single steps in bf16 1.06e-2 / 5.8e-2 / 3.6e-2 / 9.3e-2, runs of two and
+// three 0.48e-2 / 4.8e-2 / 3.4e-2 / 6.8e-2; one run of five reaches 0.1 to 20 and is not taken, nor are runs of matrices lower than 256.
+// That takes fp16 for A and Q (bounded: |A| <= 1.3, |Q| <= 8.2, a run's product <= 39) and the order Q (A Q), whose error in the directions
+// that A hardly has is of second order; and the product of a run's Q is computed in full: mirrored, errors were three to five times as large,
+// since rounded Q commute only nearly.  The first Q X stays bf16 x bf16, as x arrives with any scale; X is fp16 after it.
+torch::Tensor polar_express(torch::Tensor x, const c10::optional<torch::Tensor>& sumsq, const std::vector<std::vector<double>>& coeffs) {
+    GM_CHECK(x.is_cuda() && x.dim() == 3 && x.scalar_type() == torch::kBFloat16 && x.is_contiguous(), "polar_express wants contiguous bf16 matrices [n, m, k]");
+    for (const auto& c : coeffs) GM_CHECK(c.size() == 3, "polar_express: three coefficients a step");
+    const int64_t n = x.size(0), m = x.size(1), k = x.size(2);
+    GM_CHECK(m <= k && !coeffs.empty(), "polar_express wants wide matrices and at least one step");
+    c10::cuda::CUDAGuard guard(x.device());
+    const int steps = static_cast<int>(coeffs.size());
+    const int64_t mt = (m + 255) / 256, kt = (k + 255) / 256;
+    const bool runs = m >= 256 && ((k >= 3 * m && n * mt * kt >= sm_count()) || (k >= 2 * m && n * mt * (mt + 1) / 2 >= 3 * sm_count()));
+    const auto half = x.options().dtype(torch::kHalf);
+    torch::Tensor small[4];
+    for (int i = 0; i < (runs ? 4 : 2); ++i) small[i] = gm::out_empty({n, m, m}, half);
+    torch::Tensor y = gm::out_empty({n, m, k}, half);
+    const auto product = [&](const torch::Tensor& a, const torch::Tensor& b, torch::Tensor d) {        // a and b symmetric: a b^T = a b
+        gemm_run(a, b, d, false, false, 1.0, 0.0, c10::nullopt, false, gm::GEMM_DENSE, c10::nullopt, c10::nullopt, c10::nullopt, true, c10::nullopt, 0, false, true);
+    };
+    torch::Tensor in = x;
+    for (int first = 0; first < steps;) {
+        const int count = !runs ? 1 : first == 0 ? std::min(2, steps) : std::min(3, steps - first);
+        const bool raw = first == 0 && sumsq.has_value();                      // not normalised yet: the epilogues do it
+        const auto type = in.scalar_type();                                    // of the factor that meets X
+        const torch::Tensor& gram = small[0];
+        gemm_run(in, in, small[0], false, false, 1.0, 0.0, c10::nullopt, false, gm::GEMM_DENSE, c10::nullopt, c10::nullopt, c10::nullopt, true,
+                 raw ? sumsq : c10::nullopt, raw ? 2 : 0, false, true);
+        int q = 1, total = 1, spare = 2;                                       // buffers of the step's Q, of the run's product, and a free one
+        for (int j = 0; j < count; ++j) {
+            if (j > 0) {
+                product(gram, small[q], small[spare]);
+                product(small[q], small[spare], gram);
+            }
+            const auto& c = coeffs[first + j];
+            const int next = j == 0 ? q : spare;
+            torch::Tensor poly = small[next];
+            if (count == 1) poly = poly.view(type);
+            gemm_run(gram, gram, poly, false, false, c[2], c[1], gram, false, gm::GEMM_DENSE, c10::nullopt, c10::nullopt, c10::nullopt, true, c10::nullopt, 0, false,
+                     true, c[0]);
+            if (j > 0) {
+                const int to = q == total ? 3 : q;                             // the last Q is not needed any more
+                torch::Tensor both = j == count - 1 ? small[to].view(type) : small[to];
+                gemm_run(poly, small[total], both, false, true, 1.0, 0.0, c10::nullopt, false, gm::GEMM_DENSE, c10::nullopt, c10::nullopt, c10::nullopt, false,
+                         c10::nullopt, 0, false, true);
+                spare = total;
+                total = to;
+                q = next;
+            }
+        }
+        const bool done = first + count == steps;
+        torch::Tensor out = in.data_ptr() == y.data_ptr() ? x : y;
+        out = out.view(done ? torch::kBFloat16 : torch::kHalf);
+        gemm_run(small[total].view(type), in, out, false, true, 1.0, 0.0, c10::nullopt, false, gm::GEMM_DENSE, c10::nullopt, c10::nullopt, c10::nullopt, false,
+                 raw ? sumsq : c10::nullopt, raw ? 1 : 0, false, true);
+        in = out;
+        first += count;
+    }
+    return in;
 }
 
 // ---- MXFP8 ----------------------------------------------------------------------------------------
@@ -422,6 +502,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           py::arg("mode") = 0, py::arg("tile_expert") = py::none(), py::arg("num_m_tiles") = py::none(),
           py::arg("seg_ends") = py::none(), py::arg("symmetric") = false,
           py::arg("batch_sumsq") = py::none(), py::arg("scale_mode") = 0);
+    m.def("polar_express", &polar_express, py::arg("x"), py::arg("sumsq"), py::arg("coeffs"));
     m.def("mxfp8_quantize", &mxfp8_quantize, py::arg("x"), py::arg("rows_limit") = py::none());
     m.def("mxfp8_quantize_weight", &mxfp8_quantize_weight);
     m.def("gemm_mxfp8", &gemm_mxfp8, py::arg("a"), py::arg("sfa"), py::arg("b"), py::arg("sfb"), py::arg("d"), py::arg("alpha") = 1.0,

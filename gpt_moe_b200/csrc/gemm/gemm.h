@@ -26,6 +26,8 @@ struct GemmParams {
                                  // diagonal are computed and every off-diagonal tile is also stored transposed
     const float* batch_sumsq;    // DENSE, optional: per-batch sum of squares; s = 1 / (sqrt(sumsq[z]) * 1.02 + 1e-6) is Muon's Frobenius
     int scale_mode;              // normalisation of an operand, folded into the epilogue: 1 -> alpha * s and beta * s, 2 -> alpha * s * s
+    int in_f16, out_f16;         // DENSE: A, B and C are fp16 instead of bf16; a 16-bit output is fp16
+    float diag;                  // symmetric with C through TMA: added to the diagonal of the result
     int b_shared;                // DENSE: one B for every problem of the batch
     int* status;                 // device word; kernels write a non-zero code if a bounded wait gives up
 };

@@ -44,6 +44,28 @@ constexpr uint32_t TMEM_COLS = 512;
 constexpr int SLAB_BYTES = BM * 128;              // one slab of [128 rows][128 bytes]
 constexpr int STAGING_BYTES = 2 * SLAB_BYTES;    // two slabs; the staging area holds two such buffers
 
+constexpr uint32_t kIdescBf16Operands = (1u << 7) | (1u << 10);      // operand formats of the instruction descriptor: 1 = bf16, 0 = fp16
+
+// eight 16-bit values, bf16 or fp16 (uniform over the grid), to and from fp32
+__device__ __forceinline__ void unpack_16bit(const uint4& raw, int f16, float* v) {
+    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const float2 f = f16 ? __half22float2(*reinterpret_cast<const __half2*>(&w[e])) : __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[e]));
+        v[2 * e] = f.x;
+        v[2 * e + 1] = f.y;
+    }
+}
+__device__ __forceinline__ uint4 pack_16bit(const float* v, int f16) {
+    uint4 o;
+    if (f16) {
+        o.x = pack_half2(v[0], v[1]); o.y = pack_half2(v[2], v[3]); o.z = pack_half2(v[4], v[5]); o.w = pack_half2(v[6], v[7]);
+    } else {
+        o.x = pack_bf16x2(v[0], v[1]); o.y = pack_bf16x2(v[2], v[3]); o.z = pack_bf16x2(v[4], v[5]); o.w = pack_bf16x2(v[6], v[7]);
+    }
+    return o;
+}
+
 struct TileCoord {
     int m0, n0;        // element offsets of the tile in the output
     int az, bz, dz;    // z (batch / expert) coordinates for A, B, D
@@ -190,7 +212,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         }
     } else if (warp == 1) {
         if (lane == 0 && cta_rank == 0) {
-            constexpr uint32_t idesc = make_idesc_bf16(2 * BM, BN, A_MN, B_MN);
+            const uint32_t idesc = make_idesc_bf16(2 * BM, BN, A_MN, B_MN) & ~(p.in_f16 ? kIdescBf16Operands : 0u);
             // K-major: 8-row groups are 1024 B apart, 16 K-elements = 32 B.  MN-major: 64-element column slabs are
             // BK*128 B apart (leading offset), 8-K-row groups 1024 B apart, 16 K-rows = 2048 B.
             constexpr uint32_t a_lbo = A_MN ? BK * 128 : 16, b_lbo = B_MN ? BK * 128 : 16;
@@ -270,20 +292,21 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                 if (ok && !mbar_wait(&c_full[fetched & 1], (fetched >> 1) & 1)) { atomicExch(p.status, 105); ok = false; }
                 uint8_t* slab = staging + (use & 3) * SLAB_BYTES;
                 uint8_t* slab_row = slab + row_in_tile * 128;
+                // column of this chunk that lies on the diagonal in this thread's row (p.diag is added there; -1: none)
+                const int on_diag = p.diag != 0.f ? t.m0 + row_in_tile - (t.n0 + round * 64 + half * 32) : -1;
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     uint4* piece = reinterpret_cast<uint4*>(slab_row + (((half * 4 + q) ^ sw) << 4));
                     const uint4 cv = *piece;
-                    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&cv);
                     float v[8];
+                    unpack_16bit(cv, p.in_f16, v);
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const float2 f = __bfloat1622float2(h[e]);
-                        v[2 * e] = __uint_as_float(r[8 * q + 2 * e]) * alpha + beta * f.x;
-                        v[2 * e + 1] = __uint_as_float(r[8 * q + 2 * e + 1]) * alpha + beta * f.y;
+                    for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(r[8 * q + e]) * alpha + beta * v[e];
+                    if (on_diag >= 8 * q && on_diag < 8 * q + 8) {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) v[e] += on_diag == 8 * q + e ? p.diag : 0.f;
                     }
-                    uint4 o;
-                    o.x = pack_bf16x2(v[0], v[1]); o.y = pack_bf16x2(v[2], v[3]); o.z = pack_bf16x2(v[4], v[5]); o.w = pack_bf16x2(v[6], v[7]);
+                    const uint4 o = pack_16bit(v, p.out_f16);
                     *piece = o;
                     if (mirror) { r[4 * q] = o.x; r[4 * q + 1] = o.y; r[4 * q + 2] = o.z; r[4 * q + 3] = o.w; }      // kept packed for the transposed store
                 }
@@ -415,10 +438,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                                 if (col0 + i < t.n_limit) v[i] += beta * __bfloat162float(c[i]);
                         }
                     }
-                    if (mirror) {
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) r[j][i] = __float_as_uint(v[i]);      // kept for the transposed store below
-                    }
                     // 16-byte pieces of this thread's row go to piece index (i ^ row%8) of the 128-byte slab row
                     if (p.out_fp32) {
 #pragma unroll
@@ -427,12 +446,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                     } else {
 #pragma unroll
                         for (int q = 0; q < 4; ++q) {
-                            uint4 o;
-                            o.x = pack_bf16x2(v[8 * q], v[8 * q + 1]);
-                            o.y = pack_bf16x2(v[8 * q + 2], v[8 * q + 3]);
-                            o.z = pack_bf16x2(v[8 * q + 4], v[8 * q + 5]);
-                            o.w = pack_bf16x2(v[8 * q + 6], v[8 * q + 7]);
+                            const uint4 o = pack_16bit(v + 8 * q, p.out_f16);
                             *reinterpret_cast<uint4*>(slab_row + (((j * 4 + q) ^ sw) << 4)) = o;
+                            // kept packed for the transposed store below
+                            r[j][4 * q] = o.x; r[j][4 * q + 1] = o.y; r[j][4 * q + 2] = o.z; r[j][4 * q + 3] = o.w;
                         }
                     }
                 }
@@ -455,7 +472,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                 }
                 ++stores;
                 if (mirror) {
-                    // The same 128 x 128 block goes out transposed (bf16 only): element (row, c) of this round lands in row c of
+                    // The same 128 x 128 block goes out transposed (16-bit results only): element (row, c) of this round lands in row c of
                     // the transposed block, and 64 of this CTA's rows make one 128-byte slab row, so the two slabs are the
                     // column ranges [m0, m0 + 64) and [m0 + 64, m0 + 128) of the mirrored tile.
                     uint8_t* tbuf = staging + (stores & 1) * STAGING_BYTES;
@@ -468,8 +485,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 #pragma unroll
                         for (int i = 0; i < 32; ++i) {
                             const int cl = (half * 2 + j) * 32 + i;
-                            *reinterpret_cast<__nv_bfloat16*>(tcol + cl * 128 + ((piece ^ (i & 7)) << 4)) =
-                                __float2bfloat16_rn(__uint_as_float(r[j][i]));
+                            *reinterpret_cast<uint16_t*>(tcol + cl * 128 + ((piece ^ (i & 7)) << 4)) =
+                                static_cast<uint16_t>(r[j][(i >> 3) * 4 + ((i & 7) >> 1)] >> ((i & 1) * 16));
                         }
                     }
                     fence_proxy_async();

@@ -1,0 +1,45 @@
+"""Polar Express on the small side (`polar_express` in csrc/bindings.cpp): runs of steps and single steps against 64 bits."""
+import pytest
+import torch
+
+from gpt_moe_b200.ops import reference as ref
+
+pytestmark = pytest.mark.gpu
+
+
+def _exact(g):
+    x = g.double()
+    x = x / (x.norm(dim=(-2, -1), keepdim=True) * 1.02 + 1e-6)
+    for a, b, c in ref.POLAR_EXPRESS_COEFFS:
+        gram = x @ x.mT
+        x = a * x + (b * gram + c * (gram @ gram)) @ x
+    return x
+
+
+def _error(x, exact):
+    return ((x.double() - exact).norm(dim=(-2, -1)) / exact.norm(dim=(-2, -1))).max().item()
+
+
+# (batch, rows, columns): runs with whole tiles, with ragged ones, at the least height, just too few tiles for runs, just too narrow for them
+# (single steps with the fp16 Gram matrices), one row of pieces
+@pytest.mark.parametrize("shape", [(16, 768, 1536), (12, 520, 2056), (64, 256, 704), (8, 256, 768), (16, 768, 1528), (3, 8, 768)])
+@pytest.mark.parametrize("spectrum", ["gaussian", "decaying"])
+def test_polar_express_is_no_further_from_64_bits_than_single_steps_in_bf16(shape, spectrum):
+    from gpt_moe_b200.ops import cuda_ops
+    torch.manual_seed(9)
+    n, m, k = shape
+    g = torch.randn(n, m, k, device="cuda")
+    if spectrum == "decaying":
+        u, v = torch.linalg.qr(torch.randn(n, m, m, device="cuda"))[0], torch.linalg.qr(torch.randn(n, k, m, device="cuda"))[0]
+        g = (u * torch.exp(-12 * torch.arange(1, m + 1, device="cuda") / m)) @ v.mT
+    raw = (g * 3e-4).bfloat16()
+    sumsq = raw.float().pow(2).sum(dim=(-2, -1))
+    exact = _exact(raw)
+    got = cuda_ops.polar_express_bf16(raw.clone(), sumsq)
+    assert got.dtype == torch.bfloat16 and got.shape == raw.shape
+    # the same steps one by one with every matrix rounded to bf16; a tenth for the luck of single roundings, and 2^-8 for the output's own
+    plain = _error(ref.polar_express(raw, dtype=torch.bfloat16), exact)
+    assert _error(got, exact) < 1.1 * plain + 2 ** -8
+    normalised = (raw.double() / (raw.double().norm(dim=(-2, -1), keepdim=True) * 1.02 + 1e-6)).bfloat16()
+    assert _error(cuda_ops.polar_express_bf16(normalised.clone()), _exact(normalised * 1.0)) < 1.1 * plain + 2 ** -6
+    cuda_ops.check_status()
