@@ -89,6 +89,24 @@ CUtensorMap operand_map(const torch::Tensor& t, bool mn_major, int tile_rows_k_m
     return cached_map(t.data_ptr(), 2, cols, rows, batch, rs, bs, 64, mn_major ? 64 : tile_rows_k_major, 128);
 }
 
+// Shares of the contraction for a bf16 result whose output tiles fill the CTA pairs badly (the input gradient of the LM head contracts over
+// the vocabulary into 12 to 128 tiles).  Estimates in us, fitted on this part: a pair takes 0.42 for a block of 64 and 2 for a tile's
+// read-out, summing the shares costs a launch and their bytes.  1024 x 768 x 50304: 297 us whole, 72 in shares;
+// 3840 rows 310 and 217, 8192 rows 552 and 432; at 12544 rows (147 tiles for 74 pairs, 603) whole tiles are the better form.
+int bf16_splits(int64_t m, int64_t n, int64_t k, int sms) {
+    const int64_t tiles = ((m + 255) / 256) * ((n + 255) / 256), blocks = (k + 63) / 64, pairs = std::max(1, sms / 2);
+    const auto estimate = [&](int64_t s) {
+        const double sum = s > 1 ? 4.0 + static_cast<double>(m) * n * (8 * s + 2) / 6.0e6 : 0.0;
+        return ((tiles * s + pairs - 1) / pairs) * (((blocks + s - 1) / s) * 0.42 + 2.0) + sum;
+    };
+    int64_t best = 1;
+    for (int64_t s = 2; s <= 8 && blocks / s >= 16; ++s)
+        if (estimate(s) < estimate(best)) best = s;
+    if (best == 1 || estimate(best) > 0.93 * estimate(1)) return 1;
+    const int64_t per = (blocks + best - 1) / best;
+    return static_cast<int>((blocks + per - 1) / per);                        // every share has work
+}
+
 // D[.., M, N] = alpha * op(A) op(B)^T + beta * C, optionally accumulated into an fp32 D.
 //   a_mn = false: a is [.., M, K];  a_mn = true: a is [.., K, M]   (same for b with N)
 //   mode 0 (dense): a, b and d with the same batch, or one 2-D b for a whole batch
@@ -174,11 +192,26 @@ void gemm_run(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d, 
             p.split_k = static_cast<int>(std::min<int64_t>(sm_count() / tiles, k_blocks / 8));
         if (p.split_k > 1 && !accumulate) d.zero_();
     }
+    // a bf16 result: the shares go to fp32 slabs of their own and are summed in order
+    torch::Tensor parts;
+    if (mode == gm::GEMM_DENSE && d.scalar_type() == torch::kBFloat16 && !half_types && p.batch == 1 && d.dim() == 2 && p.C == nullptr && !p.symmetric &&
+        p.batch_sumsq == nullptr && p.M > 0 && p.N > 0) {
+        const int splits = bf16_splits(p.M, p.N, p.K, sm_count());
+        if (splits > 1) {
+            parts = gm::out_empty({splits, p.M, (p.N + 3) / 4 * 4}, d.options().dtype(torch::kFloat32));
+            p.split_k = splits;
+            p.split_slabs = 1;
+            p.out_fp32 = 1;
+            p.ldd = parts.stride(1);
+            p.d_batch_stride = parts.stride(0);
+        }
+    }
     const CUtensorMap& ta = operand_map(a, a_mn, 128, in_type);
     const CUtensorMap& tb = operand_map(b, b_mn, 128, in_type);
     const int eb = p.out_fp32 ? 4 : 2;
-    const CUtensorMap& td = cached_map(d.data_ptr(), eb, p.N, p.M, d.dim() == 3 ? d.size(0) : 1, p.ldd * eb,
-                                       d.dim() == 3 ? d.stride(0) * eb : 0, 128 / eb, 128, 128);
+    const bool slabs = parts.defined();
+    const CUtensorMap& td = cached_map(slabs ? parts.data_ptr() : d.data_ptr(), eb, p.N, p.M, slabs ? p.split_k : d.dim() == 3 ? d.size(0) : 1, p.ldd * eb,
+                                       slabs || d.dim() == 3 ? p.d_batch_stride * eb : 0, 128 / eb, 128, 128);
     // C of the output's shape comes through TMA; any other (broadcast over the batch or over rows, beside an fp32 output) is read by the threads
     CUtensorMap tc, tmirror;
     const bool tma_c = p.C != nullptr && mode == gm::GEMM_DENSE && !p.out_fp32 && !a_mn && p.K > 0 && c->dim() == d.dim() && c->sizes() == d.sizes() &&
@@ -192,6 +225,11 @@ void gemm_run(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d, 
     cudaError_t e = gm::launch_gemm_bf16(ta, tb, td, tma_c ? &tc : nullptr, tma_c && p.symmetric ? &tmirror : nullptr, p, a_mn, b_mn, sm_count(),
                                          current_stream());
     GM_CHECK(e == cudaSuccess, cudaGetErrorString(e));
+    if (slabs) {
+        gm::launch_split_sum(parts.data_ptr<float>(), p.split_k, p.M, p.N, static_cast<int>(p.ldd), d.data_ptr(), d.stride(-2), current_stream());
+        e = cudaGetLastError();
+        GM_CHECK(e == cudaSuccess, cudaGetErrorString(e));
+    }
 }
 void gemm_bf16(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d, bool a_mn, bool b_mn, double alpha, double beta,
                const c10::optional<torch::Tensor>& c, bool accumulate, int64_t mode, const c10::optional<torch::Tensor>& tile_expert,

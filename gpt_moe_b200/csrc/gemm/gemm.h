@@ -19,6 +19,7 @@ struct GemmParams {
     float alpha, beta;
     int out_fp32, accumulate;    // accumulate: D += result (fp32 output only)
     int split_k;                 // >1: the K loop is shared by this many CTAs per tile, partials meet in a TMA reduce-add (fp32 output)
+    int split_slabs;             // with split_k: every share stores its partial sums as problem `share` of D [split_k, M, N] instead (fp32, batch 1)
     const int* tile_expert;      // GROUPED_M: expert of each 128-row tile
     const int* num_m_tiles;      // GROUPED_M: number of 128-row tiles (device scalar)
     const int* seg_ends;         // GROUPED_K: cumulative padded row ends per expert
@@ -45,6 +46,9 @@ bool make_tensor_map(CUtensorMap* out, const void* base, int elem_bytes, uint64_
 // `tmirror`: with it, for symmetric results, the map of D with a 64-row box.
 cudaError_t launch_gemm_bf16(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const CUtensorMap* tc, const CUtensorMap* tmirror,
                              const GemmParams& p, bool a_mn, bool b_mn, int sms, cudaStream_t stream);
+
+// d [rows, cols] bf16 (row pitch ldd, a multiple of 8) = the sum over s of parts [splits, rows, ldp] fp32, in this order
+void launch_split_sum(const float* parts, int splits, long long rows, int cols, int ldp, void* d, long long ldd, cudaStream_t s);
 
 // Block-scaled MXFP8 GEMM: D[M,N] (bf16) = alpha * A[M,K] B[N,K]^T, e4m3 operands, UE8M0 scales per 32 elements of K.
 // Scales are stored as 512-byte records [row block of 128][K block of 128]; byte (r % 32) * 16 + (r / 32) * 4 + g of a record

@@ -141,6 +141,7 @@ __device__ __forceinline__ TileCoord tile_coord(const GemmParams& p, int tile, i
         t.k_begin += first * BK;
         t.k_blocks = count;
         t.store_zeros = false;
+        if (p.split_slabs) t.dz = split;
     }
     return t;
 }
@@ -360,7 +361,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         const int my_chunks = chunks_per_round / 2;               // per warp half
         const int rounds = (BN / 32) / chunks_per_round;
         const int cols_per_slab = 128 / elem;
-        const bool reduce = p.accumulate || p.split_k > 1;
+        const bool reduce = p.accumulate || (p.split_k > 1 && !p.split_slabs);
         const int sw = row_in_tile & 7;
         int acc = 0; uint32_t acc_ph = 0;
         uint32_t stores = 0;                                       // committed store groups: selects the staging buffer
@@ -526,6 +527,39 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         tc_fence_after();
         tmem_dealloc_pair(tmem_base, TMEM_COLS);
     }
+}
+
+// The shares of a split contraction, summed in their order (the same bits every time) and rounded once.  A thread owns four columns; bound by
+// the copy rate: six shares of 1024 x 768 take 6 us, four of 7680 x 768 21.
+__global__ void __launch_bounds__(256)
+split_sum_kernel(const float* __restrict__ parts, int splits, long long rows, int cols, int ldp, __nv_bfloat16* __restrict__ d, long long ldd) {
+    const int quads = (cols + 3) >> 2;
+    const long long slab = rows * ldp, total = rows * quads;
+    for (long long i = blockIdx.x * 256LL + threadIdx.x; i < total; i += gridDim.x * 256LL) {
+        const long long row = i / quads;
+        const int col = static_cast<int>(i - row * quads) * 4;
+        const float* src = parts + row * ldp + col;
+        float4 v = *reinterpret_cast<const float4*>(src);
+#pragma unroll 4
+        for (int s = 1; s < splits; ++s) {
+            const float4 w = *reinterpret_cast<const float4*>(src + s * slab);
+            v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
+        }
+        __nv_bfloat16* dst = d + row * ldd + col;
+        if (col + 4 <= cols) {
+            *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
+        } else {
+            const float t[3] = {v.x, v.y, v.z};
+#pragma unroll
+            for (int e = 0; e < 3; ++e)
+                if (col + e < cols) dst[e] = __float2bfloat16_rn(t[e]);
+        }
+    }
+}
+
+void launch_split_sum(const float* parts, int splits, long long rows, int cols, int ldp, void* d, long long ldd, cudaStream_t s) {
+    const long long blocks = (rows * ((cols + 3) / 4) + 255) / 256;
+    split_sum_kernel<<<static_cast<int>(blocks < 8192 ? blocks : 8192), 256, 0, s>>>(parts, splits, rows, cols, ldp, static_cast<__nv_bfloat16*>(d), ldd);
 }
 
 constexpr int GEMM_SMEM_BYTES = STAGES * STAGE_BYTES + 2 * STAGING_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/;

@@ -837,7 +837,7 @@ class _LinearCrossEntropyFn(torch.autograd.Function):
     """mean CE of (x @ W^T) against targets without materialising all logits: rows are processed in chunks;
     each chunk's logits are overwritten in place by their gradient, which immediately feeds the dX and dW GEMMs."""
 
-    CHUNK = 8192
+    CHUNK = 12544        # 49 pair tiles of 256 rows: the input gradient of a 768-wide head fills the CTA pairs twice (147 tiles for 74 pairs)
 
     @staticmethod
     def forward(ctx, x: Tensor, weight: Tensor, targets: Tensor, ignore_index: int) -> Tensor:

@@ -1,0 +1,27 @@
+"""bf16 products whose contraction is shared by several CTA pairs (`bf16_splits` in csrc/bindings.cpp): fp32 slabs summed in order."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+# the LM head's input gradient at two row counts; a last share that is shorter than the others; rows and columns outside whole tiles, the
+# result a slice of a wider matrix; just long enough for two shares and just too short
+@pytest.mark.parametrize("m,n,k", [(1024, 768, 50304), (3840, 768, 8192), (200, 104, 6152), (33, 8, 2048), (64, 264, 2112), (64, 264, 1984)])
+@pytest.mark.parametrize("b_mn", [False, True])
+def test_shared_contraction(m, n, k, b_mn):
+    from gpt_moe_b200.ops import cuda_ops
+    torch.manual_seed(8)
+    c = cuda_ops.ext()
+    a = torch.randn(m, k, device="cuda").bfloat16()
+    b = torch.randn((k, n) if b_mn else (n, k), device="cuda").bfloat16()
+    wide = torch.full((m + 1, n + 24), 5.0, device="cuda", dtype=torch.bfloat16)
+    c.gemm_bf16(a, b, wide[:m, 8: 8 + n], False, b_mn, 0.25)
+    want = 0.25 * (a.double() @ (b.double() if b_mn else b.double().t()))
+    # one rounding to bf16 (2^-9 relative at most) over sums that are fp32
+    assert ((wide[:m, 8: 8 + n].double() - want).abs() <= 2 ** -8 * want.abs() + 1e-5 * k ** 0.5).all()
+    assert (wide[m] == 5).all() and (wide[:, :8] == 5).all() and (wide[:, 8 + n:] == 5).all()
+    again = torch.empty(m, n, device="cuda", dtype=torch.bfloat16)
+    c.gemm_bf16(a, b, again, False, b_mn, 0.25)
+    assert torch.equal(again, wide[:m, 8: 8 + n])                  # the shares are summed in the same order every time
+    cuda_ops.check_status()
