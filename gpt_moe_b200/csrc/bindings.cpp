@@ -381,8 +381,8 @@ void gemm_mxfp8(const torch::Tensor& a, const torch::Tensor& sfa, const torch::T
     p.status = status_tensor(a.device().index()).data_ptr<int>();
     const uint64_t ab = a.dim() == 3 ? a.size(0) : 1, bb = b.dim() == 3 ? b.size(0) : 1;
     const CUtensorMap& ta = cached_map(a.data_ptr(), 1, p.K, a.size(-2), ab, p.K, a.size(-2) * static_cast<uint64_t>(p.K), 128, 128, 128);
-    const CUtensorMap& tb = cached_map(b.data_ptr(), 1, p.K, p.N, bb, p.K, static_cast<uint64_t>(p.N) * p.K, 128, 128, 128);
-    const CUtensorMap& td = cached_map(d.data_ptr(), 2, p.N, p.M, d.dim() == 3 ? d.size(0) : 1, d.stride(-2) * 2, d.dim() == 3 ? d.stride(0) * 2 : 0, 64, 128, 128);
+    const CUtensorMap& tb = cached_map(b.data_ptr(), 1, p.K, p.N, bb, p.K, static_cast<uint64_t>(p.N) * p.K, 128, gm::mxfp8_b_box_rows(p), 128);
+    const CUtensorMap& td = cached_map(d.data_ptr(), 2, p.N, p.M, d.dim() == 3 ? d.size(0) : 1, d.stride(-2) * 2, d.dim() == 3 ? d.stride(0) * 2 : 0, 64, 32, 128);
     // scale arrays as [records, 128 words]: one TMA row per 512-byte record, no swizzle
     GM_CHECK(reinterpret_cast<uintptr_t>(sfa.data_ptr()) % 16 == 0 && reinterpret_cast<uintptr_t>(sfb.data_ptr()) % 16 == 0, "scale arrays must be 16-byte aligned");
     const CUtensorMap& tsfa = cached_map(sfa.data_ptr(), 4, 128, sfa.numel() / 512, 1, 512, 0, 128, 1, 0);

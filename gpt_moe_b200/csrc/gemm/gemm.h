@@ -66,6 +66,8 @@ struct Mxfp8Params {
     int* status;
 };
 
+// rows in the box of B's map (each CTA of a pair stages half of a tile's columns)
+int mxfp8_b_box_rows(const Mxfp8Params& p);
 // tsfa / tsfb: maps over the scale arrays seen as [records, 128] 32-bit words (one 512-byte record per row), box {128, 1}
 cudaError_t launch_gemm_mxfp8(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const CUtensorMap& tsfa,
                               const CUtensorMap& tsfb, const Mxfp8Params& p, int sms, cudaStream_t stream);

@@ -161,7 +161,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     uint64_t* c_full = acc_empty + 2;                              // TMA_C: [2] slab of C landed
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(c_full + 2);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int cta_rank = static_cast<int>(cluster_ctarank());     // 0 = leader of the pair
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
@@ -178,41 +178,42 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     tc_fence_before();
     cluster_sync_all();                                            // both CTAs' barriers exist before either signals the other
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = uniform(*tmem_slot);
 
     int m_tiles, n_tiles;
-    const int tiles = total_tiles(p, m_tiles, n_tiles);
+    const int tiles = uniform(total_tiles(p, m_tiles, n_tiles));
     const int first_tile = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
     bool ok = true;
 
     if (warp == 0) {
-        if (lane == 0) {
-            int s = 0; uint32_t ph = 0;
-            for (int tile = first_tile; tile < tiles && ok; tile += tile_step) {
-                const TileCoord t = tile_coord(p, tile, cta_rank, m_tiles, n_tiles);
-                for (int kb = 0; kb < t.k_blocks; ++kb) {
-                    if (!mbar_wait(&empty[s], ph ^ 1)) { atomicExch(p.status, 101); ok = false; break; }
-                    if (cta_rank == 0) mbar_expect_tx(&full[s], 2 * STAGE_BYTES);      // both CTAs' copies land on the leader's barrier
-                    uint8_t* a_dst = smem + s * STAGE_BYTES;
-                    uint8_t* b_dst = a_dst + A_BYTES;
-                    const int k = t.k_begin + kb * BK;
-                    const int bn0 = t.n0 + cta_rank * BN_HALF;                          // this CTA stages its half of the B tile
-                    if (A_MN) {
-                        for (int i = 0; i < BM / 64; ++i) tma_load_3d_pair(a_dst + i * (64 * BK * 2), &tmap_a, &full[s], t.m0 + 64 * i, k, t.az);
-                    } else {
-                        tma_load_3d_pair(a_dst, &tmap_a, &full[s], k, t.m0, t.az);
-                    }
-                    if (B_MN) {
-                        for (int i = 0; i < BN_HALF / 64; ++i) tma_load_3d_pair(b_dst + i * (64 * BK * 2), &tmap_b, &full[s], bn0 + 64 * i, k, t.bz);
-                    } else {
-                        tma_load_3d_pair(b_dst, &tmap_b, &full[s], k, bn0, t.bz);
-                    }
-                    if (++s == STAGES) { s = 0; ph ^= 1; }
+        const uint32_t on = elect_one();
+        int s = 0; uint32_t ph = 0;
+        for (int tile = first_tile; tile < tiles && ok; tile += tile_step) {
+            const TileCoord t = tile_coord(p, tile, cta_rank, m_tiles, n_tiles);
+            const int k_blocks = uniform(t.k_blocks), k_begin = uniform(t.k_begin), bz = uniform(t.bz);
+            for (int kb = 0; kb < k_blocks; ++kb) {
+                if (!warp_wait(&empty[s], ph ^ 1)) { atomicExch(p.status, 101); ok = false; break; }
+                if (cta_rank == 0 && on) mbar_expect_tx(&full[s], 2 * STAGE_BYTES);      // both CTAs' copies land on the leader's barrier
+                uint8_t* a_dst = smem + s * STAGE_BYTES;
+                uint8_t* b_dst = a_dst + A_BYTES;
+                const int k = k_begin + kb * BK;
+                const int bn0 = t.n0 + cta_rank * BN_HALF;                          // this CTA stages its half of the B tile
+                if (A_MN) {
+                    for (int i = 0; i < BM / 64; ++i) tma_load_3d_pair(a_dst + i * (64 * BK * 2), &tmap_a, &full[s], t.m0 + 64 * i, k, t.az, on);
+                } else {
+                    tma_load_3d_pair(a_dst, &tmap_a, &full[s], k, t.m0, t.az, on);
                 }
+                if (B_MN) {
+                    for (int i = 0; i < BN_HALF / 64; ++i) tma_load_3d_pair(b_dst + i * (64 * BK * 2), &tmap_b, &full[s], bn0 + 64 * i, k, bz, on);
+                } else {
+                    tma_load_3d_pair(b_dst, &tmap_b, &full[s], k, bn0, bz, on);
+                }
+                if (++s == STAGES) { s = 0; ph ^= 1; }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && cta_rank == 0) {
+        if (cta_rank == 0) {
+            const uint32_t on = elect_one();
             const uint32_t idesc = make_idesc_bf16(2 * BM, BN, A_MN, B_MN) & ~(p.in_f16 ? kIdescBf16Operands : 0u);
             // K-major: 8-row groups are 1024 B apart, 16 K-elements = 32 B.  MN-major: 64-element column slabs are
             // BK*128 B apart (leading offset), 8-K-row groups 1024 B apart, 16 K-rows = 2048 B.
@@ -220,25 +221,24 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             constexpr uint32_t a_kstep = A_MN ? 2048 : 32, b_kstep = B_MN ? 2048 : 32;
             int s = 0; uint32_t ph = 0; int acc = 0; uint32_t acc_ph = 0;
             for (int tile = first_tile; tile < tiles && ok; tile += tile_step) {
-                const TileCoord t = tile_coord(p, tile, cta_rank, m_tiles, n_tiles);
-                if (t.k_blocks == 0) continue;
-                if (!mbar_wait(&acc_empty[acc], acc_ph ^ 1)) { atomicExch(p.status, 102); ok = false; break; }
+                const int k_blocks = uniform(tile_coord(p, tile, cta_rank, m_tiles, n_tiles).k_blocks);
+                if (k_blocks == 0) continue;
+                if (!warp_wait(&acc_empty[acc], acc_ph ^ 1)) { atomicExch(p.status, 102); ok = false; break; }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * BN;
-                for (int kb = 0; kb < t.k_blocks; ++kb) {
-                    if (!mbar_wait(&full[s], ph)) { atomicExch(p.status, 103); ok = false; break; }
+                for (int kb = 0; kb < k_blocks; ++kb) {
+                    if (!warp_wait(&full[s], ph)) { atomicExch(p.status, 103); ok = false; break; }
                     tc_fence_after();
                     const uint32_t a_addr = smem_u32(smem + s * STAGE_BYTES), b_addr = a_addr + A_BYTES;
-                    for (int k4 = 0; k4 < BK / 16; ++k4) {
-                        const uint64_t adesc = make_smem_desc(a_addr + k4 * a_kstep, a_lbo, 1024);
-                        const uint64_t bdesc = make_smem_desc(b_addr + k4 * b_kstep, b_lbo, 1024);
-                        umma_f16_pair(d_tmem, adesc, bdesc, idesc, (kb | k4) != 0);
-                    }
-                    umma_commit_pair(&empty[s]);
+                    const uint64_t adesc = make_smem_desc(a_addr, a_lbo, 1024), bdesc = make_smem_desc(b_addr, b_lbo, 1024);
+#pragma unroll
+                    for (int k4 = 0; k4 < BK / 16; ++k4)          // the address field counts 16-byte units
+                        umma_f16_pair(d_tmem, adesc + k4 * (a_kstep >> 4), bdesc + k4 * (b_kstep >> 4), idesc, (kb | k4) != 0, on);
+                    umma_commit_pair(&empty[s], on);
                     if (++s == STAGES) { s = 0; ph ^= 1; }
                 }
                 if (!ok) break;
-                umma_commit_pair(&acc_full[acc]);
+                umma_commit_pair(&acc_full[acc], on);
                 if (++acc == 2) { acc = 0; acc_ph ^= 1; }
             }
         }

@@ -34,7 +34,8 @@ constexpr int FA_BYTES = FM * FK, FB_BYTES = FN_HALF * FK, SF_BYTES = SF_RECORD_
 constexpr int FSTAGE_TX = FA_BYTES + FB_BYTES + 3 * SF_BYTES;        // bytes one CTA receives per stage
 constexpr int FSTAGE_BYTES = 34 * 1024;                                // stage pitch: tiles stay 1024-byte aligned
 constexpr int F_THREADS = 320;
-constexpr int F_STAGING = 2 * FM * 128;                                // one staging buffer: two slabs of [128 rows][128 bytes]
+constexpr int F_SLAB = 32 * 128;                                       // a warp's staging slab: [32 rows][128 bytes]
+constexpr int F_STAGING = 8 * 2 * F_SLAB;                              // two for each epilogue warp
 constexpr uint32_t F_TMEM_COLS = 512;
 constexpr uint32_t COL_SFA = 256, COL_SFB = 264;                       // after the 256-column accumulator
 constexpr int F_GROUP_M = 4;                                           // raster: pair rows that share a column sweep
@@ -49,16 +50,21 @@ __device__ __forceinline__ uint64_t make_sf_desc(uint32_t smem_addr) {
 }
 
 __device__ __forceinline__ void umma_mxf8_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t sfa, uint32_t sfb,
-                                               uint32_t accumulate) {
+                                               uint32_t accumulate, uint32_t on) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, q;\n\t"
         "setp.ne.b32 p, %6, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%4], [%5], p;\n\t}\n"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate) : "memory");
+        "setp.ne.b32 q, %7, 0;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%4], [%5], p;\n\t}\n"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate), "r"(on) : "memory");
 }
 // shared -> TMEM copy of a 512-byte scale record in BOTH CTAs of the pair (each from its own shared memory, same offset)
-__device__ __forceinline__ void tmem_cp_sf_pair(uint32_t taddr, uint64_t s_desc) {
-    asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(s_desc) : "memory");
+__device__ __forceinline__ void tmem_cp_sf_pair(uint32_t taddr, uint64_t s_desc, uint32_t on) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %2, 0;\n\t"
+        "@q tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;\n\t}\n"
+        ::"r"(taddr), "l"(s_desc), "r"(on) : "memory");
 }
 
 struct FTile { int m0, n0, bz, z, m_limit; };
@@ -93,13 +99,13 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* staging = smem + FSTAGES * FSTAGE_BYTES;
-    uint64_t* full = reinterpret_cast<uint64_t*>(staging + 2 * F_STAGING);
+    uint64_t* full = reinterpret_cast<uint64_t*>(staging + F_STAGING);
     uint64_t* empty = full + FSTAGES;
     uint64_t* acc_full = empty + FSTAGES;
     uint64_t* acc_empty = acc_full + 1;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int cta_rank = static_cast<int>(cluster_ctarank());
     if (threadIdx.x == 0) {
         for (int s = 0; s < FSTAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
@@ -113,65 +119,65 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     tc_fence_before();
     cluster_sync_all();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = uniform(*tmem_slot);
 
     int m_pairs, n_tiles;
-    const int tiles = f_total_tiles(p, m_pairs, n_tiles);
+    const int tiles = uniform(f_total_tiles(p, m_pairs, n_tiles));
     const int k_blocks = (p.K + FK - 1) / FK;
     const int first_tile = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
     bool ok = true;
 
     if (warp == 0) {
-        if (lane == 0) {
-            int s = 0; uint32_t ph = 0;
-            for (int tile = first_tile; tile < tiles && ok; tile += tile_step) {
-                const FTile t = f_tile(p, tile, cta_rank, m_pairs, n_tiles);
-                // record index of (row block, K block 0) in the [records, 128 words] scale tensors
-                const int sfa_rec = (t.z * p.sfa_row_blocks + t.m0 / 128) * k_blocks;
-                const int sfb_rec = (t.bz * p.sfb_row_blocks + t.n0 / 128) * k_blocks;
-                const bool second_b = t.n0 / 128 + 1 < p.sfb_row_blocks;     // the tile's upper 128 columns exist at all
-                for (int kb = 0; kb < k_blocks; ++kb) {
-                    if (!mbar_wait(&empty[s], ph ^ 1)) { atomicExch(p.status, 401); ok = false; break; }
-                    if (cta_rank == 0) mbar_expect_tx(&full[s], 2 * FSTAGE_TX);
-                    uint8_t* a_dst = smem + s * FSTAGE_BYTES;
-                    uint8_t* b_dst = a_dst + FA_BYTES;
-                    uint8_t* sf_dst = b_dst + FB_BYTES;
-                    tma_load_3d_pair(a_dst, &tmap_a, &full[s], kb * FK, t.m0, t.z);
-                    tma_load_3d_pair(b_dst, &tmap_b, &full[s], kb * FK, t.n0 + cta_rank * FN_HALF, t.bz);
-                    // rows beyond the tensors (last row block of A, a B tile narrower than 256) read as zeros: their products are clipped
-                    tma_load_3d_pair(sf_dst, &tmap_sfa, &full[s], 0, sfa_rec + kb, 0);
-                    tma_load_3d_pair(sf_dst + SF_BYTES, &tmap_sfb, &full[s], 0, sfb_rec + kb, 0);
-                    tma_load_3d_pair(sf_dst + 2 * SF_BYTES, &tmap_sfb, &full[s], 0, second_b ? sfb_rec + k_blocks + kb : sfb_rec + kb, 0);
-                    if (++s == FSTAGES) { s = 0; ph ^= 1; }
-                }
+        const uint32_t on = elect_one();
+        int s = 0; uint32_t ph = 0;
+        for (int tile = first_tile; tile < tiles && ok; tile += tile_step) {
+            const FTile t = f_tile(p, tile, cta_rank, m_pairs, n_tiles);
+            // record index of (row block, K block 0) in the [records, 128 words] scale tensors
+            const int sfa_rec = (t.z * p.sfa_row_blocks + t.m0 / 128) * k_blocks;
+            const int bz = uniform(t.bz);
+            const int sfb_rec = (bz * p.sfb_row_blocks + t.n0 / 128) * k_blocks;
+            const bool second_b = t.n0 / 128 + 1 < p.sfb_row_blocks;     // the tile's upper 128 columns exist at all
+            for (int kb = 0; kb < k_blocks; ++kb) {
+                if (!warp_wait(&empty[s], ph ^ 1)) { atomicExch(p.status, 401); ok = false; break; }
+                if (cta_rank == 0 && on) mbar_expect_tx(&full[s], 2 * FSTAGE_TX);
+                uint8_t* a_dst = smem + s * FSTAGE_BYTES;
+                uint8_t* b_dst = a_dst + FA_BYTES;
+                uint8_t* sf_dst = b_dst + FB_BYTES;
+                tma_load_3d_pair(a_dst, &tmap_a, &full[s], kb * FK, t.m0, t.z, on);
+                tma_load_3d_pair(b_dst, &tmap_b, &full[s], kb * FK, t.n0 + cta_rank * FN_HALF, bz, on);
+                // rows beyond the tensors (last row block of A, a B tile narrower than 256) read as zeros: their products are clipped
+                tma_load_3d_pair(sf_dst, &tmap_sfa, &full[s], 0, sfa_rec + kb, 0, on);
+                tma_load_3d_pair(sf_dst + SF_BYTES, &tmap_sfb, &full[s], 0, sfb_rec + kb, 0, on);
+                tma_load_3d_pair(sf_dst + 2 * SF_BYTES, &tmap_sfb, &full[s], 0, second_b ? sfb_rec + k_blocks + kb : sfb_rec + kb, 0, on);
+                if (++s == FSTAGES) { s = 0; ph ^= 1; }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && cta_rank == 0) {
+        if (cta_rank == 0) {
+            const uint32_t on = elect_one();
             constexpr uint32_t idesc = make_idesc_mxf8(2 * FM, FN);
             int s = 0; uint32_t ph = 0; uint32_t acc_ph = 0;
             for (int tile = first_tile; tile < tiles && ok; tile += tile_step) {
-                if (!mbar_wait(acc_empty, acc_ph ^ 1)) { atomicExch(p.status, 402); ok = false; break; }
+                if (!warp_wait(acc_empty, acc_ph ^ 1)) { atomicExch(p.status, 402); ok = false; break; }
                 tc_fence_after();
                 for (int kb = 0; kb < k_blocks; ++kb) {
-                    if (!mbar_wait(&full[s], ph)) { atomicExch(p.status, 403); ok = false; break; }
+                    if (!warp_wait(&full[s], ph)) { atomicExch(p.status, 403); ok = false; break; }
                     tc_fence_after();
                     const uint32_t a_addr = smem_u32(smem + s * FSTAGE_BYTES), b_addr = a_addr + FA_BYTES, sf_addr = b_addr + FB_BYTES;
-                    tmem_cp_sf_pair(tmem_base + COL_SFA, make_sf_desc(sf_addr));
-                    tmem_cp_sf_pair(tmem_base + COL_SFB, make_sf_desc(sf_addr + SF_BYTES));
-                    tmem_cp_sf_pair(tmem_base + COL_SFB + 4, make_sf_desc(sf_addr + 2 * SF_BYTES));
+                    const uint64_t sf_desc = make_sf_desc(sf_addr), adesc = make_smem_desc(a_addr, 16, 1024), bdesc = make_smem_desc(b_addr, 16, 1024);
+                    tmem_cp_sf_pair(tmem_base + COL_SFA, sf_desc, on);
+                    tmem_cp_sf_pair(tmem_base + COL_SFB, sf_desc + (SF_BYTES >> 4), on);
+                    tmem_cp_sf_pair(tmem_base + COL_SFB + 4, sf_desc + (2 * SF_BYTES >> 4), on);
 #pragma unroll
-                    for (int g = 0; g < FK / 32; ++g) {
-                        const uint64_t adesc = make_smem_desc(a_addr + g * 32, 16, 1024);
-                        const uint64_t bdesc = make_smem_desc(b_addr + g * 32, 16, 1024);
+                    for (int g = 0; g < FK / 32; ++g) {              // the address field counts 16-byte units
                         const uint32_t id = idesc | (static_cast<uint32_t>(g) << 29) | (static_cast<uint32_t>(g) << 4);
-                        umma_mxf8_pair(tmem_base, adesc, bdesc, id, tmem_base + COL_SFA, tmem_base + COL_SFB, (kb | g) != 0);
+                        umma_mxf8_pair(tmem_base, adesc + 2 * g, bdesc + 2 * g, id, tmem_base + COL_SFA, tmem_base + COL_SFB, (kb | g) != 0, on);
                     }
-                    umma_commit_pair(&empty[s]);
+                    umma_commit_pair(&empty[s], on);
                     if (++s == FSTAGES) { s = 0; ph ^= 1; }
                 }
                 if (!ok) break;
-                umma_commit_pair(acc_full);
+                umma_commit_pair(acc_full, on);
                 acc_ph ^= 1;
             }
         }
@@ -180,9 +186,8 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         // two warps of a quadrant take the two 64-column halves of every 128-column round.
         const int quad = warp & 3;
         const int half = (warp - 2) >> 2;
-        const int row_in_tile = quad * 32 + lane;
-        const bool leader = threadIdx.x == 64;
-        const int sw = row_in_tile & 7;
+        const int sw = lane & 7;
+        uint8_t* slabs = staging + (warp - 2) * 2 * F_SLAB;
         uint32_t acc_ph = 0;
         uint32_t stores = 0;
         for (int tile = first_tile; tile < tiles; tile += tile_step) {
@@ -202,12 +207,12 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             if (lane == 0) mbar_arrive_cluster(acc_empty, 0);     // the accumulator is free: the next tile's MMAs may start
 #pragma unroll
             for (int round = 0; round < 2; ++round) {
-                const int round_col0 = t.n0 + round * 128;
-                if (round_col0 >= p.N) break;                      // uniform across the CTA
-                uint8_t* buf = staging + (stores & 1) * F_STAGING;
-                if (leader) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-                asm volatile("bar.sync 1, 256;" ::: "memory");
-                uint8_t* slab_row = buf + half * (FM * 128) + row_in_tile * 128;
+                const int col = t.n0 + round * 128 + half * 64;
+                if (col >= p.N || t.m0 + quad * 32 >= t.m_limit) break;        // uniform across the warp
+                uint8_t* slab = slabs + (stores & 1) * F_SLAB;
+                // the store of two slabs ago has finished reading this one
+                if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+                __syncwarp();
 #pragma unroll
                 for (int j = 0; j < 2; ++j) {
 #pragma unroll
@@ -217,24 +222,20 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                         o.y = pack_bf16x2(__uint_as_float(r[round][j][8 * q + 2]) * p.alpha, __uint_as_float(r[round][j][8 * q + 3]) * p.alpha);
                         o.z = pack_bf16x2(__uint_as_float(r[round][j][8 * q + 4]) * p.alpha, __uint_as_float(r[round][j][8 * q + 5]) * p.alpha);
                         o.w = pack_bf16x2(__uint_as_float(r[round][j][8 * q + 6]) * p.alpha, __uint_as_float(r[round][j][8 * q + 7]) * p.alpha);
-                        *reinterpret_cast<uint4*>(slab_row + (((j * 4 + q) ^ sw) << 4)) = o;
+                        *reinterpret_cast<uint4*>(slab + lane * 128 + (((j * 4 + q) ^ sw) << 4)) = o;
                     }
                 }
                 fence_proxy_async();
-                asm volatile("bar.sync 1, 256;" ::: "memory");
-                if (leader) {
-                    for (int sl = 0; sl < 2; ++sl) {
-                        const int col = round_col0 + sl * 64;
-                        if (col >= p.N || t.m0 >= t.m_limit) break;
-                        asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
-                                     ::"l"(&tmap_d), "r"(smem_u32(buf + sl * (FM * 128))), "r"(col), "r"(t.m0), "r"(t.z) : "memory");
-                    }
+                __syncwarp();
+                if (lane == 0) {
+                    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
+                                 ::"l"(&tmap_d), "r"(smem_u32(slab)), "r"(col), "r"(t.m0 + quad * 32), "r"(t.z) : "memory");
                     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                 }
                 ++stores;
             }
         }
-        if (leader) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     }
 
     // common teardown: every path (including a timed-out wait) reaches it, so TMEM is always released
@@ -250,20 +251,222 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     }
 }
 
-constexpr int F_SMEM = FSTAGES * FSTAGE_BYTES + 2 * F_STAGING + 1024 + 256;
+// ---- short contractions: A stays ---------------------------------------------------------------------------------------------
+// With K <= 1024 the kernel above is bound by its operand stream: a 256 x 256 tile of K = 768 pulls 2 x 192 KB through L2 in the time of 24
+// MMAs, and its one accumulator makes the next tile wait for the read-out.  Here a pair walks CONSECUTIVE tiles of an output row with the
+// row's A (128 x K per CTA, at most 128 KB) and its scales resident, so that only B streams (half the bytes), and tiles are 192 columns wide:
+// with A in place a narrower tile moves no more bytes, and two accumulators of 192 columns leave room for the scale factors (384 + 64 of
+// 512 columns), so MMAs of one tile run under the read-out of the other.
+//   warp 0    : TMA producer - A and its scale records K block by K block when the row changes (each block as soon as the row before has
+//               done with it), B halves (96 rows) and the scale records of B through a ring
+//   warp 1    : MMA issuer (leader CTA) - M256 N192 K32; scale factors go through four TMEM buffers in turn
+//   warps 2-13: epilogue - a warp owns 32 rows x 64 columns, stages them in a slab of its own and stores by itself
+// The scales of a tile's 192 columns lie in two 128-row records; every other tile starts in the middle of one, two TMEM columns further on.
+// us against the kernel above as it was (operands of one lane, see umma_f16 in ptx.cuh; CUDA events, launch included): 32768 x 2304 x 768 81 -> 60,
+// 34816 x 6144 x 768 198 -> 158, 34816 x 3072 x 768 129 -> 105.  With parts switched off the second takes 92 without loads and stores (the
+// MMAs: 59 tiles of 24 x 98 clocks), 118 without loads and MMAs (428 MB of results at 3.9 TB/s): products and result stores are what is
+// left.  Storing by the threads, through the same slabs, took 163.
+constexpr int RN = 192, RN_HALF = RN / 2, R_MAX_KB = 8, R_MAX_STAGES = 8;
+constexpr int R_THREADS = 64 + 12 * 32;
+constexpr int RB_BYTES = RN_HALF * FK, RB_STAGE = RB_BYTES + 2 * SF_BYTES;
+constexpr int R_STAGING = 12 * F_SLAB;
+constexpr uint32_t R_COL_SF = 2 * RN, R_SF_BUFFERS = 4;                // 16 columns a buffer: A at 0, B at 8
+
+__host__ __device__ constexpr int resident_fixed_bytes(int k_blocks) { return k_blocks * (FA_BYTES + SF_BYTES) + R_STAGING + 1024 + 512; }
+__host__ __device__ constexpr int resident_stages(int k_blocks) {
+    const int n = (232448 - resident_fixed_bytes(k_blocks)) / RB_STAGE;
+    return n < R_MAX_STAGES ? n : R_MAX_STAGES;
+}
+
+__global__ void __launch_bounds__(R_THREADS, 1)
+gemm_mxfp8_resident_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+                           const __grid_constant__ CUtensorMap tmap_d, const __grid_constant__ CUtensorMap tmap_sfa,
+                           const __grid_constant__ CUtensorMap tmap_sfb, const Mxfp8Params p) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    const int k_blocks = p.K / FK;                                 // K is a multiple of 128
+    const int stages = resident_stages(k_blocks);
+    uint8_t* ring = smem + k_blocks * FA_BYTES;
+    uint8_t* staging = ring + stages * RB_STAGE;
+    uint8_t* sfa_smem = staging + R_STAGING;
+    uint64_t* a_full = reinterpret_cast<uint64_t*>(sfa_smem + k_blocks * SF_BYTES);
+    uint64_t* a_empty = a_full + R_MAX_KB;
+    uint64_t* b_full = a_empty + R_MAX_KB;
+    uint64_t* b_empty = b_full + R_MAX_STAGES;
+    uint64_t* acc_full = b_empty + R_MAX_STAGES;
+    uint64_t* acc_empty = acc_full + 2;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+
+    const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int cta_rank = static_cast<int>(cluster_ctarank());
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < k_blocks; ++s) { mbar_init(&a_full[s], 1); mbar_init(&a_empty[s], 1); }
+        for (int s = 0; s < stages; ++s) { mbar_init(&b_full[s], 1); mbar_init(&b_empty[s], 1); }
+        for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 24); }      // one arrival per epilogue warp of each CTA
+        fence_barrier_init();
+        tma_prefetch_desc(&tmap_a); tma_prefetch_desc(&tmap_b); tma_prefetch_desc(&tmap_d);
+        tma_prefetch_desc(&tmap_sfa); tma_prefetch_desc(&tmap_sfb);
+    }
+    if (warp == 1) { tmem_alloc_pair(tmem_slot, F_TMEM_COLS); tmem_relinquish_pair(); }
+    tc_fence_before();
+    cluster_sync_all();
+    tc_fence_after();
+    const uint32_t tmem_base = uniform(*tmem_slot);
+
+    const int n_tiles = (p.N + RN - 1) / RN;
+    const int m_pairs = p.grouped ? (*p.num_m_tiles + 1) / 2 : (p.M + 2 * FM - 1) / (2 * FM);
+    const int m_limit = p.grouped ? *p.num_m_tiles * FM : p.M;
+    const long long tiles = static_cast<long long>(m_pairs) * n_tiles * (p.grouped ? 1 : p.batch);
+    const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    const int begin = uniform(static_cast<int>(tiles * pair / pairs)), end = uniform(static_cast<int>(tiles * (pair + 1) / pairs));
+    bool ok = true;
+
+    if (warp == 0) {
+        const uint32_t on = elect_one();
+        int s = 0; uint32_t ph = 0, a_ph = 0;
+        for (int tile = begin; tile < end && ok; ++tile) {
+            const int row = tile / n_tiles, n0 = (tile - row * n_tiles) * RN;
+            const int z = p.grouped ? 0 : row / m_pairs;
+            const int m0 = 2 * (row - z * m_pairs) * FM + cta_rank * FM;
+            const int bz = p.grouped ? uniform(p.tile_expert[m0 / FM & ~1]) : z;      // expert segments are padded to 256 rows: one expert per pair
+            const bool first = tile == begin || n0 == 0;
+            const int sfa_rec = (z * p.sfa_row_blocks + m0 / 128) * k_blocks;
+            const int sfb_rec = (bz * p.sfb_row_blocks + n0 / 128) * k_blocks;
+            const bool second_b = n0 / 128 + 1 < p.sfb_row_blocks;
+            for (int kb = 0; kb < k_blocks; ++kb) {
+                if (first) {
+                    if (!warp_wait(&a_empty[kb], a_ph ^ 1)) { atomicExch(p.status, 411); ok = false; break; }
+                    if (cta_rank == 0 && on) mbar_expect_tx(&a_full[kb], 2 * (FA_BYTES + SF_BYTES));
+                    tma_load_3d_pair(smem + kb * FA_BYTES, &tmap_a, &a_full[kb], kb * FK, m0, z, on);
+                    tma_load_3d_pair(sfa_smem + kb * SF_BYTES, &tmap_sfa, &a_full[kb], 0, sfa_rec + kb, 0, on);
+                }
+                if (!warp_wait(&b_empty[s], ph ^ 1)) { atomicExch(p.status, 412); ok = false; break; }
+                if (cta_rank == 0 && on) mbar_expect_tx(&b_full[s], 2 * RB_STAGE);
+                uint8_t* b_dst = ring + s * RB_STAGE;
+                tma_load_3d_pair(b_dst, &tmap_b, &b_full[s], kb * FK, n0 + cta_rank * RN_HALF, bz, on);
+                tma_load_3d_pair(b_dst + RB_BYTES, &tmap_sfb, &b_full[s], 0, sfb_rec + kb, 0, on);
+                tma_load_3d_pair(b_dst + RB_BYTES + SF_BYTES, &tmap_sfb, &b_full[s], 0, second_b ? sfb_rec + k_blocks + kb : sfb_rec + kb, 0, on);
+                if (++s == stages) { s = 0; ph ^= 1; }
+            }
+            if (first) a_ph ^= 1;
+        }
+    } else if (warp == 1) {
+        if (cta_rank == 0) {
+            const uint32_t on = elect_one();
+            constexpr uint32_t idesc = make_idesc_mxf8(2 * FM, RN);
+            int s = 0; uint32_t ph = 0, a_ph = 0, acc_ph = 0, sf_buffer = 0; int acc = 0;
+            for (int tile = begin; tile < end && ok; ++tile) {
+                const int nt = tile % n_tiles;
+                const bool first = tile == begin || nt == 0, last = tile == end - 1 || nt == n_tiles - 1;
+                const uint32_t sfb_shift = (nt * RN & 127) >> 5;
+                if (!warp_wait(&acc_empty[acc], acc_ph ^ 1)) { atomicExch(p.status, 413); ok = false; break; }
+                tc_fence_after();
+                for (int kb = 0; kb < k_blocks; ++kb) {
+                    if ((first && !warp_wait(&a_full[kb], a_ph)) || !warp_wait(&b_full[s], ph)) { atomicExch(p.status, 414); ok = false; break; }
+                    tc_fence_after();
+                    const uint32_t a_addr = smem_u32(smem + kb * FA_BYTES), b_addr = smem_u32(ring + s * RB_STAGE);
+                    const uint32_t sfa = tmem_base + R_COL_SF + sf_buffer * 16, sfb = sfa + 8;
+                    sf_buffer = (sf_buffer + 1) % R_SF_BUFFERS;
+                    const uint64_t sfb_desc = make_sf_desc(b_addr + RB_BYTES), adesc = make_smem_desc(a_addr, 16, 1024), bdesc = make_smem_desc(b_addr, 16, 1024);
+                    tmem_cp_sf_pair(sfa, make_sf_desc(smem_u32(sfa_smem + kb * SF_BYTES)), on);
+                    tmem_cp_sf_pair(sfb, sfb_desc, on);
+                    tmem_cp_sf_pair(sfb + 4, sfb_desc + (SF_BYTES >> 4), on);
+#pragma unroll
+                    for (int g = 0; g < FK / 32; ++g) {              // the address field counts 16-byte units
+                        const uint32_t id = idesc | (static_cast<uint32_t>(g) << 29) | (static_cast<uint32_t>(g) << 4);
+                        umma_mxf8_pair(tmem_base + acc * RN, adesc + 2 * g, bdesc + 2 * g, id, sfa, sfb + sfb_shift, (kb | g) != 0, on);
+                    }
+                    umma_commit_pair(&b_empty[s], on);
+                    if (last) umma_commit_pair(&a_empty[kb], on);
+                    if (++s == stages) { s = 0; ph ^= 1; }
+                }
+                if (!ok) break;
+                umma_commit_pair(&acc_full[acc], on);
+                if (++acc == 2) { acc = 0; acc_ph ^= 1; }
+                if (last) a_ph ^= 1;
+            }
+        }
+    } else {
+        const int quad = warp & 3, group = (warp - 2) >> 2;         // TMEM lanes 32 quad .. 32 quad + 31, columns 64 group .. 64 group + 63
+        const int sw = lane & 7;
+        uint8_t* slab = staging + (warp - 2) * F_SLAB;
+        uint32_t acc_ph = 0; int acc = 0;
+        for (int tile = begin; tile < end; ++tile) {
+            const int row = tile / n_tiles, col = (tile - row * n_tiles) * RN + group * 64;
+            const int z = p.grouped ? 0 : row / m_pairs;
+            const int m0 = (2 * (row - z * m_pairs) + cta_rank) * FM + quad * 32;
+            if (ok && !mbar_wait(&acc_full[acc], acc_ph)) { atomicExch(p.status, 415); ok = false; }
+            tc_fence_after();
+            uint32_t r[2][32];
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+                tmem_ld_32x32b_x32(tmem_base + acc * RN + group * 64 + j * 32 + (static_cast<uint32_t>(quad * 32) << 16), r[j]);
+            tmem_ld_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(&acc_empty[acc], 0);
+            if (++acc == 2) { acc = 0; acc_ph ^= 1; }
+            if (col >= p.N || m0 >= m_limit) continue;              // uniform across the warp
+            if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");      // the tile before has left the slab
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    uint4 o;
+                    o.x = pack_bf16x2(__uint_as_float(r[j][8 * q]) * p.alpha, __uint_as_float(r[j][8 * q + 1]) * p.alpha);
+                    o.y = pack_bf16x2(__uint_as_float(r[j][8 * q + 2]) * p.alpha, __uint_as_float(r[j][8 * q + 3]) * p.alpha);
+                    o.z = pack_bf16x2(__uint_as_float(r[j][8 * q + 4]) * p.alpha, __uint_as_float(r[j][8 * q + 5]) * p.alpha);
+                    o.w = pack_bf16x2(__uint_as_float(r[j][8 * q + 6]) * p.alpha, __uint_as_float(r[j][8 * q + 7]) * p.alpha);
+                    *reinterpret_cast<uint4*>(slab + lane * 128 + (((j * 4 + q) ^ sw) << 4)) = o;
+                }
+            }
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) {
+                asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
+                             ::"l"(&tmap_d), "r"(smem_u32(slab)), "r"(col), "r"(m0), "r"(z) : "memory");
+                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            }
+        }
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    }
+
+    // common teardown: every path (including a timed-out wait) reaches it, so TMEM is always released
+    tc_fence_before();
+    cluster_sync_all();
+    if (warp == 1) {
+        if (*reinterpret_cast<volatile int*>(p.status) != 0) {
+            const long long start = clock64();
+            while (clock64() - start < 200000) {}
+        }
+        tc_fence_after();
+        tmem_dealloc_pair(tmem_base, F_TMEM_COLS);
+    }
+}
+
+bool mxfp8_resident(const Mxfp8Params& p) {
+    const int k_blocks = p.K / FK, tiles = (p.N + RN - 1) / RN;
+    return k_blocks <= R_MAX_KB && tiles >= 2 && 8 * tiles * RN <= 9 * p.N;
+}
+int mxfp8_b_box_rows(const Mxfp8Params& p) { return mxfp8_resident(p) ? RN_HALF : FN_HALF; }
+
+constexpr int F_SMEM = FSTAGES * FSTAGE_BYTES + F_STAGING + 1024 + 256;
 
 cudaError_t launch_gemm_mxfp8(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const CUtensorMap& tsfa,
                               const CUtensorMap& tsfb, const Mxfp8Params& p, int sms, cudaStream_t stream) {
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(gemm_mxfp8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, F_SMEM);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_mxfp8_resident_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
         if (e != cudaSuccess) return e;
         configured = true;
     }
+    const bool resident = mxfp8_resident(p);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(sms & ~1);
-    cfg.blockDim = dim3(F_THREADS);
-    cfg.dynamicSmemBytes = F_SMEM;
+    cfg.blockDim = dim3(resident ? R_THREADS : F_THREADS);
+    cfg.dynamicSmemBytes = resident ? resident_fixed_bytes(p.K / FK) + resident_stages(p.K / FK) * RB_STAGE : F_SMEM;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -272,6 +475,7 @@ cudaError_t launch_gemm_mxfp8(const CUtensorMap& ta, const CUtensorMap& tb, cons
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
+    if (resident) return cudaLaunchKernelEx(&cfg, gemm_mxfp8_resident_kernel, ta, tb, td, tsfa, tsfb, p);
     return cudaLaunchKernelEx(&cfg, gemm_mxfp8_kernel, ta, tb, td, tsfa, tsfb, p);
 }
 
