@@ -136,11 +136,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     uint64_t* bar_qdo = bars + 5;                     // [QDO_STAGES]
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_qdo + QDO_STAGES);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int kv_tile = p.long_first ? blockIdx.z : blockIdx.x, kv_head = p.long_first ? blockIdx.x : blockIdx.y;
     const int batch = p.long_first ? blockIdx.y : blockIdx.z;
     const int kv0 = kv_tile * TILE;
-    const int window = p.window_ptr ? min(max(*p.window_ptr, 0), p.seq_len) : p.window;
+    const int window = uniform(p.window_ptr ? min(max(*p.window_ptr, 0), p.seq_len) : p.window);
     const int q_tiles_total = (p.seq_len + TILE - 1) / TILE;
     int last_q_tile = (kv0 + TILE - 1 + window) / TILE;
     if (last_q_tile > q_tiles_total - 1) last_q_tile = q_tiles_total - 1;
@@ -157,80 +157,78 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = uniform(*tmem_slot);
     bool ok = true;
 
     if (warp == 8) {
-        if (lane == 0) {
+        {
+            const uint32_t on = elect_one();
             constexpr uint32_t idesc_sdp = make_idesc_bf16(TILE, TILE, false, false);
             constexpr uint32_t idesc_dv = make_idesc_bf16(TILE, HD, true, true);
             constexpr uint32_t idesc_dk = make_idesc_bf16(TILE, DQK, true, true);
             constexpr uint32_t idesc_dq = make_idesc_bf16(TILE, DQK, false, true);
-            const uint32_t k_addr = smem_u32(sk), v_addr = smem_u32(sv), q_addr = smem_u32(sq), do_addr = smem_u32(sdo);
-            const uint32_t p_addr = smem_u32(sp), ds_addr = smem_u32(sds);
+            // descriptors formed once (K-major and MN-major forms of the same tiles); the address field counts 16-byte units
+            const uint64_t k_kmaj = make_smem_desc(smem_u32(sk), 16, 1024), v_kmaj = make_smem_desc(smem_u32(sv), 16, 1024);
+            const uint64_t q_kmaj = make_smem_desc(smem_u32(sq), 16, 1024), do_kmaj = make_smem_desc(smem_u32(sdo), 16, 1024);
+            const uint64_t q_mn = make_smem_desc(smem_u32(sq), TILE * 128, 1024), do_mn = make_smem_desc(smem_u32(sdo), TILE * 128, 1024);
+            const uint64_t k_mn = make_smem_desc(smem_u32(sk), TILE * 128, 1024);
+            const uint64_t p_mn = make_smem_desc(smem_u32(sp), TILE * 128, 1024), ds_mn = make_smem_desc(smem_u32(sds), TILE * 128, 1024);
+            const uint64_t ds_kmaj = make_smem_desc(smem_u32(sds), 16, 1024);
             auto load_qdo = [&](int it) {
                 const int st = it % QDO_STAGES;
                 const int head = kv_head * p.group + it / n_q;
                 const int q0 = (kv_tile + it % n_q) * TILE;
-                mbar_expect_tx(&bar_qdo[st], QK_BYTES + T_BYTES);
+                if (on) mbar_expect_tx(&bar_qdo[st], QK_BYTES + T_BYTES);
 #pragma unroll
                 for (int sl = 0; sl < QK_SLABS; ++sl)
-                    tma_load_3d(sq + st * QK_BYTES + sl * T_BYTES, &tmap_q, &bar_qdo[st], head * DQK + 64 * sl, q0, batch);
-                tma_load_3d(sdo + st * T_BYTES, &tmap_do, &bar_qdo[st], head * HD, q0, batch);
+                    tma_load_3d(sq + st * QK_BYTES + sl * T_BYTES, &tmap_q, &bar_qdo[st], head * DQK + 64 * sl, q0, batch, on);
+                tma_load_3d(sdo + st * T_BYTES, &tmap_do, &bar_qdo[st], head * HD, q0, batch, on);
             };
-            mbar_expect_tx(bar_kv, QK_BYTES + T_BYTES);
+            if (on) mbar_expect_tx(bar_kv, QK_BYTES + T_BYTES);
 #pragma unroll
-            for (int sl = 0; sl < QK_SLABS; ++sl) tma_load_3d(sk + sl * T_BYTES, &tmap_k, bar_kv, kv_head * DQK + 64 * sl, kv0, batch);
-            tma_load_3d(sv, &tmap_v, bar_kv, kv_head * p.v_head, kv0, batch);
+            for (int sl = 0; sl < QK_SLABS; ++sl) tma_load_3d(sk + sl * T_BYTES, &tmap_k, bar_kv, kv_head * DQK + 64 * sl, kv0, batch, on);
+            tma_load_3d(sv, &tmap_v, bar_kv, kv_head * p.v_head, kv0, batch, on);
             for (int it = 0; it < QDO_STAGES && it < n_iter; ++it) load_qdo(it);
-            if (!mbar_wait(bar_kv, 0)) { atomicExch(p.status, 301); ok = false; }
+            if (!warp_wait(bar_kv, 0)) { atomicExch(p.status, 301); ok = false; }
             auto issue_sdp = [&](int it) -> bool {               // S = Q K^T ; dP = dO V^T for iteration `it`
                 const int st = it % QDO_STAGES;
-                if (!mbar_wait(&bar_qdo[st], (it / QDO_STAGES) & 1)) return false;
+                if (!warp_wait(&bar_qdo[st], (it / QDO_STAGES) & 1)) return false;
                 tc_fence_after();
-                const uint32_t qa = q_addr + st * QK_BYTES, da = do_addr + st * T_BYTES;
+                const uint64_t qa = q_kmaj + st * (QK_BYTES >> 4), da = do_kmaj + st * (T_BYTES >> 4);
 #pragma unroll
                 for (int sl = 0; sl < QK_SLABS; ++sl)
 #pragma unroll
                     for (int k4 = 0; k4 < 4; ++k4)
-                        umma_f16(tmem_base + COL_S, make_smem_desc(qa + sl * T_BYTES + k4 * 32, 16, 1024),
-                                 make_smem_desc(k_addr + sl * T_BYTES + k4 * 32, 16, 1024), idesc_sdp, (sl | k4) != 0);
+                        umma_f16(tmem_base + COL_S, qa + sl * (T_BYTES >> 4) + k4 * 2, k_kmaj + sl * (T_BYTES >> 4) + k4 * 2, idesc_sdp, (sl | k4) != 0, on);
 #pragma unroll
-                for (int k4 = 0; k4 < HD / 16; ++k4)
-                    umma_f16(tmem_base + COL_DP, make_smem_desc(da + k4 * 32, 16, 1024), make_smem_desc(v_addr + k4 * 32, 16, 1024), idesc_sdp, k4 != 0);
-                umma_commit(bar_sdp);
+                for (int k4 = 0; k4 < HD / 16; ++k4) umma_f16(tmem_base + COL_DP, da + k4 * 2, v_kmaj + k4 * 2, idesc_sdp, k4 != 0, on);
+                umma_commit(bar_sdp, on);
                 return true;
             };
             if (ok && n_iter > 0 && !issue_sdp(0)) { atomicExch(p.status, 302); ok = false; }
             for (int it = 0; it < n_iter && ok; ++it) {
                 const uint32_t ph = it & 1;
                 const int st = it % QDO_STAGES;
-                const uint32_t qa = q_addr + st * QK_BYTES, da = do_addr + st * T_BYTES;
-                if (!mbar_wait(bar_pds, ph)) { atomicExch(p.status, 303); ok = false; break; }
+                const uint64_t qa = q_mn + st * (QK_BYTES >> 4), da = do_mn + st * (T_BYTES >> 4);
+                if (!warp_wait(bar_pds, ph)) { atomicExch(p.status, 303); ok = false; break; }
                 tc_fence_after();
 #pragma unroll
-                for (int k8 = 0; k8 < TILE / 16; ++k8) {        // dV += P^T dO   (contraction over the 128 query rows)
-                    umma_f16(tmem_base + COL_DV, make_smem_desc(p_addr + k8 * 2048, TILE * 128, 1024),
-                             make_smem_desc(da + k8 * 2048, TILE * 128, 1024), idesc_dv, (it | k8) != 0);
-                }
+                for (int k8 = 0; k8 < TILE / 16; ++k8)          // dV += P^T dO   (contraction over the 128 query rows)
+                    umma_f16(tmem_base + COL_DV, p_mn + k8 * 128, da + k8 * 128, idesc_dv, (it | k8) != 0, on);
 #pragma unroll
-                for (int k8 = 0; k8 < TILE / 16; ++k8) {        // dK += dS^T Q
-                    umma_f16(tmem_base + COL_DK, make_smem_desc(ds_addr + k8 * 2048, TILE * 128, 1024),
-                             make_smem_desc(qa + k8 * 2048, TILE * 128, 1024), idesc_dk, (it | k8) != 0);
-                }
+                for (int k8 = 0; k8 < TILE / 16; ++k8)          // dK += dS^T Q
+                    umma_f16(tmem_base + COL_DK, ds_mn + k8 * 128, qa + k8 * 128, idesc_dk, (it | k8) != 0, on);
 #pragma unroll
-                for (int k8 = 0; k8 < TILE / 16; ++k8) {        // dQ = dS K      (contraction over the 128 keys)
-                    umma_f16(tmem_base + COL_DQ, make_smem_desc(ds_addr + (k8 >> 2) * (TILE * 128) + (k8 & 3) * 32, 16, 1024),
-                             make_smem_desc(k_addr + k8 * 2048, TILE * 128, 1024), idesc_dq, k8 != 0);
-                }
-                umma_commit(bar_mma);
+                for (int k8 = 0; k8 < TILE / 16; ++k8)          // dQ = dS K      (contraction over the 128 keys)
+                    umma_f16(tmem_base + COL_DQ, ds_kmaj + (k8 >> 2) * (TILE * 128 >> 4) + (k8 & 3) * 2, k_mn + k8 * 128, idesc_dq, k8 != 0, on);
+                umma_commit(bar_mma, on);
                 // S / dP of this iteration were consumed before bar_pds: the next pair can queue behind the three products
                 // (narrow heads; with wide heads dQ sits in the S columns until the softmax warps have read it out)
                 if (!WIDE && it + 1 < n_iter && !issue_sdp(it + 1)) { atomicExch(p.status, 302); ok = false; break; }
-                if (!mbar_wait(bar_mma, ph)) { atomicExch(p.status, 304); ok = false; break; }
+                if (!warp_wait(bar_mma, ph)) { atomicExch(p.status, 304); ok = false; break; }
                 if (it + QDO_STAGES < n_iter) load_qdo(it + QDO_STAGES);      // this stage's Q / dO tiles are consumed
                 if (WIDE && it + 1 < n_iter) {
-                    if (!mbar_wait(bar_dq, ph)) { atomicExch(p.status, 307); ok = false; break; }
+                    if (!warp_wait(bar_dq, ph)) { atomicExch(p.status, 307); ok = false; break; }
                     tc_fence_after();
                     if (!issue_sdp(it + 1)) { atomicExch(p.status, 302); ok = false; break; }
                 }

@@ -5,19 +5,20 @@
 // of one (batch, kv head) and walks the query tiles that see them; S = Q K^T and dP = dO V^T into TMEM, P and dS to shared memory, dV += P^T dO, dK += dS^T Q, dQ = dS K reduced into a
 // fp32 buffer by TMA).  What differs is the order.  In attn_bwd.cu one iteration is a chain: S/dP -> softmax warps -> three
 // gradient products -> dQ read-out, and the S/dP of the next iteration queue behind the gradient products, so the tensor
-// core idles while the softmax warps work and the other way round (a tcgen05.mma with N = 64 takes about 56 clocks to issue
-// whatever its size, so the 24 gradient MMAs of an iteration alone occupy the issuing thread for some 2000 clocks).  Here:
-//   warp 8 (1 thread)  issues S/dP of iteration i+1 as soon as the softmax warps have READ S/dP of iteration i from TMEM
+// core idles while the softmax warps work and the other way round.  Here:
+//   warp 8             issues S/dP of iteration i+1 as soon as the softmax warps have READ S/dP of iteration i from TMEM
 //                    (bar_sread)
-//   warp 10 (1 thread) waits for P/dS of iteration i in shared memory and issues the three gradient products (its own thread so
-//                    that neither chain waits behind the other's barrier; with one thread issuing both in turn the time was the same)
+//   warp 10            waits for P/dS of iteration i in shared memory and issues the three gradient products (its own warp so
+//                    that neither chain waits behind the other's barrier)
 //   softmax warps    read S/dP of iteration i, form P and dS as packed bf16 in REGISTERS (64 per thread), release S/dP, and
 //                    only then wait for the gradient products of iteration i-1 (which still read the P/dS tiles in shared
-//                    memory), drain dQ of iteration i-1, and store P/dS of iteration i
+//                    memory), store P/dS of iteration i, and drain dQ of iteration i-1 while the products of iteration i
+//                    write the other of two dQ tiles
 //   loader warp      K, V once; Q / dO through a three-deep ring, a stage refilled when the gradient products that read it
 //                    have completed
 // so the exponentials of iteration i+1 run under the gradient products of iteration i.  Measured on 16 x 2048 tokens, 12 heads,
-// window 1024 (delta pre-pass and dQ zero-fill included): 470-476 us against 541 us for attn_bwd.cu.
+// window 1024 (delta pre-pass and dQ zero-fill included): 445 us against 516 us for attn_bwd.cu (476 and 545 with one issuing lane).  An iteration
+// takes 4000 clocks: the softmax warps' arithmetic 1450, their stores of P and dS 680, the dQ read-out 760 to 1200; products wait for them.
 // Reference counterpart: the backward of FlexAttention (model/attention/self_attention.py:250-255) as generated by Inductor.
 #include "../common/ptx.cuh"
 #include "attn.h"
@@ -31,7 +32,7 @@ constexpr int BP_PD_BYTES = BP_TILE * BP_TILE * 2;       // P or dS tile (two 12
 constexpr int BP_STG_BYTES = BP_TILE * BP_HD * 4;        // dQ staging (two slabs of 32 fp32 columns)
 constexpr int BP_STAGES = 3;
 constexpr uint32_t BP_TMEM_COLS = 512;
-constexpr uint32_t BP_COL_S = 0, BP_COL_DP = 128, BP_COL_DV = 256, BP_COL_DK = 320, BP_COL_DQ = 384;
+constexpr uint32_t BP_COL_S = 0, BP_COL_DP = 128, BP_COL_DV = 256, BP_COL_DK = 320, BP_COL_DQ = 384;       // two dQ tiles, in turn
 
 __device__ __forceinline__ float bp_tanh_approx(float x) {
     float y;
@@ -104,11 +105,11 @@ attn_bwd_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     uint64_t* bar_qdo = bars + 5;                        // [BP_STAGES] Q / dO tile landed
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_qdo + BP_STAGES);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int kv_tile = p.long_first ? blockIdx.z : blockIdx.x, kv_head = p.long_first ? blockIdx.x : blockIdx.y;
     const int batch = p.long_first ? blockIdx.y : blockIdx.z;
     const int kv0 = kv_tile * BP_TILE;
-    const int window = p.window_ptr ? min(max(*p.window_ptr, 0), p.seq_len) : p.window;
+    const int window = uniform(p.window_ptr ? min(max(*p.window_ptr, 0), p.seq_len) : p.window);
     const int q_tiles_total = (p.seq_len + BP_TILE - 1) / BP_TILE;
     int last_q_tile = (kv0 + BP_TILE - 1 + window) / BP_TILE;
     if (last_q_tile > q_tiles_total - 1) last_q_tile = q_tiles_total - 1;
@@ -125,31 +126,33 @@ attn_bwd_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = uniform(*tmem_slot);
     bool ok = true;
 
     if (warp == 9) {
-        if (lane == 0) {
+        {
+            const uint32_t on = elect_one();
             auto load_qdo = [&](int it) {
                 const int st = it % BP_STAGES;
                 const int head = kv_head * p.group + it / n_q;
                 const int q0 = (kv_tile + it % n_q) * BP_TILE;
-                mbar_expect_tx(&bar_qdo[st], 2 * BP_T_BYTES);
-                tma_load_3d(sq + st * BP_T_BYTES, &tmap_q, &bar_qdo[st], head * BP_HD, q0, batch);
-                tma_load_3d(sdo + st * BP_T_BYTES, &tmap_do, &bar_qdo[st], head * BP_HD, q0, batch);
+                if (on) mbar_expect_tx(&bar_qdo[st], 2 * BP_T_BYTES);
+                tma_load_3d(sq + st * BP_T_BYTES, &tmap_q, &bar_qdo[st], head * BP_HD, q0, batch, on);
+                tma_load_3d(sdo + st * BP_T_BYTES, &tmap_do, &bar_qdo[st], head * BP_HD, q0, batch, on);
             };
-            mbar_expect_tx(bar_kv, 2 * BP_T_BYTES);
-            tma_load_3d(sk, &tmap_k, bar_kv, kv_head * BP_HD, kv0, batch);
-            tma_load_3d(sv, &tmap_v, bar_kv, kv_head * p.v_head, kv0, batch);
+            if (on) mbar_expect_tx(bar_kv, 2 * BP_T_BYTES);
+            tma_load_3d(sk, &tmap_k, bar_kv, kv_head * BP_HD, kv0, batch, on);
+            tma_load_3d(sv, &tmap_v, bar_kv, kv_head * p.v_head, kv0, batch, on);
             for (int it = 0; it < BP_STAGES && it < n_iter; ++it) load_qdo(it);
             for (int it = BP_STAGES; it < n_iter; ++it) {
                 // the stage was read by S/dP and by the gradient products of iteration it - BP_STAGES
-                if (!mbar_wait(bar_mma, (it - BP_STAGES) & 1)) { atomicExch(p.status, 311); break; }
+                if (!warp_wait(bar_mma, (it - BP_STAGES) & 1)) { atomicExch(p.status, 311); break; }
                 load_qdo(it);
             }
         }
     } else if (warp == 8 || warp == 10) {
-        if (lane == 0) {
+        {
+            const uint32_t on = elect_one();
             constexpr uint32_t idesc_sdp = make_idesc_bf16(BP_TILE, BP_TILE, false, false);
             constexpr uint32_t idesc_g = make_idesc_bf16(BP_TILE, BP_HD, true, true);         // dV, dK: A and B MN-major
             constexpr uint32_t idesc_dq = make_idesc_bf16(BP_TILE, BP_HD, false, true);       // dQ: A K-major, B MN-major
@@ -163,21 +166,21 @@ attn_bwd_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
             const uint64_t ds_kmaj = make_smem_desc(smem_u32(sds), 16, 1024);
             auto issue_sdp = [&](int it) -> bool {               // S = Q K^T ; dP = dO V^T for iteration `it`
                 const int st = it % BP_STAGES;
-                if (!mbar_wait(&bar_qdo[st], (it / BP_STAGES) & 1)) return false;
+                if (!warp_wait(&bar_qdo[st], (it / BP_STAGES) & 1)) return false;
                 tc_fence_after();
                 const uint64_t qa = q_kmaj + st * (BP_T_BYTES >> 4), da = do_kmaj + st * (BP_T_BYTES >> 4);
 #pragma unroll
-                for (int k4 = 0; k4 < 4; ++k4) umma_f16(tmem_base + BP_COL_S, qa + k4 * 2, k_kmaj + k4 * 2, idesc_sdp, k4 != 0);
+                for (int k4 = 0; k4 < 4; ++k4) umma_f16(tmem_base + BP_COL_S, qa + k4 * 2, k_kmaj + k4 * 2, idesc_sdp, k4 != 0, on);
 #pragma unroll
-                for (int k4 = 0; k4 < 4; ++k4) umma_f16(tmem_base + BP_COL_DP, da + k4 * 2, v_kmaj + k4 * 2, idesc_sdp, k4 != 0);
-                umma_commit(bar_sdp);
+                for (int k4 = 0; k4 < 4; ++k4) umma_f16(tmem_base + BP_COL_DP, da + k4 * 2, v_kmaj + k4 * 2, idesc_sdp, k4 != 0, on);
+                umma_commit(bar_sdp, on);
                 return true;
             };
-            if (!mbar_wait(bar_kv, 0)) { atomicExch(p.status, 301); ok = false; }
+            if (!warp_wait(bar_kv, 0)) { atomicExch(p.status, 301); ok = false; }
             if (warp == 8) {
                 if (ok && n_iter > 0 && !issue_sdp(0)) { atomicExch(p.status, 302); ok = false; }
                 for (int it = 0; it + 1 < n_iter && ok; ++it) {
-                    if (!mbar_wait(bar_sread, it & 1)) { atomicExch(p.status, 308); ok = false; break; }      // S / dP columns are free again
+                    if (!warp_wait(bar_sread, it & 1)) { atomicExch(p.status, 308); ok = false; break; }      // S / dP columns are free again
                     tc_fence_after();
                     if (!issue_sdp(it + 1)) { atomicExch(p.status, 302); ok = false; break; }
                 }
@@ -186,19 +189,19 @@ attn_bwd_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
                     // P / dS of the iteration are in shared memory; its Q / dO stage landed before its S / dP were issued (the wait on
                     // the stage's barrier returns at once and orders this thread's products after the copy as well)
                     const int st = it % BP_STAGES;
-                    if (!mbar_wait(bar_pds, it & 1) || !mbar_wait(&bar_qdo[st], (it / BP_STAGES) & 1)) { atomicExch(p.status, 303); ok = false; break; }
+                    if (!warp_wait(bar_pds, it & 1) || !warp_wait(&bar_qdo[st], (it / BP_STAGES) & 1)) { atomicExch(p.status, 303); ok = false; break; }
                     tc_fence_after();
                     const uint64_t qb = q_mn + st * (BP_T_BYTES >> 4), db = do_mn + st * (BP_T_BYTES >> 4);
 #pragma unroll
                     for (int k8 = 0; k8 < BP_TILE / 16; ++k8)        // dV += P^T dO   (contraction over the 128 query rows)
-                        umma_f16(tmem_base + BP_COL_DV, p_mn + k8 * 128, db + k8 * 128, idesc_g, (it | k8) != 0);
+                        umma_f16(tmem_base + BP_COL_DV, p_mn + k8 * 128, db + k8 * 128, idesc_g, (it | k8) != 0, on);
 #pragma unroll
                     for (int k8 = 0; k8 < BP_TILE / 16; ++k8)        // dK += dS^T Q
-                        umma_f16(tmem_base + BP_COL_DK, ds_mn + k8 * 128, qb + k8 * 128, idesc_g, (it | k8) != 0);
+                        umma_f16(tmem_base + BP_COL_DK, ds_mn + k8 * 128, qb + k8 * 128, idesc_g, (it | k8) != 0, on);
 #pragma unroll
                     for (int k8 = 0; k8 < BP_TILE / 16; ++k8)        // dQ = dS K      (contraction over the 128 keys: two 64-key slabs of dS)
-                        umma_f16(tmem_base + BP_COL_DQ, ds_kmaj + (k8 >> 2) * (BP_TILE * 128 >> 4) + (k8 & 3) * 2, k_mn + k8 * 128, idesc_dq, k8 != 0);
-                    umma_commit(bar_mma);
+                        umma_f16(tmem_base + BP_COL_DQ + (it & 1) * BP_HD, ds_kmaj + (k8 >> 2) * (BP_TILE * 128 >> 4) + (k8 & 3) * 2, k_mn + k8 * 128, idesc_dq, k8 != 0, on);
+                    umma_commit(bar_mma, on);
                 }
             }
         }
@@ -217,10 +220,8 @@ attn_bwd_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         const uint32_t s_addr = tmem_base + BP_COL_S + lane_off + half * 64, dp_addr = tmem_base + BP_COL_DP + lane_off + half * 64;
         // dQ of iteration `jt`: this thread's row, 32 of the 64 columns; scaled, staged, then one TMA reduce-add per 32-column slab
         auto drain_dq = [&](int jt) {
-            if (ok && !mbar_wait(bar_mma, jt & 1)) { atomicExch(p.status, 306); ok = false; }
-            tc_fence_after();
             uint32_t qreg[32];
-            tmem_ld_32x32b_x32(tmem_base + BP_COL_DQ + lane_off + half * 32, qreg);
+            tmem_ld_32x32b_x32(tmem_base + BP_COL_DQ + (jt & 1) * BP_HD + lane_off + half * 32, qreg);
             tmem_ld_wait();
             tc_fence_before();
             if (leader) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
@@ -280,8 +281,11 @@ attn_bwd_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
             else bp_tile_math<false, capped>(s_addr, dp_addr, wp, wd, kv0 + half * 64, qpos, w_row, c, lse2, delta, cap_a, cap_b);
             tc_fence_before();
             mbar_arrive(bar_sread);                                       // S / dP of the next iteration may be written
-            // the gradient products of the previous iteration read the P / dS tiles: wait for them, and drain their dQ
-            if (it > 0) drain_dq(it - 1);
+            // the gradient products of the previous iteration read the P / dS tiles
+            if (it > 0) {
+                if (ok && !mbar_wait(bar_mma, (it - 1) & 1)) { atomicExch(p.status, 306); ok = false; }
+                tc_fence_after();
+            }
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const int piece = (j ^ sw) << 4;
@@ -290,8 +294,15 @@ attn_bwd_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
             }
             fence_proxy_async();
             mbar_arrive(bar_pds);
+            // the previous iteration's dQ leaves while the tensor core works on this one's products, whose dQ goes to the other columns
+            // (those were read out before this thread's arrival above, so the issuing thread may overwrite them)
+            if (it > 0) drain_dq(it - 1);
         }
-        if (n_iter > 0) drain_dq(n_iter - 1);
+        if (n_iter > 0) {
+            if (ok && !mbar_wait(bar_mma, (n_iter - 1) & 1)) { atomicExch(p.status, 306); ok = false; }
+            tc_fence_after();
+            drain_dq(n_iter - 1);
+        }
         if (ok && n_iter > 0) {
             // dK, dV: TMEM lanes are the 128 keys of this CTA; each thread writes half of the columns of its key row
             const bool live = kv0 + r < p.seq_len;

@@ -119,12 +119,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_v + KV_STAGES);
     float* row_stat = reinterpret_cast<float*>(bars + 16);     // [2 halves][128 rows]
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     // heads and sequences run fastest through the grid, tiles slowest and the longest first: without a window a tile's work grows with its
     // position, and started last the longest would leave most SMs idle at the end
     const int q_tile = gridDim.z - 1 - blockIdx.z, head = blockIdx.x, batch = blockIdx.y;
     const int q0 = q_tile * AT_BM;
-    const int window = p.window_ptr ? min(max(*p.window_ptr, 0), p.seq_len) : p.window;
+    const int window = uniform(p.window_ptr ? min(max(*p.window_ptr, 0), p.seq_len) : p.window);
     const int row0 = batch * p.seq_len;
     // document masking narrows a row's look-back to the start of its document; look-backs shrink monotonically towards
     // later rows of a document, so the first row bounds the tiles to visit and the last row decides whether a tile needs masking
@@ -136,7 +136,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     }
     int kv_lo = q0 - w_first;
     if (kv_lo < 0) kv_lo = 0;
-    kv_lo &= ~(AT_BN - 1);
+    kv_lo = uniform(kv_lo & ~(AT_BN - 1));
     const int n_tiles = (q0 + AT_BM - kv_lo) / AT_BN;
     const int kv_head = head / p.group;                       // grouped-query attention: several q heads share a kv head
     const int q_col = p.q_col0 + head * DQK, k_col = p.k_col0 + kv_head * DQK, v_col = p.v_col0 + kv_head * p.v_head;
@@ -150,64 +150,65 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = uniform(*tmem_slot);
     const uint32_t tmem_s = tmem_base, tmem_p = tmem_base + AT_BN, tmem_pv = tmem_base + AT_BN + AT_BN / 2;
     bool ok = true;
 
     if (warp == 8) {
-        if (lane == 0) {
+        {
+            const uint32_t on = elect_one();
             constexpr uint32_t idesc_s = make_idesc_bf16(AT_BM, AT_BN, false, false);
             constexpr uint32_t idesc_pv = make_idesc_bf16(AT_BM, AT_D, false, true);
-            const uint32_t q_addr = smem_u32(sq), k_addr = smem_u32(sk), v_addr = smem_u32(sv);
+            // descriptors formed once; the address field counts 16-byte units
+            const uint64_t q_desc = make_smem_desc(smem_u32(sq), 16, 1024), k_desc = make_smem_desc(smem_u32(sk), 16, 1024);
+            const uint64_t v_desc = make_smem_desc(smem_u32(sv), AT_BN * 128, 1024);
             auto issue_s = [&](int st) {
 #pragma unroll
                 for (int sl = 0; sl < QK_SLABS; ++sl)
 #pragma unroll
                     for (int k4 = 0; k4 < 4; ++k4)
-                        umma_f16(tmem_s, make_smem_desc(q_addr + sl * SLAB_BYTES + k4 * 32, 16, 1024),
-                                 make_smem_desc(k_addr + st * K_BYTES + sl * SLAB_BYTES + k4 * 32, 16, 1024), idesc_s, (sl | k4) != 0);
-                umma_commit(bar_s);
+                        umma_f16(tmem_s, q_desc + sl * (SLAB_BYTES >> 4) + k4 * 2, k_desc + st * (K_BYTES >> 4) + sl * (SLAB_BYTES >> 4) + k4 * 2, idesc_s,
+                                 (sl | k4) != 0, on);
+                umma_commit(bar_s, on);
             };
             auto load_k = [&](int tile) {
                 const int st = tile % KV_STAGES;
-                mbar_expect_tx(&bar_k[st], K_BYTES);
+                if (on) mbar_expect_tx(&bar_k[st], K_BYTES);
 #pragma unroll
                 for (int sl = 0; sl < QK_SLABS; ++sl)
-                    tma_load_3d(sk + st * K_BYTES + sl * SLAB_BYTES, &tmap_k, &bar_k[st], k_col + 64 * sl, kv_lo + tile * AT_BN, batch);
+                    tma_load_3d(sk + st * K_BYTES + sl * SLAB_BYTES, &tmap_k, &bar_k[st], k_col + 64 * sl, kv_lo + tile * AT_BN, batch, on);
             };
             auto load_v = [&](int tile) {
                 const int st = tile % KV_STAGES;
-                mbar_expect_tx(&bar_v[st], V_BYTES);
-                tma_load_3d(sv + st * V_BYTES, &tmap_v, &bar_v[st], v_col, kv_lo + tile * AT_BN, batch);
+                if (on) mbar_expect_tx(&bar_v[st], V_BYTES);
+                tma_load_3d(sv + st * V_BYTES, &tmap_v, &bar_v[st], v_col, kv_lo + tile * AT_BN, batch, on);
             };
-            mbar_expect_tx(bar_q, Q_BYTES);
+            if (on) mbar_expect_tx(bar_q, Q_BYTES);
 #pragma unroll
-            for (int sl = 0; sl < QK_SLABS; ++sl) tma_load_3d(sq + sl * SLAB_BYTES, &tmap_q, bar_q, q_col + 64 * sl, q0, batch);
+            for (int sl = 0; sl < QK_SLABS; ++sl) tma_load_3d(sq + sl * SLAB_BYTES, &tmap_q, bar_q, q_col + 64 * sl, q0, batch, on);
             for (int t = 0; t < KV_STAGES && t < n_tiles; ++t) { load_k(t); load_v(t); }
-            if (!mbar_wait(bar_q, 0) || !mbar_wait(&bar_k[0], 0)) { atomicExch(p.status, 201); ok = false; }
+            if (!warp_wait(bar_q, 0) || !warp_wait(&bar_k[0], 0)) { atomicExch(p.status, 201); ok = false; }
             if (ok) { tc_fence_after(); issue_s(0); }
             for (int j = 0; j < n_tiles && ok; ++j) {
                 const uint32_t ph = j & 1;
                 const int st = j % KV_STAGES;
                 const uint32_t st_ph = (j / KV_STAGES) & 1;
                 const bool more = j + 1 < n_tiles;
-                if (!mbar_wait(bar_s, ph)) { atomicExch(p.status, 202); ok = false; break; }
+                if (!warp_wait(bar_s, ph)) { atomicExch(p.status, 202); ok = false; break; }
                 if (j + KV_STAGES < n_tiles) load_k(j + KV_STAGES);           // S_j has consumed its key tile: refill the stage
-                if (!mbar_wait(bar_p, ph) || !mbar_wait(&bar_v[st], st_ph)) { atomicExch(p.status, 203); ok = false; break; }
+                if (!warp_wait(bar_p, ph) || !warp_wait(&bar_v[st], st_ph)) { atomicExch(p.status, 203); ok = false; break; }
                 tc_fence_after();
 #pragma unroll
-                for (int k8 = 0; k8 < AT_BN / 16; ++k8) {
-                    const uint64_t bdesc = make_smem_desc(v_addr + st * V_BYTES + k8 * 2048, AT_BN * 128, 1024);
-                    umma_f16_ta(tmem_pv, tmem_p + k8 * 8, bdesc, idesc_pv, k8 != 0);      // 16 keys = 8 packed columns
-                }
-                umma_commit(bar_o);
+                for (int k8 = 0; k8 < AT_BN / 16; ++k8)
+                    umma_f16_ta(tmem_pv, tmem_p + k8 * 8, v_desc + st * (V_BYTES >> 4) + k8 * 128, idesc_pv, k8 != 0, on);      // 16 keys = 8 packed columns
+                umma_commit(bar_o, on);
                 if (more) {
                     const int nst = (j + 1) % KV_STAGES;
-                    if (!mbar_wait(&bar_k[nst], ((j + 1) / KV_STAGES) & 1)) { atomicExch(p.status, 204); ok = false; break; }
+                    if (!warp_wait(&bar_k[nst], ((j + 1) / KV_STAGES) & 1)) { atomicExch(p.status, 204); ok = false; break; }
                     tc_fence_after();
                     issue_s(nst);
                 }
-                if (!mbar_wait(bar_o, ph)) { atomicExch(p.status, 205); ok = false; break; }
+                if (!warp_wait(bar_o, ph)) { atomicExch(p.status, 205); ok = false; break; }
                 if (j + KV_STAGES < n_tiles) load_v(j + KV_STAGES);           // PV_j has consumed its value tile
             }
         }

@@ -6,14 +6,13 @@
 // tensor core works on the other:
 //   warps 0-3   softmax of tile A: thread = query row, running maximum / sum in registers, P written to TMEM as packed bf16 pairs
 //   warps 4-7   the same for tile B
-//   warp  8, 9  MMA issue for tile A and for tile B (one thread each):  S_x = Q_x K^T  (M128 N128 K64),
-//               O_x += P_x V  (M128 N64 K128, A from TMEM).  A thread serving both tiles in turn spent 1850 clocks per
-//               (query tile, key tile) - eight N = 64 instructions 960, four N = 128 instructions 275, four commits 130 each,
-//               waits on complete barriers 100 each - against 512 clocks of tensor-core work, so each tile has its own
-//               thread, the descriptors are formed once and advanced by adding to their address field, and one commit per
-//               step announces both the PV product of the step and the S product of the next one.  (The kernel time did
-//               not change with that alone: the softmax of a tile, 1700 clocks, is the longer part of its chain.)
-//   warp  10    TMA loads (one thread): Q once, then the K and V tile of a ring stage as it comes free
+//   warp  8, 9  MMA issue for tile A and for tile B (a whole warp each, see umma_f16 in ptx.cuh):  S_x = Q_x K^T  (M128 N128 K64),
+//               O_x += P_x V  (M128 N64 K128, A from TMEM).  Once P of a key tile is announced its S columns are free, so the next
+//               key tile's S is issued before this one's P V; the softmax waits for P V only before it touches O or P again.
+//               16 x 2048 tokens, 12 heads, window 1024: 225 us with one issuing lane, 195 with a warp (that order of the products included).
+//               What is left (clock64 in one CTA of nine key tiles): 3150 clocks a key tile - the second softmax pass 1750, the first 550,
+//               waiting for S 700 - and 3500 and 6500 clocks before the first and after the last one.
+//   warp  10    TMA loads (one elected lane): Q once, then the K and V tile of a ring stage as it comes free
 // O stays in TMEM for the whole CTA and the PV product accumulates into it.  The running maximum a row's exponentials are
 // taken against is only moved when the row's maximum has grown by more than 2^8 since it was last moved; then (rarely
 // after the first tiles) the row's O is rescaled in TMEM by its softmax thread.  The stale reference only changes the
@@ -110,9 +109,10 @@ __device__ __forceinline__ void dual_zero16(uint32_t p_addr) {
     tmem_st_32x32b_x16(p_addr, zeros);
 }
 
-template <bool CAP>
+template <bool CAP, class PreviousProduct>
 __device__ __forceinline__ void dual_softmax_tile(uint32_t s_addr, uint32_t p_addr, uint32_t o_addr, int kv0, int qpos, int warp_q0, int window,
-                                                  bool edge_tile, float c, float step, float& m_ref, float& l, bool first, float cap_a, float cap_b) {
+                                                  bool edge_tile, float c, float step, float& m_ref, float& l, bool first, float cap_a, float cap_b,
+                                                  const PreviousProduct& previous_product) {
     int cls[4] = {CHUNK_FULL, CHUNK_FULL, CHUNK_FULL, CHUNK_FULL};
     if (edge_tile) {
 #pragma unroll
@@ -138,10 +138,11 @@ __device__ __forceinline__ void dual_softmax_tile(uint32_t s_addr, uint32_t p_ad
         if (cls[3] != CHUNK_EMPTY) { dual_prepare_chunk<CAP>(s3, cls[3], kv0 + 96, qpos, window, cap_a, cap_b); dual_max32(s3, mx); }
     }
     const float m_tile = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * c;
+    previous_product();                            // complete from here on: O may be rescaled and P overwritten
     const bool grow = m_tile > m_ref + step;       // also true for the first finite maximum (m_ref = -inf)
     if (__any_sync(0xffffffffu, grow)) {
         const float alpha = grow ? exp2f(m_ref - m_tile) : 1.f;
-        if (!first) {                 // the previous PV product is complete: the commit that announced this S came after it
+        if (!first) {
 #pragma unroll
             for (int hh = 0; hh < 2; ++hh) {
                 uint32_t o[32];
@@ -195,19 +196,19 @@ attn_fwd_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     uint8_t* sv = sk + DU_STAGES * DU_TILE_BYTES;         // DU_STAGES value tiles
     uint64_t* bars = reinterpret_cast<uint64_t*>(sv + DU_STAGES * DU_TILE_BYTES);
     uint64_t* bar_q = bars + 0;
-    uint64_t* bar_s = bars + 1;                           // [2] S_x complete (and every product of tile x issued before it)
+    uint64_t* bar_s = bars + 1;                           // [2] S_x complete
     uint64_t* bar_p = bars + 3;                           // [2] P_x written, S_x consumed (128 arrivals)
-    uint64_t* bar_o = bars + 5;                           // [2] last PV product of tile x complete
+    uint64_t* bar_o = bars + 5;                           // [2] PV product of tile x complete
     uint64_t* bar_full = bars + 7;                        // [STAGES] key and value tile landed
     uint64_t* bar_free = bar_full + DU_STAGES;            // [STAGES] both query tiles are done with the stage (2 arrivals)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_free + DU_STAGES);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     // heads and sequences run fastest through the grid, tiles slowest and the longest first: without a window a tile's work grows with its
     // position, and started last the longest would leave most SMs idle at the end
     const int head = blockIdx.x, batch = blockIdx.y;
     const int q0 = (gridDim.z - 1 - blockIdx.z) * 2 * DU_BM;
-    const int window = p.window_ptr ? min(max(*p.window_ptr, 0), p.seq_len) : p.window;
+    const int window = uniform(p.window_ptr ? min(max(*p.window_ptr, 0), p.seq_len) : p.window);
     const int row0 = batch * p.seq_len;
     // key tiles (units of 128 keys) of each query tile: from the tile holding the first key its first row sees to its diagonal tile
     const int first_a = q0 - window, first_b = q0 + DU_BM - window;
@@ -226,26 +227,28 @@ attn_fwd_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = uniform(*tmem_slot);
     bool ok = true;
 
     if (warp == 10) {
-        if (lane == 0) {
-            mbar_expect_tx(bar_q, 2 * DU_TILE_BYTES);
-            tma_load_3d(sq, &tmap_q, bar_q, q_col, q0, batch);
-            tma_load_3d(sq + DU_TILE_BYTES, &tmap_q, bar_q, q_col, q0 + DU_BM, batch);
+        {
+            const uint32_t on = elect_one();
+            if (on) mbar_expect_tx(bar_q, 2 * DU_TILE_BYTES);
+            tma_load_3d(sq, &tmap_q, bar_q, q_col, q0, batch, on);
+            tma_load_3d(sq + DU_TILE_BYTES, &tmap_q, bar_q, q_col, q0 + DU_BM, batch, on);
             const int total = hi_a + 1 - lo_a + 1;                // key tiles lo_a .. hi_a + 1
             for (int u = 0; u < total; ++u) {
                 const int st = u % DU_STAGES, use = u / DU_STAGES;
                 const int key_row = (lo_a + u) * DU_BN;
-                if (use > 0 && !mbar_wait(&bar_free[st], (use - 1) & 1)) { atomicExch(p.status, 211); break; }
-                mbar_expect_tx(&bar_full[st], 2 * DU_TILE_BYTES);
-                tma_load_3d(sk + st * DU_TILE_BYTES, &tmap_k, &bar_full[st], k_col, key_row, batch);
-                tma_load_3d(sv + st * DU_TILE_BYTES, &tmap_v, &bar_full[st], v_col, key_row, batch);
+                if (use > 0 && !warp_wait(&bar_free[st], (use - 1) & 1)) { atomicExch(p.status, 211); break; }
+                if (on) mbar_expect_tx(&bar_full[st], 2 * DU_TILE_BYTES);
+                tma_load_3d(sk + st * DU_TILE_BYTES, &tmap_k, &bar_full[st], k_col, key_row, batch, on);
+                tma_load_3d(sv + st * DU_TILE_BYTES, &tmap_v, &bar_full[st], v_col, key_row, batch, on);
             }
         }
     } else if (warp >= 8) {
-        if (lane == 0) {
+        {
+            const uint32_t on = elect_one();
             const int x = warp - 8;
             const int n_x = x == 0 ? hi_a - lo_a + 1 : hi_a + 1 - lo_b + 1;
             const int u0 = x == 0 ? 0 : lo_b - lo_a;              // ring position of this tile's first key tile
@@ -260,27 +263,26 @@ attn_fwd_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
             const uint32_t tmem_o = tmem_base + DU_COL_O + x * DU_D;
             auto issue_s = [&](int u) -> bool {
                 const int st = u % DU_STAGES;
-                if (!mbar_wait(&bar_full[st], (u / DU_STAGES) & 1)) return false;
+                if (!warp_wait(&bar_full[st], (u / DU_STAGES) & 1)) return false;
                 tc_fence_after();
                 const uint64_t kd = k_desc + st * (DU_TILE_BYTES >> 4);
 #pragma unroll
-                for (int k4 = 0; k4 < 4; ++k4) umma_f16(tmem_s, q_desc + k4 * 2, kd + k4 * 2, idesc_s, k4 != 0);
-                umma_commit(&bar_s[x]);
+                for (int k4 = 0; k4 < 4; ++k4) umma_f16(tmem_s, q_desc + k4 * 2, kd + k4 * 2, idesc_s, k4 != 0, on);
+                umma_commit(&bar_s[x], on);
                 return true;
             };
-            if (!mbar_wait(bar_q, 0) || !issue_s(u0)) { atomicExch(p.status, 213); ok = false; }
+            if (!warp_wait(bar_q, 0) || !issue_s(u0)) { atomicExch(p.status, 213); ok = false; }
             for (int i = 0; i < n_x && ok; ++i) {
-                if (!mbar_wait(&bar_p[x], i & 1)) { atomicExch(p.status, 215); ok = false; break; }
+                if (!warp_wait(&bar_p[x], i & 1)) { atomicExch(p.status, 215); ok = false; break; }
                 tc_fence_after();
+                // S of the next key tile goes first: its columns are free (S_x was consumed before P_x was announced), and the softmax warps
+                // work on it while this tile's P V product runs
+                if (i + 1 < n_x && !issue_s(u0 + i + 1)) { atomicExch(p.status, 217); ok = false; break; }
                 const uint64_t vd = v_desc + ((u0 + i) % DU_STAGES) * (DU_TILE_BYTES >> 4);   // landed: S of this tile waited for the stage
 #pragma unroll
                 for (int k8 = 0; k8 < DU_BN / 16; ++k8)
-                    umma_f16_ta(tmem_o, tmem_p + k8 * 8, vd + k8 * 128, idesc_pv, (i | k8) != 0);      // 16 keys = 8 packed columns
-                if (i + 1 < n_x) {
-                    if (!issue_s(u0 + i + 1)) { atomicExch(p.status, 217); ok = false; }
-                } else {
-                    umma_commit(&bar_o[x]);
-                }
+                    umma_f16_ta(tmem_o, tmem_p + k8 * 8, vd + k8 * 128, idesc_pv, (i | k8) != 0, on);      // 16 keys = 8 packed columns
+                umma_commit(&bar_o[x], on);
             }
         }
     } else {
@@ -297,32 +299,39 @@ attn_fwd_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         const float c = p.scale_log2e;
         constexpr bool capped = CAPPED;
         const float cap_a = capped ? p.softcap / p.scale : 0.f, cap_b = capped ? p.scale / p.softcap : 0.f;
-        // With a reference that lags, the largest probabilities are no longer 1, which bf16 holds exactly, and windowed outputs lie up to 4 %
-        // further from 64 bits than with the exact maximum of the library kernel that lengths outside whole pairs of tiles used to run:
-        // those rescale whenever the maximum grows (5 x 1000 tokens, window 256: 2.04e-3 instead of 2.10e-3, 28 us; the single-tile kernel 31)
-        const float step = p.seq_len % (2 * DU_BM) == 0 ? DU_RESCALE_STEP : 0.f;
+        // With a reference that lags, the largest probabilities are no longer 1, which bf16 holds exactly, and outputs lie up to 4 % further
+        // from 64 bits than with the exact maximum: it lags only in windowed or short calls of whole pairs of tiles; the others rescale
+        // whenever the maximum grows (5 x 1000 tokens, window 256: 2.04e-3 instead of 2.10e-3)
+        const bool lags = p.seq_len % (2 * DU_BM) == 0 && (p.window <= p.seq_len / 2 || p.seq_len <= 16 * DU_BM);
+        const float step = lags ? DU_RESCALE_STEP : 0.f;
         float m_ref = -INFINITY, l = 0.f;
-        for (int i = 0; i < n_x && ok; ++i) {
+        for (int i = 0; i < n_x; ++i) {
             const int tile = lo_x + i;
             const int kv0 = tile * DU_BN;
-            if (!mbar_wait(&bar_s[x], i & 1)) { atomicExch(p.status, 218); ok = false; break; }
+            if (ok && !mbar_wait(&bar_s[x], i & 1)) { atomicExch(p.status, 218); ok = false; }
             tc_fence_after();
-            if (i > 0 && r == 0) {
-                // this S was committed after the PV product of the previous key tile: tile x is done with that ring stage.  A key
-                // tile the other query tile does not read (before B's first, after A's diagonal) gets both arrivals from here
-                const int done = tile - 1;
-                uint64_t* fb = &bar_free[(done - lo_a) % DU_STAGES];
-                mbar_arrive(fb);
-                if (x == 0 ? done < lo_b : done > hi_a) mbar_arrive(fb);
-            }
+            const auto previous_product = [&] {
+                if (i == 0) return;
+                if (ok && !mbar_wait(&bar_o[x], (i - 1) & 1)) { atomicExch(p.status, 219); ok = false; }
+                tc_fence_after();
+                if (r == 0) {
+                    // tile x is done with the ring stage of the previous key tile.  A key tile the other query tile does not read
+                    // (before B's first, after A's diagonal) gets both arrivals from here
+                    const int done = tile - 1;
+                    uint64_t* fb = &bar_free[(done - lo_a) % DU_STAGES];
+                    mbar_arrive(fb);
+                    if (x == 0 ? done < lo_b : done > hi_a) mbar_arrive(fb);
+                }
+            };
             // tiles strictly inside the band need no mask; the diagonal tile and the tile at the window edge do
             const bool need_mask = (kv0 + DU_BN - 1 > q0x) || (q0x + DU_BM - 1 - kv0 > window);
-            dual_softmax_tile<capped>(s_addr, p_addr, o_addr, kv0, qpos, q0x + quad * 32, window, need_mask, c, step, m_ref, l, i == 0, cap_a, cap_b);
+            dual_softmax_tile<capped>(s_addr, p_addr, o_addr, kv0, qpos, q0x + quad * 32, window, need_mask, c, step, m_ref, l, i == 0, cap_a, cap_b,
+                                      previous_product);
             tmem_st_wait();
             tc_fence_before();
             mbar_arrive(&bar_p[x]);
         }
-        if (ok && !mbar_wait(&bar_o[x], 0)) { atomicExch(p.status, 220); ok = false; }
+        if (ok && !mbar_wait(&bar_o[x], (n_x - 1) & 1)) { atomicExch(p.status, 220); ok = false; }
         if (ok) {
             tc_fence_after();
             float o[DU_D];
@@ -387,14 +396,12 @@ attn_fwd_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
 }
 
 bool attn_fwd_dual_supported(const AttnParams& p) {
-    // Windowed calls, where two query tiles share most of their keys: 16 x 2048 tokens, window 1024 225 us against 238 for the single-tile
-    // kernel, 16 x 1000, window 256 70 against 81; also with an odd number of tiles, where half of the last CTA idles, once there are
-    // nine (16 x 1152, window 256 84 against 91).  Without a window the single-tile kernel's finer grain fills the end of the grid better:
-    // 16384 tokens 955 us against 1060, 4 x 4096 285 against 303, 8 x 1100 57 against 65; up to 16 tiles an even number is better here
-    // (64 x 184 tokens 51 against 60, 5 x 1000 33 against 35).
+    // us, this kernel / the single-tile one: 16 x 2048 tokens, window 1024 195 / 248, 16384 tokens 865 / 978, 4 x 4096 251 / 293, 2 x 3000 86 / 97,
+    // 64 x 184 48 / 64, 8 x 1100 58 / 60, 1 x 1024 25 / 24, 3 x 300 17 / 16.  Of an odd number of tiles the last CTA idles by half, which a short
+    // window does not repay below nine tiles (16 x 1152, window 256 84 / 91).
     const int tiles = (p.seq_len + DU_BM - 1) / DU_BM;
     const bool windowed = p.window <= p.seq_len / 2;
-    return p.qk_dim == 64 && p.doc_start == nullptr && (windowed ? tiles % 2 == 0 || tiles >= 9 : tiles % 2 == 0 && tiles <= 16);
+    return p.qk_dim == 64 && p.doc_start == nullptr && (windowed ? tiles % 2 == 0 || tiles >= 9 : true);
 }
 
 template <bool CAPPED>

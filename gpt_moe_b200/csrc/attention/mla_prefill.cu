@@ -190,7 +190,7 @@ mla_prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const _
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_v + PF_STAGES);
     float* row_stat = reinterpret_cast<float*>(bars + 16);           // [2 halves][128 rows]
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int head = blockIdx.x, batch = blockIdx.y, q0 = (gridDim.z - 1 - blockIdx.z) * PF_M;      // the rows that see most first
     const int kv_head = head / p.group;
     const int first_pos = p.start + q0;                              // position of the tile's first query
@@ -208,12 +208,13 @@ mla_prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const _
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = uniform(*tmem_slot);
     const uint32_t tmem_s = tmem_base, tmem_ph = tmem_base + 128, tmem_pl = tmem_base + 192, tmem_pv = tmem_base + 256;
     bool ok = true;
 
     if (warp == 8) {
-        if (lane == 0) {
+        {
+            const uint32_t on = elect_one();
             constexpr uint32_t idesc_s = make_idesc_bf16(PF_M, PF_N, false, false);
             constexpr uint32_t idesc_pv = make_idesc_bf16(PF_M, 64, false, true);
             const uint64_t q_desc = make_smem_desc(smem_u32(sq), 16, 1024), k_desc = make_smem_desc(smem_u32(sk), 16, 1024);
@@ -225,54 +226,54 @@ mla_prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const _
                     constexpr int q_slab[5] = {0, 2, 3, 0, 1}, k_slab[5] = {1, 0, 2, 0, 2};
 #pragma unroll
                     for (int k4 = 0; k4 < 4; ++k4)
-                        umma_f16(tmem_s, q_desc + q_slab[part] * (PF_SLAB >> 4) + k4 * 2, kd + k_slab[part] * (PF_SLAB >> 4) + k4 * 2, idesc_s, (part | k4) != 0);
+                        umma_f16(tmem_s, q_desc + q_slab[part] * (PF_SLAB >> 4) + k4 * 2, kd + k_slab[part] * (PF_SLAB >> 4) + k4 * 2, idesc_s, (part | k4) != 0, on);
                 }
-                umma_commit(bar_s);
+                umma_commit(bar_s, on);
             };
             auto load_k = [&](int tile) {
                 const int st = tile % PF_STAGES;
                 uint8_t* dst = sk + st * PF_K_BYTES;
-                mbar_expect_tx(&bar_k[st], PF_K_BYTES);
-                tma_load_3d(dst, &tmap_kh, &bar_k[st], kv_head * 64, lo + tile * PF_N, batch);
-                tma_load_3d(dst + PF_SLAB, &tmap_kl, &bar_k[st], kv_head * 64, lo + tile * PF_N, batch);
-                tma_load_3d(dst + 2 * PF_SLAB, &tmap_rope, &bar_k[st], 0, lo + tile * PF_N, batch);
+                if (on) mbar_expect_tx(&bar_k[st], PF_K_BYTES);
+                tma_load_3d(dst, &tmap_kh, &bar_k[st], kv_head * 64, lo + tile * PF_N, batch, on);
+                tma_load_3d(dst + PF_SLAB, &tmap_kl, &bar_k[st], kv_head * 64, lo + tile * PF_N, batch, on);
+                tma_load_3d(dst + 2 * PF_SLAB, &tmap_rope, &bar_k[st], 0, lo + tile * PF_N, batch, on);
             };
             auto load_v = [&](int tile) {
                 const int st = tile % PF_STAGES;
                 uint8_t* dst = sv + st * PF_V_BYTES;
-                mbar_expect_tx(&bar_v[st], PF_V_BYTES);
-                tma_load_3d(dst, &tmap_vh, &bar_v[st], kv_head * 64, lo + tile * PF_N, batch);
-                tma_load_3d(dst + PF_SLAB, &tmap_vl, &bar_v[st], kv_head * 64, lo + tile * PF_N, batch);
+                if (on) mbar_expect_tx(&bar_v[st], PF_V_BYTES);
+                tma_load_3d(dst, &tmap_vh, &bar_v[st], kv_head * 64, lo + tile * PF_N, batch, on);
+                tma_load_3d(dst + PF_SLAB, &tmap_vl, &bar_v[st], kv_head * 64, lo + tile * PF_N, batch, on);
             };
-            mbar_expect_tx(bar_q, PF_Q_BYTES);
+            if (on) mbar_expect_tx(bar_q, PF_Q_BYTES);
 #pragma unroll
             for (int sl = 0; sl < 4; ++sl)
-                tma_load_3d(sq + sl * PF_SLAB, &tmap_q, bar_q, head * 128 + (sl & 1) * 64, q0, batch + (sl >> 1) * gridDim.y);
+                tma_load_3d(sq + sl * PF_SLAB, &tmap_q, bar_q, head * 128 + (sl & 1) * 64, q0, batch + (sl >> 1) * gridDim.y, on);
             for (int t = 0; t < PF_STAGES && t < n_tiles; ++t) { load_k(t); load_v(t); }
-            if (!mbar_wait(bar_q, 0) || !mbar_wait(&bar_k[0], 0)) { atomicExch(p.status, 231); ok = false; }
+            if (!warp_wait(bar_q, 0) || !warp_wait(&bar_k[0], 0)) { atomicExch(p.status, 231); ok = false; }
             if (ok) { tc_fence_after(); issue_s(0); }
             for (int j = 0; j < n_tiles && ok; ++j) {
                 const uint32_t ph = j & 1;
                 const int st = j % PF_STAGES;
                 const uint32_t st_ph = (j / PF_STAGES) & 1;
-                if (!mbar_wait(bar_s, ph)) { atomicExch(p.status, 232); ok = false; break; }
+                if (!warp_wait(bar_s, ph)) { atomicExch(p.status, 232); ok = false; break; }
                 if (j + PF_STAGES < n_tiles) load_k(j + PF_STAGES);            // S_j has consumed its key tile: refill the stage
-                if (!mbar_wait(bar_p, ph) || !mbar_wait(&bar_v[st], st_ph)) { atomicExch(p.status, 233); ok = false; break; }
+                if (!warp_wait(bar_p, ph) || !warp_wait(&bar_v[st], st_ph)) { atomicExch(p.status, 233); ok = false; break; }
                 tc_fence_after();
                 const uint64_t vd = v_desc + st * (PF_V_BYTES >> 4);
 #pragma unroll
                 for (int part = 0; part < 3; ++part)                 // P low x V high, P high x V low, P high x V high
 #pragma unroll
                     for (int k8 = 0; k8 < PF_N / 16; ++k8)
-                        umma_f16_ta(tmem_pv, (part == 0 ? tmem_pl : tmem_ph) + k8 * 8, vd + (part == 1 ? (PF_SLAB >> 4) : 0) + k8 * 128, idesc_pv, (part | k8) != 0);
-                umma_commit(bar_o);
+                        umma_f16_ta(tmem_pv, (part == 0 ? tmem_pl : tmem_ph) + k8 * 8, vd + (part == 1 ? (PF_SLAB >> 4) : 0) + k8 * 128, idesc_pv, (part | k8) != 0, on);
+                umma_commit(bar_o, on);
                 if (j + 1 < n_tiles) {
                     const int nst = (j + 1) % PF_STAGES;
-                    if (!mbar_wait(&bar_k[nst], ((j + 1) / PF_STAGES) & 1)) { atomicExch(p.status, 234); ok = false; break; }
+                    if (!warp_wait(&bar_k[nst], ((j + 1) / PF_STAGES) & 1)) { atomicExch(p.status, 234); ok = false; break; }
                     tc_fence_after();
                     issue_s(nst);
                 }
-                if (!mbar_wait(bar_o, ph)) { atomicExch(p.status, 235); ok = false; break; }
+                if (!warp_wait(bar_o, ph)) { atomicExch(p.status, 235); ok = false; break; }
                 if (j + PF_STAGES < n_tiles) load_v(j + PF_STAGES);            // PV_j has consumed its value tile
             }
         }

@@ -92,6 +92,7 @@ def forward_dual(q0, window, seq_len, rng, max_delay, stages=4, starved=None):
     readers = [0] * stages                 # products in flight that read the stage
     s_owner = ["free", "free"]             # S_x columns: free -> product in flight -> ready for the softmax -> free
     p_ready = [False, False]
+    pv_running = [False, False]            # a product in flight reads P_x and accumulates into O_x
     finished = []
 
     def loader():
@@ -132,16 +133,17 @@ def forward_dual(q0, window, seq_len, rng, max_delay, stages=4, starved=None):
             p_ready[x] = False
             st = (u0[x] + i) % stages
             assert stage_tile[st] == u0[x] + i, "PV reads a stage that does not hold its value tile"
-            readers[st] += 1
-            last = i + 1 == n[x]
-
-            def pv_done(st=st, last=last):
-                readers[st] -= 1
-                if last:
-                    bar_o[x].arrive()
-            mma[x].push(pv_done)
-            if not last:
+            if i + 1 < n[x]:                            # the next tile's S goes first
                 yield from issue_s(u0[x] + i + 1)
+            assert stage_tile[st] == u0[x] + i, "PV reads a stage that does not hold its value tile"
+            readers[st] += 1
+            pv_running[x] = True
+
+            def pv_done(st=st):
+                readers[st] -= 1
+                pv_running[x] = False
+                bar_o[x].arrive()
+            mma[x].push(pv_done)
         finished.append(f"issuer{x}")
 
     def softmax(x):
@@ -149,17 +151,21 @@ def forward_dual(q0, window, seq_len, rng, max_delay, stages=4, starved=None):
         for i in range(n[x]):
             yield bar_s[x], i
             assert s_owner[x] == "ready"
+            yield None                                 # the maximum of the row
             if i > 0:
+                yield bar_o[x], i - 1
+                assert not pv_running[x]
                 done = lo_x + i - 1
                 fb = bar_free[(done - lo_a) % stages]
                 fb.arrive()
                 if (done < lo_b) if x == 0 else (done > hi_a):
                     fb.arrive()
             yield None                                 # the arithmetic: other roles run meanwhile
+            assert not pv_running[x], "P or O touched while a product still uses them"
             s_owner[x] = "free"
             p_ready[x] = True
             bar_p[x].arrive()
-        yield bar_o[x], 0
+        yield bar_o[x], n[x] - 1
         finished.append(f"softmax{x}")
 
     roles = {"loader": loader(), "issuer0": issuer(0), "issuer1": issuer(1), "softmax0": softmax(0), "softmax1": softmax(1)}
@@ -197,7 +203,7 @@ def backward_pipe(n_iter, rng, max_delay, stages=3, starved=None):
     readers = [0] * stages
     sdp = {"state": "free"}               # S / dP columns of TMEM
     pds = {"holds": None, "readers": 0}   # P / dS tiles in shared memory
-    dq = {"holds": None}                  # dQ columns of TMEM
+    dq = [{"holds": None}, {"holds": None}]       # dQ columns of TMEM, two tiles in turn
     drained = []
     finished = []
 
@@ -250,24 +256,24 @@ def backward_pipe(n_iter, rng, max_delay, stages=3, starved=None):
             yield bar_pds, it
             yield bar_qdo[st], it // stages
             assert stage_iter[st] == it and pds["holds"] == it
-            assert dq["holds"] is None, "dQ overwritten before the previous tile's dQ was drained"
+            assert dq[it & 1]["holds"] is None, "dQ overwritten before the dQ of two tiles ago was drained"
             readers[st] += 1
             pds["readers"] += 1
-            dq["holds"] = ("mma", it)
+            dq[it & 1]["holds"] = ("mma", it)
 
             def done(st=st, it=it):
                 readers[st] -= 1
                 pds["readers"] -= 1
-                dq["holds"] = it
+                dq[it & 1]["holds"] = it
                 bar_mma.arrive()
             mma_g.push(done)
         finished.append("gradient_issuer")
 
     def softmax():
         def drain(jt):
-            yield bar_mma, jt
-            assert dq["holds"] == jt
-            dq["holds"] = None
+            yield None
+            assert dq[jt & 1]["holds"] == jt
+            dq[jt & 1]["holds"] = None
             drained.append(jt)
         for it in range(n_iter):
             yield bar_sdp, it
@@ -276,11 +282,14 @@ def backward_pipe(n_iter, rng, max_delay, stages=3, starved=None):
             sdp["state"] = "free"
             bar_sread.arrive()
             if it > 0:
-                yield from drain(it - 1)
+                yield bar_mma, it - 1
             assert pds["readers"] == 0, "P/dS stored while the previous gradient products still read the tiles"
             pds["holds"] = it
             bar_pds.arrive()
+            if it > 0:
+                yield from drain(it - 1)
         if n_iter > 0:
+            yield bar_mma, n_iter - 1
             yield from drain(n_iter - 1)
         finished.append("softmax")
 
