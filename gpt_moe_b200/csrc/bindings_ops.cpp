@@ -616,6 +616,93 @@ Tensor attention_branch(const Tensor& x, const Tensor& w_qkv, const Tensor& w_ou
     return y;
 }
 
+// The tensors of a layer of `trunk`.
+enum TrunkTensor { W_QKV, W_OUT, ROPE_COS, ROPE_SIN, Q_SCALE, K_SCALE, ATTN_BETA, ATTN_NORM, W_ROUTER, W_UP, W_DOWN, MLP_BETA, NEXT_NORM, TRUNK_TENSORS };
+
+// Consecutive blocks of a model without gradients as one call: per block the QKV product, rotation and QK-norm, attention, output projection, residual
+// update and norm, the routed experts, residual update and norm, 14 launches.  x [rows, hidden] fp32 is the residual stream, h its first norm (bf16);
+// returns the stream and its norm behind the last block.  Every layer works in the same buffers: a call per branch with tensors of its own cost 111 us of host time a layer here
+// (and as much again in Python around it), which is more than the kernels of a few hundred rows take.
+std::vector<Tensor> trunk(const Tensor& x, const Tensor& h0, const std::vector<std::vector<OptTensor>>& layers, const std::vector<int64_t>& windows,
+             const std::vector<std::array<double, 2>>& norm_eps, int64_t batch, int64_t heads, int64_t kv_heads, int64_t top_k, double qk_eps, double qk_min,
+             double qk_max, double scale, double softcap, bool qk_rms, bool renormalise, const std::string& activation, const OptTensor& doc_start) {
+    c10::cuda::CUDAGuard guard(x.device());
+    check_bf16(h0, "h");
+    GM_CHECK(x.is_cuda() && x.scalar_type() == torch::kFloat32 && x.is_contiguous() && x.dim() == 2 && h0.sizes() == x.sizes(), "trunk: x fp32 and h bf16 [rows, hidden]");
+    GM_CHECK(windows.size() == layers.size() && norm_eps.size() == layers.size(), "trunk: a window and two epsilons per layer");
+    const int64_t rows = x.size(0), hidden = x.size(1), dim = 64, turned = (heads + kv_heads) * dim, width = turned + kv_heads * dim;
+    GM_CHECK(batch > 0 && rows > 0 && rows % batch == 0 && norm_dim_supported(hidden) && heads > 0 && kv_heads > 0 && heads % kv_heads == 0 && top_k >= 1, "trunk: sizes");
+    const int64_t seq = rows / batch, slots = rows * top_k;
+    const int kind = act_kind(activation);
+    int64_t experts = 0, up = 0, inner = 0;
+    for (const auto& t : layers) {
+        GM_CHECK(t.size() == TRUNK_TENSORS, "trunk: tensors of a layer");
+        for (int i : {W_QKV, W_OUT, W_ROUTER, W_UP, W_DOWN}) {
+            GM_CHECK(t[i].has_value(), "trunk: a weight is missing");
+            check_bf16(*t[i], "weight");
+        }
+        for (int i : {ATTN_BETA, MLP_BETA}) GM_CHECK(t[i].has_value() && t[i]->numel() == 1, "trunk: a scale of each branch");
+        for (int i : {ATTN_NORM, NEXT_NORM}) GM_CHECK(t[i].has_value() && t[i]->numel() == hidden, "trunk: norm weights");
+        for (int i : {ROPE_COS, ROPE_SIN, Q_SCALE, K_SCALE, ATTN_BETA, ATTN_NORM, MLP_BETA, NEXT_NORM})
+            GM_CHECK(!t[i].has_value() || (t[i]->is_cuda() && t[i]->scalar_type() == torch::kFloat32 && t[i]->is_contiguous()), "trunk: fp32 tables, scales and norm weights");
+        for (int i : {ROPE_COS, ROPE_SIN}) GM_CHECK(!t[i].has_value() || (t[i]->dim() == 2 && t[i]->size(0) >= seq && t[i]->size(1) == dim / 2), "trunk: rotary tables [>= seq, 32]");
+        GM_CHECK((!t[Q_SCALE].has_value() || t[Q_SCALE]->numel() == heads) && (!t[K_SCALE].has_value() || t[K_SCALE]->numel() == kv_heads), "trunk: QK scales");
+        if (experts == 0) { experts = t[W_UP]->size(0); up = t[W_UP]->size(1); inner = t[W_DOWN]->size(2); }
+        GM_CHECK(t[W_QKV]->dim() == 2 && t[W_QKV]->size(0) == width && t[W_QKV]->size(1) == hidden && t[W_OUT]->dim() == 2 && t[W_OUT]->size(0) == hidden &&
+                 t[W_OUT]->size(1) == heads * dim && t[W_ROUTER]->dim() == 2 && t[W_ROUTER]->size(0) == experts && t[W_ROUTER]->size(1) == hidden &&
+                 t[W_UP]->dim() == 3 && t[W_UP]->size(0) == experts && t[W_UP]->size(1) == up && t[W_UP]->size(2) == hidden && t[W_DOWN]->dim() == 3 &&
+                 t[W_DOWN]->size(0) == experts && t[W_DOWN]->size(1) == hidden && t[W_DOWN]->size(2) == inner, "trunk: weight shapes, the same in every layer");
+    }
+    if (layers.empty()) return {x, h0};
+    GM_CHECK(inner * (kind == 4 ? 2 : 1) == up && inner % 8 == 0, "trunk: expert widths");
+    const auto bf = h0.options(), f32 = x.options(), i32 = x.options().dtype(torch::kInt32);
+    const int64_t cap = (slots + 255) / 256 * 256 + experts * 256, chunks = (slots + 1023) / 1024;
+    Tensor stream_a = gm::out_empty_like(x), stream_b = gm::out_empty_like(x), h = gm::out_empty_like(h0);
+    Tensor qkv = gm::out_empty({rows, width}, bf), rotated = gm::out_empty({rows, turned}, bf), branch = gm::out_empty({rows, hidden}, bf);
+    Tensor logits = gm::out_empty({rows, experts}, bf), top_idx = gm::out_empty({slots}, i32.dtype(torch::kInt64)), gates = gm::out_empty({rows, top_k}, f32);
+    Tensor packed = gm::out_empty({cap, hidden}, bf), pre = gm::out_empty({cap, up}, bf), act = gm::out_empty({cap, inner}, bf);
+    Tensor hist = gm::out_empty({2, chunks, experts}, i32), dest = gm::out_empty({slots}, i32), src = gm::out_empty({cap}, i32);
+    Tensor seg = gm::out_empty({experts}, i32), counts = gm::out_empty({experts}, i32), tiles = gm::out_empty({cap / 128}, i32), meta = gm::out_empty({2}, i32);
+    const auto part = [&](const Tensor& of, int64_t first, int64_t n) {
+        return of.as_strided({batch, seq, n, dim}, {seq * of.size(1), of.size(1), dim, 1}, first * dim);
+    };
+    const Tensor q = part(rotated, 0, heads), k = part(rotated, heads, kv_heads), v = part(qkv, heads + kv_heads, kv_heads);
+    long long* top = reinterpret_cast<long long*>(top_idx.data_ptr<int64_t>());
+    const cudaStream_t s = stream();
+    const void* residual = x.data_ptr();
+    const Tensor* normed = &h0;
+    const auto update = [&](const OptTensor& beta, const OptTensor& weight, double eps) {       // residual += beta * branch; h = norm(residual)
+        void* to = residual == stream_a.data_ptr() ? stream_b.data_ptr() : stream_a.data_ptr();
+        launch_rmsnorm_fwd(residual, true, branch.data_ptr(), nullptr, fptr(beta), to, fptr(weight), h.data_ptr(), nullptr, nullptr, nullptr, static_cast<int>(rows),
+                           static_cast<int>(hidden), static_cast<float>(eps), s);
+        residual = to;
+        normed = &h;
+    };
+    for (size_t l = 0; l < layers.size(); ++l) {
+        const auto& t = layers[l];
+        gemm_plain(*normed, *t[W_QKV], qkv);
+        rope_qknorm_fwd(qkv, rotated, t[ROPE_COS], t[ROPE_SIN], t[Q_SCALE], t[K_SCALE], seq, heads, kv_heads, dim, qk_eps, qk_rms, qk_min, qk_max, 0);
+        const Tensor o = attention_out(q, k, v, windows[l], scale, softcap, doc_start);
+        gemm_plain(o.view({rows, heads * dim}), *t[W_OUT], branch);
+        update(t[ATTN_BETA], t[ATTN_NORM], norm_eps[l][0]);
+        gemm_plain(h, *t[W_ROUTER], logits);
+        GM_CHECK(launch_router_fwd(logits.data_ptr(), true, top, gates.data_ptr<float>(), nullptr, nullptr, nullptr, nullptr, nullptr, static_cast<int>(rows),
+                                   static_cast<int>(experts), static_cast<int>(top_k), renormalise, s), "router kernel: at most 128 experts, top-k at most 8");
+        launch_route(top, static_cast<int>(slots), static_cast<int>(experts), hist.data_ptr<int>(), hist.data_ptr<int>() + chunks * experts, counts.data_ptr<int>(),
+                     seg.data_ptr<int>(), tiles.data_ptr<int>(), meta.data_ptr<int>(), dest.data_ptr<int>(), src.data_ptr<int>(), s);
+        launch_gather_rows(h.data_ptr(), src.data_ptr<int>(), meta.data_ptr<int>(), packed.data_ptr(), nullptr, nullptr, static_cast<int>(hidden),
+                           static_cast<int>(top_k), static_cast<int>(cap), static_cast<int>(rows), s);
+        gemm_by_expert(packed, *t[W_UP], pre, tiles, meta);
+        launch_activation_fwd(pre.data_ptr(), act.data_ptr(), meta.data_ptr<int>(), nullptr, nullptr, static_cast<int>(cap), static_cast<int>(inner), kind, s);
+        gemm_by_expert(act, *t[W_DOWN], packed, tiles, meta);
+        launch_combine_fwd(packed.data_ptr(), dest.data_ptr<int>(), gates.data_ptr<float>(), branch.data_ptr(), static_cast<int>(rows), static_cast<int>(hidden),
+                           static_cast<int>(top_k), static_cast<int>(cap), s);
+        update(t[MLP_BETA], t[NEXT_NORM], norm_eps[l][1]);
+    }
+    check_launch("trunk");
+    return {residual == stream_a.data_ptr() ? stream_a : stream_b, h};
+}
+
 // Router projection -> routing -> gather -> grouped up GEMM -> activation -> grouped down GEMM -> gated combine.
 Tensor moe_branch(const Tensor& x, const Tensor& w_router, int64_t top_k, bool renormalise, const Tensor& w_up, const Tensor& w_down,
                   const std::string& activation) {
@@ -905,6 +992,7 @@ void register_kernels(pybind11::module_& m) {
     m.def("embedding_grad", &embedding_grad);
     m.def("attention_branch", &attention_branch);
     m.def("moe_branch", &moe_branch);
+    m.def("trunk", &trunk);
     m.def("continuation_logprob", &continuation_logprob);
     m.def("adamw", &adamw);
     m.def("muon_prepare", &muon_prepare);

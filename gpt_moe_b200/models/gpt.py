@@ -27,9 +27,10 @@ from torch.utils.checkpoint import checkpoint
 
 from ..config.training import PHASES, ROLES
 from ..ops import api
-from .attention import AttentionContext
-from .block import Block, apply_norm, make_norm
+from .attention import AttentionContext, SelfAttention
+from .block import Block, apply_norm, make_norm, norm_eps
 from .linear import Linear
+from .moe import MoE
 
 
 def validate_linear_config(linear_config, use_moe: bool) -> List[str]:
@@ -232,6 +233,78 @@ class GPT(nn.Module):
         return {"adamw": adamw, "muon": muon}
 
     # ---- forward ------------------------------------------------------------------------------
+    @staticmethod
+    def _plain_forward(x: Tensor, ctx: AttentionContext) -> bool:
+        """Whether blocks over this residual stream may run as composed native calls at all."""
+        if not x.is_cuda or x.dtype != torch.float32 or x.dim() != 3 or x.numel() == 0 or ctx.attn_mask is not None:
+            return False
+        from ..ops import cuda_ops
+        d = x.shape[2]
+        return d % 128 == 0 and d // 128 in (1, 2, 4, 6, 8, 12, 16) and cuda_ops.plain_call() and cuda_ops.no_global_hooks()
+
+    @staticmethod
+    def _plain_layer(block: nn.Module, next_norm: nn.Module, x: Tensor, ctx: AttentionContext):
+        """What `trunk` (csrc/bindings_ops.cpp) needs of one block and the norm behind it, for a forward pass without gradients over a residual
+        stream x: ((what the layers of one call share), tensors, window, epsilons).  None unless the block would take its composed calls: the
+        conditions are theirs (SelfAttention._fused_rope_attention, MoE._forward_plain, cuda_ops.residual_rms_norm)."""
+        from ..ops import cuda_ops
+        from ..ops.attention_cuda import _window_int
+        if type(block) is not Block:
+            return None
+        parts, t, d = block._modules, x.shape[1], x.shape[2]
+        attn, mlp = parts["attn"], parts["mlp"]
+        if type(attn) is not SelfAttention or type(mlp) is not MoE or not cuda_ops.unhooked(attn, mlp):
+            return None
+        proj, router, experts = attn._modules, mlp._modules["router"], mlp.num_experts
+        heads, kv_heads, q_proj, out_proj = attn.n_heads, attn.n_kv_heads, proj["q_proj"], proj["out_proj"]
+        if (attn.head_size != 64 or heads + kv_heads > 64 or heads % kv_heads or (t % 128 and attn.softcap != 0.0) or not attn.is_causal
+                or mlp._modules.get("shared_expert") is not None or mlp.ep_size > 1 or (mlp.training and mlp.load_balance_weight > 0)
+                or experts % 8 or experts > 128 or mlp.top_k > 8):
+            return None
+        table = mlp._modules["experts"]._modules
+        mlps = [table[str(e)]._modules for e in range(experts)]
+        ups, downs = [m["up_proj"] for m in mlps], [m["down_proj"] for m in mlps]
+        for m in (out_proj, router, ups[0], downs[0]):
+            if type(m) is not Linear or m._parameters.get("bias") is not None or m.precision != "default":
+                return None
+        norm = parts["ln_2"]
+        (alpha_a, beta_a), (alpha_m, beta_m) = block._scales("attn"), block._scales("mlp")
+        if (q_proj.precision != "default" or q_proj._parameters.get("bias") is not None or not cuda_ops.unhooked(out_proj, router)
+                or not (isinstance(norm, nn.RMSNorm) and isinstance(next_norm, nn.RMSNorm)) or alpha_a is not None or alpha_m is not None
+                or beta_a is None or beta_m is None):
+            return None
+        norms = [norm._parameters.get("weight"), next_norm._parameters.get("weight")]
+        w_up, w_down = [m._parameters.get("weight") for m in ups], [m._parameters.get("weight") for m in downs]
+        if any(w is None for w in norms) or any(w is None for w in w_up) or any(w is None for w in w_down) or w_up[0].shape[0] % 16:
+            return None
+        rotary, scales, fp32 = proj.get("rotary"), attn._parameters, cuda_ops.as_fp32
+        use_norm = attn.use_qk_norm
+        tensors = [
+            cuda_ops.bf16_weight((q_proj._parameters["weight"], proj["k_proj"]._parameters["weight"], proj["v_proj"]._parameters["weight"])),
+            cuda_ops.bf16_weight((out_proj._parameters["weight"],)),
+            None if rotary is None else rotary._buffers["cos_cached"], None if rotary is None else rotary._buffers["sin_cached"],
+            fp32(scales["q_scale"]) if use_norm else None, fp32(scales["k_scale"]) if use_norm else None, fp32(beta_a), fp32(norms[0]),
+            cuda_ops.bf16_weight((router._parameters["weight"],)), cuda_ops.stacked_weight(w_up), cuda_ops.stacked_weight(w_down), fp32(beta_m),
+            fp32(norms[1])]
+        shared = (heads, kv_heads, mlp.top_k, attn.qk_eps, max(attn.qk_scale_min, -3.0e38), min(attn.qk_scale_max, 3.0e38), 64 ** -0.5, attn.softcap,
+                  attn.qk_norm_type == "rms", not (mlp.top_k == 1 or mlp.full_softmax_gating), table["0"].activation_name)
+        window = None if (attn.is_full_attention or not attn.use_flex_attention) else _window_int(ctx.window)
+        return shared + (tensors[9].shape,), tensors, t if window is None else window, (norm_eps(norm, x.dtype), norm_eps(next_norm, x.dtype))
+
+    @staticmethod
+    def _plain_blocks(layers: list, x: Tensor, h: Tensor, ctx: AttentionContext) -> Tuple[Tensor, Tensor]:
+        """Residual stream and its next norm after the blocks that `_plain_layer` described."""
+        from ..ops import cuda_ops
+        b, t, d = x.shape
+        if ctx.document_ids is not None and ctx.doc_start is None:
+            from ..ops.attention_tc import document_starts
+            ctx.doc_start = document_starts(ctx.document_ids)
+        cuda_ops.count_path("attention:tcgen05", len(layers))
+        heads, kv_heads, *rest = layers[0][0][:-1]
+        x, h = cuda_ops.ext().trunk(x.reshape(b * t, d), h.reshape(b * t, d), [l[1] for l in layers], [l[2] for l in layers], [l[3] for l in layers], b,
+                                    heads, kv_heads, *rest, None if ctx.document_ids is None else ctx.doc_start)
+        return x.view(b, t, d), h.view(b, t, d)
+
     def _attention_context(self, attn_mask: Optional[Tensor], document_ids: Optional[Tensor],
                            ignore_doc_mask: bool, batch: int, seq_len: int, device) -> AttentionContext:
         if attn_mask is not None:
@@ -263,18 +336,29 @@ class GPT(nn.Module):
         if chain:
             # residual update + following RMSNorm as one op per link (see Block.forward_prenormed)
             h = apply_norm(blocks[0].ln_1, x)
+            plain = h.dtype == torch.bfloat16 and self._plain_forward(x, ctx)
+            # blocks that one native call can run without gradients wait here; one, two, four .. at a time, so that the GPU is at work while
+            # the host collects the next ones
+            waiting, at_a_time = [], 1
             hook = getattr(self, "block_grad_hook", None) if grad_mode else None
             for i, block in enumerate(blocks):
                 if hook is not None and h.requires_grad:
                     # the gradient of a block's normalised input is the last thing its backward produces
                     h.register_hook(lambda grad, layer=i, fn=hook: fn(layer))
                 next_norm = blocks[i + 1].ln_1 if i + 1 < len(blocks) else self.transformer.ln_f
+                layer = self._plain_layer(block, next_norm, x, ctx) if plain else None
+                if waiting and (layer is None or layer[0] != waiting[0][0] or len(waiting) == at_a_time):
+                    x, h = self._plain_blocks(waiting, x, h, ctx)
+                    waiting, at_a_time = [], 2 * at_a_time
+                if layer is not None:
+                    waiting.append(layer)
+                    continue
                 next_q = getattr(blocks[i + 1].attn, "q_proj", None) if i + 1 < len(blocks) else None
                 next_mxfp8 = next_q is not None and next_q.precision in ("mxfp8", "fp8") and hasattr(blocks[i + 1].attn, "k_proj")
                 x, h, block_balance = block.forward_prenormed(x, h, ctx, next_norm, next_mxfp8)
                 if block_balance is not None:
                     balance_loss = block_balance if balance_loss is None else balance_loss + block_balance
-            x = h
+            x = self._plain_blocks(waiting, x, h, ctx)[1] if waiting else h
         elif self.activation_offloader is not None and grad_mode:
             x, balance_loss = self.activation_offloader.run(self.transformer.h, x, ctx)
         else:

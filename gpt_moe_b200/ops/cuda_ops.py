@@ -64,9 +64,9 @@ def ext():
 _path_counts: dict = {}
 
 
-def count_path(name: str) -> None:
+def count_path(name: str, times: int = 1) -> None:
     """Record that an op ran on path `name` (`attention:tcgen05`, `attention:sdpa`, `linear:torch`, ...)."""
-    _path_counts[name] = _path_counts.get(name, 0) + 1
+    _path_counts[name] = _path_counts.get(name, 0) + times
 
 
 def path_counts() -> dict:
@@ -157,10 +157,18 @@ def plain_call() -> bool:
 def bypassable(*modules) -> bool:
     """Calling these modules does nothing but run their class's forward: no hooks (a process may also have global ones) and no forward
     of an instance's own.  Only then may a composed call stand in for them."""
+    return unhooked(*modules) and no_global_hooks()
+
+
+def unhooked(*modules) -> bool:
     for m in modules:
         own = m.__dict__
         if own["_forward_hooks"] or own["_forward_pre_hooks"] or own["_backward_hooks"] or own["_backward_pre_hooks"] or "forward" in own:
             return False
+    return True
+
+
+def no_global_hooks() -> bool:
     return not _nn_module._has_any_global_hook()
 
 

@@ -1,0 +1,89 @@
+"""All blocks of a forward pass without gradients as one native call (`trunk`): the bits of the blocks' own calls, and only where they apply."""
+import pytest
+import torch
+
+from gpt_moe_b200.config import get_preset
+from gpt_moe_b200.models.gpt import GPT
+from gpt_moe_b200.ops import cuda_ops
+
+pytestmark = pytest.mark.gpu
+
+# name: (model options, tokens, whether the one call serves it)
+CASES = {
+    "one token": ({}, 1, True),
+    "odd length": ({}, 77, True),
+    "grouped heads, full attention in one layer": (dict(n_kv_heads=4, full_attention_layers=[1], global_attn_dim=768, global_n_kv_heads=4), 300, True),
+    "two experts a token, gates renormalised": (dict(moe_top_k=2), 130, True),
+    "relu2": (dict(activation="relu2"), 40, True),
+    "capped logits": (dict(use_attn_logit_softcapping=True, attn_logit_softcap=20.0), 128, True),
+    "no rotation": (dict(pos_encoding_type="learned"), 64, True),
+    "a scale on the residual": (dict(use_weighted_residual_path=True), 64, False),
+    "dense feed-forward": (dict(use_moe=False), 64, False),
+}
+
+
+def _model(**options):
+    torch.manual_seed(1)
+    gc, tc = get_preset("small")
+    gc.n_layers, gc.mlp_hidden_dim, gc.weighted_main_path_init = 3, 256, 0.3
+    for name, value in options.items():
+        assert hasattr(gc, name), name
+        setattr(gc, name, value)
+    tc.seq_len_train = tc.seq_len_val = 512
+    tc.resolve(1)
+    model = GPT(gc, tc).cuda().eval()
+    model.set_sliding_window(48)
+    model.set_precision_phase("evaluation")
+    return model, gc
+
+
+def _served(model):
+    """Layers that went into the native call, one entry per call of the model's."""
+    seen, inner = [], model._plain_blocks
+    model._plain_blocks = lambda layers, *args: (seen.append(len(layers)), inner(layers, *args))[1]
+    return seen
+
+
+def _apart(model):
+    model._plain_forward = lambda *args: False
+
+
+@pytest.mark.parametrize("case", CASES)
+def test_trunk_has_the_bits_of_the_blocks_own_calls(case):
+    options, t, served = CASES[case]
+    model, gc = _model(**options)
+    ids = torch.randint(0, gc.vocab_size, (3, t), device="cuda")
+    with torch.no_grad():
+        seen = _served(model)
+        got = model(ids)
+        assert sum(seen) == (3 if served else 0)
+        _apart(model)
+        assert torch.equal(got, model(ids))
+    cuda_ops.check_status()
+
+
+def test_trunk_steps_aside_for_whoever_looks_at_a_block():
+    model, gc = _model()
+    ids = torch.randint(0, gc.vocab_size, (2, 33), device="cuda")
+    with torch.no_grad():
+        want, seen = model(ids), _served(model)
+        for module, apart in ((model.transformer.h[1].attn, 1), (model.transformer.h[2].mlp, 1), (model.transformer.h[0].attn.out_proj, 1),
+                              (model.transformer.h[0].mlp.router, 1)):
+            calls = []
+            handle = module.register_forward_hook(lambda *args: calls.append(1))
+            seen.clear()
+            assert torch.equal(model(ids), want) and sum(seen) == 3 - apart and calls      # the other blocks stay in the native call
+            handle.remove()
+        own = model.transformer.h[1].mlp.forward
+        model.transformer.h[1].mlp.forward = lambda x: (0 * own(x)[0], None)
+        seen.clear()
+        assert not torch.equal(model(ids), want) and sum(seen) == 2
+        del model.transformer.h[1].mlp.forward
+        # weights changed in place are seen by the next call
+        seen.clear()
+        assert torch.equal(model(ids), want) and sum(seen) == 3
+        model.transformer.h[1].attn.out_proj.weight.mul_(2)
+        changed = model(ids)
+        _apart(model)
+        assert not torch.equal(changed, want) and torch.equal(changed, model(ids))
+    cuda_ops.check_status()
