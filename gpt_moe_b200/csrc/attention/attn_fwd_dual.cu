@@ -397,11 +397,11 @@ attn_fwd_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
 
 bool attn_fwd_dual_supported(const AttnParams& p) {
     // us, this kernel / the single-tile one: 16 x 2048 tokens, window 1024 195 / 248, 16384 tokens 865 / 978, 4 x 4096 251 / 293, 2 x 3000 86 / 97,
-    // 64 x 184 48 / 64, 8 x 1100 58 / 60, 1 x 1024 25 / 24, 3 x 300 17 / 16.  Of an odd number of tiles the last CTA idles by half, which a short
+    // 64 x 184 48 / 64, 8 x 1100 58 / 60, 1 x 1024 25 / 24, 3 x 300 17 / 16, 8 x 45 8.6 / 7.1.  Of an odd number of tiles the last CTA idles by half, which a short
     // window does not repay below nine tiles (16 x 1152, window 256 84 / 91).
     const int tiles = (p.seq_len + DU_BM - 1) / DU_BM;
     const bool windowed = p.window <= p.seq_len / 2;
-    return p.qk_dim == 64 && p.doc_start == nullptr && (windowed ? tiles % 2 == 0 || tiles >= 9 : true);
+    return p.qk_dim == 64 && p.doc_start == nullptr && (windowed ? tiles % 2 == 0 || tiles >= 9 : tiles > 1);
 }
 
 template <bool CAPPED>

@@ -102,11 +102,84 @@ route_place_kernel(const long long* __restrict__ idx, const int* __restrict__ ch
     }
 }
 
+// All three in one block for at most ROUTE_CHUNK slots (a step of sampling, a short prompt), the same tables: three launches of a few
+// hundred slots took 8 us and the gaps between them.
+__global__ void __launch_bounds__(ROUTE_CHUNK)
+route_small_kernel(const long long* __restrict__ idx, int* __restrict__ counts, int* __restrict__ seg_ends, int* __restrict__ tile_expert,
+                   int* __restrict__ meta, int* __restrict__ dest, int* __restrict__ src_of_row, int slots, int experts) {
+    __shared__ int warp_count[32][MAX_EXPERTS];
+    __shared__ int cnt[MAX_EXPERTS], pstart[MAX_EXPERTS + 1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int i = threadIdx.x; i < 32 * MAX_EXPERTS; i += blockDim.x) (&warp_count[0][0])[i] = 0;
+    const int slot = threadIdx.x;
+    int e = slot < slots ? static_cast<int>(idx[slot]) : experts;           // `experts` = sentinel for idle lanes
+    if (!GM_IN_BOUNDS(e >= 0 && e <= experts && (slot >= slots || e < experts), 901)) e = experts;
+    __syncthreads();
+    const unsigned same = __match_any_sync(0xffffffffu, e);
+    const int rank = __popc(same & ((1u << lane) - 1u));
+    if (e < experts && rank == 0) warp_count[warp][e] = __popc(same);
+    __syncthreads();
+    if (threadIdx.x < experts) {           // exclusive prefix over the 32 warps, per expert
+        int run = 0;
+#pragma unroll
+        for (int w = 0; w < 32; ++w) {
+            const int c = warp_count[w][threadIdx.x];
+            warp_count[w][threadIdx.x] = run;
+            run += c;
+        }
+        cnt[threadIdx.x] = run;
+        counts[threadIdx.x] = run;
+    }
+    __syncthreads();
+    if (warp == 0) {                       // padded segments: four experts a lane, prefix over the lanes
+        int size[MAX_EXPERTS / 32], sum = 0;
+#pragma unroll
+        for (int i = 0; i < MAX_EXPERTS / 32; ++i) {
+            const int x = lane * (MAX_EXPERTS / 32) + i;
+            size[i] = x < experts ? (cnt[x] + SEG_PAD - 1) / SEG_PAD * SEG_PAD : 0;
+            sum += size[i];
+        }
+        int before = sum;
+#pragma unroll
+        for (int s = 1; s < 32; s <<= 1) {
+            const int other = __shfl_up_sync(0xffffffffu, before, s);
+            if (lane >= s) before += other;
+        }
+        const int total = __shfl_sync(0xffffffffu, before, 31);
+        before -= sum;
+#pragma unroll
+        for (int i = 0; i < MAX_EXPERTS / 32; ++i) {
+            const int x = lane * (MAX_EXPERTS / 32) + i;
+            if (x < experts) {
+                pstart[x] = before;
+                before += size[i];
+                seg_ends[x] = before;
+            }
+        }
+        if (lane == 0) { pstart[experts] = total; meta[0] = total / 128; meta[1] = total; }
+    }
+    __syncthreads();
+    if (e < experts) {
+        const int row = pstart[e] + warp_count[warp][e] + rank;
+        dest[slot] = row;
+        src_of_row[row] = slot;
+    }
+    for (int x = warp; x < experts; x += 32) {                              // a warp marks an expert's pad rows and tiles
+        const int from = pstart[x] + cnt[x], to = pstart[x + 1];
+        for (int r = from + lane; r < to; r += 32) src_of_row[r] = -1;
+        for (int t = pstart[x] / 128 + lane; t < to / 128; t += 32) tile_expert[t] = x;
+    }
+}
+
 bool launch_route(const long long* idx, int slots, int experts, int* chunk_hist, int* chunk_start, int* counts, int* seg_ends,
                   int* tile_expert, int* meta, int* dest, int* src_of_row, cudaStream_t s) {
     if (experts > MAX_EXPERTS || slots < 0) return false;
     // slots == 0 (an expert-parallel rank that received no rows this step): the plan alone yields empty segments and zero tiles
     const int chunks = (slots + ROUTE_CHUNK - 1) / ROUTE_CHUNK;
+    if (chunks == 1) {
+        route_small_kernel<<<1, ROUTE_CHUNK, 0, s>>>(idx, counts, seg_ends, tile_expert, meta, dest, src_of_row, slots, experts);
+        return true;
+    }
     if (chunks > 0) route_count_kernel<<<chunks, ROUTE_CHUNK, 0, s>>>(idx, chunk_hist, slots, experts);
     route_plan_kernel<<<1, 128, 0, s>>>(chunk_hist, chunk_start, counts, seg_ends, tile_expert, meta, src_of_row, chunks, experts);
     if (chunks > 0) route_place_kernel<<<chunks, ROUTE_CHUNK, 0, s>>>(idx, chunk_start, dest, src_of_row, slots, experts);
