@@ -500,7 +500,7 @@ torch::Tensor attn_bwd(const torch::Tensor& q, const torch::Tensor& k, const tor
     p.single_tile = unpipelined ? 1 : 0;
     p.window_ptr = window_word(window_tensor);
     const CUtensorMap& tdq = cached_map(dq.data_ptr(), 4, static_cast<uint64_t>(H) * D, T, B, static_cast<uint64_t>(H) * D * 4,
-                                        static_cast<uint64_t>(T) * H * D * 4, 32, 128, 128);
+                                        static_cast<uint64_t>(T) * H * D * 4, 32, D == 64 && !unpipelined ? 32 : 128, 128);      // rows that leave at a time
     cudaError_t e = gm::launch_attn_bwd(head_map(q, 128), head_map(k, 128), head_map(v, 128, true), head_map(d_out, 128), tdq, p,
                                         d_out.data_ptr(), out.data_ptr(), token_pitch(d_out), token_pitch(out), delta.data_ptr<float>(),
                                         current_stream());

@@ -193,108 +193,141 @@ def test_forward_model_notices_a_ring_that_is_too_shallow():
         forward_dual(1280, 1024, 2048, random.Random(seed), 3, stages=2)
 
 
-# ---- backward: score products of the next query tile ahead of the gradient products ------------------------------------------------
+# ---- backward: transposed scores, P and dS in TMEM, dQ drained by warps of its own -------------------------------------------------
 
 def backward_pipe(n_iter, rng, max_delay, stages=3, starved=None):
-    bar_kv, bar_sdp, bar_sread, bar_pds, bar_mma = Barrier(1), Barrier(1), Barrier(1), Barrier(1), Barrier(1)   # 256-thread barriers as one
-    bar_qdo = [Barrier(1) for _ in range(stages)]
-    tma, mma_s, mma_g = AsyncQueue(rng, max_delay), AsyncQueue(rng, max_delay), AsyncQueue(rng, max_delay)
-    stage_iter = [None] * stages
-    readers = [0] * stages
-    sdp = {"state": "free"}               # S / dP columns of TMEM
-    pds = {"holds": None, "readers": 0}   # P / dS tiles in shared memory
-    dq = [{"holds": None}, {"holds": None}]       # dQ columns of TMEM, two tiles in turn
-    drained = []
-    finished = []
+    one = ("kv", "s", "p", "dv", "dp", "ds", "dk", "mma", "dq", "end")           # many-thread barriers as one arrival
+    bar = {name: Barrier(1) for name in one}
+    ring = {name: [Barrier(1) for _ in range(stages)] for name in ("qdo", "free", "stat")}
+    tma, mma = AsyncQueue(rng, max_delay), AsyncQueue(rng, max_delay)
+    stage_iter, readers = [None] * stages, [0] * stages
+    stats = [None] * stages
+    s_cols, dp_cols = {"state": "free"}, {"state": "free"}      # S; dP, then dS in the same columns
+    p_cols = {"holds": None, "reader": False}
+    ds_tile = [{"holds": None, "reader": False}, {"holds": None, "reader": False}]
+    dq_cols = {"holds": None}
+    drained, finished = [], []
+
+    def commit(*names):
+        def done():
+            for b in names:
+                b.arrive()
+        mma.push(done)
 
     def loader():
-        tma.push(bar_kv.arrive)
-
-        def load(it):
+        tma.push(bar["kv"].arrive)
+        for it in range(n_iter):
             st = it % stages
+            if it >= stages:
+                yield ring["free"][st], it // stages - 1
             assert readers[st] == 0, "a Q/dO stage is refilled while a product still reads it"
             stage_iter[st] = None
 
             def landed(st=st, it=it):
                 stage_iter[st] = it
-                bar_qdo[st].arrive()
+                ring["qdo"][st].arrive()
             tma.push(landed)
-        for it in range(min(stages, n_iter)):
-            load(it)
-        for it in range(stages, n_iter):
-            yield bar_mma, it - stages
-            load(it)
         finished.append("loader")
 
-    def issue_sdp(it):
-        st = it % stages
-        yield bar_qdo[st], it // stages
-        assert stage_iter[st] == it
-        assert sdp["state"] == "free", "S/dP overwritten before the softmax warps have read them"
-        sdp["state"] = "mma"
+    def product(st, it, start, done):
+        assert stage_iter[st] == it and stats[st] == it, "a product reads a stage that holds another tile"
+        start()
         readers[st] += 1
 
-        def done(st=st):
+        def complete():
             readers[st] -= 1
-            sdp["state"] = "ready"
-            bar_sdp.arrive()
-        mma_s.push(done)
+            done()
+        mma.push(complete)
 
-    def score_issuer():
-        yield bar_kv, 0
-        if n_iter > 0:
-            yield from issue_sdp(0)
-        for it in range(n_iter - 1):
-            yield bar_sread, it
-            yield from issue_sdp(it + 1)
-        finished.append("score_issuer")
+    def issuer():
+        def issue_s(it):
+            assert s_cols["state"] == "free", "S overwritten before the softmax warps have read it"
+            product(it % stages, it, lambda: s_cols.update(state="mma"), lambda: s_cols.update(state=it))
+            commit(bar["s"])
 
-    def gradient_issuer():
-        yield bar_kv, 0
+        def issue_dp(it):
+            assert dp_cols["state"] == "free", "dP overwrites dS before dK has used it"
+            product(it % stages, it, lambda: dp_cols.update(state="mma"), lambda: dp_cols.update(state=it))
+            commit(bar["dp"])
+
+        yield bar["kv"], 0
+        yield ring["qdo"][0], 0
+        yield ring["stat"][0], 0
+        issue_s(0)
+        issue_dp(0)
         for it in range(n_iter):
-            st = it % stages
-            yield bar_pds, it
-            yield bar_qdo[st], it // stages
-            assert stage_iter[st] == it and pds["holds"] == it
-            assert dq[it & 1]["holds"] is None, "dQ overwritten before the dQ of two tiles ago was drained"
-            readers[st] += 1
-            pds["readers"] += 1
-            dq[it & 1]["holds"] = ("mma", it)
+            st, nxt, more = it % stages, (it + 1) % stages, it + 1 < n_iter
+            yield bar["p"], it
+            if more:
+                yield ring["qdo"][nxt], (it + 1) // stages
+                yield ring["stat"][nxt], (it + 1) // stages
+                issue_s(it + 1)
+            assert p_cols["holds"] == it
+            product(st, it, lambda: p_cols.update(reader=True), lambda: p_cols.update(reader=False))
+            commit(bar["dv"])
+            yield bar["ds"], it
+            assert dp_cols["state"] == ("dS", it) and ds_tile[it & 1]["holds"] == it
+            product(st, it, lambda: None, lambda: dp_cols.update(state="free"))
+            commit(bar["dk"])
+            if it > 0:
+                yield bar["dq"], it - 1
+            assert dq_cols["holds"] is None, "dQ overwritten before it was drained"
+            ds_tile[it & 1]["reader"] = True
 
-            def done(st=st, it=it):
-                readers[st] -= 1
-                pds["readers"] -= 1
-                dq[it & 1]["holds"] = it
-                bar_mma.arrive()
-            mma_g.push(done)
-        finished.append("gradient_issuer")
+            def dq_done(it=it):
+                ds_tile[it & 1]["reader"] = False
+                dq_cols["holds"] = it
+            mma.push(dq_done)
+            commit(ring["free"][st], bar["mma"])
+            if more:
+                yield bar["dk"], it
+                issue_dp(it + 1)
+        commit(bar["end"])
+        finished.append("issuer")
+
+    def drain():
+        def put(jt):
+            stats[jt % stages] = jt
+            ring["stat"][jt % stages].arrive()
+        for jt in range(min(stages, n_iter)):
+            put(jt)
+        for jt in range(n_iter):
+            yield bar["mma"], jt
+            assert dq_cols["holds"] == jt
+            yield None
+            dq_cols["holds"] = None
+            drained.append(jt)
+            bar["dq"].arrive()
+            if jt + stages < n_iter:
+                assert readers[jt % stages] == 0, "statistics replaced while a product still reads them"
+                put(jt + stages)
+        finished.append("drain")
 
     def softmax():
-        def drain(jt):
-            yield None
-            assert dq[jt & 1]["holds"] == jt
-            dq[jt & 1]["holds"] = None
-            drained.append(jt)
         for it in range(n_iter):
-            yield bar_sdp, it
-            assert sdp["state"] == "ready"
-            yield None                                 # P and dS formed in registers
-            sdp["state"] = "free"
-            bar_sread.arrive()
+            yield ring["stat"][it % stages], it // stages
+            yield bar["s"], it
+            assert s_cols["state"] == it and stats[it % stages] == it
+            yield None                                 # P formed
             if it > 0:
-                yield bar_mma, it - 1
-            assert pds["readers"] == 0, "P/dS stored while the previous gradient products still read the tiles"
-            pds["holds"] = it
-            bar_pds.arrive()
-            if it > 0:
-                yield from drain(it - 1)
-        if n_iter > 0:
-            yield bar_mma, n_iter - 1
-            yield from drain(n_iter - 1)
+                yield bar["dv"], it - 1
+            assert not p_cols["reader"], "P overwritten while dV still reads it"
+            p_cols["holds"] = it
+            s_cols["state"] = "free"
+            bar["p"].arrive()
+            yield bar["dp"], it
+            assert dp_cols["state"] == it and stats[it % stages] == it
+            yield None                                 # dS formed
+            assert not ds_tile[it & 1]["reader"], "dS stored while dQ of two tiles ago still reads it"
+            ds_tile[it & 1]["holds"] = it
+            dp_cols["state"] = ("dS", it)
+            bar["ds"].arrive()
+        yield bar["end"], 0
+        assert not any(readers) and drained[: n_iter - 1] == list(range(n_iter - 1))
         finished.append("softmax")
 
-    roles = {"loader": loader(), "score_issuer": score_issuer(), "gradient_issuer": gradient_issuer(), "softmax": softmax()}
-    run(roles, [tma, mma_s, mma_g], rng, starved=starved, starve=0.95)
+    roles = {"loader": loader(), "issuer": issuer(), "drain": drain(), "softmax": softmax()}
+    run(roles, [tma, mma], rng, starved=starved, starve=0.95)
     assert len(finished) == 4 and drained == list(range(n_iter))
 
 
@@ -315,7 +348,7 @@ def test_forward_protocol_survives_a_role_that_lags_far_behind(starved):
         forward_dual(q0, 1024, 2048, rng, 5, starved=starved)
 
 
-@pytest.mark.parametrize("starved", ["loader", "score_issuer", "gradient_issuer", "softmax"])
+@pytest.mark.parametrize("starved", ["loader", "issuer", "drain", "softmax"])
 def test_backward_protocol_survives_a_role_that_lags_far_behind(starved):
     rng = random.Random(sum(map(ord, starved)))
     for n_iter in (1, 3, 4, 9, 18):
