@@ -27,7 +27,7 @@ struct AttnParams {
     float* lse;                     // [batch, heads, seq] natural-log LSE of the scaled scores
     // backward
     const float* delta;             // [batch, heads, seq] rowsum(dO * O)
-    float* dq_accum;                // [tokens, heads*qk_dim] fp32, zero-initialised; reduced into by TMA
+    float* dq_accum;                // [tokens, heads*qk_dim] fp32, cleared by the delta pass; reduced into by TMA
     void* dk;                       // [tokens, kv_heads*qk_dim] bf16; dv is [tokens, kv_heads*64] with its own pitch
     void* dv;
     long long dkv_stride, dv_stride;
@@ -52,6 +52,9 @@ cudaError_t launch_attn_bwd_pipe(const CUtensorMap& tq, const CUtensorMap& tk, c
 cudaError_t launch_attn_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
                             const CUtensorMap& tdq, const AttnParams& p, const void* d_out, const void* out, long long do_stride,
                             long long o_stride, float* delta, cudaStream_t stream);
+
+// dq [tokens, width] fp32 -> bf16 rows of `pitch` values (width and pitch multiples of 8, 16-byte aligned)
+cudaError_t launch_attn_dq_store(const float* dq, void* out, long long tokens, int width, long long pitch, cudaStream_t s);
 
 // Prefill over expanded latent keys (mla_prefill.cu): maps with 64 x 128 boxes of the queries [2 terms x B, T, H * 128], the key and value terms
 // [B, S, Hk * 64] and the rotary keys [B, S, 64]; positions count from `base`.

@@ -33,10 +33,11 @@ constexpr int QDO_STAGES = 2;
 constexpr uint32_t BW_TMEM_COLS = 512;
 constexpr uint32_t COL_S = 0, COL_DP = 128, COL_DV = 256, COL_DK = 320, COL_DQ64 = 384;   // DQK = 128: dK spans 320..447, dQ aliases S
 
-// delta[b, h, t] = sum_d dO[t, h, d] * O[t, h, d]; eight lanes (16 bytes each) per (token, head), four heads per warp pass
+// delta[b, h, t] = sum_d dO[t, h, d] * O[t, h, d]; eight lanes (16 bytes each) per (token, head), four heads per warp pass.  The same pass
+// clears the row of dQ that the backward adds to (a fill of its own took 10 us of 16384 tokens' 16 heads, and a launch)
 __global__ void __launch_bounds__(256)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ d_out, const __nv_bfloat16* __restrict__ out, float* __restrict__ delta,
-                  long long tokens, int heads, int seq_len, long long do_stride, long long o_stride) {
+                  long long tokens, int heads, int seq_len, long long do_stride, long long o_stride, float* __restrict__ dq, int qk_dim) {
     const int lane = threadIdx.x & 31;
     const int sub = lane >> 3, li = lane & 7;
     const int groups = (heads + 3) / 4;
@@ -46,6 +47,8 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ d_out, const __nv_bfloat16* 
         const int h = static_cast<int>(idx - tok * groups) * 4 + sub;
         float s = 0.f;
         if (h < heads) {
+            float4* clear = reinterpret_cast<float4*>(dq + (tok * heads + h) * qk_dim);
+            for (int i = li; i < qk_dim / 4; i += 8) clear[i] = make_float4(0.f, 0.f, 0.f, 0.f);
             const uint4 ra = *reinterpret_cast<const uint4*>(d_out + tok * do_stride + h * HD + li * 8);
             const uint4 rb = *reinterpret_cast<const uint4*>(out + tok * o_stride + h * HD + li * 8);
             const __nv_bfloat162* pa = reinterpret_cast<const __nv_bfloat162*>(&ra);
@@ -60,6 +63,26 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ d_out, const __nv_bfloat16* 
         for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         if (li == 0 && h < heads) delta[((tok / seq_len) * heads + h) * seq_len + tok % seq_len] = s;
     }
+}
+
+// dQ [tokens, width] fp32 as bf16 rows `pitch` values apart (a slice of a packed gradient row): 32 bytes in, 16 out a thread.  Torch's copy
+// between these layouts took 41 us for 16384 x 1024, this 18.
+__global__ void __launch_bounds__(256)
+attn_dq_store_kernel(const float* __restrict__ dq, __nv_bfloat16* __restrict__ out, long long tokens, int width, long long pitch) {
+    const int per_row = width / 8;
+    const long long total = tokens * per_row;
+    for (long long i = blockIdx.x * 256LL + threadIdx.x; i < total; i += gridDim.x * 256LL) {
+        const long long tok = i / per_row;
+        const int col = static_cast<int>(i - tok * per_row) * 8;
+        const float4 a = *reinterpret_cast<const float4*>(dq + i * 8), b = *reinterpret_cast<const float4*>(dq + i * 8 + 4);
+        *reinterpret_cast<uint4*>(out + tok * pitch + col) = make_uint4(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w), pack_bf16x2(b.x, b.y), pack_bf16x2(b.z, b.w));
+    }
+}
+
+cudaError_t launch_attn_dq_store(const float* dq, void* out, long long tokens, int width, long long pitch, cudaStream_t s) {
+    const long long blocks = (tokens * (width / 8) + 255) / 256;
+    attn_dq_store_kernel<<<static_cast<int>(blocks < 4736 ? blocks : 4736), 256, 0, s>>>(dq, static_cast<__nv_bfloat16*>(out), tokens, width, pitch);
+    return cudaGetLastError();
 }
 
 __device__ __forceinline__ float tanh_approx_bwd(float x) {
@@ -395,7 +418,7 @@ cudaError_t launch_attn_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const 
     p.long_first = p.window > p.seq_len / 2 && ctas > 148;
     const long long tokens = static_cast<long long>(p.batch) * p.seq_len;
     attn_delta_kernel<<<1184, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(d_out), static_cast<const __nv_bfloat16*>(out), delta,
-                                                tokens, p.heads, p.seq_len, do_stride, o_stride);
+                                                tokens, p.heads, p.seq_len, do_stride, o_stride, p.dq_accum, p.qk_dim);
     const bool capped = p.softcap > 0.f;
     if (p.qk_dim == 128)
         return capped ? launch_bwd_variant<128, true>(tq, tk, tv, tdo, tdq, p, stream) : launch_bwd_variant<128, false>(tq, tk, tv, tdo, tdq, p, stream);

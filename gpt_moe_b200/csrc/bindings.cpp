@@ -70,6 +70,9 @@ CUtensorMap cached_map(const void* ptr, int elem_bytes, uint64_t cols, uint64_t 
     auto it = cache.find(key);
     if (it != cache.end()) return it->second;
     if (cache.size() > 8192) cache.clear();
+    // the encoder is a driver call and wants a current context, which a thread that has not launched anything yet (autograd's, on its first
+    // node) does not have
+    GM_CHECK(cudaSetDevice(at::cuda::current_device()) == cudaSuccess, "cudaSetDevice failed");
     CUtensorMap map;
     GM_CHECK(reinterpret_cast<uintptr_t>(ptr) % 16 == 0, "TMA base address must be 16-byte aligned");
     GM_CHECK(row_stride_bytes % 16 == 0 && (batch == 1 || batch_stride_bytes % 16 == 0), "TMA strides must be multiples of 16 bytes");
@@ -469,11 +472,12 @@ std::vector<torch::Tensor> attn_fwd(const torch::Tensor& q, const torch::Tensor&
 
 // Backward.  `unpipelined`: keep the call on the kernel that issues its products in program order (the other is checked against it).
 // q, k, v, out, d_out: [B,T,H(kv),64] bf16 views; lse [B,H,T].  dk, dv: [B,T,Hkv,64] bf16 views that are written
-// (they may be column slices of a packed gradient buffer).  Returns dq as fp32 [B,T,H,64].
+// (they may be column slices of a packed gradient buffer).  Returns dq as fp32 [B,T,H,64]; `dq_out`: a bf16 view of that shape
+// (contiguous heads, e.g. the first columns of the same buffer) that gets its values as well.
 torch::Tensor attn_bwd(const torch::Tensor& q, const torch::Tensor& k, const torch::Tensor& v, const torch::Tensor& out,
                        const torch::Tensor& d_out, const torch::Tensor& lse, torch::Tensor& dk, torch::Tensor& dv, int64_t window,
                        double scale, double softcap, const c10::optional<torch::Tensor>& doc_start, bool unpipelined,
-                       const c10::optional<torch::Tensor>& window_tensor) {
+                       const c10::optional<torch::Tensor>& window_tensor, const c10::optional<torch::Tensor>& dq_out) {
     c10::cuda::CUDAGuard guard(q.device());
     const int B = q.size(0), T = q.size(1), H = q.size(2), D = q.size(3), Hkv = k.size(2);
     GM_CHECK((D == 64 || D == 128) && k.size(3) == D && v.size(3) == 64 && T >= 1 && H % Hkv == 0,
@@ -492,7 +496,7 @@ torch::Tensor attn_bwd(const torch::Tensor& q, const torch::Tensor& k, const tor
     p.doc_start = doc_start_ptr(doc_start, static_cast<int64_t>(B) * T);
     p.lse = const_cast<float*>(lse.data_ptr<float>());
     auto delta = gm::out_empty({B, H, T}, lse.options());
-    auto dq = gm::out_zeros({B, T, H, D}, lse.options());
+    auto dq = gm::out_empty({B, T, H, D}, lse.options());
     p.delta = delta.data_ptr<float>();
     p.dq_accum = dq.data_ptr<float>();
     p.dk = dk.data_ptr(); p.dv = dv.data_ptr(); p.dv_head = static_cast<int>(head_pitch(dv)); p.dkv_stride = token_pitch(dk); p.dv_stride = token_pitch(dv);
@@ -505,6 +509,13 @@ torch::Tensor attn_bwd(const torch::Tensor& q, const torch::Tensor& k, const tor
                                         d_out.data_ptr(), out.data_ptr(), token_pitch(d_out), token_pitch(out), delta.data_ptr<float>(),
                                         current_stream());
     GM_CHECK(e == cudaSuccess, cudaGetErrorString(e));
+    if (dq_out.has_value()) {
+        const torch::Tensor& o = *dq_out;
+        GM_CHECK(o.is_cuda() && o.scalar_type() == torch::kBFloat16 && o.sizes() == q.sizes() && o.stride(3) == 1 && o.stride(2) == D && o.stride(1) % 8 == 0 &&
+                 o.stride(0) == T * o.stride(1) && reinterpret_cast<uintptr_t>(o.data_ptr()) % 16 == 0, "dq_out: bf16 view of q's shape, contiguous heads, aligned rows");
+        e = gm::launch_attn_dq_store(dq.data_ptr<float>(), o.data_ptr(), static_cast<long long>(B) * T, H * D, o.stride(1), current_stream());
+        GM_CHECK(e == cudaSuccess, cudaGetErrorString(e));
+    }
     return dq;
 }
 
@@ -549,6 +560,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           py::arg("doc_start") = py::none(), py::arg("quantize") = false, py::arg("single_tile") = false, py::arg("window_tensor") = py::none());
     m.def("attn_bwd", &attn_bwd, py::arg("q"), py::arg("k"), py::arg("v"), py::arg("out"), py::arg("d_out"), py::arg("lse"), py::arg("dk"),
           py::arg("dv"), py::arg("window"), py::arg("scale"), py::arg("softcap") = 0.0, py::arg("doc_start") = py::none(),
-          py::arg("unpipelined") = false, py::arg("window_tensor") = py::none());
+          py::arg("unpipelined") = false, py::arg("window_tensor") = py::none(), py::arg("dq_out") = py::none());
     gm::register_kernels(m);
 }

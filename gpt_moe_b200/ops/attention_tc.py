@@ -58,12 +58,9 @@ class _AttentionFn(torch.autograd.Function):
             dq32 = ext().attn_bwd(q, k, v, out, d_out, lse, dk, dv, window, scale, softcap, ctx.doc_start)
             return dq32.to(q.dtype), dk, dv, None, None, None, None
         # one packed gradient buffer [B, T, (H + 2 Hkv) * 64]: dk and dv are written in place by the kernel, dq is converted into it
-        packed = torch.empty((b, t, (h + 2 * hk) * d), dtype=q.dtype, device=q.device)
-        dk = packed[..., h * d: (h + hk) * d].unflatten(-1, (hk, d))
-        dv = packed[..., (h + hk) * d:].unflatten(-1, (hk, d))
-        dq32 = ext().attn_bwd(q, k, v, out, d_out, lse, dk, dv, window, scale, softcap, ctx.doc_start)
-        dq = packed[..., : h * d].unflatten(-1, (h, d))
-        dq.copy_(dq32)
+        packed = torch.empty((b, t, h + 2 * hk, d), dtype=q.dtype, device=q.device)
+        dq, dk, dv = packed[:, :, :h], packed[:, :, h: h + hk], packed[:, :, h + hk:]
+        ext().attn_bwd(q, k, v, out, d_out, lse, dk, dv, window, scale, softcap, ctx.doc_start, dq_out=dq)
         return dq, dk, dv, None, None, None, None
 
 
