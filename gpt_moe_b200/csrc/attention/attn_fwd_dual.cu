@@ -38,6 +38,9 @@ constexpr uint32_t DU_TMEM_COLS = 512;
 constexpr uint32_t DU_COL_S = 0, DU_COL_P = 256, DU_COL_O = 384;
 constexpr int DU_POLY_PER_8 = 2;                         // exponentials of every 8 evaluated as a polynomial on the FMA pipe (0 or an even number;
                                                          // 232 us with 2, 241 us with 0 on 16 x 2048 tokens, 12 heads, window 1024)
+constexpr int DU_TURN_TILES = 12;                        // from this many key tiles on the two query tiles take turns at their exponentials: started together
+                                                         // they stay in step, share the MUFU in the second pass and leave it idle in the rest
+                                                         // (16384 tokens 904 -> 816 us, 4 x 4096 270 -> 256; nine key tiles 199 -> 200, two 48 -> 53)
 constexpr float DU_RESCALE_STEP = 8.f;                   // log2 units the row maximum may outgrow its reference before O is rescaled
 
 // Capping and masking of 32 scores (columns kv0 .. kv0 + 31 of the key tile) in place.
@@ -109,10 +112,10 @@ __device__ __forceinline__ void dual_zero16(uint32_t p_addr) {
     tmem_st_32x32b_x16(p_addr, zeros);
 }
 
-template <bool CAP, class PreviousProduct>
+template <bool CAP, class PreviousProduct, class Turn>
 __device__ __forceinline__ void dual_softmax_tile(uint32_t s_addr, uint32_t p_addr, uint32_t o_addr, int kv0, int qpos, int warp_q0, int window,
                                                   bool edge_tile, float c, float step, float& m_ref, float& l, bool first, float cap_a, float cap_b,
-                                                  const PreviousProduct& previous_product) {
+                                                  const PreviousProduct& previous_product, const Turn& my_turn) {
     int cls[4] = {CHUNK_FULL, CHUNK_FULL, CHUNK_FULL, CHUNK_FULL};
     if (edge_tile) {
 #pragma unroll
@@ -161,6 +164,7 @@ __device__ __forceinline__ void dual_softmax_tile(uint32_t s_addr, uint32_t p_ad
     const uint64_t c2 = pack2(c, c), neg_base2 = pack2(-base, -base);
     uint64_t sum2[2] = {0ull, 0ull};                        // two packed pairs of partial row sums (bit pattern of 0.f, 0.f)
     uint32_t s2[32];
+    my_turn();
     tmem_ld_32x32b_x32(s_addr + 64, s2);
     if (cls[0] != CHUNK_EMPTY) dual_exp32(s0, p_addr, c2, neg_base2, sum2); else dual_zero16(p_addr);
     tmem_ld_wait();
@@ -185,7 +189,7 @@ __device__ __forceinline__ void dual_softmax_tile(uint32_t s_addr, uint32_t p_ad
     l += (t0 + t1) + (t2 + t3);
 }
 
-template <bool CAPPED>
+template <bool CAPPED, bool TURNS>
 __global__ void __launch_bounds__(DU_THREADS, 1)
 attn_fwd_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                      const __grid_constant__ CUtensorMap tmap_v, const AttnParams p) {
@@ -304,12 +308,18 @@ attn_fwd_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         // whenever the maximum grows (5 x 1000 tokens, window 256: 2.04e-3 instead of 2.10e-3)
         const bool lags = p.seq_len % (2 * DU_BM) == 0 && (p.window <= p.seq_len / 2 || p.seq_len <= 16 * DU_BM);
         const float step = lags ? DU_RESCALE_STEP : 0.f;
+        const int n_a = hi_a - lo_a + 1;                       // key tiles of A; B has as many or one more
+        const bool in_turn = TURNS && n_a >= DU_TURN_TILES;
+        if (in_turn && x == 1) asm volatile("bar.arrive 1, 256;" ::: "memory");
         float m_ref = -INFINITY, l = 0.f;
         for (int i = 0; i < n_x; ++i) {
             const int tile = lo_x + i;
             const int kv0 = tile * DU_BN;
             if (ok && !mbar_wait(&bar_s[x], i & 1)) { atomicExch(p.status, 218); ok = false; }
             tc_fence_after();
+            const auto my_turn = [&] {
+                if (in_turn && i < n_a) asm volatile("bar.sync %0, 256;" ::"r"(1 + x) : "memory");
+            };
             const auto previous_product = [&] {
                 if (i == 0) return;
                 if (ok && !mbar_wait(&bar_o[x], (i - 1) & 1)) { atomicExch(p.status, 219); ok = false; }
@@ -326,60 +336,59 @@ attn_fwd_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
             // tiles strictly inside the band need no mask; the diagonal tile and the tile at the window edge do
             const bool need_mask = (kv0 + DU_BN - 1 > q0x) || (q0x + DU_BM - 1 - kv0 > window);
             dual_softmax_tile<capped>(s_addr, p_addr, o_addr, kv0, qpos, q0x + quad * 32, window, need_mask, c, step, m_ref, l, i == 0, cap_a, cap_b,
-                                      previous_product);
+                                      previous_product, my_turn);
+            if (in_turn && (x == 0 || i + 1 < n_a)) asm volatile("bar.arrive %0, 256;" ::"r"(2 - x) : "memory");
             tmem_st_wait();
             tc_fence_before();
             mbar_arrive(&bar_p[x]);
         }
         if (ok && !mbar_wait(&bar_o[x], (n_x - 1) & 1)) { atomicExch(p.status, 220); ok = false; }
-        if (ok) {
-            tc_fence_after();
-            float o[DU_D];
+        tc_fence_after();
+        float o[DU_D];
 #pragma unroll
-            for (int hh = 0; hh < 2; ++hh) tmem_ld_32x32b_x32(o_addr + hh * 32, *reinterpret_cast<uint32_t(*)[32]>(&o[32 * hh]));
-            tmem_ld_wait();
-            if (qpos < p.seq_len) {                           // rows past the sequence end were computed on zeros
-                const float inv = 1.f / l;
-                const long long token = static_cast<long long>(row0) + qpos;
-                __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.out) + token * p.out_stride + head * DU_D;
+        for (int hh = 0; hh < 2; ++hh) tmem_ld_32x32b_x32(o_addr + hh * 32, *reinterpret_cast<uint32_t(*)[32]>(&o[32 * hh]));
+        tmem_ld_wait();
+        if (ok && qpos < p.seq_len) {                     // rows past the sequence end were computed on zeros
+            const float inv = 1.f / l;
+            const long long token = static_cast<long long>(row0) + qpos;
+            __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.out) + token * p.out_stride + head * DU_D;
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    uint4 w;
-                    w.x = pack_bf16x2(o[8 * q] * inv, o[8 * q + 1] * inv);
-                    w.y = pack_bf16x2(o[8 * q + 2] * inv, o[8 * q + 3] * inv);
-                    w.z = pack_bf16x2(o[8 * q + 4] * inv, o[8 * q + 5] * inv);
-                    w.w = pack_bf16x2(o[8 * q + 6] * inv, o[8 * q + 7] * inv);
-                    *reinterpret_cast<uint4*>(out + 8 * q) = w;
-                }
-                if (p.out_q != nullptr) {
-                    // the thread's 64 output columns are two MXFP8 blocks of the token-major row: quantise the bf16 values just stored
-                    // (reference: attention output quantised straight from its own layout, model/linear/fp8/custom/output_projection.py:16-49)
-                    const int width = p.heads * DU_D;
-#pragma unroll
-                    for (int blk = 0; blk < 2; ++blk) {
-                        float amax = 0.f;
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) { o[32 * blk + i] = round_bf16(o[32 * blk + i] * inv); amax = fmaxf(amax, fabsf(o[32 * blk + i])); }
-                        const uint32_t e8 = e8m0_from_amax(amax);
-                        const float qs = inv_scale_from_e8m0(e8);
-                        const int col = head * DU_D + 32 * blk;
-                        uint8_t* dst = p.out_q + token * width + col;
-                        const float* ob = o + 32 * blk;
-#pragma unroll
-                        for (int q = 0; q < 2; ++q) {
-                            uint4 w;
-                            w.x = pack_e4m3x4(ob[16 * q] * qs, ob[16 * q + 1] * qs, ob[16 * q + 2] * qs, ob[16 * q + 3] * qs);
-                            w.y = pack_e4m3x4(ob[16 * q + 4] * qs, ob[16 * q + 5] * qs, ob[16 * q + 6] * qs, ob[16 * q + 7] * qs);
-                            w.z = pack_e4m3x4(ob[16 * q + 8] * qs, ob[16 * q + 9] * qs, ob[16 * q + 10] * qs, ob[16 * q + 11] * qs);
-                            w.w = pack_e4m3x4(ob[16 * q + 12] * qs, ob[16 * q + 13] * qs, ob[16 * q + 14] * qs, ob[16 * q + 15] * qs);
-                            *reinterpret_cast<uint4*>(dst + 16 * q) = w;
-                        }
-                        p.out_sf[sf_offset(token, col >> 5, (width + 127) >> 7)] = static_cast<uint8_t>(e8);
-                    }
-                }
-                // natural-log LSE of the scaled scores, layout [batch, head, seq]; m_ref is the reference the sum l was taken against
-                p.lse[(static_cast<long long>(batch) * p.heads + head) * p.seq_len + qpos] = m_ref * 0.69314718056f + __logf(l);
+            for (int q = 0; q < 8; ++q) {
+                uint4 w;
+                w.x = pack_bf16x2(o[8 * q] * inv, o[8 * q + 1] * inv);
+                w.y = pack_bf16x2(o[8 * q + 2] * inv, o[8 * q + 3] * inv);
+                w.z = pack_bf16x2(o[8 * q + 4] * inv, o[8 * q + 5] * inv);
+                w.w = pack_bf16x2(o[8 * q + 6] * inv, o[8 * q + 7] * inv);
+                *reinterpret_cast<uint4*>(out + 8 * q) = w;
             }
+            if (p.out_q != nullptr) {
+                // the thread's 64 output columns are two MXFP8 blocks of the token-major row: quantise the bf16 values just stored
+                // (reference: attention output quantised straight from its own layout, model/linear/fp8/custom/output_projection.py:16-49)
+                const int width = p.heads * DU_D;
+#pragma unroll
+                for (int blk = 0; blk < 2; ++blk) {
+                    float amax = 0.f;
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) { o[32 * blk + i] = round_bf16(o[32 * blk + i] * inv); amax = fmaxf(amax, fabsf(o[32 * blk + i])); }
+                    const uint32_t e8 = e8m0_from_amax(amax);
+                    const float qs = inv_scale_from_e8m0(e8);
+                    const int col = head * DU_D + 32 * blk;
+                    uint8_t* dst = p.out_q + token * width + col;
+                    const float* ob = o + 32 * blk;
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        uint4 w;
+                        w.x = pack_e4m3x4(ob[16 * q] * qs, ob[16 * q + 1] * qs, ob[16 * q + 2] * qs, ob[16 * q + 3] * qs);
+                        w.y = pack_e4m3x4(ob[16 * q + 4] * qs, ob[16 * q + 5] * qs, ob[16 * q + 6] * qs, ob[16 * q + 7] * qs);
+                        w.z = pack_e4m3x4(ob[16 * q + 8] * qs, ob[16 * q + 9] * qs, ob[16 * q + 10] * qs, ob[16 * q + 11] * qs);
+                        w.w = pack_e4m3x4(ob[16 * q + 12] * qs, ob[16 * q + 13] * qs, ob[16 * q + 14] * qs, ob[16 * q + 15] * qs);
+                        *reinterpret_cast<uint4*>(dst + 16 * q) = w;
+                    }
+                    p.out_sf[sf_offset(token, col >> 5, (width + 127) >> 7)] = static_cast<uint8_t>(e8);
+                }
+            }
+            // natural-log LSE of the scaled scores, layout [batch, head, seq]; m_ref is the reference the sum l was taken against
+            p.lse[(static_cast<long long>(batch) * p.heads + head) * p.seq_len + qpos] = m_ref * 0.69314718056f + __logf(l);
         }
     }
 
@@ -404,10 +413,10 @@ bool attn_fwd_dual_supported(const AttnParams& p) {
     return p.qk_dim == 64 && p.doc_start == nullptr && (windowed ? tiles % 2 == 0 || tiles >= 9 : tiles > 1);
 }
 
-template <bool CAPPED>
+template <bool CAPPED, bool TURNS>
 static cudaError_t launch_dual_variant(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnParams& p, cudaStream_t stream) {
     constexpr int smem = (2 + 2 * DU_STAGES) * DU_TILE_BYTES + 1024 + 256;
-    auto kernel = attn_fwd_dual_kernel<CAPPED>;
+    auto kernel = attn_fwd_dual_kernel<CAPPED, TURNS>;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -420,7 +429,9 @@ static cudaError_t launch_dual_variant(const CUtensorMap& tq, const CUtensorMap&
 }
 
 cudaError_t launch_attn_fwd_dual(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnParams& p, cudaStream_t stream) {
-    return p.softcap > 0.f ? launch_dual_variant<true>(tq, tk, tv, p, stream) : launch_dual_variant<false>(tq, tk, tv, p, stream);
+    const bool turns = (p.window < p.seq_len ? p.window : p.seq_len) >= DU_TURN_TILES * DU_BN;
+    if (p.softcap > 0.f) return turns ? launch_dual_variant<true, true>(tq, tk, tv, p, stream) : launch_dual_variant<true, false>(tq, tk, tv, p, stream);
+    return turns ? launch_dual_variant<false, true>(tq, tk, tv, p, stream) : launch_dual_variant<false, false>(tq, tk, tv, p, stream);
 }
 
 }  // namespace gm
