@@ -212,20 +212,21 @@ void gemm_run(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d, 
     const CUtensorMap& ta = operand_map(a, a_mn, 128, in_type);
     const CUtensorMap& tb = operand_map(b, b_mn, 128, in_type);
     const int eb = p.out_fp32 ? 4 : 2;
-    const bool slabs = parts.defined();
-    const CUtensorMap& td = cached_map(slabs ? parts.data_ptr() : d.data_ptr(), eb, p.N, p.M, slabs ? p.split_k : d.dim() == 3 ? d.size(0) : 1, p.ldd * eb,
-                                       slabs || d.dim() == 3 ? p.d_batch_stride * eb : 0, 128 / eb, 128, 128);
     // C of the output's shape comes through TMA; any other (broadcast over the batch or over rows, beside an fp32 output) is read by the threads
     CUtensorMap tc, tmirror;
     const bool tma_c = p.C != nullptr && mode == gm::GEMM_DENSE && !p.out_fp32 && !a_mn && p.K > 0 && c->dim() == d.dim() && c->sizes() == d.sizes() &&
                        p.ldc > 0 && (p.batch == 1 || p.c_batch_stride > 0);
+    const bool slabs = parts.defined();
+    const CUtensorMap& td = cached_map(slabs ? parts.data_ptr() : d.data_ptr(), eb, p.N, p.M, slabs ? p.split_k : d.dim() == 3 ? d.size(0) : 1, p.ldd * eb,
+                                       slabs || d.dim() == 3 ? p.d_batch_stride * eb : 0, 128 / eb, tma_c ? 128 : 32, 128);        // a warp stores its 32 rows, beside a C through TMA the CTA its 128
     GM_CHECK((!p.in_f16 || p.C == nullptr || tma_c) && (diag == 0.0 || (tma_c && symmetric)), "GEMM: an fp16 C or a diagonal term needs C in the layout of the output");
     p.diag = static_cast<float>(diag);
     if (tma_c) {
         tc = cached_map(p.C, 2, p.N, p.M, p.batch, p.ldc * 2, d.dim() == 3 ? p.c_batch_stride * 2 : 0, 64, 128, 128);
-        if (p.symmetric) tmirror = cached_map(p.D, 2, p.N, p.M, p.batch, p.ldd * 2, d.dim() == 3 ? p.d_batch_stride * 2 : 0, 64, 64, 128);
     }
-    cudaError_t e = gm::launch_gemm_bf16(ta, tb, td, tma_c ? &tc : nullptr, tma_c && p.symmetric ? &tmirror : nullptr, p, a_mn, b_mn, sm_count(),
+    // the transposed blocks of a symmetric result: 64 rows of 128 bytes beside a C through TMA, else 64 rows of a warp's 32 columns
+    if (p.symmetric) tmirror = cached_map(p.D, 2, p.N, p.M, p.batch, p.ldd * 2, d.dim() == 3 ? p.d_batch_stride * 2 : 0, tma_c ? 64 : 32, 64, tma_c ? 128 : 0);
+    cudaError_t e = gm::launch_gemm_bf16(ta, tb, td, tma_c ? &tc : nullptr, p.symmetric ? &tmirror : nullptr, p, a_mn, b_mn, sm_count(),
                                          current_stream());
     GM_CHECK(e == cudaSuccess, cudaGetErrorString(e));
     if (slabs) {

@@ -43,7 +43,8 @@ bool make_tensor_map(CUtensorMap* out, const void* base, int elem_bytes, uint64_
                      int swizzle_bytes);
 
 // `tc`: map of C in the layout of D (64 x 128 box) when the epilogue may fetch it by TMA (dense, bf16 output, K > 0, A K-major), else null;
-// `tmirror`: with it, for symmetric results, the map of D with a 64-row box.
+// `tmirror`: for symmetric results, the map of D for the transposed blocks: boxes of 64 rows, with `tc` 64 columns (128-byte swizzle), else 32
+// (no swizzle).  `td`: boxes of 128 bytes, with `tc` 128 rows, else 32.
 cudaError_t launch_gemm_bf16(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const CUtensorMap* tc, const CUtensorMap* tmirror,
                              const GemmParams& p, bool a_mn, bool b_mn, int sms, cudaStream_t stream);
 
