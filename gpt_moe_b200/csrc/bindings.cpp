@@ -210,12 +210,12 @@ void gemm_run(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d, 
         }
     }
     const CUtensorMap& ta = operand_map(a, a_mn, 128, in_type);
-    const CUtensorMap& tb = operand_map(b, b_mn, 128, in_type);
     const int eb = p.out_fp32 ? 4 : 2;
     // C of the output's shape comes through TMA; any other (broadcast over the batch or over rows, beside an fp32 output) is read by the threads
     CUtensorMap tc, tmirror;
     const bool tma_c = p.C != nullptr && mode == gm::GEMM_DENSE && !p.out_fp32 && !a_mn && p.K > 0 && c->dim() == d.dim() && c->sizes() == d.sizes() &&
                        p.ldc > 0 && (p.batch == 1 || p.c_batch_stride > 0);
+    const CUtensorMap& tb = operand_map(b, b_mn, gm::gemm_bf16_tile_width(p, a_mn, tma_c, sm_count()) / 2, in_type);
     const bool slabs = parts.defined();
     const CUtensorMap& td = cached_map(slabs ? parts.data_ptr() : d.data_ptr(), eb, p.N, p.M, slabs ? p.split_k : d.dim() == 3 ? d.size(0) : 1, p.ldd * eb,
                                        slabs || d.dim() == 3 ? p.d_batch_stride * eb : 0, 128 / eb, tma_c ? 128 : 32, 128);        // a warp stores its 32 rows, beside a C through TMA the CTA its 128

@@ -35,9 +35,13 @@
 
 namespace gm {
 
-constexpr int BM = 128, BN = 256, BK = 64, STAGES = 5;
-constexpr int BN_HALF = BN / 2;
-constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN_HALF * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
+constexpr int BM = 128, BK = 64;
+// columns of a pair's tile and the ring that goes with them: 256, or 128 where those leave half of the CTA pairs without a tile
+template <int WIDTH>
+struct Tiling {
+    static constexpr int BN = WIDTH, BN_HALF = BN / 2, STAGES = WIDTH == 256 ? 5 : 6;
+    static constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN_HALF * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
+};
 constexpr int GEMM_THREADS = 320;           // warp 0 TMA, warp 1 MMA, warps 2-9 epilogue
 constexpr int GROUP_M = 4;               // in pair tiles (256 rows each)
 constexpr uint32_t TMEM_COLS = 512;
@@ -76,6 +80,7 @@ struct TileCoord {
 
 // Work is enumerated in PAIR tiles (two vertically adjacent 128-row tiles, one per CTA of the pair); `m_tiles` counts
 // the 128-row tiles rounded up to an even number.
+template <int BN>
 __device__ __forceinline__ int total_tiles(const GemmParams& p, int& m_tiles, int& n_tiles) {
     n_tiles = (p.N + BN - 1) / BN;
     if (p.mode == GEMM_GROUPED_M) {
@@ -87,6 +92,7 @@ __device__ __forceinline__ int total_tiles(const GemmParams& p, int& m_tiles, in
     return m_tiles / 2 * n_tiles * p.batch * p.split_k;
 }
 
+template <int BN>
 __device__ __forceinline__ TileCoord tile_coord(const GemmParams& p, int tile, int cta_rank, int m_tiles, int n_tiles) {
     TileCoord t;
     int split = 0;
@@ -146,11 +152,13 @@ __device__ __forceinline__ TileCoord tile_coord(const GemmParams& p, int tile, i
     return t;
 }
 
-template <bool A_MN, bool B_MN, bool TMA_C>
+template <bool A_MN, bool B_MN, bool TMA_C, int WIDTH>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                  const __grid_constant__ CUtensorMap tmap_d, const __grid_constant__ CUtensorMap tmap_c,
                  const __grid_constant__ CUtensorMap tmap_mirror, const GemmParams p) {
+    using Tile = Tiling<WIDTH>;
+    constexpr int BN = Tile::BN, BN_HALF = Tile::BN_HALF, STAGES = Tile::STAGES, A_BYTES = Tile::A_BYTES, STAGE_BYTES = Tile::STAGE_BYTES;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* staging = smem + STAGES * STAGE_BYTES;
@@ -181,7 +189,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     const uint32_t tmem_base = uniform(*tmem_slot);
 
     int m_tiles, n_tiles;
-    const int tiles = uniform(total_tiles(p, m_tiles, n_tiles));
+    const int tiles = uniform(total_tiles<BN>(p, m_tiles, n_tiles));
     const int first_tile = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
     bool ok = true;
 
@@ -189,7 +197,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         const uint32_t on = elect_one();
         int s = 0; uint32_t ph = 0;
         for (int tile = first_tile; tile < tiles && ok; tile += tile_step) {
-            const TileCoord t = tile_coord(p, tile, cta_rank, m_tiles, n_tiles);
+            const TileCoord t = tile_coord<BN>(p, tile, cta_rank, m_tiles, n_tiles);
             const int k_blocks = uniform(t.k_blocks), k_begin = uniform(t.k_begin), bz = uniform(t.bz);
             for (int kb = 0; kb < k_blocks; ++kb) {
                 if (!warp_wait(&empty[s], ph ^ 1)) { atomicExch(p.status, 101); ok = false; break; }
@@ -221,7 +229,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             constexpr uint32_t a_kstep = A_MN ? 2048 : 32, b_kstep = B_MN ? 2048 : 32;
             int s = 0; uint32_t ph = 0; int acc = 0; uint32_t acc_ph = 0;
             for (int tile = first_tile; tile < tiles && ok; tile += tile_step) {
-                const int k_blocks = uniform(tile_coord(p, tile, cta_rank, m_tiles, n_tiles).k_blocks);
+                const int k_blocks = uniform(tile_coord<BN>(p, tile, cta_rank, m_tiles, n_tiles).k_blocks);
                 if (k_blocks == 0) continue;
                 if (!warp_wait(&acc_empty[acc], acc_ph ^ 1)) { atomicExch(p.status, 102); ok = false; break; }
                 tc_fence_after();
@@ -261,9 +269,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             mbar_expect_tx(&c_full[k & 1], SLAB_BYTES);
             tma_load_3d(staging + (slab & 3) * SLAB_BYTES, &tmap_c, &c_full[k & 1], t.n0 + round * 64, t.m0, t.dz);
         };
-        if (leader && first_tile < tiles) fetch_c(tile_coord(p, first_tile, cta_rank, m_tiles, n_tiles), 0, 0, 0);
+        if (leader && first_tile < tiles) fetch_c(tile_coord<BN>(p, first_tile, cta_rank, m_tiles, n_tiles), 0, 0, 0);
         for (int tile = first_tile; tile < tiles; tile += tile_step) {
-            const TileCoord t = tile_coord(p, tile, cta_rank, m_tiles, n_tiles);
+            const TileCoord t = tile_coord<BN>(p, tile, cta_rank, m_tiles, n_tiles);
             const int rounds = min(BN / 64, (t.n_limit - t.n0 + 63) / 64);
             float alpha = p.alpha, beta = p.beta;
             if (p.batch_sumsq != nullptr) {                   // an operand is an un-normalised Muon update: scale the result instead
@@ -280,7 +288,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                     asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
                     const uint32_t next = use + (mirror ? 2 : 1);
                     if (round + 1 < rounds) fetch_c(t, round + 1, next, fetched + 1);
-                    else if (tile + tile_step < tiles) fetch_c(tile_coord(p, tile + tile_step, cta_rank, m_tiles, n_tiles), 0, next, fetched + 1);
+                    else if (tile + tile_step < tiles) fetch_c(tile_coord<BN>(p, tile + tile_step, cta_rank, m_tiles, n_tiles), 0, next, fetched + 1);
                 }
                 uint32_t r[32];
                 tmem_ld_32x32b_x32(tmem_base + acc * BN + (round * 2 + half) * 32 + (static_cast<uint32_t>(quad * 32) << 16), r);
@@ -383,7 +391,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         };
         for (int tile = first_tile; tile < tiles; tile += tile_step) {
-            const TileCoord t = tile_coord(p, tile, cta_rank, m_tiles, n_tiles);
+            const TileCoord t = tile_coord<BN>(p, tile, cta_rank, m_tiles, n_tiles);
             const bool have_acc = t.k_blocks != 0;
             if (!have_acc && !(t.store_zeros && !p.accumulate)) continue;      // nothing to add, nothing to clear
             const int row0 = t.m0 + quad * 32;
@@ -399,15 +407,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                 tc_fence_after();
             }
 #pragma unroll
-            for (int sl = 0; sl < 2; ++sl) {
-                const int col = t.n0 + half * 128 + sl * 64;
+            for (int sl = 0; sl < BN / 128; ++sl) {
+                const int col = t.n0 + half * BN_HALF + sl * 64;
                 uint32_t r[2][32];
                 if (have_acc) {
 #pragma unroll
                     for (int j = 0; j < 2; ++j)
-                        tmem_ld_32x32b_x32(tmem_base + acc * BN + half * 128 + sl * 64 + j * 32 + (static_cast<uint32_t>(quad * 32) << 16), r[j]);
+                        tmem_ld_32x32b_x32(tmem_base + acc * BN + half * BN_HALF + sl * 64 + j * 32 + (static_cast<uint32_t>(quad * 32) << 16), r[j]);
                     tmem_ld_wait();
-                    if (sl == 1) {                                              // accumulator fully read: release it early
+                    if (sl == BN / 128 - 1) {                                   // accumulator fully read: release it early
                         tc_fence_before();
                         __syncwarp();
                         if (lane == 0) mbar_arrive_cluster(&acc_empty[acc], 0);
@@ -524,12 +532,11 @@ void launch_split_sum(const float* parts, int splits, long long rows, int cols, 
     split_sum_kernel<<<static_cast<int>(blocks < 8192 ? blocks : 8192), 256, 0, s>>>(parts, splits, rows, cols, ldp, static_cast<__nv_bfloat16*>(d), ldd);
 }
 
-constexpr int GEMM_SMEM_BYTES = STAGES * STAGE_BYTES + 2 * STAGING_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/;
-
-template <bool A_MN, bool B_MN, bool TMA_C>
+template <bool A_MN, bool B_MN, bool TMA_C, int WIDTH>
 static cudaError_t launch_variant(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const CUtensorMap& tc, const CUtensorMap& tm,
                                   const GemmParams& p, int sms, cudaStream_t stream) {
-    auto kernel = gemm_bf16_kernel<A_MN, B_MN, TMA_C>;
+    constexpr int GEMM_SMEM_BYTES = Tiling<WIDTH>::STAGES * Tiling<WIDTH>::STAGE_BYTES + 2 * STAGING_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/;
+    auto kernel = gemm_bf16_kernel<A_MN, B_MN, TMA_C, WIDTH>;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM_BYTES);
@@ -551,13 +558,24 @@ static cudaError_t launch_variant(const CUtensorMap& ta, const CUtensorMap& tb, 
     return cudaLaunchKernelEx(&cfg, kernel, ta, tb, td, tc, tm, p);
 }
 
+// Half the width where even so every tile has a CTA pair of its own: the chain of loads, products and read-out that such a launch consists of is
+// then half as long.  us with cold caches, 256 / 128 columns: 360 x 2304 x 768 11.6 / 9.0, 1024 x 2048 x 1024 13.3 / 10.3, 1024 x 1024 x 1024 12.7 / 9.6,
+// 2048 rows of eight experts x 768 x 3072 26.8 / 22.3.  Rows of a grouped product are the most there can be, p.M.
+int gemm_bf16_tile_width(const GemmParams& p, bool a_mn, bool c_by_tma, int sms) {
+    const long long halves = static_cast<long long>((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + 127) / 128) * (p.mode == GEMM_GROUPED_M ? 1 : p.batch);
+    const bool plain = !a_mn && !c_by_tma && !p.symmetric && !p.out_fp32 && p.split_k == 1 && p.mode != GEMM_GROUPED_K;
+    return plain && p.N > 128 && halves <= sms / 2 ? 128 : 256;
+}
+
 cudaError_t launch_gemm_bf16(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const CUtensorMap* tc, const CUtensorMap* tmirror,
                              const GemmParams& p, bool a_mn, bool b_mn, int sms, cudaStream_t stream) {
     const CUtensorMap& tm = tmirror != nullptr ? *tmirror : td;
+    if (gemm_bf16_tile_width(p, a_mn, tc != nullptr, sms) == 128)
+        return b_mn ? launch_variant<false, true, false, 128>(ta, tb, td, td, tm, p, sms, stream) : launch_variant<false, false, false, 128>(ta, tb, td, td, tm, p, sms, stream);
     if (tc != nullptr && !a_mn)
-        return b_mn ? launch_variant<false, true, true>(ta, tb, td, *tc, tm, p, sms, stream) : launch_variant<false, false, true>(ta, tb, td, *tc, tm, p, sms, stream);
-    if (a_mn) return b_mn ? launch_variant<true, true, false>(ta, tb, td, td, tm, p, sms, stream) : launch_variant<true, false, false>(ta, tb, td, td, tm, p, sms, stream);
-    return b_mn ? launch_variant<false, true, false>(ta, tb, td, td, tm, p, sms, stream) : launch_variant<false, false, false>(ta, tb, td, td, tm, p, sms, stream);
+        return b_mn ? launch_variant<false, true, true, 256>(ta, tb, td, *tc, tm, p, sms, stream) : launch_variant<false, false, true, 256>(ta, tb, td, *tc, tm, p, sms, stream);
+    if (a_mn) return b_mn ? launch_variant<true, true, false, 256>(ta, tb, td, td, tm, p, sms, stream) : launch_variant<true, false, false, 256>(ta, tb, td, td, tm, p, sms, stream);
+    return b_mn ? launch_variant<false, true, false, 256>(ta, tb, td, td, tm, p, sms, stream) : launch_variant<false, false, false, 256>(ta, tb, td, td, tm, p, sms, stream);
 }
 
 }  // namespace gm
