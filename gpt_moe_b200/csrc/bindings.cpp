@@ -13,6 +13,7 @@
 #include "gemm/gemm.h"
 #include "attention/attn.h"
 #include "kernels.h"
+#include "kernels_decl.h"
 
 namespace {
 
@@ -264,6 +265,16 @@ torch::Tensor polar_express(torch::Tensor x, const c10::optional<torch::Tensor>&
     GM_CHECK(m <= k && !coeffs.empty(), "polar_express wants wide matrices and at least one step");
     c10::cuda::CUDAGuard guard(x.device());
     const int steps = static_cast<int>(coeffs.size());
+    if (gm::polar_small_supported(m, k, steps) && n > 0 && reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0) {
+        GM_CHECK(!sumsq.has_value() || (sumsq->is_cuda() && sumsq->scalar_type() == torch::kFloat32 && sumsq->is_contiguous() && sumsq->numel() == n) ,
+                 "polar_express: one fp32 sum of squares per matrix");
+        std::vector<float> flat;
+        for (const auto& c : coeffs) flat.insert(flat.end(), c.begin(), c.end());
+        const cudaError_t e = gm::launch_polar_small(x.data_ptr(), sumsq.has_value() ? sumsq->data_ptr<float>() : nullptr, static_cast<int>(n), static_cast<int>(m),
+                                                     static_cast<int>(k), flat.data(), steps, current_stream());
+        GM_CHECK(e == cudaSuccess, cudaGetErrorString(e));
+        return x;
+    }
     const int64_t mt = (m + 255) / 256, kt = (k + 255) / 256;
     const bool runs = m >= 256 && ((k >= 3 * m && n * mt * kt >= sm_count()) || (k >= 2 * m && n * mt * (mt + 1) / 2 >= 3 * sm_count()));
     const auto half = x.options().dtype(torch::kHalf);

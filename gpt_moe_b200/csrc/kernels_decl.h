@@ -99,6 +99,10 @@ void launch_cast_bf16(const float* src, void* dst, long long n, cudaStream_t s);
 
 void launch_muon_normalize(void* packed, const float* sumsq, int n_mats, long long per_matrix, cudaStream_t s);
 
+// fused/polar_small.cu: Polar Express in place on n matrices [m, k] bf16 of few rows; coeffs: three per step (host memory)
+bool polar_small_supported(long long m, long long k, int steps);
+cudaError_t launch_polar_small(void* x, const float* sumsq, int n, int m, int k, const float* coeffs, int steps, cudaStream_t s);
+
 // comm/fused_comm.cu
 bool launch_rs_muon_prepare(const float* const* grads, float* const* bufs, void* packed, float* sumsq, int n_mats, int rows, int cols,
                             long long g_stride, long long b_stride, float momentum, int nesterov, int transpose,

@@ -21,8 +21,9 @@ def _error(x, exact):
 
 
 # (batch, rows, columns): runs with whole tiles, with ragged ones, at the least height, just too few tiles for runs, just too narrow for them
-# (single steps with the fp16 Gram matrices), one row of pieces
-@pytest.mark.parametrize("shape", [(16, 768, 1536), (12, 520, 2056), (64, 256, 704), (8, 256, 768), (16, 768, 1528), (3, 8, 768)])
+# (single steps with the fp16 Gram matrices); few rows (one launch): every height, as wide as high, more matrices than SMs
+@pytest.mark.parametrize("shape", [(16, 768, 1536), (12, 520, 2056), (64, 256, 704), (8, 256, 768), (16, 768, 1528), (3, 8, 768),
+                                   (4, 32, 1536), (2, 24, 264), (150, 16, 16)])
 @pytest.mark.parametrize("spectrum", ["gaussian", "decaying"])
 def test_polar_express_is_no_further_from_64_bits_than_single_steps_in_bf16(shape, spectrum):
     from gpt_moe_b200.ops import cuda_ops
