@@ -621,7 +621,8 @@ enum TrunkTensor { W_QKV, W_OUT, ROPE_COS, ROPE_SIN, Q_SCALE, K_SCALE, ATTN_BETA
 
 // Consecutive blocks of a model without gradients as one call: per block the QKV product, rotation and QK-norm, attention, output projection, residual
 // update and norm, the routed experts, residual update and norm, 14 launches.  x [rows, hidden] fp32 is the residual stream, h its first norm (bf16);
-// returns the stream and its norm behind the last block.  Every layer works in the same buffers: a call per branch with tensors of its own cost 111 us of host time a layer here
+// returns the stream and its norm behind the last block.  Pad rows of the experts' buffers hold whatever lay there: their products are rows
+// that nothing reads.  Every layer works in the same buffers: a call per branch with tensors of its own cost 111 us of host time a layer here
 // (and as much again in Python around it), which is more than the kernels of a few hundred rows take.
 std::vector<Tensor> trunk(const Tensor& x, const Tensor& h0, const std::vector<std::vector<OptTensor>>& layers, const std::vector<int64_t>& windows,
              const std::vector<std::array<double, 2>>& norm_eps, int64_t batch, int64_t heads, int64_t kv_heads, int64_t top_k, double qk_eps, double qk_min,
@@ -691,9 +692,9 @@ std::vector<Tensor> trunk(const Tensor& x, const Tensor& h0, const std::vector<s
         launch_route(top, static_cast<int>(slots), static_cast<int>(experts), hist.data_ptr<int>(), hist.data_ptr<int>() + chunks * experts, counts.data_ptr<int>(),
                      seg.data_ptr<int>(), tiles.data_ptr<int>(), meta.data_ptr<int>(), dest.data_ptr<int>(), src.data_ptr<int>(), s);
         launch_gather_rows(h.data_ptr(), src.data_ptr<int>(), meta.data_ptr<int>(), packed.data_ptr(), nullptr, nullptr, static_cast<int>(hidden),
-                           static_cast<int>(top_k), static_cast<int>(cap), static_cast<int>(rows), s);
+                           static_cast<int>(top_k), static_cast<int>(cap), static_cast<int>(rows), s, true);
         gemm_by_expert(packed, *t[W_UP], pre, tiles, meta);
-        launch_activation_fwd(pre.data_ptr(), act.data_ptr(), meta.data_ptr<int>(), nullptr, nullptr, static_cast<int>(cap), static_cast<int>(inner), kind, s);
+        launch_activation_fwd(pre.data_ptr(), act.data_ptr(), meta.data_ptr<int>(), nullptr, nullptr, static_cast<int>(cap), static_cast<int>(inner), kind, s, src.data_ptr<int>());
         gemm_by_expert(act, *t[W_DOWN], packed, tiles, meta);
         launch_combine_fwd(packed.data_ptr(), dest.data_ptr<int>(), gates.data_ptr<float>(), branch.data_ptr(), static_cast<int>(rows), static_cast<int>(hidden),
                            static_cast<int>(top_k), static_cast<int>(cap), s);

@@ -205,17 +205,18 @@ __device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
 // own (reference: gather + activation + quantise in one kernel, model/linear/fp8/custom/grouped.py:15-84).  A thread holds 8
 // consecutive elements, so a 32-element block is 4 adjacent lanes.
 
-// packed[row] = hidden[src_of_row[row] / k] (zeros for pad rows); one warp per row, 16-byte vectors
+// packed[row] = hidden[src_of_row[row] / k] (pad rows: zeros, or with `skip_pads` left as they are); one warp per row, 16-byte vectors
 __global__ void __launch_bounds__(256)
 gather_rows_kernel(const __nv_bfloat16* __restrict__ hidden, const int* __restrict__ src_of_row, const int* __restrict__ meta,
                    __nv_bfloat16* __restrict__ packed, uint8_t* __restrict__ q, uint8_t* __restrict__ sf, int d, int top_k, int cap_rows,
-                   int tokens) {
+                   int tokens, int skip_pads) {
     const int lane = threadIdx.x & 31;
     const int total = min(meta[1], cap_rows);
     const int vecs = d / 8, k_blocks = (d + 127) >> 7;
     for (int row = blockIdx.x * 8 + (threadIdx.x >> 5); row < total; row += gridDim.x * 8) {
         int src = src_of_row[row];
         if (!GM_IN_BOUNDS(src < 0 || src / top_k < tokens, 902)) src = -1;                    // checked build: treated as a pad row
+        if (src < 0 && skip_pads) continue;                                                    // warp-uniform
         uint4* out = reinterpret_cast<uint4*>(packed + static_cast<long long>(row) * d);
         const uint4* in = reinterpret_cast<const uint4*>(hidden + static_cast<long long>(src < 0 ? 0 : src / top_k) * d);
         for (int base = 0; base < vecs; base += 32) {                  // warp-uniform trip count: the quantiser shuffles
@@ -238,10 +239,10 @@ gather_rows_kernel(const __nv_bfloat16* __restrict__ hidden, const int* __restri
 }
 
 void launch_gather_rows(const void* hidden, const int* src_of_row, const int* meta, void* packed, void* q, void* sf, int d, int top_k,
-                        int cap_rows, int tokens, cudaStream_t s) {
+                        int cap_rows, int tokens, cudaStream_t s, bool skip_pads) {
     gather_rows_kernel<<<1184, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(hidden), src_of_row, meta,
                                             static_cast<__nv_bfloat16*>(packed), static_cast<uint8_t*>(q), static_cast<uint8_t*>(sf), d, top_k,
-                                            cap_rows, tokens);
+                                            cap_rows, tokens, skip_pads ? 1 : 0);
 }
 
 // out[t] = sum_k gates[t,k] * y[dest[t*k+k']]   (fp32 accumulation, bf16 result); one warp per token
@@ -369,6 +370,8 @@ __device__ __forceinline__ void emit_quantized8(const uint4& stored, bool active
     }
 }
 
+// src_of_row (forward, optional): rows without a slot are left as they are - where nothing reads pad rows, as in a pass without gradients.  360
+// tokens of eight experts fill 360 of 2048 rows: a pass over all of them took 15.3 us at 4096 hidden columns, this one 6.3 us.
 // IDX: type of the flat piece index.  Both kernels move 6 to 12 bytes per element and were short of issue slots, not of bandwidth: a 64-bit
 // division per piece cost more instructions than some of the rest (34816 rows, h = 3072, with the MXFP8 copy: forward 160 -> 151 us, backward
 // 246 -> 240 us).  The sigmoid keeps its IEEE division: the approximate one takes 125 and 217 us, and loses bits (and everything of a gate
@@ -376,7 +379,7 @@ __device__ __forceinline__ void emit_quantized8(const uint4& stored, bool active
 template <bool SWIGLU, typename IDX>
 __global__ void __launch_bounds__(256)
 activation_fwd_kernel(const __nv_bfloat16* __restrict__ pre, __nv_bfloat16* __restrict__ act, const int* __restrict__ meta,
-                      uint8_t* __restrict__ q, uint8_t* __restrict__ sf, int rows, int h, int kind) {
+                      uint8_t* __restrict__ q, uint8_t* __restrict__ sf, int rows, int h, int kind, const int* __restrict__ src_of_row) {
     const int total = meta ? min(meta[1], rows) : rows;
     const IDX per_row = h / 8;
     const IDX n = static_cast<IDX>(total) * per_row;
@@ -390,7 +393,7 @@ activation_fwd_kernel(const __nv_bfloat16* __restrict__ pre, __nv_bfloat16* __re
         const int c = active ? static_cast<int>(i - row * per_row) * 8 : 0;
         const long long r = static_cast<long long>(row);
         uint4 stored = make_uint4(0, 0, 0, 0);
-        if (active) {
+        if (active && (src_of_row == nullptr || src_of_row[row] >= 0)) {
             float a[8], o[8];
             unpack8(*reinterpret_cast<const uint4*>(pre + r * in_w + c), a);
             if (SWIGLU) {
@@ -455,10 +458,11 @@ activation_bwd_kernel(const __nv_bfloat16* __restrict__ dact, const __nv_bfloat1
 }
 
 template <bool SWIGLU>
-static void launch_act_fwd(const __nv_bfloat16* pre, __nv_bfloat16* act, const int* meta, uint8_t* q, uint8_t* sf, int rows, int h, int kind, cudaStream_t s) {
+static void launch_act_fwd(const __nv_bfloat16* pre, __nv_bfloat16* act, const int* meta, uint8_t* q, uint8_t* sf, int rows, int h, int kind,
+                           const int* src_of_row, cudaStream_t s) {
     // 32-bit indices while the grid's last step past the end stays below 2^32
-    if (static_cast<long long>(rows) * (h / 8) < (1LL << 31)) activation_fwd_kernel<SWIGLU, uint32_t><<<2368, 256, 0, s>>>(pre, act, meta, q, sf, rows, h, kind);
-    else activation_fwd_kernel<SWIGLU, long long><<<2368, 256, 0, s>>>(pre, act, meta, q, sf, rows, h, kind);
+    if (static_cast<long long>(rows) * (h / 8) < (1LL << 31)) activation_fwd_kernel<SWIGLU, uint32_t><<<2368, 256, 0, s>>>(pre, act, meta, q, sf, rows, h, kind, src_of_row);
+    else activation_fwd_kernel<SWIGLU, long long><<<2368, 256, 0, s>>>(pre, act, meta, q, sf, rows, h, kind, src_of_row);
 }
 template <bool SWIGLU>
 static void launch_act_bwd(const __nv_bfloat16* dact, const __nv_bfloat16* pre, __nv_bfloat16* dpre, const int* meta, uint8_t* q, uint8_t* sf, int rows, int h,
@@ -467,9 +471,10 @@ static void launch_act_bwd(const __nv_bfloat16* dact, const __nv_bfloat16* pre, 
     else activation_bwd_kernel<SWIGLU, long long><<<2368, 256, 0, s>>>(dact, pre, dpre, meta, q, sf, rows, h, kind);
 }
 
-void launch_activation_fwd(const void* pre, void* act, const int* meta, void* q, void* sf, int rows, int h, int kind, cudaStream_t s) {
+void launch_activation_fwd(const void* pre, void* act, const int* meta, void* q, void* sf, int rows, int h, int kind, cudaStream_t s,
+                           const int* src_of_row) {
     auto* f = kind == 4 ? launch_act_fwd<true> : launch_act_fwd<false>;
-    f(static_cast<const __nv_bfloat16*>(pre), static_cast<__nv_bfloat16*>(act), meta, static_cast<uint8_t*>(q), static_cast<uint8_t*>(sf), rows, h, kind, s);
+    f(static_cast<const __nv_bfloat16*>(pre), static_cast<__nv_bfloat16*>(act), meta, static_cast<uint8_t*>(q), static_cast<uint8_t*>(sf), rows, h, kind, src_of_row, s);
 }
 void launch_activation_bwd(const void* dact, const void* pre, void* dpre, const int* meta, void* q, void* sf, int rows, int h, int kind,
                            cudaStream_t s) {

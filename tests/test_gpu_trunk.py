@@ -62,6 +62,22 @@ def test_trunk_has_the_bits_of_the_blocks_own_calls(case):
     cuda_ops.check_status()
 
 
+@pytest.mark.parametrize("tokens", [1, 37, 130, 400])
+def test_trunk_does_not_read_rows_that_hold_no_slot(tokens):
+    """Pad rows of the experts' buffers are left as they are; here every byte the allocator has to give is part of a NaN."""
+    model, gc = _model(moe_top_k=2)
+    ids = torch.randint(0, gc.vocab_size, (1, tokens), device="cuda")
+    with torch.no_grad():
+        _apart(model)
+        want = model(ids)
+        del model._plain_forward
+        torch.cuda.empty_cache()
+        held = [torch.full((size,), 255, dtype=torch.uint8, device="cuda") for size in (1 << 10, 1 << 16, 1 << 19, 1 << 20, 12 << 20, 20 << 20, 40 << 20) for _ in range(12)]
+        del held
+        assert torch.equal(model(ids), want)
+    cuda_ops.check_status()
+
+
 def test_trunk_steps_aside_for_whoever_looks_at_a_block():
     model, gc = _model()
     ids = torch.randint(0, gc.vocab_size, (2, 33), device="cuda")
