@@ -17,6 +17,15 @@ namespace gm {
 
 constexpr long long kWaitBudgetCycles = 2000000000LL;   // ~1 s at B200 clocks
 
+// ---- a kernel that starts while the one before it on its stream drains ----------------------------
+// `grid_wait` (every thread of a kernel launched with the programmatic-serialization attribute, before it reads or writes global memory): the
+// kernel before has ended and its results are visible; no effect in other launches.  `grid_trigger`: this block no longer
+// holds back the start of such a successor, which begins when every block has said so or ended - so no block that has yet to
+// start can be kept from an SM by one that waits for it.  The wait is for the whole kernel either way.  A waiting kernel reads through
+// pointers that are NOT `const __restrict__`: the compiler may move loads through those across the wait.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- bounds-checked build ------------------------------------------------------------------------
 // With -DGM_CHECK_BOUNDS=1 (the `_C_checked` build, GM_CHECK_BOUNDS=1 in the environment) every data-dependent index that a
 // kernel takes from a tensor (an expert id, a routed row, a target class) is tested before it is used:

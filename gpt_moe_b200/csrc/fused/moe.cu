@@ -210,6 +210,7 @@ __global__ void __launch_bounds__(256)
 gather_rows_kernel(const __nv_bfloat16* __restrict__ hidden, const int* __restrict__ src_of_row, const int* __restrict__ meta,
                    __nv_bfloat16* __restrict__ packed, uint8_t* __restrict__ q, uint8_t* __restrict__ sf, int d, int top_k, int cap_rows,
                    int tokens, int skip_pads) {
+    grid_trigger();
     const int lane = threadIdx.x & 31;
     const int total = min(meta[1], cap_rows);
     const int vecs = d / 8, k_blocks = (d + 127) >> 7;
@@ -380,6 +381,7 @@ template <bool SWIGLU, typename IDX>
 __global__ void __launch_bounds__(256)
 activation_fwd_kernel(const __nv_bfloat16* __restrict__ pre, __nv_bfloat16* __restrict__ act, const int* __restrict__ meta,
                       uint8_t* __restrict__ q, uint8_t* __restrict__ sf, int rows, int h, int kind, const int* __restrict__ src_of_row) {
+    grid_trigger();
     const int total = meta ? min(meta[1], rows) : rows;
     const IDX per_row = h / 8;
     const IDX n = static_cast<IDX>(total) * per_row;

@@ -47,6 +47,7 @@ rmsnorm_fwd_kernel(const TX* __restrict__ x, const __nv_bfloat16* __restrict__ b
                    const float* __restrict__ beta, TX* __restrict__ x_out, const float* __restrict__ w,
                    __nv_bfloat16* __restrict__ y, float* __restrict__ rstd, uint8_t* __restrict__ yq, uint8_t* __restrict__ ysf,
                    int rows, int d, float eps) {
+    grid_trigger();
     const int lane = threadIdx.x & 31;
     const int row = blockIdx.x * NORM_WARPS + (threadIdx.x >> 5);
     if (row >= rows) return;                       // whole warps leave together: a warp owns one row
