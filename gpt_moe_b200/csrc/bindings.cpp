@@ -175,6 +175,8 @@ void gemm_run(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d, 
         GM_CHECK(reinterpret_cast<uintptr_t>(p.C) % 16 == 0 && p.c_batch_stride % 8 == 0, "C must lie on 16-byte boundaries");      // read 16 bytes at a time
     }
     GM_CHECK(p.ldd % 8 == 0 && (p.C == nullptr || p.ldc % 8 == 0), "output row pitch must be a multiple of 8 elements");
+    // here, not only in the tensor map: a shared contraction's map describes its slabs, and the sum stores to D by itself
+    GM_CHECK(reinterpret_cast<uintptr_t>(p.D) % 16 == 0, "the GEMM output must lie on a 16-byte boundary");
     if (symmetric) {      // the caller vouches that alpha * A B^T + beta * C is symmetric; only the upper triangle of tiles is computed
         GM_CHECK(mode == gm::GEMM_DENSE && p.M == p.N && !p.out_fp32 && !accumulate, "symmetric GEMM: dense, square, bf16 output");
         p.symmetric = 1;

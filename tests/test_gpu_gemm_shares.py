@@ -25,3 +25,16 @@ def test_shared_contraction(m, n, k, b_mn):
     c.gemm_bf16(a, b, again, False, b_mn, 0.25)
     assert torch.equal(again, wide[:m, 8: 8 + n])                  # the shares are summed in the same order every time
     cuda_ops.check_status()
+
+
+@pytest.mark.parametrize("m,n,k", [(64, 264, 8192), (64, 264, 64)])          # shared by several pairs, and whole
+@pytest.mark.parametrize("offset", [1, 2, 4])
+def test_an_output_off_the_16_byte_grid_is_refused(m, n, k, offset):
+    """Before any launch: the sum over the shares stores 8 bytes at a time."""
+    from gpt_moe_b200.ops import cuda_ops
+    a, b = torch.zeros(m, k, device="cuda").bfloat16(), torch.zeros(n, k, device="cuda").bfloat16()
+    wide = torch.full((m, n + 8), 5.0, device="cuda", dtype=torch.bfloat16)
+    with pytest.raises(RuntimeError, match="16-byte"):
+        cuda_ops.ext().gemm_bf16(a, b, wide[:, offset: offset + n])
+    assert (wide == 5).all()
+    cuda_ops.check_status()
