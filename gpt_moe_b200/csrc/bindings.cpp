@@ -257,9 +257,15 @@ void gemm_bf16(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d,
 // Rounding noise of A grows by a^2 a step against the smallest singular values.  Error against 64 bits (2-norm; matrices 768 x 3072:
 // Gaussian / rank 8 plus noise / singular values 1/i / exp(-12 i / m)): single steps in bf16 1.06e-2 / 5.8e-2 / 3.6e-2 / 9.3e-2, runs of two and
 // three 0.48e-2 / 4.8e-2 / 3.4e-2 / 6.8e-2; one run of five reaches 0.1 to 20 and is not taken, nor are runs of matrices lower than 256.
-// That takes fp16 for A and Q (bounded: |A| <= 1.3, |Q| <= 8.2, a run's product <= 39) and the order Q (A Q), whose error in the directions
+// That takes fp16 for A and Q and the order Q (A Q), whose error in the directions
 // that A hardly has is of second order; and the product of a run's Q is computed in full: mirrored, errors were three to five times as large,
 // since rounded Q commute only nearly.  The first Q X stays bf16 x bf16, as x arrives with any scale; X is fp16 after it.
+// fp16 has 2^-24 as its smallest step, so every fp16 matrix is held times a power of two that the next product's alpha takes off: singular values
+// up to 1 (of x as it comes; the polynomials diverge from 1.03 on) give |A| <= 3.97, |Q| <= 8.16, a run's product <= 33.0 and |X| <= 1.99 in every step, and
+// the powers leave a factor of two to 65504.  Without them rows of 1e-5 of the others lost a tenth to a quarter of their result (error of these
+// rows 0.22; bf16 steps 0.010, with the powers 0.0040: 16 of 768 x 1536), rows of 1e-6 all of it, and so did matrices of norm 1e-11 (0.23, 0.005, 0.004).
+// Rows of 1e-8 (0.007 to 0.009 in emulation) and norms of 1e-15 are farther than bf16 steps are: their results lie at 1e-5 of a row's usual size and less.
+constexpr double kPolarGram = 8192.0, kPolarFactor = 4096.0, kPolarRun = 1024.0, kPolarX = 16384.0;
 torch::Tensor polar_express(torch::Tensor x, const c10::optional<torch::Tensor>& sumsq, const std::vector<std::vector<double>>& coeffs) {
     GM_CHECK(x.is_cuda() && x.dim() == 3 && x.scalar_type() == torch::kBFloat16 && x.is_contiguous(), "polar_express wants contiguous bf16 matrices [n, m, k]");
     for (const auto& c : coeffs) GM_CHECK(c.size() == 3, "polar_express: three coefficients a step");
@@ -283,18 +289,20 @@ torch::Tensor polar_express(torch::Tensor x, const c10::optional<torch::Tensor>&
     torch::Tensor small[4];
     for (int i = 0; i < (runs ? 4 : 2); ++i) small[i] = gm::out_empty({n, m, m}, half);
     torch::Tensor y = gm::out_empty({n, m, k}, half);
-    const auto product = [&](const torch::Tensor& a, const torch::Tensor& b, torch::Tensor d) {        // a and b symmetric: a b^T = a b
-        gemm_run(a, b, d, false, false, 1.0, 0.0, c10::nullopt, false, gm::GEMM_DENSE, c10::nullopt, c10::nullopt, c10::nullopt, true, c10::nullopt, 0, false, true);
+    const auto product = [&](const torch::Tensor& a, const torch::Tensor& b, torch::Tensor d) {        // a and b symmetric: a b^T = a b; A times a Q
+        gemm_run(a, b, d, false, false, 1.0 / kPolarFactor, 0.0, c10::nullopt, false, gm::GEMM_DENSE, c10::nullopt, c10::nullopt, c10::nullopt, true, c10::nullopt, 0, false, true);
     };
     torch::Tensor in = x;
+    double in_scale = 1.0;                                                     // what X is held times
     for (int first = 0; first < steps;) {
         const int count = !runs ? 1 : first == 0 ? std::min(2, steps) : std::min(3, steps - first);
         const bool raw = first == 0 && sumsq.has_value();                      // not normalised yet: the epilogues do it
         const auto type = in.scalar_type();                                    // of the factor that meets X
         const torch::Tensor& gram = small[0];
-        gemm_run(in, in, small[0], false, false, 1.0, 0.0, c10::nullopt, false, gm::GEMM_DENSE, c10::nullopt, c10::nullopt, c10::nullopt, true,
+        gemm_run(in, in, small[0], false, false, kPolarGram / (in_scale * in_scale), 0.0, c10::nullopt, false, gm::GEMM_DENSE, c10::nullopt, c10::nullopt, c10::nullopt, true,
                  raw ? sumsq : c10::nullopt, raw ? 2 : 0, false, true);
         int q = 1, total = 1, spare = 2;                                       // buffers of the step's Q, of the run's product, and a free one
+        double total_scale = kPolarFactor;
         for (int j = 0; j < count; ++j) {
             if (j > 0) {
                 product(gram, small[q], small[spare]);
@@ -304,24 +312,27 @@ torch::Tensor polar_express(torch::Tensor x, const c10::optional<torch::Tensor>&
             const int next = j == 0 ? q : spare;
             torch::Tensor poly = small[next];
             if (count == 1) poly = poly.view(type);
-            gemm_run(gram, gram, poly, false, false, c[2], c[1], gram, false, gm::GEMM_DENSE, c10::nullopt, c10::nullopt, c10::nullopt, true, c10::nullopt, 0, false,
-                     true, c[0]);
+            gemm_run(gram, gram, poly, false, false, c[2] * kPolarFactor / (kPolarGram * kPolarGram), c[1] * kPolarFactor / kPolarGram, gram, false, gm::GEMM_DENSE, c10::nullopt, c10::nullopt, c10::nullopt, true, c10::nullopt, 0, false,
+                     true, c[0] * kPolarFactor);
             if (j > 0) {
                 const int to = q == total ? 3 : q;                             // the last Q is not needed any more
                 torch::Tensor both = j == count - 1 ? small[to].view(type) : small[to];
-                gemm_run(poly, small[total], both, false, true, 1.0, 0.0, c10::nullopt, false, gm::GEMM_DENSE, c10::nullopt, c10::nullopt, c10::nullopt, false,
+                gemm_run(poly, small[total], both, false, true, kPolarRun / (kPolarFactor * total_scale), 0.0, c10::nullopt, false, gm::GEMM_DENSE, c10::nullopt, c10::nullopt, c10::nullopt, false,
                          c10::nullopt, 0, false, true);
                 spare = total;
                 total = to;
+                total_scale = kPolarRun;
                 q = next;
             }
         }
         const bool done = first + count == steps;
         torch::Tensor out = in.data_ptr() == y.data_ptr() ? x : y;
         out = out.view(done ? torch::kBFloat16 : torch::kHalf);
-        gemm_run(small[total].view(type), in, out, false, true, 1.0, 0.0, c10::nullopt, false, gm::GEMM_DENSE, c10::nullopt, c10::nullopt, c10::nullopt, false,
+        const double out_scale = done ? 1.0 : kPolarX;
+        gemm_run(small[total].view(type), in, out, false, true, out_scale / (total_scale * in_scale), 0.0, c10::nullopt, false, gm::GEMM_DENSE, c10::nullopt, c10::nullopt, c10::nullopt, false,
                  raw ? sumsq : c10::nullopt, raw ? 1 : 0, false, true);
         in = out;
+        in_scale = out_scale;
         first += count;
     }
     return in;

@@ -44,3 +44,37 @@ def test_polar_express_is_no_further_from_64_bits_than_single_steps_in_bf16(shap
     normalised = (raw.double() / (raw.double().norm(dim=(-2, -1), keepdim=True) * 1.02 + 1e-6)).bfloat16()
     assert _error(cuda_ops.polar_express_bf16(normalised.clone()), _exact(normalised * 1.0)) < 1.1 * plain + 2 ** -6
     cuda_ops.check_status()
+
+
+# runs of steps, single steps, and the kernel for few rows
+@pytest.mark.parametrize("shape", [(16, 768, 1536), (8, 256, 768), (3, 512, 512), (4, 32, 768)])
+@pytest.mark.parametrize("weak", [1e-4, 1e-5, 1e-6, 1e-7])
+def test_rows_far_below_the_others_keep_their_direction(shape, weak):
+    """A 2-norm over the matrix does not see them: the error is taken over the weak rows alone."""
+    from gpt_moe_b200.ops import cuda_ops
+    torch.manual_seed(10)
+    n, m, k = shape
+    g = torch.randn(n, m, k, device="cuda")
+    rows = torch.arange(m, device="cuda") % 8 == 3
+    g[:, rows] *= weak
+    raw = g.bfloat16()
+    exact = _exact(raw)
+    got = cuda_ops.polar_express_bf16(raw.clone(), raw.float().pow(2).sum(dim=(-2, -1)))
+    plain = ref.polar_express(raw, dtype=torch.bfloat16)
+    for part in (rows, ~rows):            # bounds as above
+        assert _error(got[:, part], exact[:, part]) < 1.1 * _error(plain[:, part], exact[:, part]) + 2 ** -8
+    cuda_ops.check_status()
+
+
+@pytest.mark.parametrize("shape", [(16, 768, 1536), (3, 512, 512), (4, 32, 768)])
+@pytest.mark.parametrize("norm", [1e-9, 1e-11, 1e-13])
+def test_matrices_that_are_nearly_zero_keep_their_direction(shape, norm):
+    """The momentum of an expert that has seen no token for long: 1 / (1.02 norm + 1e-6) no longer brings its norm to one."""
+    from gpt_moe_b200.ops import cuda_ops
+    torch.manual_seed(11)
+    g = torch.randn(shape, device="cuda")
+    raw = (g * (norm / g.norm(dim=(-2, -1), keepdim=True))).bfloat16()
+    exact = _exact(raw)
+    got = cuda_ops.polar_express_bf16(raw.clone(), raw.float().pow(2).sum(dim=(-2, -1)))
+    assert _error(got, exact) < 1.1 * _error(ref.polar_express(raw, dtype=torch.bfloat16), exact) + 2 ** -8
+    cuda_ops.check_status()
