@@ -246,7 +246,8 @@ void gemm_bf16(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d,
 }
 
 // ---- Polar Express ------------------------------------------------------------------------------------
-// Five steps X <- (a I + b A + c A^2) X, A = X X^T, on a batch of wide bf16 matrices x [n, m, k], m <= k; the result is bf16, and x is scratch.
+// Five steps X <- (a I + b A + c A^2) X, A = X X^T, on a batch of bf16 matrices x [n, m, k], wide ones (m <= k) as
+// a rule; the result is bf16, and a contiguous x is scratch.
 // The polynomials of consecutive steps commute, so a run of steps is carried out on the small m x m side: with Q = a I + b A + c A^2
 // the next Gram matrix is Q A Q, and the product of the run's Q goes to X once.  A run costs one X X^T and one Q X whatever its length,
 // where every step paid for both.  Runs of two and three steps are 18 products, 14 of them small, single steps 15 with 5 small ones.
@@ -267,13 +268,15 @@ void gemm_bf16(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d,
 // Rows of 1e-8 (0.007 to 0.009 in emulation) and norms of 1e-15 are farther than bf16 steps are: their results lie at 1e-5 of a row's usual size and less.
 constexpr double kPolarGram = 8192.0, kPolarFactor = 4096.0, kPolarRun = 1024.0, kPolarX = 16384.0;
 torch::Tensor polar_express(torch::Tensor x, const c10::optional<torch::Tensor>& sumsq, const std::vector<std::vector<double>>& coeffs) {
-    GM_CHECK(x.is_cuda() && x.dim() == 3 && x.scalar_type() == torch::kBFloat16 && x.is_contiguous(), "polar_express wants contiguous bf16 matrices [n, m, k]");
+    GM_CHECK(x.is_cuda() && x.dim() == 3 && x.scalar_type() == torch::kBFloat16 && x.stride(2) == 1 && x.stride(1) % 8 == 0 && (x.size(0) <= 1 || x.stride(0) % 8 == 0) &&
+             reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0, "polar_express wants bf16 matrices [n, m, k] of contiguous rows on 16-byte boundaries");
+    if (!x.is_contiguous()) x = x.contiguous();                               // a batch or row pitch of its own
     for (const auto& c : coeffs) GM_CHECK(c.size() == 3, "polar_express: three coefficients a step");
     const int64_t n = x.size(0), m = x.size(1), k = x.size(2);
-    GM_CHECK(m <= k && !coeffs.empty(), "polar_express wants wide matrices and at least one step");
+    GM_CHECK(!coeffs.empty(), "polar_express wants at least one step");
     c10::cuda::CUDAGuard guard(x.device());
     const int steps = static_cast<int>(coeffs.size());
-    if (gm::polar_small_supported(m, k, steps) && n > 0 && reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0) {
+    if (gm::polar_small_supported(m, k, steps) && n > 0) {
         GM_CHECK(!sumsq.has_value() || (sumsq->is_cuda() && sumsq->scalar_type() == torch::kFloat32 && sumsq->is_contiguous() && sumsq->numel() == n) ,
                  "polar_express: one fp32 sum of squares per matrix");
         std::vector<float> flat;

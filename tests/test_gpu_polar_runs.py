@@ -78,3 +78,19 @@ def test_matrices_that_are_nearly_zero_keep_their_direction(shape, norm):
     got = cuda_ops.polar_express_bf16(raw.clone(), raw.float().pow(2).sum(dim=(-2, -1)))
     assert _error(got, exact) < 1.1 * _error(ref.polar_express(raw, dtype=torch.bfloat16), exact) + 2 ** -8
     cuda_ops.check_status()
+
+
+# runs, single steps, few rows in one launch, and more rows than columns
+@pytest.mark.parametrize("shape", [(16, 768, 1536), (3, 512, 520), (4, 16, 264), (2, 264, 136)])
+def test_matrices_with_a_pitch_of_their_own(shape):
+    from gpt_moe_b200.ops import cuda_ops
+    torch.manual_seed(12)
+    n, m, k = shape
+    wide = torch.randn(n, m + 2, k + 24, device="cuda").bfloat16()
+    x = wide[:, 1: m + 1, 8: k + 8]
+    sumsq = x.float().pow(2).sum(dim=(-2, -1))
+    assert torch.equal(cuda_ops.polar_express_bf16(x, sumsq), cuda_ops.polar_express_bf16(x.contiguous(), sumsq))
+    exact = _exact(x)
+    plain = _error(ref.polar_express(x, dtype=torch.bfloat16), exact)
+    assert _error(cuda_ops.polar_express_bf16(x, sumsq), exact) < 1.1 * plain + 2 ** -8
+    cuda_ops.check_status()
