@@ -400,12 +400,13 @@ attn_fwd_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
 }
 
 bool attn_fwd_dual_supported(const AttnParams& p) {
-    // us, this kernel / the single-tile one: 16 x 2048 tokens, window 1024 195 / 248, 16384 tokens 865 / 978, 4 x 4096 251 / 293, 2 x 3000 86 / 97,
-    // 64 x 184 48 / 64, 8 x 1100 58 / 60, 1 x 1024 25 / 24, 3 x 300 17 / 16, 8 x 45 8.6 / 7.1.  Of an odd number of tiles the last CTA idles by half, which a short
-    // window does not repay below nine tiles (16 x 1152, window 256 84 / 91).
+    // us, this kernel / the single-tile one (12 heads unless said otherwise): 16 x 2048 tokens, window 1024 205 / 248, 16384 tokens, 16 heads 815 / 978, 4 x 4096,
+    // 16 heads 251 / 293, 64 x 129 51 / 66, 8 x 500 25 / 30, 16 x 700 57 / 69, 16 x 1000 86 / 100.  Of an odd number of tiles the last CTA idles by half: with three
+    // that is a quarter of the work (64 x 300 109 / 103, 16 x 384 36 / 33, 8 x 300 25 / 23, equal at 1 x and 3 x 300), with five no more (16 x 600 55 / 57, 8 x 640 33 / 35,
+    // 4 x 600, 16 heads 26 / 27), 16 x 896 84 / 84, 16 x 1152 114 / 117, 8 x 1408 79 / 84.  A short window does not repay it below nine tiles (16 x 1152, window 256 80 / 96).
     const int tiles = (p.seq_len + DU_BM - 1) / DU_BM;
     const bool windowed = p.window <= p.seq_len / 2;
-    return p.qk_dim == 64 && p.doc_start == nullptr && (windowed ? tiles % 2 == 0 || tiles >= 9 : tiles > 1);
+    return p.qk_dim == 64 && p.doc_start == nullptr && (tiles % 2 == 0 || tiles >= (windowed ? 9 : 5));
 }
 
 template <bool CAPPED, bool TURNS>
