@@ -241,14 +241,15 @@ attn_bwd_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         const int quad = warp & 3;                       // TMEM lanes 32 quad .. + 31: query rows of the dQ tile
         const int r = quad * 32 + lane, sw = lane & 7;
         uint8_t* mine = stg + quad * (BP_STG_BYTES / 4);
-        // statistics of query row r of iteration `jt`, [batch, head, seq].  Rows past the sequence end are zeros; a huge
-        // log-sum-exp makes their probabilities 0
-        const float per_scale = 1.f / p.scale;
+        // statistics of query row r of iteration `jt`, [batch, head, seq].  Rows past the sequence end are zeros; a huge log-sum-exp makes
+        // their probabilities 0 - over the scale a constant, as 1e30 over a scale of 1e-12 would be infinite and the second of its terms a NaN
+        const float per_scale = 1.f / p.scale, never = copysignf(1e38f, -p.scale);
         float lse = 1e30f, delta = 0.f;
+        bool live = false;
         int first_key = 0, need_mask = 0;
         auto fetch_stats = [&](int jt) {
             const int head = kv_head * p.group + jt / n_q, q0 = (kv_tile + jt % n_q) * BP_TILE, qpos = q0 + r;
-            const bool live = qpos < p.seq_len;
+            live = qpos < p.seq_len;
             const long long stat = (static_cast<long long>(batch) * p.heads + head) * p.seq_len + qpos;
             lse = live ? p.lse[stat] : 1e30f;
             delta = live ? p.delta[stat] : 0.f;
@@ -264,7 +265,7 @@ attn_bwd_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         auto put_stats = [&](int jt) {
             const int st = jt % BP_STAGES;
             if (CAPPED) reinterpret_cast<float*>(aug_lse + st * BP_AUG_BYTES)[r] = lse * 1.4426950408889634f;
-            else reinterpret_cast<uint4*>(aug_lse + st * BP_AUG_BYTES)[r] = bp_terms(-lse * per_scale);
+            else reinterpret_cast<uint4*>(aug_lse + st * BP_AUG_BYTES)[r] = bp_terms(live ? -lse * per_scale : never);
             reinterpret_cast<uint4*>(aug_delta + st * BP_AUG_BYTES)[r] = bp_terms(-delta);
             int* mask = reinterpret_cast<int*>(masks + st * BP_MASK_BYTES);
             mask[r] = first_key;

@@ -110,3 +110,20 @@ def test_three_tiles_without_a_window_take_the_single_tile_kernel(t):
     out, lse = cuda_ops.ext().attn_fwd(q, k, v, t, 0.125)
     single, single_lse = cuda_ops.ext().attn_fwd(q, k, v, t, 0.125, single_tile=True)
     assert torch.equal(out, single) and torch.equal(lse, single_lse)
+
+
+@pytest.mark.parametrize("t", [200, 256])
+@pytest.mark.parametrize("scale", [1e-12, 1e-6, 4.0])
+def test_gradients_at_any_scale(t, scale):
+    """Rows past the end of the last tile have no probabilities, however small the scale that their statistics are divided by."""
+    torch.manual_seed(11)
+    q, k, v = (torch.randn(2, t, n, 64, device="cuda").bfloat16().requires_grad_() for n in (4, 2, 2))
+    g = torch.randn(2, t, 4, 64, device="cuda").bfloat16()
+    out = attention_cuda.attention(q, k, v, scale=scale)
+    grads = torch.autograd.grad(out, (q, k, v), g)
+    want_in = [x.detach().double().requires_grad_() for x in (q, k, v)]
+    want = ref.attention(*want_in, causal=True, scale=scale)
+    assert rel(out, want) < 6e-3
+    for got, exp in zip(grads, torch.autograd.grad(want, want_in, g.double())):
+        assert rel(got, exp) < 1e-2
+    cuda_ops.check_status()
