@@ -640,7 +640,8 @@ std::vector<Tensor> trunk(const Tensor& x, const Tensor& h0, const std::vector<s
         GM_CHECK(t.size() == TRUNK_TENSORS, "trunk: tensors of a layer");
         for (int i : {W_QKV, W_OUT, W_ROUTER, W_UP, W_DOWN}) {
             GM_CHECK(t[i].has_value(), "trunk: a weight is missing");
-            check_bf16(*t[i], "weight");
+            if (i != W_OUT && i != W_ROUTER) check_bf16(*t[i], "weight");      // these two may be parameters as they are, whose rows may have a pitch
+            GM_CHECK(t[i]->is_cuda() && t[i]->scalar_type() == torch::kBFloat16, "trunk: bf16 weights");
         }
         for (int i : {ATTN_BETA, MLP_BETA}) GM_CHECK(t[i].has_value() && t[i]->numel() == 1, "trunk: a scale of each branch");
         for (int i : {ATTN_NORM, NEXT_NORM}) GM_CHECK(t[i].has_value() && t[i]->numel() == hidden, "trunk: norm weights");

@@ -249,7 +249,7 @@ class GPT(nn.Module):
         conditions are theirs (SelfAttention._fused_rope_attention, MoE._forward_plain, cuda_ops.residual_rms_norm)."""
         from ..ops import cuda_ops
         from ..ops.attention_cuda import _window_int
-        if type(block) is not Block:
+        if type(block) is not Block or "forward_prenormed" in block.__dict__:
             return None
         parts, t, d = block._modules, x.shape[1], x.shape[2]
         attn, mlp = parts["attn"], parts["mlp"]
@@ -265,11 +265,12 @@ class GPT(nn.Module):
         mlps = [table[str(e)]._modules for e in range(experts)]
         ups, downs = [m["up_proj"] for m in mlps], [m["down_proj"] for m in mlps]
         for m in (out_proj, router, ups[0], downs[0]):
-            if type(m) is not Linear or m._parameters.get("bias") is not None or m.precision != "default":
+            # (a bias that is no plain parameter is not in the table at all)
+            if type(m) is not Linear or m._parameters.get("bias", m) is not None or m.precision != "default":
                 return None
         norm = parts["ln_2"]
         (alpha_a, beta_a), (alpha_m, beta_m) = block._scales("attn"), block._scales("mlp")
-        if (q_proj.precision != "default" or q_proj._parameters.get("bias") is not None or not cuda_ops.unhooked(out_proj, router)
+        if (q_proj.precision != "default" or q_proj.bias is not None or not cuda_ops.unhooked(out_proj, router)
                 or not (isinstance(norm, nn.RMSNorm) and isinstance(next_norm, nn.RMSNorm)) or alpha_a is not None or alpha_m is not None
                 or beta_a is None or beta_m is None):
             return None
@@ -280,7 +281,8 @@ class GPT(nn.Module):
         rotary, scales, fp32 = proj.get("rotary"), attn._parameters, cuda_ops.as_fp32
         use_norm = attn.use_qk_norm
         tensors = [
-            cuda_ops.bf16_weight((q_proj._parameters["weight"], proj["k_proj"]._parameters["weight"], proj["v_proj"]._parameters["weight"])),
+            # as attributes: these three may be pruned or parametrised, their weights then being no plain parameters
+            cuda_ops.bf16_weight((q_proj.weight, proj["k_proj"].weight, proj["v_proj"].weight)),
             cuda_ops.bf16_weight((out_proj._parameters["weight"],)),
             None if rotary is None else rotary._buffers["cos_cached"], None if rotary is None else rotary._buffers["sin_cached"],
             fp32(scales["q_scale"]) if use_norm else None, fp32(scales["k_scale"]) if use_norm else None, fp32(beta_a), fp32(norms[0]),

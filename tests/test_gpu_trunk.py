@@ -1,6 +1,8 @@
 """All blocks of a forward pass without gradients as one native call (`trunk`): the bits of the blocks' own calls, and only where they apply."""
 import pytest
 import torch
+import torch.nn.utils.parametrize
+import torch.nn.utils.prune
 
 from gpt_moe_b200.config import get_preset
 from gpt_moe_b200.models.gpt import GPT
@@ -102,4 +104,52 @@ def test_trunk_steps_aside_for_whoever_looks_at_a_block():
         changed = model(ids)
         _apart(model)
         assert not torch.equal(changed, want) and torch.equal(changed, model(ids))
+    cuda_ops.check_status()
+
+
+class _Twice(torch.nn.Module):
+    def forward(self, w):
+        return 2 * w
+
+
+def _parametrised_weight(block):
+    torch.nn.utils.parametrize.register_parametrization(block.attn.k_proj, "weight", _Twice())
+
+
+def _pruned_weight(block):
+    torch.nn.utils.prune.random_unstructured(block.attn.q_proj, "weight", 0.5)
+
+
+def _parametrised_bias(block):
+    block.attn.q_proj.register_parameter("bias", torch.nn.Parameter(torch.randn(block.attn.attn_dim, device="cuda")))
+    torch.nn.utils.parametrize.register_parametrization(block.attn.q_proj, "bias", _Twice())
+
+
+def _rows_with_a_pitch(block):
+    for module in (block.attn.out_proj, block.mlp.router):
+        rows, cols = module.weight.shape
+        wide = torch.zeros(rows, cols + 8, device="cuda", dtype=torch.bfloat16)
+        wide[:, :cols] = module.weight.detach()
+        module.weight = torch.nn.Parameter(wide[:, :cols])
+
+
+def _own_step(block):
+    inner = block.forward_prenormed
+    block.forward_prenormed = lambda x, h, *rest: inner(x, 2 * h, *rest)
+
+
+# change of the middle block: layers that stay in the native call
+@pytest.mark.parametrize("change,served", [(_parametrised_weight, 3), (_pruned_weight, 3), (_parametrised_bias, 2), (_rows_with_a_pitch, 3), (_own_step, 2)])
+def test_trunk_takes_modules_as_the_blocks_own_calls_do(change, served):
+    model, gc = _model()
+    ids = torch.randint(0, gc.vocab_size, (2, 40), device="cuda")
+    with torch.no_grad():
+        plain = model(ids)
+        change(model.transformer.h[1])
+        seen = _served(model)
+        got = model(ids)
+        assert sum(seen) == served
+        _apart(model)
+        assert torch.equal(got, model(ids))
+        assert torch.equal(got, plain) == (change is _rows_with_a_pitch)
     cuda_ops.check_status()
