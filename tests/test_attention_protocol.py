@@ -1,7 +1,7 @@
 """Host-side model of the barrier protocols of the two pipelined attention kernels (no GPU needed).
 
 `csrc/attention/attn_fwd_dual.cu` and `csrc/attention/attn_bwd_pipe.cu` each run four or five sequential roles (loader, MMA issuers,
-softmax groups) that meet only on mbarriers.  The roles are transcribed here as generators over the same barriers with the
+softmax groups) that meet on mbarriers and, where the forward's two softmax groups take turns, on two named barriers.  The roles are transcribed here as generators over the same barriers with the
 hardware's phase-parity semantics, asynchronous work (TMA copies, tcgen05 products) completes after a random delay, in order per
 issuing thread, and a random scheduler interleaves the roles.  The model checks, for every tile geometry the launchers can
 produce, that every role finishes (no wait can stay unsatisfied: on the GPU that would be a bounded wait giving up), and that
@@ -26,6 +26,29 @@ class Barrier:
 
     def done(self, parity):
         return (self.phase & 1) != (parity & 1)
+
+
+class NamedBarrier:
+    """`bar.sync` by one group of 128 threads and `bar.arrive` by another, 256 in all.  Unlike an mbarrier's, the wait has no limit; and a group that
+    comes twice before the other has come would complete the barrier by itself."""
+
+    def __init__(self):
+        self.here, self.phase = set(), 0
+
+    def arrive(self, group):
+        assert group not in self.here, "a group arrives twice in one phase of a named barrier"
+        self.here.add(group)
+        if len(self.here) == 2:
+            self.here.clear()
+            self.phase += 1
+
+    def sync(self, group):
+        before = self.phase
+        self.arrive(group)
+        yield self, before
+
+    def done(self, before):
+        return self.phase > before
 
 
 class AsyncQueue:
@@ -76,8 +99,14 @@ def run(roles, queues, rng, limit=400000, starved=None, starve=0.0):
 
 # ---- forward: two query tiles per CTA -------------------------------------------------------------------------------------------
 
-def forward_dual(q0, window, seq_len, rng, max_delay, stages=4, starved=None):
+TURN_TILES = 12                             # DU_TURN_TILES in csrc/attention/attn_fwd_dual.cu
+
+
+def forward_dual(q0, window, seq_len, rng, max_delay, stages=4, starved=None, turns=None, without=None):
+    """`turns`: the launcher's choice of the kernel with turns (by the host's window, which may exceed a device-resident one).  `without`: a part
+    of the turn protocol that is left out, which has to show."""
     tile = 128
+    turns = min(window, seq_len) >= TURN_TILES * tile if turns is None else turns
     first_a, first_b = q0 - window, q0 + tile - window
     lo_a, lo_b = (first_a // tile if first_a > 0 else 0), (first_b // tile if first_b > 0 else 0)
     hi_a = q0 // tile
@@ -93,6 +122,8 @@ def forward_dual(q0, window, seq_len, rng, max_delay, stages=4, starved=None):
     s_owner = ["free", "free"]             # S_x columns: free -> product in flight -> ready for the softmax -> free
     p_ready = [False, False]
     pv_running = [False, False]            # a product in flight reads P_x and accumulates into O_x
+    in_turn, my_turn = turns and n[0] >= TURN_TILES, [NamedBarrier(), NamedBarrier()]      # named barriers 1 and 2
+    exponentials = [False, False]
     finished = []
 
     def loader():
@@ -148,6 +179,8 @@ def forward_dual(q0, window, seq_len, rng, max_delay, stages=4, starved=None):
 
     def softmax(x):
         lo_x = lo_a if x == 0 else lo_b
+        if in_turn and x == 1 and without != "first arrival":
+            my_turn[0].arrive(1)
         for i in range(n[x]):
             yield bar_s[x], i
             assert s_owner[x] == "ready"
@@ -160,7 +193,15 @@ def forward_dual(q0, window, seq_len, rng, max_delay, stages=4, starved=None):
                 fb.arrive()
                 if (done < lo_b) if x == 0 else (done > hi_a):
                     fb.arrive()
+            if in_turn and i < n[0]:
+                yield from my_turn[x].sync(x)
+                exponentials[x] = True
+                assert not all(exponentials), "both query tiles at their exponentials in one turn"
             yield None                                 # the arithmetic: other roles run meanwhile
+            exponentials[x] = False
+            last = n[0] if without == "last turn's rule" else n[0] - 1
+            if in_turn and (x == 0 or i < last):
+                my_turn[1 - x].arrive(x)
             assert not pv_running[x], "P or O touched while a product still uses them"
             s_owner[x] = "free"
             p_ready[x] = True
@@ -170,7 +211,7 @@ def forward_dual(q0, window, seq_len, rng, max_delay, stages=4, starved=None):
 
     roles = {"loader": loader(), "issuer0": issuer(0), "issuer1": issuer(1), "softmax0": softmax(0), "softmax1": softmax(1)}
     run(roles, [tma] + mma, rng, starved=starved, starve=0.95)
-    assert len(finished) == 5
+    assert len(finished) == 5 and not any(b.here for b in my_turn)
 
 
 @pytest.mark.parametrize("seq_len,window", [(256, 0), (256, 1000), (512, 128), (768, 77), (1024, 300), (2048, 1024), (2048, 1000), (2048, 5000),
@@ -181,6 +222,22 @@ def test_forward_with_two_query_tiles_never_stalls_and_never_reuses_a_live_buffe
     for q0 in range(0, seq_len, 256):
         for _ in range(3):
             forward_dual(q0, min(window, seq_len), seq_len, rng, max_delay)
+
+
+@pytest.mark.parametrize("max_delay", [0, 3, 40])
+@pytest.mark.parametrize("window", [1535, 1536, 1537, 1663, 1664, 2000, 4096])      # B has as many key tiles as A, or one more; eleven, twelve, thirteen ..
+def test_forward_turns_end_for_every_count_of_key_tiles(window, max_delay):
+    rng = random.Random(window * 3 + max_delay)
+    for q0 in range(1024, 3584, 256):
+        for starved in (None, "softmax0", "softmax1", "issuer0", "issuer1"):
+            forward_dual(q0, window, 4096, rng, max_delay, starved=starved, turns=True)
+
+
+@pytest.mark.parametrize("without", ["first arrival", "last turn's rule"])
+def test_forward_model_notices_a_turn_that_is_not_passed_on(without):
+    for seed in range(5):
+        with pytest.raises(AssertionError):
+            forward_dual(2048, 2000, 4096, random.Random(seed), 3, without=without)
 
 
 def test_forward_model_notices_a_ring_that_is_too_shallow():
@@ -195,7 +252,8 @@ def test_forward_model_notices_a_ring_that_is_too_shallow():
 
 # ---- backward: transposed scores, P and dS in TMEM, dQ drained by warps of its own -------------------------------------------------
 
-def backward_pipe(n_iter, rng, max_delay, stages=3, starved=None):
+def backward_pipe(n_iter, rng, max_delay, stages=3, starved=None, without=None):
+    """`without`: a wait that is left out, which has to show."""
     one = ("kv", "s", "p", "dv", "dp", "ds", "dk", "mma", "dq", "end")           # many-thread barriers as one arrival
     bar = {name: Barrier(1) for name in one}
     ring = {name: [Barrier(1) for _ in range(stages)] for name in ("qdo", "free", "stat")}
@@ -269,7 +327,7 @@ def backward_pipe(n_iter, rng, max_delay, stages=3, starved=None):
             assert dp_cols["state"] == ("dS", it) and ds_tile[it & 1]["holds"] == it
             product(st, it, lambda: None, lambda: dp_cols.update(state="free"))
             commit(bar["dk"])
-            if it > 0:
+            if it > 0 and without != "dq":
                 yield bar["dq"], it - 1
             assert dq_cols["holds"] is None, "dQ overwritten before it was drained"
             ds_tile[it & 1]["reader"] = True
@@ -280,7 +338,8 @@ def backward_pipe(n_iter, rng, max_delay, stages=3, starved=None):
             mma.push(dq_done)
             commit(ring["free"][st], bar["mma"])
             if more:
-                yield bar["dk"], it
+                if without != "dk":
+                    yield bar["dk"], it
                 issue_dp(it + 1)
         commit(bar["end"])
         finished.append("issuer")
@@ -309,7 +368,7 @@ def backward_pipe(n_iter, rng, max_delay, stages=3, starved=None):
             yield bar["s"], it
             assert s_cols["state"] == it and stats[it % stages] == it
             yield None                                 # P formed
-            if it > 0:
+            if it > 0 and without != "dv":
                 yield bar["dv"], it - 1
             assert not p_cols["reader"], "P overwritten while dV still reads it"
             p_cols["holds"] = it
@@ -337,6 +396,14 @@ def test_pipelined_backward_never_stalls_and_never_reuses_a_live_buffer(n_iter, 
     rng = random.Random(n_iter * 17 + max_delay)
     for _ in range(5):
         backward_pipe(n_iter, rng, max_delay)
+
+
+@pytest.mark.parametrize("broken", [dict(without="dk"), dict(without="dq", starved="drain"), dict(without="dv"), dict(stages=1)])
+def test_backward_model_notices_what_is_missing(broken):
+    """dP issued before dK has read dS; dQ before a slow drain has taken the last one; P stored before dV has read it; one Q / dO stage."""
+    with pytest.raises(AssertionError):
+        for seed in range(20):
+            backward_pipe(9, random.Random(seed), 40, **broken)
 
 
 @pytest.mark.parametrize("starved", ["loader", "issuer0", "issuer1", "softmax0", "softmax1"])
