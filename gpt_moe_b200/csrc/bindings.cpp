@@ -94,14 +94,18 @@ CUtensorMap operand_map(const torch::Tensor& t, bool mn_major, int tile_rows_k_m
 }
 
 // Shares of the contraction for a bf16 result whose output tiles fill the CTA pairs badly (the input gradient of the LM head contracts over
-// the vocabulary into 12 to 128 tiles).  Estimates in us, fitted on this part: a pair takes 0.42 for a block of 64 and 2 for a tile's
-// read-out, summing the shares costs a launch and their bytes.  1024 x 768 x 50304: 297 us whole, 72 in shares;
-// 3840 rows 310 and 217, 8192 rows 552 and 432; at 12544 rows (147 tiles for 74 pairs, 603) whole tiles are the better form.
-int bf16_splits(int64_t m, int64_t n, int64_t k, int sms) {
-    const int64_t tiles = ((m + 255) / 256) * ((n + 255) / 256), blocks = (k + 63) / 64, pairs = std::max(1, sms / 2);
+// the vocabulary into 12 to 128 tiles).  Estimates in us, fitted to 45 to 12544 rows of 768 to 2048 columns with contractions of 2048 to 50304 (cold caches,
+// launches from a graph; 8 % off on average, the choice 2 % above the best of 1 to 8 shares): a launch takes 3.4; a block of 64 takes a pair 0.29,
+// up to 0.38 when all pairs pull operands from L2, and a tile's read-out 1.8; tiles of 128 columns (`narrow`) 0.18 to 0.23 and 2.7; the sum costs a
+// launch in a gap, 4.5, and its bytes at 14 TB/s, as the slabs still lie in L2.  us, whole / in shares: 1024 x 768 x 50304 159 / 64, 4096 rows 247 / 220,
+// 9472 545 / 480; 360 x 768 x 8192 30 / 18; 360 x 1024 x 2048 12 / 15 and 2048 x 1024 x 4096 20 / 23 stay whole.
+int bf16_splits(int64_t m, int64_t n, int64_t k, bool narrow, int sms) {
+    const int64_t rows = (m + 255) / 256, tiles = rows * ((n + 255) / 256), blocks = (k + 63) / 64, pairs = std::max(1, sms / 2);
+    const auto busy = [&](int64_t items) { return static_cast<double>(std::min(items, pairs)) / pairs; };
     const auto estimate = [&](int64_t s) {
-        const double sum = s > 1 ? 4.0 + static_cast<double>(m) * n * (8 * s + 2) / 6.0e6 : 0.0;
-        return ((tiles * s + pairs - 1) / pairs) * (((blocks + s - 1) / s) * 0.42 + 2.0) + sum;
+        if (s == 1 && narrow) return 3.4 + blocks * (0.18 + 0.053 * busy(rows * ((n + 127) / 128))) + 2.7;
+        const double sum = s > 1 ? 4.5 + static_cast<double>(m) * n * (8 * s + 2) / 14.0e6 : 0.0;
+        return 3.4 + ((tiles * s + pairs - 1) / pairs) * (((blocks + s - 1) / s) * (0.287 + 0.097 * busy(tiles * s)) + 1.8) + sum;
     };
     int64_t best = 1;
     for (int64_t s = 2; s <= 8 && blocks / s >= 16; ++s)
@@ -202,7 +206,7 @@ void gemm_run(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d, 
     torch::Tensor parts;
     if (mode == gm::GEMM_DENSE && d.scalar_type() == torch::kBFloat16 && !half_types && p.batch == 1 && d.dim() == 2 && p.C == nullptr && !p.symmetric &&
         p.batch_sumsq == nullptr && p.M > 0 && p.N > 0) {
-        const int splits = bf16_splits(p.M, p.N, p.K, sm_count());
+        const int splits = bf16_splits(p.M, p.N, p.K, gm::gemm_bf16_tile_width(p, a_mn, false, sm_count()) == 128, sm_count());
         if (splits > 1) {
             parts = gm::out_empty({splits, p.M, (p.N + 3) / 4 * 4}, d.options().dtype(torch::kFloat32));
             p.split_k = splits;
@@ -579,6 +583,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           py::arg("mode") = 0, py::arg("tile_expert") = py::none(), py::arg("num_m_tiles") = py::none(),
           py::arg("seg_ends") = py::none(), py::arg("symmetric") = false,
           py::arg("batch_sumsq") = py::none(), py::arg("scale_mode") = 0);
+    m.def("bf16_splits", &bf16_splits, py::arg("m"), py::arg("n"), py::arg("k"), py::arg("narrow"), py::arg("sms"));
     m.def("polar_express", &polar_express, py::arg("x"), py::arg("sumsq"), py::arg("coeffs"));
     m.def("mxfp8_quantize", &mxfp8_quantize, py::arg("x"), py::arg("rows_limit") = py::none());
     m.def("mxfp8_quantize_weight", &mxfp8_quantize_weight);

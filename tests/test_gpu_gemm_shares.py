@@ -38,3 +38,31 @@ def test_an_output_off_the_16_byte_grid_is_refused(m, n, k, offset):
         cuda_ops.ext().gemm_bf16(a, b, wide[:, offset: offset + n])
     assert (wide == 5).all()
     cuda_ops.check_status()
+
+
+def test_contractions_that_a_sum_would_not_repay_stay_whole():
+    """us, whole / the best of 2 to 8 shares: 360 x 1024 x 2048 12 / 14, 1536 x 768 x 3072 16 / 18, 2048 x 1024 x 4096 20 / 23; the others gain."""
+    from gpt_moe_b200.ops import cuda_ops
+    splits = cuda_ops.ext().bf16_splits
+    for m, n, k in ((360, 1024, 2048), (1536, 768, 3072), (2048, 1024, 4096)):
+        assert splits(m, n, k, True, 148) == 1
+    for m, n, k, narrow in ((360, 768, 8192, True), (1024, 768, 50304, True), (2048, 768, 50304, True), (9472, 768, 50304, False)):
+        assert splits(m, n, k, narrow, 148) > 1
+
+
+# where shares begin: few columns with long enough a contraction; a last share shorter than the others; rows of several tiles
+@pytest.mark.parametrize("m,n,k", [(64, 264, 4096), (300, 520, 5000), (33, 8, 4160), (1100, 264, 9000)])
+@pytest.mark.parametrize("b_mn", [False, True])
+def test_shared_contractions_at_the_line(m, n, k, b_mn):
+    from gpt_moe_b200.ops import cuda_ops
+    torch.manual_seed(9)
+    c = cuda_ops.ext()
+    assert c.bf16_splits(m, n, k, n > 128, 148) > 1
+    a = torch.randn(m, k, device="cuda").bfloat16()
+    b = torch.randn((k, n) if b_mn else (n, k), device="cuda").bfloat16()
+    wide = torch.full((m + 1, n + 24), 5.0, device="cuda", dtype=torch.bfloat16)
+    c.gemm_bf16(a, b, wide[:m, 8: 8 + n], False, b_mn)
+    want = a.double() @ (b.double() if b_mn else b.double().t())
+    assert ((wide[:m, 8: 8 + n].double() - want).abs() <= 2 ** -8 * want.abs() + 1e-5 * k ** 0.5).all()      # as above
+    assert (wide[m] == 5).all() and (wide[:, :8] == 5).all() and (wide[:, 8 + n:] == 5).all()
+    cuda_ops.check_status()
