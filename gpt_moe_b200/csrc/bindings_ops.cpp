@@ -322,20 +322,21 @@ MlaCachedArgs mla_cached_args(const Tensor& query, const Tensor& low, const Tens
 // Whether a call expands the visible cache instead of running the absorbed form: heads of 64 + 64 columns with 64-wide values, no
 // soft-capping, at least 8 new tokens a sequence (fewer were not measured), and the cheaper of the two by an estimate of their kernels in us:
 //   absorbed   its (query row, position) products, 2 rank + rope wide, and W_k and W_v once per (token, head);
-//   expanded   the positions that one CTA of the attention walks, times the waves of CTAs, and every position's kv heads (product, split).
-// The constants are a fit to 266 calls of each form (8, 16 and 32 heads on 1 to 32 kv heads, ranks 256 to 1024, 1 to 32 sequences of 8 to 512
-// new tokens over 192 to 8000 positions, with room left in the cache): it is 9 % off on average, and taking the form it names costs 0.5 %
-// over taking the better one each time (at worst 25 %, one call of 60 against 48 us).  For 16 heads, rank 512, 2 x 512 over 2012 it says
-// 1091 : 133.  The expansion holds 1 KB per position and kv head, 4 GB at the limit; longer calls stay absorbed.
+//   expanded   the positions that one CTA of the attention walks, times the waves of CTAs, every position's kv heads (product over the rank, split),
+//              every position once, and W's terms.
+// The constants are a fit to 606 calls of each form that lie within 2.5 times of one another (16 and 32 heads on 4 to 16 kv heads, ranks 256 to 1024,
+// 1 to 8 sequences of 8 to 256 new tokens over 8 to 8256 positions; cold caches, launches from a graph): 13 and 6 % off on average.  Over these and 330 more
+// the form it names costs 0.4 % over the better one each time (at worst 27 %, one call of 178 against 140 us).  The absorbed form has the benefit of
+// 5 %.  The expansion holds 1 KB per position and kv head, 4 GB at the limit; longer calls stay absorbed.
 bool mla_prefill_wanted(int64_t B, int64_t T, int64_t heads, int64_t kv_heads, int64_t end, int64_t window, int64_t r, int64_t dr, int64_t content,
                         int64_t value, double softcap) {
     if (T < 8 || r % 64 != 0 || dr != 64 || content != 64 || value != 64 || softcap > 0.0) return false;
     const double visible = static_cast<double>(window < 0 ? end : std::min(end, window + T));
     if (B * visible * kv_heads > 4194304.0) return false;
     const double rows = static_cast<double>(B * T * heads), waves = std::max(1.0, heads * B * ((T + 127) / 128) / 148.0);
-    const double absorbed = 26.0 + 21.5e-9 * rows * visible * (2 * r + dr) + 3.5e-5 * rows * r;
-    const double expanded = 45.0 + 0.0235 * visible * waves + 6.3e-4 * B * visible * kv_heads;
-    return absorbed > expanded;
+    const double absorbed = 26.4 + 21.1e-9 * rows * visible * (2 * r + dr) + 3.9e-5 * rows * r, positions = B * visible;
+    const double expanded = 34.3 + 0.0196 * visible * waves + (2.18e-7 * r + 3.8e-4) * positions * kv_heads + 5.5e-4 * positions + 7.3e-4 * kv_heads * r;
+    return absorbed > 1.05 * expanded;
 }
 
 bool mla_prefill_aligned(const MlaCachedArgs& a) {

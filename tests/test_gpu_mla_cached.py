@@ -187,6 +187,15 @@ def test_a_context_in_fp32_has_the_bits_of_fp32(b, t, h, hkv, r, dr, s):
     assert rel(got, want) < 6e-7                                  # 2e-7 to 4e-7 with fp32 products and sums throughout
 
 
+# low ranks and few positions, measured in us absorbed / expanded: 150 / 85, 320 / 177, 93 / 73, 50 / 38, 138 / 110; and the other way: 297 / 357, 39 / 78
+@pytest.mark.parametrize("b,t,h,hkv,end,r,expanded", [(4, 24, 32, 8, 1524, 256, True), (4, 24, 32, 8, 4024, 256, True), (1, 64, 32, 8, 1564, 256, True),
+                                                      (4, 16, 16, 4, 16, 512, True), (4, 32, 16, 16, 1532, 512, True), (2, 48, 16, 16, 8048, 512, False),
+                                                      (1, 16, 16, 16, 1516, 512, False)])
+def test_the_form_follows_what_the_expansion_costs(b, t, h, hkv, end, r, expanded):
+    from gpt_moe_b200.ops import cuda_ops
+    assert cuda_ops.ext().mla_prefill_wanted(b, t, h, hkv, end, -1, r, 64, 64, 64, 0.0) == expanded
+
+
 @pytest.mark.parametrize("expanded", [True, False])
 @pytest.mark.parametrize("b,t,h,hkv,r,start", [(1, 500, 8, 8, 256, 300), (2, 130, 16, 4, 512, 360)])
 def test_only_the_output_is_rounded_to_bf16(b, t, h, hkv, r, start, expanded):
