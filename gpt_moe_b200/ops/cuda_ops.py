@@ -13,6 +13,7 @@ Conventions
 """
 from __future__ import annotations
 
+import functools
 from typing import List, Optional, Sequence, Tuple
 
 import torch
@@ -841,11 +842,22 @@ def set_loss_scale(scale: float) -> None:
     _loss_scale = float(scale)
 
 
+@functools.lru_cache(maxsize=64)
+def loss_chunk_rows(width: int, vocab: int, sms: int, gradients: bool) -> int:
+    """Rows of a chunk of the LM-head loss: 8192, and with gradients up to 12544, where the tiles of the input gradient (256 x 256, one to a CTA pair)
+    come closest to whole waves: 12544 for 768 columns on 148 SMs (147 tiles for 2 x 74 pairs), 9472 for 512, 1024 and 2048.  us forward and
+    backward, 32768 rows, chunks of 8192 / 9472 / 12544: 768 columns 8018 / 8041 / 7910, 512 6313 / 6163 / 6216, 1024 10160 / 9753 / 10042, 2048 17816 / 17551 /
+    18080.  More than 8192 rows only while their bf16 logits stay below 1.25 GiB (0.82 GB of 50304 columns at 8192 rows, 1.26 GB at 12544)."""
+    if not gradients:
+        return 8192
+    pairs, tiles = max(1, sms // 2), -(-width // 256)
+    most = max(32, min(49, (5 << 28) // (512 * vocab)))
+    return 256 * max(range(32, most + 1), key=lambda rows: (rows * tiles / (-(-rows * tiles // pairs) * pairs), rows))
+
+
 class _LinearCrossEntropyFn(torch.autograd.Function):
     """mean CE of (x @ W^T) against targets without materialising all logits: rows are processed in chunks;
     each chunk's logits are overwritten in place by their gradient, which immediately feeds the dX and dW GEMMs."""
-
-    CHUNK = 12544        # 49 pair tiles of 256 rows: the input gradient of a 768-wide head fills the CTA pairs twice (147 tiles for 74 pairs)
 
     @staticmethod
     def forward(ctx, x: Tensor, weight: Tensor, targets: Tensor, ignore_index: int) -> Tensor:
@@ -864,7 +876,7 @@ class _LinearCrossEntropyFn(torch.autograd.Function):
         accumulate = _take_accumulate_flag((weight,)) if target_buf is not None else False
         if need_grad and target_buf is None:
             dw = torch.empty(w.shape, dtype=torch.float32, device=x.device)
-        chunk = min(_LinearCrossEntropyFn.CHUNK, rows)
+        chunk = min(loss_chunk_rows(w.shape[1], vocab, torch.cuda.get_device_properties(x.device).multi_processor_count, need_grad), rows)
         logits = torch.empty((chunk, vocab), dtype=BF16, device=x.device)
         for start in range(0, rows, chunk):
             n = min(chunk, rows - start)
