@@ -127,3 +127,20 @@ def test_gradients_at_any_scale(t, scale):
     for got, exp in zip(grads, torch.autograd.grad(want, want_in, g.double())):
         assert rel(got, exp) < 1e-2
     cuda_ops.check_status()
+
+
+# twelve key tiles and more, where the two query tiles take turns at their exponentials: B with as many key tiles as A and with one more
+@pytest.mark.parametrize("softcap", [0.0, 15.0])
+@pytest.mark.parametrize("t,window", [(2048, 2048), (2304, 1536), (3072, 1700)])
+def test_turns_of_the_query_tiles(t, window, softcap):
+    torch.manual_seed(12)
+    q, k = (2 * torch.nn.functional.rms_norm(torch.randn(1, t, 2, 64, device="cuda"), (64,)).bfloat16() for _ in range(2))
+    v = torch.randn(1, t, 2, 64, device="cuda").bfloat16()
+    out, lse = cuda_ops.ext().attn_fwd(q, k, v, window, 0.125, softcap)
+    want = ref.attention(q.double(), k.double(), v.double(), causal=True, window=window, scale=0.125, softcap_value=softcap)
+    # bf16 probabilities and result; the cap is the hardware's tanh (2^-11 of the cap, an exponent of e)
+    assert rel(out, want) < (6e-3 if softcap else 3e-3)
+    word = torch.tensor([window], dtype=torch.int32, device="cuda")           # the kernel's own look-back, shorter than the one the host decides by
+    again, again_lse = cuda_ops.ext().attn_fwd(q, k, v, t, 0.125, softcap, window_tensor=word)
+    assert torch.equal(out, again) and torch.equal(lse, again_lse)
+    cuda_ops.check_status()
