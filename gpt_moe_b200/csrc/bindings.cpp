@@ -218,9 +218,9 @@ void gemm_run(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d, 
     }
     const CUtensorMap& ta = operand_map(a, a_mn, 128, in_type);
     const int eb = p.out_fp32 ? 4 : 2;
-    // C of the output's shape comes through TMA; any other (broadcast over the batch or over rows, beside an fp32 output) is read by the threads
+    // C of the output's shape comes through TMA; any other (broadcast over the batch or over rows, beside an fp32 output or an MN-major operand) is read by the threads
     CUtensorMap tc, tmirror;
-    const bool tma_c = p.C != nullptr && mode == gm::GEMM_DENSE && !p.out_fp32 && !a_mn && p.K > 0 && c->dim() == d.dim() && c->sizes() == d.sizes() &&
+    const bool tma_c = p.C != nullptr && mode == gm::GEMM_DENSE && !p.out_fp32 && !a_mn && !b_mn && p.K > 0 && c->dim() == d.dim() && c->sizes() == d.sizes() &&
                        p.ldc > 0 && (p.batch == 1 || p.c_batch_stride > 0);
     const CUtensorMap& tb = operand_map(b, b_mn, gm::gemm_bf16_tile_width(p, a_mn, tma_c, sm_count()) / 2, in_type);
     const bool slabs = parts.defined();

@@ -44,7 +44,7 @@ bool make_tensor_map(CUtensorMap* out, const void* base, int elem_bytes, uint64_
 
 // columns of a pair's tile; B's map has boxes of half as many rows
 int gemm_bf16_tile_width(const GemmParams& p, bool a_mn, bool c_by_tma, int sms);
-// `tc`: map of C in the layout of D (64 x 128 box) when the epilogue may fetch it by TMA (dense, bf16 output, K > 0, A K-major), else null;
+// `tc`: map of C in the layout of D (64 x 128 box) when the epilogue may fetch it by TMA (dense, 16-bit output, K > 0, both operands K-major), else null;
 // `tmirror`: for symmetric results, the map of D for the transposed blocks: boxes of 64 rows, with `tc` 64 columns (128-byte swizzle), else 32
 // (no swizzle).  `td`: boxes of 128 bytes, with `tc` 128 rows, else 32.
 cudaError_t launch_gemm_bf16(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const CUtensorMap* tc, const CUtensorMap* tmirror,

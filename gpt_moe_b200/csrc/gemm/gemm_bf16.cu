@@ -252,11 +252,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             }
         }
     } else if (TMA_C) {
-        // Epilogue of D = alpha * acc + beta * C for dense bf16 outputs.  C arrives by TMA in the slab the result is staged in: rounds of 64
+        // Epilogue of D = alpha * acc + beta * C for dense 16-bit outputs.  C arrives by TMA in the slab the result is staged in: rounds of 64
         // columns walk a ring of four slabs [128 rows][128 bytes], the slab of the next round is requested while this one is worked
         // on, and every thread replaces the 16-byte pieces of its row in place.  (Read by the threads themselves, 64 bytes of a row
-        // each, C cost 32 cache lines per load in the chain between accumulator and store: 96 products of 768 x 6144 x 768 took 802 us,
-        // 629 now against 600 without C; 128 of 768 x 3072 x 768 627, 454 and 427; 128 symmetric ones of 768^3 134 and 103.)
+        // each, C cost 32 cache lines per load in the chain between accumulator and store: 128 symmetric products of 768^3 took 134 us, 103 now.)
         const int quad = warp & 3;
         const int half = (warp - 2) >> 2;                          // 32 of a round's 64 columns
         const int row_in_tile = quad * 32 + lane;
@@ -575,8 +574,7 @@ cudaError_t launch_gemm_bf16(const CUtensorMap& ta, const CUtensorMap& tb, const
     const CUtensorMap& tm = tmirror != nullptr ? *tmirror : td;
     if (gemm_bf16_tile_width(p, a_mn, tc != nullptr, sms) == 128)
         return b_mn ? launch_variant<false, true, false, 128>(ta, tb, td, td, tm, p, sms, stream) : launch_variant<false, false, false, 128>(ta, tb, td, td, tm, p, sms, stream);
-    if (tc != nullptr && !a_mn)
-        return b_mn ? launch_variant<false, true, true, 256>(ta, tb, td, *tc, tm, p, sms, stream) : launch_variant<false, false, true, 256>(ta, tb, td, *tc, tm, p, sms, stream);
+    if (tc != nullptr) return launch_variant<false, false, true, 256>(ta, tb, td, *tc, tm, p, sms, stream);
     if (a_mn) return b_mn ? launch_variant<true, true, false, 256>(ta, tb, td, td, tm, p, sms, stream) : launch_variant<true, false, false, 256>(ta, tb, td, td, tm, p, sms, stream);
     return b_mn ? launch_variant<false, true, false, 256>(ta, tb, td, td, tm, p, sms, stream) : launch_variant<false, false, false, 256>(ta, tb, td, td, tm, p, sms, stream);
 }

@@ -97,7 +97,7 @@ def main() -> None:
         if not args.case.startswith("attn_bwd"):
             fn = lambda: c.attn_fwd(q.detach(), k.detach(), v.detach(), 1024, d ** -0.5, single_tile=args.single_tile)
             flops = 4 * d * keys * b_ * h
-        else:                                        # the binding itself: delta pre-pass, zeroed fp32 dQ, the backward kernel
+        else:                                        # the binding itself: delta pre-pass (which clears the fp32 dQ), the backward kernel
             qd, kd, vd = q.detach(), k.detach(), v.detach()
             out, lse = c.attn_fwd(qd, kd, vd, 1024, d ** -0.5)
             g = torch.randn_like(out)
@@ -123,12 +123,12 @@ def main() -> None:
         a = torch.empty(96, 768, 768, device=dev, dtype=torch.bfloat16)
         fn = lambda: c.gemm_bf16(x, x, a, symmetric=args.case == "gemm_xxt")
         flops = 2 * 96 * 768 * 768 * 6144                 # of the full product: the symmetric form does two thirds of it
-    elif args.case == "gemm_addend":             # Polar Express' B X + a X for 96 matrices [768, 6144], the addend fetched by TMA
-        b = torch.randn(96, 768, 768, device=dev).mul_(0.03).bfloat16()
-        x = torch.randn(96, 768, 6144, device=dev).bfloat16()
-        y = torch.empty_like(x)
-        fn = lambda: c.gemm_bf16(b, x, y, False, True, 1.0, 0.3, x)
-        flops = 2 * 96 * 768 * 768 * 6144
+    elif args.case == "gemm_addend":             # Polar Express' b A + c A A on 96 Gram matrices [768, 768], the addend fetched by TMA
+        x = torch.randn(96, 768, 768, device=dev).mul_(0.03).bfloat16()
+        a = torch.bmm(x, x.mT)
+        y = torch.empty_like(a)
+        fn = lambda: c.gemm_bf16(a, a, y, False, False, 0.5, -2.8, a, symmetric=True)
+        flops = 2 * 96 * 768 ** 3                         # of the full product: the symmetric form does two thirds of it
     elif args.case in ("mla_decode", "mla_prefill"):   # attention of new tokens over a latent cache with room left, 16 heads, rank 512, from the
         b_, new, seen = (32, 1, 8000) if args.case == "mla_decode" else (2, 512, 2012)      # projections to the attention output
         latent, rope = (torch.randn(b_, seen + 100, n, device=dev).bfloat16() for n in (512, 64))
