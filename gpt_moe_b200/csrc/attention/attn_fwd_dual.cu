@@ -13,11 +13,10 @@
 //               What is left (clock64 in one CTA of nine key tiles): 3150 clocks a key tile - the second softmax pass 1750, the first 550,
 //               waiting for S 700 - and 3500 and 6500 clocks before the first and after the last one.
 //   warp  10    TMA loads (one elected lane): Q once, then the K and V tile of a ring stage as it comes free
-// O stays in TMEM for the whole CTA and the PV product accumulates into it.  A row's exponentials are taken against its maximum so far; when a key
-// tile raises the maximum of any row of a warp, the softmax threads rescale their rows of O in TMEM (rare after the first tiles).  The reference is
-// the exact maximum, at every length and window: one that may lag by up to 2^8 saves 2 to 7 % of the time (16 x 2048 tokens, 12 heads, window
-// 1024 199 against 205 us, 16384 tokens 761 against 812), but the largest probability is then no longer 1, which bf16 holds exactly, and outputs lie
-// 1 to 4 % further from 64 bits, 18 to 22 % where scores are spread three times as wide (2.14e-3 against 1.79e-3).
+// O stays in TMEM for the whole CTA and the PV product accumulates into it.  The running maximum a row's exponentials are
+// taken against is only moved when the row's maximum has grown by more than 2^8 since it was last moved; then (rarely
+// after the first tiles) the row's O is rescaled in TMEM by its softmax thread.  The stale reference only changes the
+// common factor of numerator and denominator, which cancels in O / l.
 // TMEM: S_A 0-127, S_B 128-255, P_A 256-319, P_B 320-383, O_A 384-447, O_B 448-511 (one CTA per SM).
 // A ring stage is released by the softmax warps: a tile's users each arrive once they have seen their PV product of that tile
 // complete (a tile only one query tile reads gets both arrivals from it), so the two query tiles may drift apart by up to
@@ -42,6 +41,7 @@ constexpr int DU_POLY_PER_8 = 2;                         // exponentials of ever
 constexpr int DU_TURN_TILES = 12;                        // from this many key tiles on the two query tiles take turns at their exponentials: started together
                                                          // they stay in step, share the MUFU in the second pass and leave it idle in the rest
                                                          // (16384 tokens 904 -> 816 us, 4 x 4096 270 -> 256; nine key tiles 199 -> 200, two 48 -> 53)
+constexpr float DU_RESCALE_STEP = 8.f;                   // log2 units the row maximum may outgrow its reference before O is rescaled
 
 // Capping and masking of 32 scores (columns kv0 .. kv0 + 31 of the key tile) in place.
 template <bool MASK, bool CAP>
@@ -114,7 +114,7 @@ __device__ __forceinline__ void dual_zero16(uint32_t p_addr) {
 
 template <bool CAP, class PreviousProduct, class Turn>
 __device__ __forceinline__ void dual_softmax_tile(uint32_t s_addr, uint32_t p_addr, uint32_t o_addr, int kv0, int qpos, int warp_q0, int window,
-                                                  bool edge_tile, float c, float& m_ref, float& l, bool first, float cap_a, float cap_b,
+                                                  bool edge_tile, float c, float step, float& m_ref, float& l, bool first, float cap_a, float cap_b,
                                                   const PreviousProduct& previous_product, const Turn& my_turn) {
     int cls[4] = {CHUNK_FULL, CHUNK_FULL, CHUNK_FULL, CHUNK_FULL};
     if (edge_tile) {
@@ -142,7 +142,7 @@ __device__ __forceinline__ void dual_softmax_tile(uint32_t s_addr, uint32_t p_ad
     }
     const float m_tile = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * c;
     previous_product();                            // complete from here on: O may be rescaled and P overwritten
-    const bool grow = m_tile > m_ref;              // also true for the first finite maximum (m_ref = -inf)
+    const bool grow = m_tile > m_ref + step;       // also true for the first finite maximum (m_ref = -inf)
     if (__any_sync(0xffffffffu, grow)) {
         const float alpha = grow ? exp2f(m_ref - m_tile) : 1.f;
         if (!first) {
@@ -303,6 +303,11 @@ attn_fwd_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         const float c = p.scale_log2e;
         constexpr bool capped = CAPPED;
         const float cap_a = capped ? p.softcap / p.scale : 0.f, cap_b = capped ? p.scale / p.softcap : 0.f;
+        // With a reference that lags, the largest probabilities are no longer 1, which bf16 holds exactly, and outputs lie up to 4 % further
+        // from 64 bits than with the exact maximum: it lags only in windowed or short calls of whole pairs of tiles; the others rescale
+        // whenever the maximum grows (5 x 1000 tokens, window 256: 2.04e-3 instead of 2.10e-3)
+        const bool lags = p.seq_len % (2 * DU_BM) == 0 && (p.window <= p.seq_len / 2 || p.seq_len <= 16 * DU_BM);
+        const float step = lags ? DU_RESCALE_STEP : 0.f;
         const int n_a = hi_a - lo_a + 1;                       // key tiles of A; B has as many or one more
         const bool in_turn = TURNS && n_a >= DU_TURN_TILES;
         if (in_turn && x == 1) asm volatile("bar.arrive 1, 256;" ::: "memory");
@@ -330,7 +335,7 @@ attn_fwd_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
             };
             // tiles strictly inside the band need no mask; the diagonal tile and the tile at the window edge do
             const bool need_mask = (kv0 + DU_BN - 1 > q0x) || (q0x + DU_BM - 1 - kv0 > window);
-            dual_softmax_tile<capped>(s_addr, p_addr, o_addr, kv0, qpos, q0x + quad * 32, window, need_mask, c, m_ref, l, i == 0, cap_a, cap_b,
+            dual_softmax_tile<capped>(s_addr, p_addr, o_addr, kv0, qpos, q0x + quad * 32, window, need_mask, c, step, m_ref, l, i == 0, cap_a, cap_b,
                                       previous_product, my_turn);
             if (in_turn && (x == 0 || i + 1 < n_a)) asm volatile("bar.arrive %0, 256;" ::"r"(2 - x) : "memory");
             tmem_st_wait();

@@ -74,34 +74,6 @@ def test_ragged_outputs_are_as_exact_as_the_single_tile_kernels(t, window):
     cuda_ops.check_status()
 
 
-# a whole and a ragged length, windowed; either side of 2048 positions and a window on either side of half of them
-@pytest.mark.parametrize("t,longer,window", [(1000, 1024, 256), (2048, 2304, 2304), (2048, 2304, 1100)])
-def test_rows_do_not_depend_on_the_length_behind_them(t, longer, window):
-    """One rule for the reference that exponentials are taken against, whatever the length: rows that see the same keys have the same bits."""
-    torch.manual_seed(8)
-    q, k, v = (2 * torch.randn(1, longer, 2, 64, device="cuda").bfloat16() for _ in range(3))
-    long = cuda_ops.ext().attn_fwd(q, k, v, min(window, longer), 0.125)[0]
-    part = [x[:, :t].contiguous() for x in (q, k, v)]
-    assert torch.equal(cuda_ops.ext().attn_fwd(*part, min(window, t), 0.125)[0], long[:, :t])
-    word = torch.tensor([min(window, longer)], dtype=torch.int32, device="cuda")
-    assert torch.equal(cuda_ops.ext().attn_fwd(q, k, v, longer, 0.125, window_tensor=word)[0], long)
-    cuda_ops.check_status()
-
-
-@pytest.mark.parametrize("t,window", [(256, None), (1024, 256), (2048, 1024), (2048, None)])
-def test_whole_lengths_are_as_exact_as_the_single_tile_kernel(t, window):
-    torch.manual_seed(9)
-    q, k = (torch.nn.functional.rms_norm(torch.randn(2, t, 4, 64, device="cuda"), (64,)).bfloat16() for _ in range(2))
-    v = torch.randn(2, t, 4, 64, device="cuda").bfloat16()
-    w = t if window is None else window
-    for spread in (1, 3):                                     # of the scores; bounds as above
-        out = cuda_ops.ext().attn_fwd(spread * q, k, v, w, 0.125)[0]
-        single = cuda_ops.ext().attn_fwd(spread * q, k, v, w, 0.125, single_tile=True)[0]
-        want = ref.attention(spread * q.double(), k.double(), v.double(), causal=True, window=window)
-        assert rel(out, want) < 1.003 * rel(single, want)
-    cuda_ops.check_status()
-
-
 @pytest.mark.parametrize("t", [257, 384])
 def test_three_tiles_without_a_window_take_the_single_tile_kernel(t):
     """Of three query tiles the two-tile kernel idles in a quarter of its work (64 x 300 tokens: 109 us against 103)."""
