@@ -303,10 +303,15 @@ attn_fwd_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         const float c = p.scale_log2e;
         constexpr bool capped = CAPPED;
         const float cap_a = capped ? p.softcap / p.scale : 0.f, cap_b = capped ? p.scale / p.softcap : 0.f;
-        // With a reference that lags, the largest probabilities are no longer 1, which bf16 holds exactly, and outputs lie up to 4 % further
-        // from 64 bits than with the exact maximum: it lags only in windowed or short calls of whole pairs of tiles; the others rescale
-        // whenever the maximum grows (5 x 1000 tokens, window 256: 2.04e-3 instead of 2.10e-3)
-        const bool lags = p.seq_len % (2 * DU_BM) == 0 && (p.window <= p.seq_len / 2 || p.seq_len <= 16 * DU_BM);
+        // With a reference that lags, the largest probabilities are no longer 1, which bf16 holds exactly: outputs lie up to 3 % further from 64 bits,
+        // 3 to 20 % where scores are spread three times as wide.  us and error at both spreads, lagging / exact: 16 x 2048, 12 heads, window 1024 198 / 204,
+        // 2.08e-3 / 2.05e-3, 2.14e-3 / 1.79e-3; without a window 224 / 236, 2.07e-3 / 2.04e-3, 2.13e-3 / 1.79e-3; 64 x 256 54 / 56, 1.96e-3 / 1.95e-3, 1.82e-3 / 1.76e-3.
+        // It lags where this kernel is the one that has always served the call, windowed or short calls of whole pairs of tiles; ragged and long full ones
+        // would otherwise go to the single-tile kernel, whose maximum is exact, and rescale whenever theirs grows, so that they lose nothing
+        // here (5 x 1000 tokens, window 256: 2.04e-3 instead of 2.10e-3).  Exact everywhere was taken back: other roundings in every layer move a training
+        // step's fp32 results by up to 4.8e-5.  Short is meant of the look-back in use and of the one that the host chose this kernel by.
+        const int reach = max(p.window, window);
+        const bool lags = p.seq_len % (2 * DU_BM) == 0 && (reach <= p.seq_len / 2 || p.seq_len <= 16 * DU_BM);
         const float step = lags ? DU_RESCALE_STEP : 0.f;
         const int n_a = hi_a - lo_a + 1;                       // key tiles of A; B has as many or one more
         const bool in_turn = TURNS && n_a >= DU_TURN_TILES;
@@ -405,7 +410,7 @@ attn_fwd_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
 }
 
 bool attn_fwd_dual_supported(const AttnParams& p) {
-    // us, this kernel / the single-tile one (12 heads unless said otherwise): 16 x 2048 tokens, window 1024 205 / 248, 16384 tokens, 16 heads 815 / 978, 4 x 4096,
+    // us, this kernel / the single-tile one (12 heads unless said otherwise): 16 x 2048 tokens, window 1024 198 / 251, 16384 tokens, 16 heads 815 / 978, 4 x 4096,
     // 16 heads 251 / 293, 64 x 129 51 / 66, 8 x 500 25 / 30, 16 x 700 57 / 69, 16 x 1000 86 / 100.  Of an odd number of tiles the last CTA idles by half: with three
     // that is a quarter of the work (64 x 300 109 / 103, 16 x 384 36 / 33, 8 x 300 25 / 23, equal at 1 x and 3 x 300), with five no more (16 x 600 55 / 57, 8 x 640 33 / 35,
     // 4 x 600, 16 heads 26 / 27), 16 x 896 84 / 84, 16 x 1152 114 / 117, 8 x 1408 79 / 84.  A short window does not repay it below nine tiles (16 x 1152, window 256 80 / 96).

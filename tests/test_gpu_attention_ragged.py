@@ -116,3 +116,16 @@ def test_turns_of_the_query_tiles(t, window, softcap):
     again, again_lse = cuda_ops.ext().attn_fwd(q, k, v, t, 0.125, softcap, window_tensor=word)
     assert torch.equal(out, again) and torch.equal(lse, again_lse)
     cuda_ops.check_status()
+
+
+def test_a_longer_look_back_on_the_device_keeps_the_exact_maximum():
+    """The reference of the exponentials may lag only where the look-back in use is short, not where the host's bound alone is."""
+    torch.manual_seed(13)
+    t = 2304
+    q, k = (torch.nn.functional.rms_norm(torch.randn(1, t, 4, 64, device="cuda"), (64,)).bfloat16() for _ in range(2))
+    q, v = 3 * q, torch.randn(1, t, 4, 64, device="cuda").bfloat16()
+    word = torch.tensor([t], dtype=torch.int32, device="cuda")
+    out, single = (cuda_ops.ext().attn_fwd(q, k, v, 1024, 0.125, single_tile=one, window_tensor=word)[0] for one in (False, True))
+    want = ref.attention(q.double(), k.double(), v.double(), causal=True, window=None)
+    assert rel(out, want) < 1.003 * rel(single, want)                 # bound as above
+    cuda_ops.check_status()
