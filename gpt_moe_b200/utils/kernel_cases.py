@@ -157,10 +157,11 @@ def main() -> None:
         targets = torch.randint(0, 50304, (8192,), device=dev)
         fn = lambda: c.row_nll(logits, targets, -100)
         bytes_ = 8192 * 50304 * 2
-    elif args.case == "polar":                   # five Polar Express iterations on the same batch
+    elif args.case == "polar":                   # five Polar Express iterations on such a batch; x is scratch, so every call gets a copy (0.9 GB, timed too)
         x = torch.randn(96, 768, 6144, device=dev)
         x = (x / (x.norm(dim=(-2, -1), keepdim=True) * 1.02 + 1e-6)).bfloat16()
-        fn = lambda: cuda_ops.polar_express_bf16(x)
+        work = torch.empty_like(x)
+        fn = lambda: cuda_ops.polar_express_bf16(work.copy_(x))
         flops = 5 * 96 * (4 * 768 * 768 * 6144 + 2 * 768 ** 3)
     elif args.case == "rs_muon":                 # reduce + momentum + pack for 16 matrices of 6144 x 768 (world of one)
         grads = [torch.randn(6144, 768, device=dev) for _ in range(16)]
