@@ -13,10 +13,10 @@
 //   dQ_i = dS K                              M128 N64 K128, A = the same dS tile read K-major, B = K read MN-major;
 //                                            the 128x64 fp32 result is scaled, staged in shared memory and added into
 //                                            a fp32 dQ buffer by TMA reduce-add (several key tiles contribute to one row)
-// The K and V tiles stay resident; Q / dO tiles run through a two-deep TMA ring.  Warp 8 is the control warp (loads and
-// MMA issue by one thread), warps 0-7 are the softmax warps (warps w and w+4 share TMEM quadrant w and split the key columns).
-// delta = rowsum(dO * O) comes from a small pre-pass kernel in this file.
-// Calls with 64-wide heads go to attn_bwd_pipe.cu (the same products, software-pipelined); this kernel serves 128-wide heads and is
+// The K and V tiles stay resident; Q / dO tiles run through a two-deep TMA ring.  Warp 8 is the control warp (loads and MMA issue, a whole
+// warp: see umma_f16 in ptx.cuh), warps 0-7 are the softmax warps (warps w and w+4 share TMEM quadrant w and split the key columns).
+// delta = rowsum(dO * O) comes from a small pre-pass kernel in this file, which also clears the dQ buffer.
+// Calls with 64-wide heads go to attn_bwd_pipe.cu (transposed score tiles, P and dS in TMEM); this kernel serves 128-wide heads and is
 // the one that kernel is tested against.  The delta pre-pass and the launcher of both live here.
 // Reference counterpart: the backward of FlexAttention (model/attention/self_attention.py:250-255) as generated by Inductor.
 #include "../common/ptx.cuh"

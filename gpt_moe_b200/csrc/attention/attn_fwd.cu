@@ -10,7 +10,7 @@
 //                       row-major shared-memory tile; accumulator in TMEM (64 columns)
 //   O  = O*alpha + PV   rescale-and-accumulate in registers (64 fp32 per row), normalise at the end
 // Q, K and V are read by TMA directly out of the packed projection output [tokens, (Hq+2Hkv)*64]; nothing is transposed.
-// Warp 8 is the control warp (TMA loads + MMA issue, one thread); warps 0-7 are the softmax warps: warps w and w+4
+// Warp 8 is the control warp (TMA loads + MMA issue by a whole warp, see umma_f16 in ptx.cuh); warps 0-7 are the softmax warps: warps w and w+4
 // share the 32 query rows of TMEM quadrant w and split the key columns (and the output columns) between them; the two
 // halves of a row exchange only their running maximum, through shared memory, once per key tile.  K and V each use a
 // two-deep ring of shared-memory tiles refilled as soon as the MMA reading a tile has committed; two CTAs fit per SM

@@ -258,7 +258,8 @@ void gemm_bf16(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d,
 // us, single steps with bf16 Gram matrices / here: 96 of 768 x 6144 5060 / 2870, 96 of 768 x 3072 3050 / 2060, 128 of 768 x 1536 2490 / 2310,
 // 16 of 768 x 6144 990 / 657, 16 of 768 x 3072 607 / 505, in runs; where a run's fourteen small products are launches of a few waves they
 // cost what the large ones save (24 of 1024 x 2048 1075 / 1113, 3 of 512 x 2048 286 / 308): runs are taken for X at least three times as wide
-// as high with two tiles of Q X for every CTA pair, or twice as wide with six tiles of a small product.
+// as high with two tiles of Q X for every CTA pair, or twice as wide with six tiles of a small product.  A run holds four m x m matrices where
+// single steps hold two (226 MB more for 96 of 768).
 // Rounding noise of A grows by a^2 a step against the smallest singular values.  Error against 64 bits (2-norm; matrices 768 x 3072:
 // Gaussian / rank 8 plus noise / singular values 1/i / exp(-12 i / m)): single steps in bf16 1.06e-2 / 5.8e-2 / 3.6e-2 / 9.3e-2, runs of two and
 // three 0.48e-2 / 4.8e-2 / 3.4e-2 / 6.8e-2; one run of five reaches 0.1 to 20 and is not taken, nor are runs of matrices lower than 256.

@@ -4,7 +4,8 @@
 // 256 x 256 output tiles: each CTA owns 128 of the rows and stages only HALF of the B tile, the tensor cores of
 // both SMs read both halves, so a CTA pulls 32 KB instead of 48 KB through L2 per 128 x 256 x 64 block of work -
 // the main loop of a one-CTA kernel is bound by exactly that traffic.  Roles inside each CTA:
-//   warp 0  : TMA producer   - fills a 5-stage ring of {A 128x64, B 128x64} bf16 tiles (128B swizzle); the
+//   warp 0  : TMA producer   - fills a 5-stage ring of {A 128x64, B 128x64} bf16 tiles (128B swizzle; with
+//                              128-column tiles six stages and B 64x64); the
 //                              bytes of both CTAs are counted on the leader's (even CTA's) barrier
 //   warp 1  : MMA issuer     - leader CTA only: the whole warp walks the loop, one lane's tcgen05.mma (M256 N256 K16) go into one of
 //                              two TMEM accumulators (2 x 256 columns in each CTA), commits to both CTAs
@@ -23,7 +24,7 @@
 //             epilogue stores every off-diagonal tile a second time transposed (the reference's triangle-and-mirror
 //             kernels, optimizers/polar_express.py:60-121 and :155-230)
 //   GROUPED_M rows of A belong to experts; tile -> expert table on the device picks B's z slice
-//             (expert segments are padded to 128 rows, so a tile never straddles two experts)
+//             (expert segments are padded to 256 rows, so a pair's tile never straddles two experts)
 //   GROUPED_K one output matrix per expert, contraction over that expert's (padded) row segment
 //             - the expert weight gradient; empty experts get exact zeros
 // Reference counterparts: Triton `_grouped_mm_kernel` (model/linear/default/grouped.py:12-70) and the
@@ -46,7 +47,7 @@ constexpr int GEMM_THREADS = 320;           // warp 0 TMA, warp 1 MMA, warps 2-9
 constexpr int GROUP_M = 4;               // in pair tiles (256 rows each)
 constexpr uint32_t TMEM_COLS = 512;
 constexpr int SLAB_BYTES = BM * 128;              // one slab of [128 rows][128 bytes]
-constexpr int STAGING_BYTES = 2 * SLAB_BYTES;    // two slabs; the staging area holds two such buffers
+constexpr int STAGING_BYTES = 2 * SLAB_BYTES;    // the staging area is twice this: two slabs of 4 KB for each epilogue warp, beside a C through TMA four slabs of all 128 rows
 
 constexpr uint32_t kIdescBf16Operands = (1u << 7) | (1u << 10);      // operand formats of the instruction descriptor: 1 = bf16, 0 = fp16
 
