@@ -195,7 +195,8 @@ void gemm_run(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& d, 
     p.status = status_tensor(a.device().index()).data_ptr<int>();
     // split-K: a long contraction with too few output tiles to fill the GPU (weight gradients) is shared by several CTAs per tile
     p.split_k = 1;
-    if (mode == gm::GEMM_DENSE && p.out_fp32 && may_split) {
+    // (not beside C, which every share would add)
+    if (mode == gm::GEMM_DENSE && p.out_fp32 && may_split && p.C == nullptr) {
         const int64_t tiles = ((p.M + 255) / 256) * 2 * ((p.N + 255) / 256) * p.batch;      // CTA pairs own 256-row tiles
         const int64_t k_blocks = (p.K + 63) / 64;
         if (tiles * 2 <= sm_count() && k_blocks >= 16)

@@ -66,3 +66,20 @@ def test_shared_contractions_at_the_line(m, n, k, b_mn):
     assert ((wide[:m, 8: 8 + n].double() - want).abs() <= 2 ** -8 * want.abs() + 1e-5 * k ** 0.5).all()      # as above
     assert (wide[m] == 5).all() and (wide[:, :8] == 5).all() and (wide[:, 8 + n:] == 5).all()
     cuda_ops.check_status()
+
+
+# contractions that an fp32 result would share: the addend comes in once, also on top of what the output holds.  Whole numbers below 2^24: every order
+# of the sums gives the same
+@pytest.mark.parametrize("m,n,k,b_mn", [(638, 48, 8192, False), (767, 128, 4096, True), (1062, 864, 1296, True)])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_an_addend_beside_an_fp32_result_is_added_once(m, n, k, b_mn, accumulate):
+    from gpt_moe_b200.ops import cuda_ops
+    torch.manual_seed(15)
+    a = torch.randint(-1, 2, (m, k), device="cuda").bfloat16()
+    b = torch.randint(-1, 2, (k, n) if b_mn else (n, k), device="cuda").bfloat16()
+    c = 2 * torch.randint(-60, 60, (m, n), device="cuda").bfloat16()
+    d = torch.randint(-1000, 1000, (m, n), device="cuda").float()
+    want = a.double() @ (b.double() if b_mn else b.double().t()) - 0.5 * c.double() + (d.double() if accumulate else 0)
+    cuda_ops.ext().gemm_bf16(a, b, d, False, b_mn, 1.0, -0.5, c, accumulate)
+    assert torch.equal(d.double(), want)
+    cuda_ops.check_status()
